@@ -55,6 +55,8 @@ struct Weight {
     int chunks;        // ceil(K / 64)
     float scale;       // per-tensor weight scale
     size_t bytes;      // groups * chunks * 16 * 16
+    alignas(64) unsigned char tensor_map[128];   // the tensor-core GEMM's map of it, made on first use
+    bool has_map;
 };
 
 // ---- launch helper: optional programmatic dependent launch ----------------------

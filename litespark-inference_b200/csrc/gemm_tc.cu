@@ -1,25 +1,33 @@
 // Prefill path of the ternary linear layer on the 5th-generation tensor cores (tcgen05).
 //
-//   acc[t, n] = sum_k w[n, k] * xq[t, k]      int8 x int8 -> int32 in tensor memory (exact)
+//   acc[t, n] = sum_k w[n,k] * xq[t, k]      int8 x int8 -> int32 in tensor memory (exact)
 //   y[t, n]   = float(acc) * (xscale[t] * wscale)
 //
 // Replaces, for many token rows, what the reference does with its batched kernel
 // (matmul_lut_avx512_mT, matmul_lut_avx512_extern_c.cpp:258-339) and, as the tensor-unit analogue,
 // its AMX tile GEMM (matmul_amx_int8_mT_v2, :819-933).
 //
-// One CTA owns 128 output features (the MMA's M side: one TMEM lane per feature) and TN token rows
-// (the MMA's N side: one TMEM column per token).  Per 128-wide K block, through a 4-stage ring:
-//   warp 0      TMA: 4 KB of packed 2-bit weights (128 rows x 32 bytes of the device chunk layout)
-//               and the TN x 128-byte tile of int8 activations (128-byte swizzle) -> shared memory
-//   warps 2-5   expand the packed rows to signed int8 {-1,0,+1} in the canonical K-major,
-//               128-byte-swizzled operand layout (thread = weight row; one packed word -> 16 bytes)
-//   warp 1      one thread issues 4 x tcgen05.mma.kind::i8 (M=128, N=TN, K=32) per block and
-//               commits the stage back to the producer
-// then warps 2-9 read the accumulators with tcgen05.ld (two warps per quarter of the TMEM lanes, alternate
-// 32-column slabs; warps 6-9 exist only for this) and write fp32 (and, if asked, the int32).
+// One CTA owns FM tiles of 128 output features (the MMA's M side: one TMEM lane per feature) and TN token rows
+// (the MMA's N side: one TMEM column per token).  Per 256-wide K block:
+//   warp 10     TMA: FM x 8 KB of packed 2-bit weights (128 rows x 64 bytes of the device chunk layout)
+//   warp 0      TMA: two TN x 128-byte tiles of int8 activations (128-byte swizzle); each its own shared-memory ring
+//   warps 2-9   expand the packed rows to int8 codes {0,1,2} and store them to a ring of FM x 64 columns of TENSOR
+//               MEMORY (thread = weight row = TMEM lane; four codes per column), from where the MMA takes its A
+//               operand; sum(x) of the token is subtracted once in the epilogue, as the reference's VNNI path does
+//   warp 1      one thread issues FM x 8 x tcgen05.mma.kind::i8 (A in TMEM, M=128, N=TN, K=32) per block and
+//               commits the stages back to the producer and to the expanders
+// then warps 2-9 read the accumulators with tcgen05.ld and write fp32 (and, if asked, the int32).
 // The activations are stored with the 4x4 index transpose inside every 16-element block that the
 // masked decode of a packed word implies (same trick as the CUDA-core kernel), so a packed word
-// expands with 4 x (shift, and, byte-subtract) and lands as one aligned 16-byte chunk.
+// expands with 4 x (shift, and).
+//
+// What bounds it, and why the weights go through tensor memory: with the expanded tile in shared memory a block of
+// 128 x 256 x 128 moved 104 KB through the SM's 128 bytes per cycle (expanded tile written and read, activations
+// written and read), 812 cycles for 512 of MMA; measured 850.  In tensor memory only the activations are left.
+//
+// Gated pairing (PAIR): tile 0 holds gate rows and tile 1 the up rows of the same features, so ReLU^2 / SiLU and the
+// product are formed in the epilogue.  K split: gridDim.z CTAs of one cluster take a K range each and hand their
+// int32 partial sums of the token columns they do not finish to the CTA that does, through distributed shared memory.
 //
 // Every wait on an mbarrier is bounded; on expiry the kernel records an error code, stops issuing
 // work, drains its own copies, frees its tensor memory and returns.
@@ -30,19 +38,40 @@
 
 namespace lspk {
 
-constexpr int kTcThreads = 320;          // 10 warps: TMA, MMA, 4 x expand + epilogue, 4 x epilogue only
-constexpr int kTcStages = 4;
-constexpr int kTcBK = 128;               // K elements per pipeline block
-constexpr int kTcRows = 128;             // output features per CTA
+constexpr int kTcThreads = 352;          // 11 warps: activation TMA, MMA, 8 x expand + epilogue, weight TMA
+constexpr int kTcBK = 256;               // K elements per pipeline block
+constexpr int kTcRows = 128;             // output features per tile
+constexpr int kTcWStages = 4;            // ring of packed weights
 constexpr unsigned kSpinLimit = 1u << 22;
 
-// One matrix of a launch: the matrices of a call (q/k/v; gate/up) share the activations and are covered by one
-// grid, matrix i owning the output-feature tiles [tile0, tile0 + ceil(N / 128)) of gridDim.x.
+// Shared- and tensor-memory plan of one instantiation.  FM feature tiles: two (gate and up) for the gated pairing, else
+// one.  One feature tile of up to 64 token rows takes half the tensor memory, so that two CTAs share an SM and one's
+// epilogue and start-up run under the other's MMAs; the others take all of it.
+template <bool PAIR, int TN>
+struct TcLayout {
+    static constexpr int FM = PAIR ? 2 : 1;
+    static constexpr bool kHalf = !PAIR && TN <= 64;
+    static constexpr int kX = kHalf ? (TN == 64 ? 3 : 5) : TN >= 96 ? 4 : TN == 64 ? 6 : 8;
+    static constexpr int kXBytes = TN * kTcBK;             // two swizzled tiles of TN x 128 bytes
+    static constexpr int kTileBytes = kTcRows * kTcBK / 4; // packed weights of one feature tile
+    static constexpr int kWBytes = FM * kTileBytes;
+    static constexpr int kCols = kHalf ? 256 : 512;        // tensor memory of a CTA
+    static constexpr int kACols = kTcBK / 4;               // columns of one expanded tile
+    static constexpr int kAMax = (kCols - FM * TN) / (FM * kACols);
+    static constexpr int kA = kAMax > 4 ? 4 : kAMax;       // operand ring
+    static constexpr int kSlab = TN == 32 ? 8 : 16;        // token columns an epilogue warp reads at once
+    static constexpr int kSlabs = TN / kSlab;
+    static constexpr int kMaxSplits = PAIR && TN > 64 ? 1 : kSlabs % 4 ? 2 : 4;
+    static constexpr int kRedBytes = FM * kTcRows * TN * 4 / kMaxSplits * (kMaxSplits - 1);
+    static constexpr int kSmem = kX * kXBytes + kTcWStages * kWBytes + kRedBytes + 1024;
+    static_assert(kA >= 2 && kSmem <= (kHalf ? 110 : 225) * 1024, "does not fit");
+};
+
+// One matrix of a launch: the matrices of a call (q/k/v) share the activations and are covered by one grid, matrix
+// i owning the feature tiles [tile0, next matrix's tile0) of gridDim.x.  Pairing: segment 0 gate, segment 1 up.
 struct TcSeg {
     float* out;
     int32_t* acc_out;
-    int32_t* split_ws;       // K split / gated pairing: this CTA's K range stores its int32 partial sums in slice
-                             // blockIdx.z of this workspace ([splits][M, N]); the finish kernel adds the slices
     float w_scale;
     int N;
     int tile0;
@@ -51,10 +80,11 @@ struct TcParams {
     TcSeg seg[3];
     int n_seg;
     const float* x_scales;
+    const int* x_sums;
     int M, K;
     int k_blocks;            // K blocks of the whole product
     int kb_per_split;        // K blocks per CTA along gridDim.z (== k_blocks when K is not split)
-    int epilogue;            // LSPK_EPI_STORE or LSPK_EPI_ADD
+    int epilogue;
     int* error_flag;
     unsigned long long* trace;   // optional phase trace: one record per role of CTA (0,0,0) (ids 10, 11, 12)
     int trace_cap;
@@ -92,59 +122,143 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
     return d;
 }
 
-template <int TN>
-__global__ void __launch_bounds__(kTcThreads)
+// True in exactly one lane of a converged warp.  The single-thread instructions below (bulk copies, MMAs, commits) take
+// uniform operands: behind this predicate the compiler knows that one lane runs them.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void tc_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// 32 columns of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_store_32(uint32_t addr, const uint32_t* v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
+        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+// 8, 16 or 32 columns of this thread's TMEM lane, complete on return.
+template <int W>
+__device__ __forceinline__ void tmem_load(uint32_t addr, uint32_t* v) {
+    if constexpr (W == 8) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                     : "r"(addr)
+                     : "memory");
+    } else if constexpr (W == 16) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(addr)
+            : "memory");
+    } else {
+        static_assert(W == 32, "slabs of 8, 16 or 32 columns");
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+              "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
+              "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
+              "=r"(v[30]), "=r"(v[31])
+            : "r"(addr)
+            : "memory");
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// v[j] for a run-time j without moving v to local memory.
+template <int W>
+__device__ __forceinline__ uint32_t pick(const uint32_t* v, int j) {
+    uint32_t r = v[0];
+#pragma unroll
+    for (int i = 1; i < W; ++i) r = j == i ? v[i] : r;
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+template <bool PAIR, int TN>
+__global__ void __launch_bounds__(kTcThreads, TcLayout<PAIR, TN>::kHalf ? 2 : 1)
 ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                        const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x,
                        const __grid_constant__ TcParams p) {
-    constexpr int kPackedBytes = kTcRows * kTcBK / 4;       // 4096
-    constexpr int kATileBytes = kTcRows * kTcBK;            // 16384
-    constexpr int kBTileBytes = TN * kTcBK;
-    constexpr int kStageBytes = kPackedBytes + kATileBytes + kBTileBytes;
-    constexpr uint32_t kTmemCols = TN < 32 ? 32 : TN;       // power of two >= 32
-    // instruction descriptor: D = s32, A = B = signed int8, both K-major, N = TN, M = 128
+    using L = TcLayout<PAIR, TN>;
+    constexpr int FM = L::FM;
+    constexpr int kX = L::kX, kA = L::kA, kW = kTcWStages, W = L::kSlab, kBK = kTcBK;
+    // instruction descriptor: D = s32, A = B = signed int8 (the weight codes 0, 1, 2 are their own int8 values), both
+    // K-major, N = TN, M = 128
     constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((128u >> 4) << 24);
 
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t full_w[kTcStages];     // packed weights of the stage have landed
-    __shared__ __align__(8) uint64_t full_tma[kTcStages];   // activation tile of the stage has landed
-    __shared__ __align__(8) uint64_t full_a[kTcStages];
-    __shared__ __align__(8) uint64_t empty[kTcStages];
+    __shared__ __align__(8) uint64_t full_w[kW], empty_w[kW];   // packed weights: landed / read by the expanders
+    __shared__ __align__(8) uint64_t full_x[kX], empty_x[kX];   // activations: landed / multiplied
+    __shared__ __align__(8) uint64_t full_a[kA], empty_a[kA];   // operand: expanded (and activations landed) / multiplied
     __shared__ __align__(8) uint64_t acc_ready;
+    __shared__ __align__(8) float2 tok[TN];                 // per token: quantiser scale, sum of its int8 values (bits)
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    // warps 2-9: two sets of four, each covering the 128 TMEM lanes
+    const int set = warp < 6 ? 0 : 1, quarter = warp & 3, row = quarter * 32 + lane;   // row of a tile == TMEM lane
+    // feature tile of this CTA: matrix, first feature of tile 0
     int sgi = 0;
-    if (p.n_seg > 1 && (int)blockIdx.x >= p.seg[1].tile0) sgi = 1;
-    if (p.n_seg > 2 && (int)blockIdx.x >= p.seg[2].tile0) sgi = 2;
+    if (!PAIR) {
+        if (p.n_seg > 1 && (int)blockIdx.x >= p.seg[1].tile0) sgi = 1;
+        if (p.n_seg > 2 && (int)blockIdx.x >= p.seg[2].tile0) sgi = 2;
+    }
     const TcSeg& sg = p.seg[sgi];
     const CUtensorMap* map_w = sgi == 0 ? &map_w0 : sgi == 1 ? &map_w1 : &map_w2;
     const int n0 = ((int)blockIdx.x - sg.tile0) * kTcRows;
     const int m0 = blockIdx.y * TN;
-    // K split: this CTA's K blocks are [kb0, kb0 + nkb)
-    const int kb0 = blockIdx.z * p.kb_per_split;
+    // K split over the cluster: this CTA's K blocks are [kb0, kb0 + nkb)
+    const int splits = gridDim.z, rank = blockIdx.z;
+    const int kb0 = rank * p.kb_per_split;
     const int nkb = min(p.kb_per_split, p.k_blocks - kb0);
 
-    auto a_tile = [&](int s) { return smem + (size_t)s * kStageBytes; };
-    auto b_tile = [&](int s) { return smem + (size_t)s * kStageBytes + kATileBytes; };
-    auto packed = [&](int s) { return smem + (size_t)s * kStageBytes + kATileBytes + kBTileBytes; };
+    auto x_tile = [&](int s) { return smem + (size_t)s * L::kXBytes; };
+    auto packed = [&](int s, int f) { return smem + (size_t)kX * L::kXBytes + (size_t)s * L::kWBytes + f * L::kTileBytes; };
+    int32_t* red = reinterpret_cast<int32_t*>(smem + (size_t)kX * L::kXBytes + (size_t)kW * L::kWBytes);   // from the peers
 
     if (tid == 0) {
         abort_flag = 0;
-        for (int s = 0; s < kTcStages; ++s) {
+        for (int s = 0; s < kW; ++s) {
             mbar_init(&full_w[s], 1);
-            mbar_init(&full_tma[s], 1);
-            mbar_init(&full_a[s], 4);                      // one arrival per expansion warp
-            mbar_init(&empty[s], 1);
+            mbar_init(&empty_w[s], 4 * FM);                 // one arrival per expanding warp
+        }
+        for (int s = 0; s < kX; ++s) {
+            mbar_init(&full_x[s], 1);
+            mbar_init(&empty_x[s], 1);
+        }
+        for (int s = 0; s < kA; ++s) {
+            mbar_init(&full_a[s], 4 * FM);
+            mbar_init(&empty_a[s], 1);
         }
         mbar_init(&acc_ready, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_mbar_init();
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
-                     "r"(kTmemCols)
+                     "r"((uint32_t)L::kCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -152,285 +266,304 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_a = tmem_base + FM * TN;            // columns behind the accumulators: the operand ring
     volatile int* abortp = &abort_flag;
+    if (splits > 1) cluster_arrive();                       // "this CTA runs": awaited before the first remote store
 
     grid_dependency_launch();
-    // The packed weights do not depend on the previous kernel: the producer requests the first ring of them, and
-    // the expansion warps turn them into operand tiles, while that kernel is still running.  Whoever touches the
-    // activations, the scales or the outputs waits for it first.
-    auto load_weights = [&](int kb) {
-        const int s = kb % kTcStages;
-        mbar_expect_tx(&full_w[s], kPackedBytes);
-        // inner coordinate in 4-byte units (a K block is 2 chunks x 16 rows x 16 bytes = 128 units per row
-        // group), outer coordinate = row group
-        tma_load_2d(packed(s), map_w, (kb0 + kb) * 128, n0 / kRowsPerGroup, &full_w[s]);
-    };
-
+    // The packed weights do not depend on the previous kernel: they are requested, and expanded, while it is still
+    // running.  Whoever touches the activations, the scales or the outputs waits for it first.
+    const int own = L::kSlabs / splits;                     // token slabs this CTA finishes: [rank * own, rank * own + own)
+    float res[(L::kSlabs + 1) / 2][W];                      // residual of this thread's outputs (ADD epilogue)
+    bool ok = true;
     if (warp == 0) {
-        // ---------------- producer ------------------------------------------------------------
-        if (lane == 0) {
-            PhaseTrace tr;
-            tr.begin(p.trace, p.trace_cap, 10, 0);
-            const int early = min(nkb, kTcStages);
-            for (int kb = 0; kb < early; ++kb) load_weights(kb);
-            grid_dependency_wait();
-            int issued = 0;
-            for (int kb = 0; kb < nkb; ++kb) {
-                if ((kb & 1) == 0) tr.mark();              // before the wait for blocks 0, 2, 4, ...
-                const int s = kb % kTcStages;
-                if (kb >= kTcStages && !mbar_wait(&empty[s], ((kb / kTcStages) - 1) & 1, abortp)) break;
-                if (*abortp) break;
-                if (kb >= early) load_weights(kb);
-                mbar_expect_tx(&full_tma[s], kBTileBytes);
-                tma_load_2d(b_tile(s), &map_x, (kb0 + kb) * kTcBK, m0, &full_tma[s]);
-                ++issued;
-            }
-            tr.end();
-            if (*abortp) {
-                // drain: wait (bounded) for every copy this thread started
-                const int w_issued = issued > early ? issued : early;
-                for (int kb = 0; kb < w_issued; ++kb) {
-                    const int s = kb % kTcStages;
-                    if (kb + kTcStages >= w_issued)
-                        for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&full_w[s], (kb / kTcStages) & 1); ++i) {}
-                }
-                for (int kb = 0; kb < issued; ++kb) {
-                    const int s = kb % kTcStages;
-                    if (kb + kTcStages >= issued)
-                        for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&full_tma[s], (kb / kTcStages) & 1); ++i) {}
-                }
-            }
-        }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer ------------------------------------------------------------
-        if (lane == 0) {
-            PhaseTrace tr;
-            tr.begin(p.trace, p.trace_cap, 11, 32);
-            grid_dependency_wait();
-            bool ok = true;
-            for (int kb = 0; kb < nkb && ok; ++kb) {
-                if ((kb & 1) == 0) tr.mark();
-                const int s = kb % kTcStages;
-                const uint32_t ph = (kb / kTcStages) & 1;
-                ok = mbar_wait(&full_tma[s], ph, abortp) && mbar_wait(&full_a[s], ph, abortp);
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t da = umma_desc_sw128(smem_u32(a_tile(s)));
-                const uint64_t db = umma_desc_sw128(smem_u32(b_tile(s)));
-#pragma unroll
-                for (int k4 = 0; k4 < kTcBK / 32; ++k4) {
-                    const uint32_t accumulate = (kb | k4) ? 1u : 0u;
-                    // advancing 32 int8 along K = 32 bytes = 2 descriptor address units
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                        ::"r"(tmem_base), "l"(da + (uint64_t)(k4 * 2)), "l"(db + (uint64_t)(k4 * 2)), "r"(kIdesc),
-                        "r"(accumulate)
-                        : "memory");
-                }
-                // frees the stage for the producer once the MMAs above have read it
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&empty[s]))
-                             : "memory");
-            }
-            // On the regular path this tells the epilogue warps that every MMA has completed.  After an abort
-            // nobody waits on it any more (they saw the abort flag), and the same commit + one bounded wait makes
-            // sure that no MMA issued above is still in flight when the tensor memory is freed below.
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&acc_ready))
-                         : "memory");
-            if (!ok)
-                for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&acc_ready, 0); ++i) {}
-            tr.end();
-        }
-    } else {
-        // ---------------- expand packed weights -> int8 operand tile, then epilogue ---------------
-        const int row = tid - 64;                         // 0..127: weight row inside the CTA tile
-        const int gi = row >> 4, rr = row & 15;
-        bool ok = true;
+        // ---------------- activation producer (whole warp in step, one lane issues) --------------
         PhaseTrace tr;
-        tr.begin(p.trace, p.trace_cap, 12, 64);
-        // warps 6-9 take no part in the expansion: they double the warps that drain the accumulators afterwards
-        for (int kb = 0; kb < (warp < 6 ? nkb : 0) && ok; ++kb) {
-            if ((kb & 7) == 0 && kb < 24) tr.mark();
-            const int s = kb % kTcStages;
-            // warp-uniform: every lane polls with its own counter, and the barrier below needs the whole warp
-            ok = __all_sync(0xffffffffu, mbar_wait(&full_w[s], (kb / kTcStages) & 1, abortp));
+        tr.begin(p.trace, p.trace_cap, 10, 0);
+        grid_dependency_wait();
+        int kb = 0;
+        for (; kb < nkb; ++kb) {
+            tr.mark();
+            const int s = kb % kX;
+            if (kb >= kX) ok = __all_sync(0xffffffffu, mbar_wait(&empty_x[s], ((kb / kX) - 1) & 1, abortp));
             if (!ok) break;
-            const unsigned char* pk = packed(s);
-            unsigned char* arow = a_tile(s) + (size_t)(row >> 3) * 1024 + (size_t)(row & 7) * 128;
+            if (elect_one()) {
+                mbar_expect_tx(&full_x[s], L::kXBytes);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {                  // the two 64-weight chunks of this K block
-                const uint4 w = *reinterpret_cast<const uint4*>(pk + gi * 512 + c * 256 + rr * 16);
-                const uint32_t words[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    uint4 o;
-                    o.x = __vsub4(words[m] & 0x03030303u, 0x01010101u);
-                    o.y = __vsub4((words[m] >> 2) & 0x03030303u, 0x01010101u);
-                    o.z = __vsub4((words[m] >> 4) & 0x03030303u, 0x01010101u);
-                    o.w = __vsub4((words[m] >> 6) & 0x03030303u, 0x01010101u);
-                    const int chunk = c * 4 + m;           // 16-byte chunk index inside the 128-byte row
-                    *reinterpret_cast<uint4*>(arow + ((chunk ^ (row & 7)) << 4)) = o;
-                }
+                for (int hf = 0; hf < kBK / 128; ++hf)
+                    tma_load_2d(x_tile(s) + hf * (TN * 128), &map_x, (kb0 + kb) * kBK + hf * 128, m0, &full_x[s]);
             }
-            fence_async_smem();                            // generic-proxy writes -> visible to the tensor unit
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full_a[s]);        // 4 arrivals per stage instead of 128
-        }
-        // epilogue: TMEM lane = weight row, column = token
-        grid_dependency_wait();                            // scales, residual and outputs belong to the chain
-        tr.mark();                                         // all blocks expanded
-        __syncwarp();
-        if (ok) ok = mbar_wait(&acc_ready, 0, abortp);
-        tr.mark();                                         // accumulators complete
-        ok = __all_sync(0xffffffffu, ok);              // the tensor-memory loads below need the whole warp
-        if (ok) {
-            tc_fence_after();
-            const int quarter = warp & 3;                  // TMEM lanes this warp may read
-            const int n = n0 + quarter * 32 + lane;
-#pragma unroll 1
-            // two warps share a quarter of the TMEM lanes: they take alternate 32-column slabs
-            for (int cb = warp < 6 ? 0 : 1; cb < TN / 32; cb += 2) {
-                uint32_t v[32];
-                tr.mark();                                 // previous slab stored
-                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-                      "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
-                      "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
-                      "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                tr.mark();                                 // a 32-column slab of accumulators is in registers
-                const int t0 = m0 + cb * 32;
-                const int jmax = min(32, p.M - t0);        // token rows of this slab that exist
-                // scale of token row t0 + lane (one coalesced load; handed round by shuffles below)
-                const float my_scale = (!sg.split_ws && lane < jmax) ? __fmul_rn(__ldg(p.x_scales + t0 + lane), sg.w_scale) : 0.0f;
-                float sc[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) sc[j] = __shfl_sync(0xffffffffu, my_scale, j);
-                if (n < sg.N && jmax > 0) {
-                    const size_t o0 = (size_t)t0 * sg.N + n;
-                    if (sg.split_ws) {
-                        // partial sums of this K range: exact in int32, slice blockIdx.z of the workspace
-                        int32_t* wsp = sg.split_ws + (size_t)blockIdx.z * p.M * sg.N + o0;
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (j < jmax) wsp[(size_t)j * sg.N] = (int)v[j];
-                    } else {
-                        float* outp = sg.out + o0;
-                        if (sg.acc_out) {
-                            int32_t* accp = sg.acc_out + o0;
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (j < jmax) accp[(size_t)j * sg.N] = (int)v[j];
-                        }
-                        // every load of the slab before its first store: the stores may alias the residual as far
-                        // as the compiler knows, and would otherwise serialise 32 round trips
-                        if (p.epilogue == LSPK_EPI_ADD) {
-                            float res[32];
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) res[j] = j < jmax ? outp[(size_t)j * sg.N] : 0.0f;
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (j < jmax)
-                                    outp[(size_t)j * sg.N] = __fadd_rn(res[j], __fmul_rn((float)(int)v[j], sc[j]));
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (j < jmax) outp[(size_t)j * sg.N] = __fmul_rn((float)(int)v[j], sc[j]);
-                        }
-                    }
-                }
-            }
         }
         tr.end();
+        // after an abort: wait (bounded) for every copy this warp started
+        if (!ok)
+            for (int b = max(0, kb - kX); b < kb; ++b)
+                for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&full_x[b % kX], (b / kX) & 1); ++i) {}
+        __syncwarp();
+    } else if (warp == 10) {
+        // ---------------- weight producer ---------------------------------------------------------
+        int kb = 0;
+        for (; kb < nkb; ++kb) {
+            const int s = kb % kW;
+            if (kb >= kW) ok = __all_sync(0xffffffffu, mbar_wait(&empty_w[s], ((kb / kW) - 1) & 1, abortp));
+            if (!ok) break;
+            if (elect_one()) {
+                mbar_expect_tx(&full_w[s], L::kWBytes);
+                // inner coordinate in 4-byte units (16 rows x 16 bytes per 64 of K: kBK units of 4 bytes per row
+                // group), outer coordinate = row group; a tile past the matrix reads zeros
+#pragma unroll
+                for (int f = 0; f < FM; ++f)
+                    tma_load_2d(packed(s, f), PAIR && f == 1 ? &map_w1 : map_w, (kb0 + kb) * kBK, n0 / kRowsPerGroup, &full_w[s]);
+            }
+            __syncwarp();
+        }
+        if (!ok)
+            for (int b = max(0, kb - kW); b < kb; ++b)
+                for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&full_w[b % kW], (b / kW) & 1); ++i) {}
+        __syncwarp();
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (whole warp in step, one lane issues) ----------------------
+        PhaseTrace tr;
+        tr.begin(p.trace, p.trace_cap, 11, 32);
+        for (int kb = 0; kb < nkb; ++kb) {
+            tr.mark();
+            const int s = kb % kX, sa = kb % kA;
+            // the expanders arrive here only after the activations of the block have landed too
+            ok = __all_sync(0xffffffffu, mbar_wait(&full_a[sa], (kb / kA) & 1, abortp));
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t db = umma_desc_sw128(smem_u32(x_tile(s)));
+            if (elect_one()) {
+#pragma unroll
+                for (int f = 0; f < FM; ++f) {
+#pragma unroll
+                    for (int k8 = 0; k8 < kBK / 32; ++k8) {
+                        const uint32_t accumulate = (kb | k8) ? 1u : 0u;
+                        // 32 int8 along K: 8 columns of the operand ring; in the activations 2 descriptor address
+                        // units (32 bytes), the second 128 in a swizzled tile of its own
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\t"
+                            "setp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+                            ::"r"(tmem_base + (uint32_t)(f * TN)), "r"(tmem_a + (uint32_t)((sa * FM + f) * L::kACols + k8 * 8)),
+                            "l"(db + (uint64_t)((k8 >> 2) * (TN * 128 / 16) + (k8 & 3) * 2)), "r"(kIdesc), "r"(accumulate)
+                            : "memory");
+                    }
+                }
+                tc_commit(&empty_a[sa]);                   // free the operand stage and the shared-memory stage
+                tc_commit(&empty_x[s]);                    // once the MMAs above have read them
+            }
+            __syncwarp();
+        }
+        // On the regular path this tells the epilogue warps that every MMA has completed.  After an abort
+        // nobody waits on it any more (they saw the abort flag), and the same commit + one bounded wait makes
+        // sure that no MMA issued above is still in flight when the tensor memory is freed below.
+        if (elect_one()) tc_commit(&acc_ready);
+        if (!ok)
+            for (unsigned i = 0; i < kSpinLimit && !mbar_try_wait(&acc_ready, 0); ++i) {}
+        tr.end();
+        __syncwarp();
+    } else {
+        // ---------------- expand packed weights into the tensor-memory operand ring ---------------
+        // With two feature tiles set e expands tile e of every K block, with one the sets take alternate blocks.
+        const unsigned char* pk = packed(0, FM == 2 ? set : 0) + (row >> 4) * (kBK * 4) + (row & 15) * 16;
+        const uint32_t ta = tmem_a + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(FM == 2 ? set * L::kACols : 0);
+        constexpr int kStep = FM == 2 ? 1 : 2;
+        PhaseTrace tr;
+        tr.begin(p.trace, p.trace_cap, 12, 64);
+        uint4 w[kBK / 64];                                 // this row's weights of the next block
+        // warp-uniform results: every lane polls with its own counter, and what follows needs the whole warp
+        auto fetch = [&](int kb) {
+            const int sw = kb % kW;
+            ok = __all_sync(0xffffffffu, mbar_wait(&full_w[sw], (kb / kW) & 1, abortp));
+            if (ok) {
+#pragma unroll
+                for (int c = 0; c < kBK / 64; ++c) w[c] = *reinterpret_cast<const uint4*>(pk + (size_t)sw * L::kWBytes + c * 256);
+            }
+        };
+        int kb = FM == 2 ? 0 : set;
+        if (kb < nkb) fetch(kb);
+        for (; kb < nkb && ok; kb += kStep) {
+            if (kb < 20) tr.mark();
+            const int sa = kb % kA;
+            if (kb >= kA) ok = __all_sync(0xffffffffu, mbar_wait(&empty_a[sa], ((kb / kA) - 1) & 1, abortp));
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int hf = 0; hf < kBK / 128; ++hf) {
+                uint32_t o[32];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const uint4 wc = w[hf * 2 + c];
+                    const uint32_t words[4] = {wc.x, wc.y, wc.z, wc.w};
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) o[c * 16 + m * 4 + j] = (words[m] >> (2 * j)) & 0x03030303u;
+                }
+                tmem_store_32(ta + (uint32_t)(sa * FM * L::kACols + hf * 32), o);
+            }
+            if (lane == 0) mbar_arrive(&empty_w[kb % kW]);
+            if (quarter == 0) ok = __all_sync(0xffffffffu, mbar_wait(&full_x[kb % kX], (kb / kX) & 1, abortp));
+            if (!ok) break;
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full_a[sa]);
+            if (kb + kStep < nkb) fetch(kb + kStep);
+        }
+        grid_dependency_wait();                            // scales, residual and outputs belong to the chain
+        tr.mark();                                         // all blocks expanded
+        for (int t = tid - 64; t < TN; t += 256)
+            tok[t] = m0 + t < p.M ? make_float2(p.x_scales[m0 + t], __int_as_float(p.x_sums[m0 + t])) : make_float2(0.f, 0.f);
+        if (!PAIR && p.epilogue == LSPK_EPI_ADD) {         // under the last MMAs
+#pragma unroll
+            for (int i = 0; i < (L::kSlabs + 1) / 2; ++i) {
+                const int t0 = m0 + (rank * own + set + 2 * i) * W, n = n0 + row;
+                const int jmax = n < sg.N && set + 2 * i < own ? min(W, p.M - t0) : 0;
+#pragma unroll
+                for (int j = 0; j < W; ++j) res[i][j] = j < jmax ? sg.out[(size_t)(t0 + j) * sg.N + n] : 0.0f;
+            }
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (ok) ok = mbar_wait(&acc_ready, 0, abortp);
+        tr.mark();                                         // accumulators complete
+        tr.end();
+        ok = __all_sync(0xffffffffu, ok);                  // the tensor-memory loads below need the whole warp
+        tc_fence_after();
+    }
+
+    // ---- epilogue: TMEM lane = feature, column = token; kSlabs slabs of W columns per feature tile ----------------
+    const bool finisher = warp >= 2 && warp < 10 && ok;
+    const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    if (splits > 1) {
+        cluster_wait();                                    // every CTA of the cluster is running
+        if (finisher) {
+            // hand the partial sums of the other CTAs' slabs to them: red[source][tile][column][row] of the owner
+            for (int i = set; i < FM * L::kSlabs; i += 2) {
+                const int f = i / L::kSlabs, sl = i % L::kSlabs, owner = sl / own;
+                if (owner == rank) continue;
+                uint32_t v[W];
+                tmem_load<W>(tlane + (uint32_t)(f * TN + sl * W), v);
+                const int src = rank < owner ? rank : rank - 1;
+                const uint32_t local = smem_u32(red + ((size_t)((src * FM + f) * own + (sl - owner * own)) * W) * kTcRows + row);
+                const uint32_t remote = map_to_rank(local, (uint32_t)owner);
+#pragma unroll
+                for (int j = 0; j < W; ++j) st_cluster_u32(remote + (uint32_t)(j * kTcRows * 4), v[j]);
+            }
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
+    if (finisher) {
+        const int n = n0 + row;
+        auto load_slab = [&](int f, int sl, uint32_t* v) {
+            tmem_load<W>(tlane + (uint32_t)(f * TN + sl * W), v);
+            if (splits > 1) {
+                const int32_t* r0 = red + ((size_t)(f * own + (sl - rank * own)) * W) * kTcRows + row;
+                for (int src = 0; src < splits - 1; ++src)
+#pragma unroll
+                    for (int j = 0; j < W; ++j) v[j] += (uint32_t)r0[((size_t)src * FM * own * W + j) * kTcRows];
+            }
+        };
+        // The element loops are straight-line code (no branch inside: with the taps and the choice of epilogue decided
+        // per element a slab of a gate/up pair took 2500 cycles, as long as two K blocks).
+        if constexpr (PAIR) {
+            const TcSeg &g = p.seg[0], &u = p.seg[1];
+#pragma unroll 1
+            for (int sl = rank * own + set; sl < rank * own + own; sl += 2) {
+                uint32_t vg[W], vu[W];
+                load_slab(0, sl, vg);
+                load_slab(1, sl, vu);
+                const int t0 = m0 + sl * W, jmax = n < g.N ? min(W, p.M - t0) : 0;
+                const size_t o0 = (size_t)t0 * g.N + n;
+                float y[W];
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    const float2 ti = tok[sl * W + j];
+                    vg[j] -= (uint32_t)__float_as_int(ti.y);
+                    vu[j] -= (uint32_t)__float_as_int(ti.y);
+                    y[j] = ti.x;
+                }
+                if (g.acc_out)
+                    for (int j = 0; j < jmax; ++j) g.acc_out[o0 + (size_t)j * g.N] = (int)pick<W>(vg, j);
+                if (u.acc_out)
+                    for (int j = 0; j < jmax; ++j) u.acc_out[o0 + (size_t)j * g.N] = (int)pick<W>(vu, j);
+                if (p.epilogue == LSPK_EPI_SILU_MUL) {
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        const float yg = __fmul_rn((float)(int)vg[j], __fmul_rn(y[j], g.w_scale));
+                        const float yu = __fmul_rn((float)(int)vu[j], __fmul_rn(y[j], u.w_scale));
+                        y[j] = __fmul_rn(__fdiv_rn(yg, __fadd_rn(expf(-yg), 1.0f)), yu);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        const float gpos = fmaxf(__fmul_rn((float)(int)vg[j], __fmul_rn(y[j], g.w_scale)), 0.0f);
+                        const float yu = __fmul_rn((float)(int)vu[j], __fmul_rn(y[j], u.w_scale));
+                        y[j] = __fmul_rn(__fmul_rn(gpos, gpos), yu);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    if (j < jmax) g.out[o0 + (size_t)j * g.N] = y[j];
+            }
+        } else {
+            const bool add = p.epilogue == LSPK_EPI_ADD;
+#pragma unroll
+            for (int i = 0; i < (L::kSlabs + 1) / 2; ++i) {
+                const int sl = rank * own + set + 2 * i;
+                if (set + 2 * i >= own) break;
+                const int t0 = m0 + sl * W, jmax = n < sg.N ? min(W, p.M - t0) : 0;
+                float* outp = sg.out + (size_t)t0 * sg.N + n;
+                uint32_t v[W];
+                load_slab(0, sl, v);
+                float y[W];
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    const float2 ti = tok[sl * W + j];
+                    v[j] -= (uint32_t)__float_as_int(ti.y);
+                    y[j] = __fmul_rn((float)(int)v[j], __fmul_rn(ti.x, sg.w_scale));
+                }
+                if (sg.acc_out)
+                    for (int j = 0; j < jmax; ++j) sg.acc_out[(size_t)(t0 + j) * sg.N + n] = (int)pick<W>(v, j);
+                if (add) {
+#pragma unroll
+                    for (int j = 0; j < W; ++j) y[j] = __fadd_rn(res[i][j], y[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    if (j < jmax) outp[(size_t)j * sg.N] = y[j];
+            }
+        }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
-        __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)L::kCols) : "memory");
     }
     if (tid == 0 && abort_flag && p.error_flag) atomicExch(p.error_flag, LSPK_ERR_DEVICE_WAIT);
 }
 
-// K split: int32 sums of all K ranges -> fp32 outputs (rescale, residual add or the gated pairing), and the
-// raw accumulators where asked for.  Up to three matrices of one call are finished by one launch; for the
-// gated epilogues segment 0 is the gate and segment 1 the up projection (same N), and only out[0] is written.
-struct FinishSeg {
-    const int32_t* ws;       // [splits][M, N]
-    float* out;
-    int32_t* acc_out;
-    float w_scale;
-    int N;
-    int splits;
-};
-struct FinishParams {
-    FinishSeg seg[3];
-    int n_seg;
-    int M;
-    int epilogue;
-    const float* x_scales;
-};
-
-// Sum of one element over the K-range slices (at most 8): all loads issued before the first add.
-__device__ __forceinline__ int sum_slices(const int32_t* first, size_t slice, int splits) {
-    int v[8];
-#pragma unroll
-    for (int z = 0; z < 8; ++z) v[z] = z < splits ? first[(size_t)z * slice] : 0;
-    return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-}
-
-__global__ void splitk_finish_kernel(const FinishParams p) {
-    grid_dependency_launch();
-    grid_dependency_wait();
-    const bool pair = p.epilogue == LSPK_EPI_RELU2_MUL || p.epilogue == LSPK_EPI_SILU_MUL;
-    const int n_seg = pair ? 1 : p.n_seg;
-    for (int sgi = 0; sgi < n_seg; ++sgi) {
-        const FinishSeg sg = p.seg[sgi];
-        const size_t total = (size_t)p.M * sg.N;
-        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-            const int t = (int)(i / sg.N);
-            const int a = sum_slices(sg.ws + i, total, sg.splits);
-            if (sg.acc_out) sg.acc_out[i] = a;
-            const float xs = p.x_scales[t];
-            const float y = __fmul_rn((float)a, __fmul_rn(xs, sg.w_scale));
-            if (pair) {
-                const int b = sum_slices(p.seg[1].ws + i, total, p.seg[1].splits);
-                if (p.seg[1].acc_out) p.seg[1].acc_out[i] = b;
-                const float u = __fmul_rn((float)b, __fmul_rn(xs, p.seg[1].w_scale));
-                if (p.epilogue == LSPK_EPI_SILU_MUL) {
-                    sg.out[i] = __fmul_rn(__fdiv_rn(y, __fadd_rn(expf(-y), 1.0f)), u);
-                } else {
-                    const float gpos = fmaxf(y, 0.0f);
-                    sg.out[i] = __fmul_rn(__fmul_rn(gpos, gpos), u);
-                }
-            } else {
-                sg.out[i] = p.epilogue == LSPK_EPI_ADD ? __fadd_rn(sg.out[i], y) : y;
-            }
-        }
-    }
-}
-
 // int8 rows [M, K] in natural order -> [M, Kp] with the 4x4 transpose inside every 16-element block
-// (Kp = K rounded up to 64, zero padded), the order the expanded weights come out in.
-__global__ void permute_rows_kernel(const int8_t* __restrict__ src, int8_t* __restrict__ dst, int M, int K, int Kp) {
+// (Kp = K rounded up to 64, zero padded), the order the expanded weights come out in, and the sum of each row.
+__global__ void __launch_bounds__(256)
+permute_rows_kernel(const int8_t* __restrict__ src, int8_t* __restrict__ dst, int* __restrict__ sums, int K, int Kp) {
+    __shared__ int part[32];
     grid_dependency_launch();
     grid_dependency_wait();
-    const size_t total = (size_t)M * Kp;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(i / Kp), kp = (int)(i % Kp);
+    const size_t t = blockIdx.x;
+    int sum = 0;
+    for (int kp = threadIdx.x; kp < Kp; kp += blockDim.x) {
         const int k = perm_index(kp);                      // the transpose is its own inverse
-        dst[i] = k < K ? src[(size_t)t * K + k] : (int8_t)0;
+        const int8_t v = k < K ? src[t * K + k] : (int8_t)0;
+        dst[t * Kp + kp] = v;
+        sum += v;
     }
+    sum = block_sum(sum, part);
+    if (threadIdx.x == 0) sums[t] = sum;
 }
 
 // ---- host side -------------------------------------------------------------------------------------
@@ -454,9 +587,8 @@ struct TcScratch {
     int8_t *xq = nullptr, *xq_perm = nullptr;
     float* xs = nullptr;
     int* err = nullptr;
-    int32_t* split_ws = nullptr;
     int* xsum = nullptr;
-    size_t cap_xq = 0, cap_perm = 0, cap_xs = 0, cap_ws = 0, cap_xsum = 0;
+    size_t cap_xq = 0, cap_perm = 0, cap_xs = 0, cap_xsum = 0;
 };
 static TcScratch g_tc;
 
@@ -487,25 +619,107 @@ int quant_scratch(size_t M, size_t K, int8_t** q, float** s, int** sums) {
     return LSPK_OK;
 }
 
-template <int TN>
+// Tensor maps.  A weight keeps its own; of the activation scratch the last few shapes are kept (a prefill uses two, at
+// most four tile widths).  Encoding one costs the host about as long as a launch.
+static int weight_map(EncodeTiledFn enc, CUtensorMap* out, Weight* w) {
+    static_assert(sizeof(CUtensorMap) == sizeof(w->tensor_map), "CUtensorMap is 128 bytes");
+    if (!w->has_map) {
+        const cuuint64_t row_words = (cuuint64_t)w->chunks * 64;          // 4-byte units per row group
+        const cuuint64_t dims[2] = {row_words, (cuuint64_t)w->groups};
+        const cuuint64_t strides[1] = {row_words * 4};
+        const cuuint32_t box[2] = {kTcBK, 8};                             // a K block of 8 row groups
+        const cuuint32_t estr[2] = {1, 1};
+        const CUresult r = enc(reinterpret_cast<CUtensorMap*>(w->tensor_map), CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, w->dev, dims,
+                               strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(LSPK_ERR_CUDA, "tensor map (weights) failed: %d", (int)r);
+        w->has_map = true;
+    }
+    memcpy(out, w->tensor_map, sizeof(*out));
+    return LSPK_OK;
+}
+static int activation_map(EncodeTiledFn enc, CUtensorMap* out, int8_t* x, int Kp, int M, int tn) {
+    struct Entry { int8_t* x; int Kp, M, tn; CUtensorMap map; };
+    static Entry kept[8];
+    static int next = 0;
+    for (const Entry& e : kept)
+        if (e.x == x && e.Kp == Kp && e.M == M && e.tn == tn) {
+            *out = e.map;
+            return LSPK_OK;
+        }
+    const cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)M};
+    const cuuint64_t strides[1] = {(cuuint64_t)Kp};
+    const cuuint32_t box[2] = {128, (cuuint32_t)tn};                      // one swizzled tile: half a K block
+    const cuuint32_t estr[2] = {1, 1};
+    Entry& e = kept[next];
+    e.x = nullptr;
+    const CUresult r = enc(&e.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(LSPK_ERR_CUDA, "tensor map (activations) failed: %d", (int)r);
+    e.x = x;
+    e.Kp = Kp;
+    e.M = M;
+    e.tn = tn;
+    next = (next + 1) % 8;
+    *out = e.map;
+    return LSPK_OK;
+}
+
+template <bool PAIR, int TN>
 static cudaError_t launch_tc(const CUtensorMap* mw, const CUtensorMap& mx, const TcParams& p, dim3 grid) {
-    constexpr size_t smem = (size_t)kTcStages * (kTcRows * kTcBK / 4 + kTcRows * kTcBK + TN * kTcBK) + 1024;
+    constexpr int smem = TcLayout<PAIR, TN>::kSmem;
     static bool attr_set = false;
-    auto kern = ternary_gemm_tc_kernel<TN>;
+    auto kern = ternary_gemm_tc_kernel<PAIR, TN>;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
+    if (grid.z > 1)
+        return launch_cluster(kern, grid, dim3(kTcThreads), smem, true, dim3(1, 1, grid.z), mw[0], mw[1], mw[2], mx, p);
     return launch(kern, grid, dim3(kTcThreads), smem, true, mw[0], mw[1], mw[2], mx, p);
 }
 
-// Tensor-core path.  Handles STORE / ADD epilogues of one or several matrices sharing the input (each matrix is
-// its own GEMM launch) and the gated gate/up pairings (two GEMMs into the int32 workspace, gate applied by the
-// finish kernel).
+// Token rows per tile and K split of a launch: the plan with the smallest time by a model of a CTA's life in SM cycles,
+// fitted to measured launches (q/k/v, o, gate/up and down of a 2560 / 6912 layer at 32 ... 1531 rows, every plan; the
+// pick is within 7 % of the best measured plan at each, on the best one at 17 of 24):
+//   a K block takes the MMA issue and execution time of the CTAs that share the SM, but not less than one turn of the
+//   pipeline; start-up, first copies and epilogue are paid per round of CTAs, a K split pays its exchange.
+// Small M therefore takes many narrow tiles and K ranges (all SMs, short chains), large M the widest tiles.
+struct TcPlan {
+    int tn, splits, kb_per;
+};
+static TcPlan plan_tiles(int tiles, bool pair, int M, int k_blocks) {
+    TcPlan best = {};
+    double best_cost = 1e30;
+    const int fm = pair ? 2 : 1;
+    for (int tn = 32; tn <= 128; tn += 32) {
+        if (tn > 32 && tn - 32 >= M) break;
+        for (int splits = 1; splits <= (pair && tn > 64 ? 1 : tn == 96 ? 2 : 4); splits *= 2) {
+            const int kb_per = (k_blocks + splits - 1) / splits;
+            if (splits > 1 && (kb_per < 2 || (splits - 1) * kb_per >= k_blocks)) continue;
+            const int ctas = tiles * ((M + tn - 1) / tn) * splits, per_sm = (ctas + sm_count() - 1) / sm_count();
+            const int occ = !pair && tn <= 64 ? 2 : 1, rounds = (per_sm + occ - 1) / occ;
+            const double mma = fm * 8 * (tn * 0.47 > 64.0 ? tn * 0.47 : 64.0) * (per_sm < occ ? per_sm : occ);
+            double cost = rounds * (kb_per * (mma > 970.0 ? mma : 970.0) + 6200.0 + 15.5 * fm * tn);
+            if (splits > 1) cost += 400.0 + 5.0 * fm * tn;
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = TcPlan{tn, splits, kb_per};
+            }
+        }
+    }
+    return best;
+}
+
+// Fewest rows this kernel takes: with one eight-row tile the mma.sync kernel (linear_mma.cu) is level with it (33 us for
+// the four products of a layer at 8 rows, here 35), with two it is behind (16 rows: 38 and 34 us; 31 rows: 55 and 36).
+constexpr int kTcMinRows = 9;
+
+// Tensor-core path: one launch for all matrices of the call (plus the row quantiser in front of it).
 int linear_tensor_core(const lspk_linear_args* a, int* handled) {
     *handled = 0;
-    if (a->M < 32) return LSPK_OK;
+    if (a->M < kTcMinRows) return LSPK_OK;
     const bool pair = a->epilogue == LSPK_EPI_RELU2_MUL || a->epilogue == LSPK_EPI_SILU_MUL;
     if (a->epilogue != LSPK_EPI_STORE && a->epilogue != LSPK_EPI_ADD && !pair) return LSPK_OK;
     if (pair && a->n_mats != 2) return LSPK_OK;
@@ -521,6 +735,7 @@ int linear_tensor_core(const lspk_linear_args* a, int* handled) {
     const float* xs = a->x_scales;
     if (int rc = grow((void**)&g_tc.xq_perm, &g_tc.cap_perm, (size_t)M * Kp)) return rc;
     g_tc.err = device_wait_flag();
+    if (int rc = grow((void**)&g_tc.xsum, &g_tc.cap_xsum, (size_t)M * 4)) return rc;
     int permuted = 0;
     if (a->prologue != LSPK_PRO_INT8) {
         if (int rc = grow((void**)&g_tc.xs, &g_tc.cap_xs, (size_t)M * 4)) return rc;
@@ -528,7 +743,7 @@ int linear_tensor_core(const lspk_linear_args* a, int* handled) {
         // fp32 rows: one kernel quantises straight into the permuted layout (unless the caller wants the
         // natural-order int8 rows back as well)
         if (!a->xq_out)
-            if (int rc = quantize_rows_permuted(a, K, Kp, g_tc.xq_perm, g_tc.xs, &permuted)) return rc;
+            if (int rc = quantize_rows_permuted(a, K, Kp, g_tc.xq_perm, g_tc.xs, &permuted, 0, g_tc.xsum)) return rc;
         if (!permuted) {
             if (int rc = grow((void**)&g_tc.xq, &g_tc.cap_xq, (size_t)M * K)) return rc;
             int rc = a->prologue == LSPK_PRO_RMSNORM_QUANT
@@ -538,119 +753,57 @@ int linear_tensor_core(const lspk_linear_args* a, int* handled) {
             xq = g_tc.xq;
         }
     }
-    if (!permuted) {
-        const size_t total = (size_t)M * Kp;
-        int grid = (int)((total + 255) / 256);
-        if (grid > sm_count() * 8) grid = sm_count() * 8;
-        LSPK_CUDA(launch(permute_rows_kernel, dim3(grid), dim3(256), 0, true, xq, g_tc.xq_perm, M, K, Kp));
-    }
+    if (!permuted)
+        LSPK_CUDA(launch(permute_rows_kernel, dim3(M), dim3(256), 0, true, xq, g_tc.xq_perm, g_tc.xsum, K, Kp));
     if (a->xq_out) LSPK_CUDA(cudaMemcpyAsync(a->xq_out, xq, (size_t)M * K, cudaMemcpyDeviceToDevice, stream()));
     if (a->xscale_out) LSPK_CUDA(cudaMemcpyAsync(a->xscale_out, xs, (size_t)M * 4, cudaMemcpyDeviceToDevice, stream()));
 
-    // ---- one grid for all matrices of the call: output-feature tiles of matrix 0, 1, 2 side by side in grid.x --
-    const int k_blocks = (Kp + kTcBK - 1) / kTcBK;
-    int n_tiles[3] = {0, 0, 0}, total_tiles = 0;
+    // ---- one grid for all matrices of the call: feature tiles of matrix 0, 1, 2 side by side in grid.x ----------
+    const Weight* w[3] = {};
     for (int i = 0; i < a->n_mats; ++i) {
-        const Weight* w = reinterpret_cast<const Weight*>(a->w[i]);
-        LSPK_REQUIRE(w && w->K == K && (a->out[i] || (pair && i == 1)),
+        w[i] = reinterpret_cast<const Weight*>(a->w[i]);
+        LSPK_REQUIRE(w[i] && w[i]->K == K && (a->out[i] || (pair && i == 1)),
                      "linear (tensor-core): matrices must share K and have outputs");
-        LSPK_REQUIRE(!pair || w->N == w0->N, "linear (tensor-core): gate and up must have the same N");
-        n_tiles[i] = (w->N + kTcRows - 1) / kTcRows;
-        total_tiles += n_tiles[i];
+        LSPK_REQUIRE(!pair || w[i]->N == w0->N, "linear (tensor-core): gate and up must have the same N");
     }
-    // Token rows per CTA tile.  A K block costs about the same whatever the tile's width (the loop is bound by
-    // its handshakes, not by the tensor pipe), so 256 rows per tile halve the work when the grid still fills
-    // the machine or the K loop is long; otherwise more, narrower tiles win.
-    const bool wide = M > 128 && (total_tiles * ((M + 255) / 256) * 2 > sm_count() || k_blocks >= 32);
-    const int TN = wide ? 256 : M > 64 ? 128 : M > 32 ? 64 : 32;
-    const int m_tiles = (M + TN - 1) / TN;
-    CUtensorMap mx;
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)M};
-        const cuuint64_t strides[1] = {(cuuint64_t)Kp};
-        const cuuint32_t box[2] = {(cuuint32_t)kTcBK, (cuuint32_t)TN};
-        const cuuint32_t estr[2] = {1, 1};
-        CUresult r = enc(&mx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, g_tc.xq_perm, dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(LSPK_ERR_CUDA, "tensor map (activations) failed: %d", (int)r);
-    }
-    // K split when the output tiles alone leave most SMs idle: every CTA then streams a fraction of the bytes and
-    // runs a fraction of the K loop; the partial sums of a K range go to their own slice of an int32 workspace
-    // and the finish kernel adds the slices (exact).  The gated pairing always goes through the workspace: its
-    // epilogue needs both products of an element.
-    int sp = 1;
-    if (total_tiles * m_tiles * 2 <= sm_count()) {
-        sp = sm_count() / (total_tiles * m_tiles);
-        if (sp > 8) sp = 8;
-        if (sp > k_blocks / 2) sp = k_blocks / 2;                       // at least two K blocks per CTA
-        if (sp < 1) sp = 1;
-    }
-    const int kb_per = (k_blocks + sp - 1) / sp;
-    const int splits = (k_blocks + kb_per - 1) / kb_per;                // no CTA without work
-    const bool via_ws = splits > 1 || pair;
-    size_t ws_off[3] = {0, 0, 0}, ws_total = 0;
-    if (via_ws) {
-        for (int i = 0; i < a->n_mats; ++i) {
-            const Weight* w = reinterpret_cast<const Weight*>(a->w[i]);
-            ws_off[i] = ws_total;
-            ws_total += (size_t)M * w->N * splits;
-        }
-        if (int rc = grow((void**)&g_tc.split_ws, &g_tc.cap_ws, ws_total * 4)) return rc;
-    }
-    CUtensorMap mw[3];
+    const int k_blocks = (Kp + kTcBK - 1) / kTcBK;
+    int tiles = 0;
+    for (int i = 0; i < (pair ? 1 : a->n_mats); ++i) tiles += (w[i]->N + kTcRows - 1) / kTcRows;
+    const TcPlan plan = plan_tiles(tiles, pair, M, k_blocks);
+    CUtensorMap mx, mw[3];
+    if (int rc = activation_map(enc, &mx, g_tc.xq_perm, Kp, M, plan.tn)) return rc;
     TcParams p = {};
-    FinishParams fp = {};
-    fp.M = M;
-    fp.epilogue = a->epilogue;
-    fp.x_scales = xs;
-    size_t finish_elems = 0;
     int tile0 = 0;
     for (int i = 0; i < a->n_mats; ++i) {
-        const Weight* w = reinterpret_cast<const Weight*>(a->w[i]);
-        const cuuint64_t row_words = (cuuint64_t)w->chunks * 64;          // 4-byte units per row group
-        const cuuint64_t dims[2] = {row_words, (cuuint64_t)w->groups};
-        const cuuint64_t strides[1] = {row_words * 4};
-        const cuuint32_t box[2] = {128, 8};                               // 512 bytes x 8 row groups
-        const cuuint32_t estr[2] = {1, 1};
-        CUresult r = enc(&mw[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, w->dev, dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(LSPK_ERR_CUDA, "tensor map (weights) failed: %d", (int)r);
-        p.seg[i] = TcSeg{a->out[i], a->acc_out[i], via_ws ? g_tc.split_ws + ws_off[i] : nullptr, w->scale, w->N, tile0};
-        tile0 += n_tiles[i];
-        if (via_ws) {
-            fp.seg[fp.n_seg++] = FinishSeg{g_tc.split_ws + ws_off[i], a->out[i], a->acc_out[i], w->scale, w->N, splits};
-            finish_elems += (size_t)M * w->N;
-        }
+        if (int rc = weight_map(enc, &mw[i], reinterpret_cast<Weight*>(a->w[i]))) return rc;
+        p.seg[i] = TcSeg{a->out[i], a->acc_out[i], w[i]->scale, w[i]->N, tile0};
+        if (!pair || i == 0) tile0 += (w[i]->N + kTcRows - 1) / kTcRows;
     }
     for (int i = a->n_mats; i < 3; ++i) mw[i] = mw[0];
     p.n_seg = a->n_mats;
     p.x_scales = xs;
+    p.x_sums = g_tc.xsum;
     p.M = M;
     p.K = K;
     p.k_blocks = k_blocks;
-    p.kb_per_split = kb_per;
+    p.kb_per_split = plan.kb_per;
     p.epilogue = a->epilogue;
     p.error_flag = g_tc.err;
     p.trace = trace_buffer();
     p.trace_cap = trace_capacity();
-    {
-        const dim3 grid(total_tiles, m_tiles, splits);
-        cudaError_t e = TN == 256 ? launch_tc<256>(mw, mx, p, grid)
-                       : TN == 128 ? launch_tc<128>(mw, mx, p, grid)
-                       : TN == 64 ? launch_tc<64>(mw, mx, p, grid)
-                                  : launch_tc<32>(mw, mx, p, grid);
-        if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "tensor-core GEMM launch failed: %s", cudaGetErrorString(e));
-    }
-    if (fp.n_seg > 0) {
-        if (pair) finish_elems /= 2;
-        int fgrid = (int)((finish_elems / (size_t)fp.n_seg + 255) / 256);
-        if (fgrid > sm_count() * 4) fgrid = sm_count() * 4;
-        if (fgrid < 1) fgrid = 1;
-        cudaError_t e = launch(splitk_finish_kernel, dim3(fgrid), dim3(256), 0, true, fp);
-        if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "tensor-core finish launch failed: %s", cudaGetErrorString(e));
-    }
+    const dim3 grid(tile0, (M + plan.tn - 1) / plan.tn, plan.splits);
+    cudaError_t e;
+    if (pair)
+        e = plan.tn == 128 ? launch_tc<true, 128>(mw, mx, p, grid)
+            : plan.tn == 96 ? launch_tc<true, 96>(mw, mx, p, grid)
+            : plan.tn == 64 ? launch_tc<true, 64>(mw, mx, p, grid)
+                            : launch_tc<true, 32>(mw, mx, p, grid);
+    else
+        e = plan.tn == 128 ? launch_tc<false, 128>(mw, mx, p, grid)
+            : plan.tn == 96 ? launch_tc<false, 96>(mw, mx, p, grid)
+            : plan.tn == 64 ? launch_tc<false, 64>(mw, mx, p, grid)
+                            : launch_tc<false, 32>(mw, mx, p, grid);
+    if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "tensor-core GEMM launch failed: %s", cudaGetErrorString(e));
     *handled = 1;
     return LSPK_OK;
 }
