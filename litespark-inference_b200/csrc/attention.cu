@@ -899,6 +899,9 @@ static int attention_launch_t(const AttnParams& p) {
         const size_t rs = (size_t)((p.Q + 2 * p.KV) * D + D) * sizeof(float);
         LSPK_CUDA(launch(rope_store_kernel<KVT>, dim3(p.T), dim3(kAttnThreads), rs, true, p));
     }
+    int handled = 0;
+    if (int rc = attention_prefill_mma(p, sizeof(KVT) == 2, &handled)) return rc;
+    if (handled) return LSPK_OK;
     if (!p.fused && !p.pos_per_row && p.T >= 2 * kRows) {
         // many consecutive rows of one sequence: kRows query rows per CTA share every key / value row they fetch
         const int nch2 = D / VEC, tpk2 = nch2 > 32 ? 32 : nch2;

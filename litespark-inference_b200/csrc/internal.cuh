@@ -121,6 +121,8 @@ struct AttnParams {
     int trace_cap;
 };
 int attention_launch(const AttnParams& p, int kv_is_fp16);
+// attention_mma.cu: tensor-core form for 16 and more consecutive rows of one sequence (rope_store_kernel has run).
+int attention_prefill_mma(const AttnParams& p, int kv_is_fp16, int* handled);
 
 // One product of a streamed batch (linear_stream.cu).  The caller fills everything above the line; stream_launch
 // fills the rest.  With `sel` set the product's matrices are chosen on the device: expert e = *sel (written by an

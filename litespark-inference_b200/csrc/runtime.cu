@@ -160,26 +160,54 @@ static int upload_table(DevTable& t, int kind, const void* host, const float* sc
     return LSPK_OK;
 }
 
+// Most prompt rows that go through the layers at once.  The products' cost per row falls with the rows of a launch (a
+// layer's four at 2560 / 6912: 45 us for 128 rows, 74 for 512, 175 for 1531) and levels off there; 2048 rows of scratch
+// are 180 MB at that shape, allocated only for prompts that long.
+constexpr int kMaxPrefillRows = 2048;
+
+// Grows the row scratch of the layers.  Graphs captured before hold the old addresses and are dropped.
+static int reserve_rows(State* s, int rows) {
+    if (rows <= s->cap_rows) return LSPK_OK;
+    const lspk_model_config& c = s->m->cfg;
+    const size_t R = (size_t)((rows + 127) / 128) * 128, H = c.hidden_size, I = c.intermediate_size, kv = s->m->kv_dim();
+    LSPK_CUDA(cudaStreamSynchronize(stream()));
+    for (auto& g : s->graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    struct Buf { void** p; size_t width; };
+    const Buf bufs[] = {{(void**)&s->x, H}, {(void**)&s->q, H}, {(void**)&s->k, kv}, {(void**)&s->v, kv}, {(void**)&s->attn, H},
+                        {(void**)&s->inter, I}, {(void**)&s->tok_rows, 1}};
+    for (const Buf& b : bufs) {
+        if (*b.p) {
+            cudaFree(*b.p);
+            s->bytes -= (size_t)s->cap_rows * b.width * 4;
+        }
+        *b.p = nullptr;
+    }
+    s->cap_rows = 0;
+    for (const Buf& b : bufs) {
+        LSPK_CUDA(cudaMalloc(b.p, R * b.width * 4));
+        s->bytes += R * b.width * 4;
+    }
+    s->cap_rows = (int)R;
+    return LSPK_OK;
+}
+
 // One transformer layer for `rows` rows held in the state's scratch buffers.
 //   one row: norm + quantiser fused into the linear kernels;
-//   otherwise rows go through the batched norm+quantise kernel once and the linear kernels (eight-row
-//   tensor-core tiles below 32 rows, the tcgen05 GEMM from there) take the int8 prologue.
+//   otherwise rows are normalised and quantised once, straight into the layout of the product that follows
+//   (eight-row tensor-core tiles for up to eight rows, the tcgen05 GEMM from there).
 //   per_row_seq: rows are different sequences (batched decode) instead of consecutive positions.
 int run_layer(State* s, int li, int rows, bool per_row_seq, int seq, bool skip_attention) {
     Model* m = s->m;
     const lspk_model_config& c = m->cfg;
     const DevLayer& L = m->layers[li];
-    const int H = c.hidden_size, I = c.intermediate_size;
     const bool bitnet = c.arch == 0;
-    // fp32 rows go to the linear layer as they are: one row is normalised and quantised inside the GEMV;
-    // more rows are quantised once, by one kernel, straight into the activation layout of the kernel that
-    // takes them (eight-row tiles below 32 rows, the tcgen05 GEMM from there).  The library scratch this
-    // uses is sized by the warm-up run that precedes every graph capture.
-    const bool fused_quant = true;
     const float eps = c.rms_norm_eps;
 
-    auto linear = [&](int n_mats, const int* which, float* const* outs, const float* src, int8_t* src_q,
-                      const DevNorm* norm, int K, int epilogue) -> int {
+    auto linear = [&](int n_mats, const int* which, float* const* outs, const float* src,
+                      const DevNorm* norm, int epilogue) -> int {
         lspk_linear_args a = {};
         for (int i = 0; i < n_mats; ++i) {
             a.w[i] = L.proj[which[i]];
@@ -189,22 +217,13 @@ int run_layer(State* s, int li, int rows, bool per_row_seq, int seq, bool skip_a
         a.M = rows;
         a.epilogue = epilogue;
         a.eps = eps;
-        if (fused_quant) {
-            a.x_f32 = src;
-            if (norm) {
-                a.prologue = LSPK_PRO_RMSNORM_QUANT;
-                a.gamma = norm->g;
-                a.gamma_is_bf16 = norm->is_bf16;
-            } else {
-                a.prologue = LSPK_PRO_QUANT;
-            }
+        a.x_f32 = src;
+        if (norm) {
+            a.prologue = LSPK_PRO_RMSNORM_QUANT;
+            a.gamma = norm->g;
+            a.gamma_is_bf16 = norm->is_bf16;
         } else {
-            int rc = norm ? lspk_rmsnorm_quantize_rows(src, norm->g, norm->is_bf16, src_q, s->xs, rows, K, eps)
-                          : lspk_quantize_rows(src, src_q, s->xs, rows, K);
-            if (rc) return rc;
-            a.prologue = LSPK_PRO_INT8;
-            a.x_i8 = src_q;
-            a.x_scales = s->xs;
+            a.prologue = LSPK_PRO_QUANT;
         }
         return lspk_linear(&a);
     };
@@ -213,7 +232,7 @@ int run_layer(State* s, int li, int rows, bool per_row_seq, int seq, bool skip_a
     {
         const int which[3] = {LSPK_PROJ_Q, LSPK_PROJ_K, LSPK_PROJ_V};
         float* outs[3] = {s->q, s->k, s->v};
-        if (int rc = linear(3, which, outs, s->x, s->xq_h, &L.norm[LSPK_NORM_INPUT], H, LSPK_EPI_STORE)) return rc;
+        if (int rc = linear(3, which, outs, s->x, &L.norm[LSPK_NORM_INPUT], LSPK_EPI_STORE)) return rc;
     }
     if (!skip_attention) {
         AttnParams p = {};
@@ -241,21 +260,19 @@ int run_layer(State* s, int li, int rows, bool per_row_seq, int seq, bool skip_a
     {
         const int which[1] = {LSPK_PROJ_O};
         float* outs[1] = {s->x};
-        if (int rc = linear(1, which, outs, s->attn, s->xq_h, bitnet ? &L.norm[LSPK_NORM_ATTN_SUB] : nullptr, H,
-                            LSPK_EPI_ADD)) return rc;
+        if (int rc = linear(1, which, outs, s->attn, bitnet ? &L.norm[LSPK_NORM_ATTN_SUB] : nullptr, LSPK_EPI_ADD)) return rc;
     }
     // MLP block: gate and up as one call with the gate (ReLU^2 or SiLU) as its epilogue at every row count
     {
         const int which[2] = {LSPK_PROJ_GATE, LSPK_PROJ_UP};
         float* outs[2] = {s->inter, nullptr};
-        if (int rc = linear(2, which, outs, s->x, s->xq_h, &L.norm[LSPK_NORM_POST_ATTN], H,
+        if (int rc = linear(2, which, outs, s->x, &L.norm[LSPK_NORM_POST_ATTN],
                             bitnet ? LSPK_EPI_RELU2_MUL : LSPK_EPI_SILU_MUL)) return rc;
     }
     {
         const int which[1] = {LSPK_PROJ_DOWN};
         float* outs[1] = {s->x};
-        if (int rc = linear(1, which, outs, s->inter, s->xq_i, bitnet ? &L.norm[LSPK_NORM_FFN_SUB] : nullptr, I,
-                            LSPK_EPI_ADD)) return rc;
+        if (int rc = linear(1, which, outs, s->inter, bitnet ? &L.norm[LSPK_NORM_FFN_SUB] : nullptr, LSPK_EPI_ADD)) return rc;
     }
     return LSPK_OK;
 }
@@ -294,6 +311,7 @@ static int enqueue_step(State* s, bool store_logits, bool host_io = false) {
 }
 
 static int build_graph(State* s, int variant) {
+    if (int rc = reserve_rows(s, s->batch)) return rc;
     if (s->graph[variant] && s->graph_gen[variant] == scratch_generation()) return LSPK_OK;
     if (s->graph[variant]) {
         // library scratch whose addresses the graph holds was moved by a later call (a larger prefill, a
@@ -493,11 +511,9 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
     s->kv_fp16 = kv_fp16 ? 1 : 0;
     s->host_pos.assign(batch, 0);
     const lspk_model_config& c = m->cfg;
-    const int H = c.hidden_size, I = c.intermediate_size, V = c.vocab_size, D = m->D(), kv = m->kv_dim();
-    s->cap_rows = batch > 128 ? batch : 128;
+    const int V = c.vocab_size, D = m->D();
     s->logits_rows = batch > 8 ? batch : 8;
     const size_t cache_bytes = (size_t)batch * s->seq_stride() * s->kv_elem();
-    const size_t R = s->cap_rows;
     int rc = 0;
     rc |= dev_alloc(&s->cache_k, cache_bytes, &s->bytes);
     rc |= dev_alloc(&s->cache_v, cache_bytes, &s->bytes);
@@ -507,19 +523,9 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
     rc |= dev_alloc((void**)&s->ctl, (size_t)(2 * batch + 1) * 4, &s->bytes);
     rc |= dev_alloc((void**)&s->best, (size_t)batch * 8, &s->bytes);
     rc |= dev_alloc((void**)&s->tokens_out, (size_t)t_max * batch * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->x, R * H * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->q, R * H * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->k, R * kv * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->v, R * kv * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->attn, R * H * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->inter, R * I * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->inter2, R * I * 4, &s->bytes);
     rc |= dev_alloc((void**)&s->logits, (size_t)s->logits_rows * V * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->xq_h, R * H, &s->bytes);
-    rc |= dev_alloc((void**)&s->xq_i, R * I, &s->bytes);
-    rc |= dev_alloc((void**)&s->xs, R * 4, &s->bytes);
-    rc |= dev_alloc((void**)&s->tok_rows, R * 4, &s->bytes);
-    if (!rc && cudaMallocHost((void**)&s->h_int, (size_t)(t_max * batch + R + 16) * 4) != cudaSuccess) rc = 1;
+    rc |= reserve_rows(s, batch > 128 ? batch : 128);
+    if (!rc && cudaMallocHost((void**)&s->h_int, (size_t)(t_max * batch + 2 * batch + 16) * 4) != cudaSuccess) rc = 1;
     if (!rc && cudaMallocHost((void**)&s->h_logits, (size_t)s->logits_rows * V * 4) != cudaSuccess) rc = 1;
     if (!rc && batch == 1) {
         // the two words of the host-fed step (see State): mapped pinned memory and its device alias
@@ -563,7 +569,7 @@ int lspk_state_free(lspk_state_t h) {
     for (auto& g : s->graph)
         if (g) cudaGraphExecDestroy(g);
     void* dev[] = {s->cache_k, s->cache_v, s->rope_cos, s->rope_sin, s->rope_cur, s->ctl, s->best, s->tokens_out, s->x, s->q, s->k,
-                   s->v, s->attn, s->inter, s->inter2, s->logits, s->xq_h, s->xq_i, s->xs, s->tok_rows};
+                   s->v, s->attn, s->inter, s->logits, s->tok_rows};
     for (void* p : dev) cudaFree(p);
     if (s->h_int) cudaFreeHost(s->h_int);
     if (s->h_logits) cudaFreeHost(s->h_logits);
@@ -697,6 +703,7 @@ int lspk_forward_prefill(lspk_state_t h, int seq, const int* tokens_host, int T,
     if (s->host_pos[seq] + T > s->t_max)
         return fail(LSPK_ERR_STATE, "prefill would exceed t_max: pos=%d T=%d t_max=%d", s->host_pos[seq], T, s->t_max);
     const DevTable& head = m->head.data ? m->head : m->emb;
+    if (int rc = reserve_rows(s, T < kMaxPrefillRows ? T : kMaxPrefillRows)) return rc;
     for (int t0 = 0; t0 < T; t0 += s->cap_rows) {
         const int rows = (T - t0) < s->cap_rows ? (T - t0) : s->cap_rows;
         memcpy(s->h_int, tokens_host + t0, (size_t)rows * 4);
@@ -720,8 +727,9 @@ int lspk_forward_prefill(lspk_state_t h, int seq, const int* tokens_host, int T,
             LSPK_CUDA(cudaMemsetAsync(s->best, 0, 8, stream()));
             if (int rc = lm_head_launch(head.kind, head.data, head.scale, s->x + (size_t)(rows - 1) * H, s->logits, 1, V, H,
                                         m->final_norm.g, m->final_norm.is_bf16, c.rms_norm_eps, s->best)) return rc;
-            LSPK_CUDA(cudaMemcpyAsync(s->h_logits, s->logits, (size_t)V * 4, cudaMemcpyDeviceToHost, stream()));
-            LSPK_CUDA(cudaMemcpyAsync(s->h_int + s->cap_rows, s->best, 8, cudaMemcpyDeviceToHost, stream()));
+            if (last_logits_host)
+                LSPK_CUDA(cudaMemcpyAsync(s->h_logits, s->logits, (size_t)V * 4, cudaMemcpyDeviceToHost, stream()));
+            LSPK_CUDA(cudaMemcpyAsync(s->h_int + rows, s->best, 8, cudaMemcpyDeviceToHost, stream()));
             LSPK_CUDA(cudaMemsetAsync(s->best, 0, 8, stream()));     // the decode step expects cleared keys
         }
         LSPK_CUDA(launch(advance_pos_kernel, dim3(1), dim3(32), 0, true, s->ctl, seq, rows));
@@ -731,7 +739,7 @@ int lspk_forward_prefill(lspk_state_t h, int seq, const int* tokens_host, int T,
             if (last_logits_host) memcpy(last_logits_host, s->h_logits, (size_t)V * 4);
             if (next_token_host) {
                 unsigned long long key = 0;
-                memcpy(&key, s->h_int + s->cap_rows, 8);
+                memcpy(&key, s->h_int + rows, 8);
                 *next_token_host = (int)(0xffffffffu - (uint32_t)(key & 0xffffffffull));
             }
         }

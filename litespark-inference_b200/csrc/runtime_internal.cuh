@@ -47,11 +47,9 @@ struct State {
     int* ctl = nullptr;               // device: pos[batch], token[batch], step
     unsigned long long* best = nullptr;   // device: argmax keys [batch]
     int* tokens_out = nullptr;        // device: [t_max * batch]
-    float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *inter = nullptr, *inter2 = nullptr;
+    float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *inter = nullptr;
     float *logits = nullptr;          // [max(batch, 8), V]
     int logits_rows = 0;
-    int8_t *xq_h = nullptr, *xq_i = nullptr;
-    float* xs = nullptr;
     int* tok_rows = nullptr;          // device token ids for a prefill chunk
     int* h_int = nullptr;             // pinned staging for ints
     float* h_logits = nullptr;        // pinned staging for logits
