@@ -23,9 +23,12 @@ template <> struct EmbTraits<0> { static constexpr int E = 8;  };   // bf16: 8 v
 template <> struct EmbTraits<1> { static constexpr int E = 16; };   // int8
 template <> struct EmbTraits<2> { static constexpr int E = 32; };   // int4, low nibble first
 
+// The s-th group of four consecutive values of a 16-byte chunk.  The integer formats go through the mantissa of 2^23
+// (bits | 0x4b000000, then minus the bias: exact) because integer-to-float conversions issue at a fraction of the add
+// rate (int4, 128256 x 2560: 115 us with them, and the table's 164 MB take 25).  int4 nibbles stay at their bit offset:
+// value e of a group comes out times 16^e, and x is staged divided by it (int4_unscale), so every product is the same.
 template <int KIND>
 __device__ __forceinline__ void decode4(const uint4& c, int s, float f[4]) {
-    // the s-th group of four consecutive values of a 16-byte chunk
     const uint32_t w[4] = {c.x, c.y, c.z, c.w};
     if (KIND == 0) {
         const uint32_t a = w[(s * 2) & 3], b = w[(s * 2 + 1) & 3];
@@ -34,14 +37,19 @@ __device__ __forceinline__ void decode4(const uint4& c, int s, float f[4]) {
         f[2] = __uint_as_float(b << 16);
         f[3] = __uint_as_float(b & 0xffff0000u);
     } else if (KIND == 1) {
-        const uint32_t a = w[s & 3];
+        const uint32_t a = w[s & 3] ^ 0x80808080u;                          // value + 128
 #pragma unroll
-        for (int e = 0; e < 4; ++e) f[e] = (float)((int)(a << (24 - 8 * e)) >> 24);
+        for (int e = 0; e < 4; ++e) f[e] = __uint_as_float(__byte_perm(a, 0x4b000000u, 0x7440 + e)) - 8388736.0f;
     } else {
-        const uint32_t a = (w[(s >> 1) & 3] >> ((s & 1) * 16)) & 0xffffu;   // two bytes = four nibbles
+        const uint32_t a = w[(s >> 1) & 3] >> ((s & 1) * 16);               // two bytes = four nibbles
 #pragma unroll
-        for (int e = 0; e < 4; ++e) f[e] = (float)((int)(a << (28 - 4 * e)) >> 28);
+        for (int e = 0; e < 4; ++e)                                         // (value + 8) << 4 e
+            f[e] = __uint_as_float((a & (0xfu << (4 * e))) ^ (0x4b000000u | (8u << (4 * e)))) - (8388608.0f + (float)(8 << (4 * e)));
     }
+}
+template <int KIND>
+__device__ __forceinline__ float staged_x(float v, int k) {
+    return KIND == 2 ? v * __uint_as_float((127u - 4u * (k & 3)) << 23) : v;
 }
 
 __device__ __forceinline__ unsigned long long argmax_key(float v, int idx) {
@@ -91,7 +99,7 @@ lm_head_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_scal
                 v = __fmul_rn(__fmul_rn(v, rrms), gm);
             }
             const int c = k / E, s = (k % E) / 4, e = k & 3;
-            dst[((size_t)s * nchunks + c) * 4 + e] = v;
+            dst[((size_t)s * nchunks + c) * 4 + e] = staged_x<KIND>(v, k);
         }
     }
     __syncthreads();
@@ -179,43 +187,108 @@ lm_head_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_scal
     }
 }
 
-// ---- several rows of x against a bf16 table on the warp-level tensor cores -------------------------
+// ---- several rows of x on the warp-level tensor cores ------------------------------------------------
 // With 2..16 rows of x the CUDA-core kernel above is bound by its fused multiply-adds (V * H * T of them)
 // and by shared-memory reads of x.  Here a warp owns 16 table rows (the MMA's M side), the rows of x are
 // the N side (one or two tiles of eight), and the table bytes go from global memory straight into A
-// fragments: lane (g, t) loads 16 bytes of row g and of row g + 8 per 32-wide K step; which eight k's a
+// fragments: lane (g, t) loads 16 bytes of row g and of row g + 8 per K step; which k's a
 // lane holds is a permutation of K that the x fragments repeat, so no shuffle is needed.
-// x stays fp32-exact: it is split into three bf16 terms (x = hi + mid + lo up to 2^-24 |x|), each product
-// bf16 x bf16 is exact in the fp32 accumulator, so the result differs from the fp32 dot product only in
-// summation order, like every other reduction here.
-constexpr int kLmmStepsInFlight = 6;      // 32-wide K steps of table data in flight per lane (12 x 16 bytes)
+// x stays fp32-exact: it is split into three 16-bit terms, each product is exact in the fp32 accumulator, so the
+// result differs from the fp32 dot product only in summation order, like every other reduction here.
+//   bf16 table   bf16 terms (8 bits each, the range of fp32)
+//   int8, int4   the integers become fp16 in registers (bits | 0x6400 is 1024 + value) and x is cut into fp16 terms (11
+//                bits each) after an exact scaling by a power of two
+constexpr int kLmmStepsInFlight = 6;      // K steps of table data in flight per lane (12 x 16 bytes)
 
-__device__ __forceinline__ void mma_bf16_16816(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+template <bool F16>
+__device__ __forceinline__ void lm_mma_16816(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    if constexpr (F16)
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 __device__ __forceinline__ uint32_t bf16_rn_bits(float v) {          // round to nearest even, as a 16-bit pattern
     const uint32_t u = __float_as_uint(v);
     return (u + 0x7fffu + ((u >> 16) & 1u)) >> 16;
 }
+// Cuts the next 16-bit term off v.
+template <bool F16>
+__device__ __forceinline__ uint16_t take_term(float& v) {
+    if constexpr (F16) {
+        const __half h = __float2half_rn(v);
+        v -= __half2float(h);
+        return __half_as_ushort(h);
+    } else {
+        const uint32_t b = bf16_rn_bits(v);
+        v -= __uint_as_float(b << 16);
+        return (uint16_t)b;
+    }
+}
 
-// NT: tiles of eight rows of x (1 or 2) a CTA holds.  Shared memory: [3 terms][8 * NT rows][H + 32] bf16.
+// How a table format meets the MMA.  KPL: values of a 16-byte load (a lane's share of a K step of 4 * KPL).
+template <int KIND> struct LmmTraits {
+    static constexpr bool kF16 = KIND != 0;
+    static constexpr int KPL = EmbTraits<KIND>::E;
+    static constexpr int kStep = 4 * KPL;
+    // row padding (16-bit elements) that spreads the 16-byte loads of a quarter warp over all banks
+    static constexpr int kPad = KIND == 0 ? 32 : KIND == 1 ? 8 : 16;
+    // element k of a row of x -> its place in shared memory.  int4: the nibbles of a word come out of the decode as
+    // (0,4) (1,5) (2,6) (3,7), and a lane's four 16-byte pieces are swapped in pairs for lanes 2 and 3 (banks)
+    static __device__ __forceinline__ int place(int k) {
+        if (KIND != 2) return k;
+        const int step = k & ~127, t = (k >> 5) & 3, word = (k >> 3) & 3, n = k & 7;
+        return step + t * 32 + ((word ^ (t >> 1)) << 3) + ((n & 3) << 1) + (n >> 2);
+    }
+};
+// A operands of 16 k's: a[0] / a[1] the two pairs of a table row, from the i-th group of a 16-byte load.
+template <int KIND>
+__device__ __forceinline__ void lmm_operand(const uint4& c, int i, uint32_t a[2]) {
+    const uint32_t w[4] = {c.x, c.y, c.z, c.w};
+    if constexpr (KIND == 0) {
+        a[0] = w[2 * i];
+        a[1] = w[2 * i + 1];
+    } else {
+        uint32_t p, q, bias;
+        if constexpr (KIND == 1) {
+            const uint32_t v = w[i] ^ 0x80808080u;
+            p = __byte_perm(v, 0x64646464u, 0x4140);
+            q = __byte_perm(v, 0x64646464u, 0x4342);
+            bias = 0x64806480u;                            // 1024 + 128
+        } else {
+            const uint32_t v = w[i >> 1] >> ((i & 1) * 8);
+            p = (v & 0x000f000fu) ^ 0x64086408u;           // 1024 + (value + 8)
+            q = ((v >> 4) & 0x000f000fu) ^ 0x64086408u;
+            bias = 0x64086408u;
+        }
+        const __half2 hb = *reinterpret_cast<const __half2*>(&bias);
+        const __half2 hp = __hsub2(*reinterpret_cast<const __half2*>(&p), hb), hq = __hsub2(*reinterpret_cast<const __half2*>(&q), hb);
+        a[0] = *reinterpret_cast<const uint32_t*>(&hp);
+        a[1] = *reinterpret_cast<const uint32_t*>(&hq);
+    }
+}
+
+// NT: tiles of eight rows of x (1 or 2) a CTA holds.  Shared memory: [3 terms][8 * NT rows][H + pad] 16-bit terms.
 // passes: more rows than a CTA holds are served side by side in ONE launch: CTA b takes the row block b % passes
 // and the table tiles of position b / passes, so the CTAs that need the same table rows run next to each other
 // and the table comes from HBM once (the second reader finds it in L2).
-template <int NT>
+template <int KIND, int NT>
 __global__ void __launch_bounds__(kLmThreads)
-lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ x, float* __restrict__ logits, int T_all, int V,
-                   int H, const void* __restrict__ norm_gamma, int gamma_is_bf16, float eps,
-                   unsigned long long* __restrict__ best_keys, int passes) {
+lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_scale, const float* __restrict__ x,
+                   float* __restrict__ logits, int T_all, int V, int H, const void* __restrict__ norm_gamma, int gamma_is_bf16,
+                   float eps, unsigned long long* __restrict__ best_keys, int passes) {
+    using TR = LmmTraits<KIND>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* xs = reinterpret_cast<uint16_t*>(smem_raw);
-    __shared__ float red[32];
     __shared__ unsigned long long s_best[kLmWarps][8 * NT];
+    __shared__ float s_unscale[8 * NT];
     unsigned long long best[NT][2];                          // greedy argmax keys of tokens 8 n + 2 t4 + {0, 1}
 #pragma unroll
     for (int n = 0; n < NT; ++n) best[n][0] = best[n][1] = 0ull;
@@ -227,9 +300,9 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ x, f
     x += (size_t)pass * R * H;
     if (logits) logits += (size_t)pass * R * V;
     if (best_keys) best_keys += pass * R;
-    const int ld = H + 32;                                 // row stride in bf16: 64 bytes of padding make the quarter-warp 16-byte loads conflict-free
-    const int steps = H / 32;                              // host guarantees H % 32 == 0
-    const size_t row_chunks = (size_t)H / 8;
+    const int ld = H + TR::kPad;
+    const int steps = H / TR::kStep;                       // host guarantees H % kStep == 0
+    const size_t row_chunks = (size_t)H / TR::KPL;
 
     // table rows of this warp's first tile can be requested before the activations exist
     auto tile_of = [&](int i) { return (cta * kLmWarps + warp) + i * ncta * kLmWarps; };
@@ -253,38 +326,49 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ x, f
     grid_dependency_launch();
     grid_dependency_wait();
 
-    // rows of x (optionally RMS-normalised) -> three bf16 terms in shared memory
-    for (int r = 0; r < R; ++r) {
-        if (r < T) {
-            const float* xr = x + (size_t)r * H;
-            float rrms = 1.0f;
-            if (norm_gamma) {
-                float ssq = 0.0f;
-                for (int k = tid; k < H; k += kLmThreads) ssq = fmaf(xr[k], xr[k], ssq);
-                ssq = block_sum(ssq, red);
-                rrms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ssq, (float)H), eps)));
-            }
-            for (int k = tid; k < H; k += kLmThreads) {
-                float v = xr[k];
-                if (norm_gamma) {
-                    const float gm = gamma_is_bf16 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(norm_gamma)[k])
-                                                   : reinterpret_cast<const float*>(norm_gamma)[k];
-                    v = __fmul_rn(__fmul_rn(v, rrms), gm);
+    auto gamma_of = [&](int k) {
+        return gamma_is_bf16 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(norm_gamma)[k])
+                             : reinterpret_cast<const float*>(norm_gamma)[k];
+    };
+    // rows of x (optionally RMS-normalised) -> three 16-bit terms in shared memory, a row per warp (no barrier)
+    for (int r = warp; r < R; r += kLmWarps) {
+        const float* xr = x + (size_t)r * H;
+        float rrms = 1.0f, scale = 1.0f;
+        if (r < T && (norm_gamma || TR::kF16)) {
+            float ssq = 0.0f, amax = 0.0f;
+            for (int k = lane * 4; k < H; k += 128) {
+                const float4 v = *reinterpret_cast<const float4*>(xr + k);
+                const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    ssq = fmaf(f[e], f[e], ssq);
+                    if (TR::kF16) amax = fmaxf(amax, fabsf(norm_gamma ? f[e] * gamma_of(k + e) : f[e]));
                 }
-                const uint32_t hi = bf16_rn_bits(v);
-                const float r1 = v - __uint_as_float(hi << 16);
-                const uint32_t mid = bf16_rn_bits(r1);
-                const float r2 = r1 - __uint_as_float(mid << 16);
-                const uint32_t lo = bf16_rn_bits(r2);
-                xs[(size_t)(0 * R + r) * ld + k] = (uint16_t)hi;
-                xs[(size_t)(1 * R + r) * ld + k] = (uint16_t)mid;
-                xs[(size_t)(2 * R + r) * ld + k] = (uint16_t)lo;
             }
-        } else {
-            for (int k = tid; k < H; k += kLmThreads) {
-                xs[(size_t)(0 * R + r) * ld + k] = 0;
-                xs[(size_t)(1 * R + r) * ld + k] = 0;
-                xs[(size_t)(2 * R + r) * ld + k] = 0;
+            if (norm_gamma) {
+                ssq = warp_sum(ssq);
+                rrms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ssq, (float)H), eps)));
+                amax *= rrms;
+            }
+            if (TR::kF16) {
+                // largest element near 2^13 (fp16 ends at 2^16), by an exact power of two
+                amax = warp_max(amax);
+                const int ex = amax > 0.0f ? max(-100, min(100, 140 - (int)(__float_as_uint(amax) >> 23))) : 0;
+                scale = __uint_as_float((uint32_t)(127 + ex) << 23);
+                if (lane == 0) s_unscale[r] = __uint_as_float((uint32_t)(127 - ex) << 23);
+            }
+        }
+        for (int k = lane * 4; k < H; k += 128) {
+            float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < T) v4 = *reinterpret_cast<const float4*>(xr + k);
+            float f[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (norm_gamma) f[e] = __fmul_rn(__fmul_rn(f[e], rrms), gamma_of(k + e));
+                if (TR::kF16) f[e] *= scale;
+                const int at = TR::place(k + e);
+#pragma unroll
+                for (int term = 0; term < 3; ++term) xs[(size_t)(term * R + r) * ld + at] = take_term<TR::kF16>(f[e]);
             }
         }
     }
@@ -316,14 +400,23 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ x, f
                 const int sidx = s0 + u;
                 if (sidx < steps) {
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) {
+                    for (int j = 0; j < TR::KPL / 8; ++j) {          // 16-byte pieces of x: two MMAs each
+                        uint32_t lo0[2], hi0[2], lo1[2], hi1[2];
+                        lmm_operand<KIND>(cur[u][0], 2 * j, lo0);
+                        lmm_operand<KIND>(cur[u][1], 2 * j, hi0);
+                        lmm_operand<KIND>(cur[u][0], 2 * j + 1, lo1);
+                        lmm_operand<KIND>(cur[u][1], 2 * j + 1, hi1);
+                        const int piece = KIND == 2 ? j ^ (t4 >> 1) : j;
 #pragma unroll
-                        for (int term = 0; term < 3; ++term) {
-                            // this lane's B data: token row (8 n + g), k = 32 sidx + 8 t4 .. + 7
-                            const uint4 b = *reinterpret_cast<const uint4*>(
-                                xs + (size_t)(term * R + 8 * n + g) * ld + (size_t)sidx * 32 + t4 * 8);
-                            mma_bf16_16816(acc[n], cur[u][0].x, cur[u][1].x, cur[u][0].y, cur[u][1].y, b.x, b.y);
-                            mma_bf16_16816(acc[n], cur[u][0].z, cur[u][1].z, cur[u][0].w, cur[u][1].w, b.z, b.w);
+                        for (int n = 0; n < NT; ++n) {
+#pragma unroll
+                            for (int term = 0; term < 3; ++term) {
+                                // this lane's B data: token row 8 n + g, the k's of its table load
+                                const uint4 b = *reinterpret_cast<const uint4*>(
+                                    xs + (size_t)(term * R + 8 * n + g) * ld + (size_t)sidx * TR::kStep + t4 * TR::KPL + piece * 8);
+                                lm_mma_16816<TR::kF16>(acc[n], lo0[0], hi0[0], lo0[1], hi0[1], b.x, b.y);
+                                lm_mma_16816<TR::kF16>(acc[n], lo1[0], hi1[0], lo1[1], hi1[1], b.z, b.w);
+                            }
                         }
                     }
                 }
@@ -337,8 +430,10 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ x, f
                 const int v = v0 + g + 8 * (c >> 1);
                 const int tok = 8 * n + 2 * t4 + (c & 1);
                 if (v < V && tok < T) {
-                    if (logits) logits[(size_t)tok * V + v] = acc[n][c];
-                    const unsigned long long key = argmax_key(acc[n][c], v);
+                    float y = acc[n][c];
+                    if (TR::kF16) y = __fmul_rn(emb_scale[v], y * s_unscale[tok]);
+                    if (logits) logits[(size_t)tok * V + v] = y;
+                    const unsigned long long key = argmax_key(y, v);
                     best[n][c & 1] = key > best[n][c & 1] ? key : best[n][c & 1];
                 }
             }
@@ -368,6 +463,24 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ x, f
     }
 }
 
+template <int KIND, int NT>
+static cudaError_t launch_lm_mma(dim3 grid, size_t smem, const uint4* emb, const float* emb_scale, const float* x, float* logits,
+                                 int T, int V, int H, const void* norm_gamma, int gamma_is_bf16, float eps,
+                                 unsigned long long* best_key, int passes) {
+    static bool attr_set = false;
+    auto kern = lm_head_mma_kernel<KIND, NT>;
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return e;
+        attr_set = true;
+    }
+    return launch(kern, grid, dim3(kLmThreads), smem, true, emb, emb_scale, x, logits, T, V, H, norm_gamma, gamma_is_bf16, eps,
+                  best_key, passes);
+}
+
+// Whether several rows go to the tensor-core kernel (a K step of it is 32, 64 or 128 wide).
+bool lm_head_rows_on_tensor_cores(int kind, int H) { return H % (kind == 0 ? 32 : kind == 1 ? 64 : 128) == 0; }
+
 // norm_gamma / best_key may be null; best_key points at T keys (one greedy argmax per row of x, combined with
 // atomicMax: the caller clears them).  Larger T is tiled here.
 int lm_head_launch(int kind, const void* emb, const float* emb_scale, const float* x, float* logits,
@@ -382,12 +495,12 @@ int lm_head_launch(int kind, const void* emb, const float* emb_scale, const floa
     LSPK_REQUIRE(H % E == 0, "lm_head: H=%d must be a multiple of %d for this embedding format", H, E);
     LSPK_REQUIRE(((uintptr_t)emb & 15) == 0, "lm_head: embedding must be 16-byte aligned");
     const int rows_per_cta = kLmWarps;
-    int grid = (V + rows_per_cta - 1) / rows_per_cta;
+    int grid = (V + rows_per_cta - 1) / rows_per_cta;      // kernels that take two rows per warp loop less
     const int cap = sm_count() * 4;
     if (grid > cap) grid = cap;
     const uint4* e4 = reinterpret_cast<const uint4*>(emb);
-    if (kind == 0 && T > 1 && H % 32 == 0 && (logits || best_key)) {
-        // several rows against the bf16 table: tensor-core kernel.  A CTA holds sixteen rows where their three bf16
+    if (T > 1 && lm_head_rows_on_tensor_cores(kind, H) && (logits || best_key) && ((uintptr_t)x & 15) == 0) {
+        // several rows: tensor-core kernel.  A CTA holds sixteen rows where their three 16-bit
         // terms fit the shared memory (H <= 2100), else eight; more rows than that are row blocks served side by
         // side in one launch (the kernel's `passes`), so the table is read from HBM once
         const int nt = ((size_t)3 * 16 * (H + 32) * 2 <= 200 * 1024 && T > 8) ? 2 : 1;
@@ -398,22 +511,17 @@ int lm_head_launch(int kind, const void* emb, const float* emb_scale, const floa
         LSPK_REQUIRE(passes <= sm_count(), "lm_head: too many rows (%d) for one launch", T);
         int per_pass = (V + 16 * kLmWarps - 1) / (16 * kLmWarps);
         if (per_pass > sm_count() / passes) per_pass = sm_count() / passes;
-        const int mgrid = per_pass * passes;
-        static bool attr1 = false, attr2 = false;
-        cudaError_t e = cudaSuccess;
-        if (nt == 1) {
-            if (!attr1) e = cudaFuncSetAttribute(lm_head_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            attr1 = attr1 || e == cudaSuccess;
-            if (e == cudaSuccess)
-                e = launch(lm_head_mma_kernel<1>, dim3(mgrid), dim3(kLmThreads), smem, true, e4, x, logits, T, V, H, norm_gamma,
-                           gamma_is_bf16, eps, best_key, passes);
-        } else {
-            if (!attr2) e = cudaFuncSetAttribute(lm_head_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            attr2 = attr2 || e == cudaSuccess;
-            if (e == cudaSuccess)
-                e = launch(lm_head_mma_kernel<2>, dim3(mgrid), dim3(kLmThreads), smem, true, e4, x, logits, T, V, H, norm_gamma,
-                           gamma_is_bf16, eps, best_key, passes);
-        }
+        const dim3 mgrid(per_pass * passes);
+        cudaError_t e;
+#define LSPK_LMM(KIND)                                                                                                      \
+        e = nt == 1 ? launch_lm_mma<KIND, 1>(mgrid, smem, e4, emb_scale, x, logits, T, V, H, norm_gamma, gamma_is_bf16, eps, \
+                                             best_key, passes)                                                              \
+                    : launch_lm_mma<KIND, 2>(mgrid, smem, e4, emb_scale, x, logits, T, V, H, norm_gamma, gamma_is_bf16, eps, \
+                                             best_key, passes)
+        if (kind == 0) LSPK_LMM(0);
+        else if (kind == 1) LSPK_LMM(1);
+        else LSPK_LMM(2);
+#undef LSPK_LMM
         if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "lm_head (mma) launch failed: %s", cudaGetErrorString(e));
         return LSPK_OK;
     }
@@ -443,9 +551,11 @@ int lm_head_launch(int kind, const void* emb, const float* emb_scale, const floa
                            norm_gamma, gamma_is_bf16, eps, bk);                                             \
         } while (0)
         if (tt == 1) {
+            // integer formats: a value of x fetched from shared memory serves two table rows (one row at a time the
+            // reads of x, 4 bytes per half a byte of int4 table, would take longer than the table)
             if (kind == 0) LSPK_LM_LAUNCH(0, 1, 10, 1);
-            else if (kind == 1) LSPK_LM_LAUNCH(1, 1, 5, 1);
-            else LSPK_LM_LAUNCH(2, 1, 3, 1);
+            else if (kind == 1) LSPK_LM_LAUNCH(1, 1, 5, 2);
+            else LSPK_LM_LAUNCH(2, 1, 3, 2);
         } else {
             // measured at V = 128256, H = 2560, 8 rows (loads in flight, table rows per warp): (4,1) 396 us,
             // (4,2) 315, (3,4) 482, (6,2) 514, (2,4) 255: with eight rows the kernel is bound by its
