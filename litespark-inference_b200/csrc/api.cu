@@ -61,6 +61,15 @@ static int* g_wait_flag = nullptr;
 int* device_wait_flag() { return g_wait_flag; }
 int bound_device() { return g_device; }
 
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && release_parked_states()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 // Lazily bind to a device the first time any entry point needs one.
 
 int ensure_init() {
@@ -155,7 +164,7 @@ int lspk_sync(void) {
 void* lspk_malloc(size_t bytes) {
     if (ensure_init()) return nullptr;
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
+    cudaError_t e = device_malloc(&p, bytes ? bytes : 16);
     if (e != cudaSuccess) {
         fail(LSPK_ERR_CUDA, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
         return nullptr;
@@ -214,7 +223,7 @@ int lspk_memset(void* dev, int value, size_t bytes) {
 
 int lspk_flush_l2(void) {
     if (int rc = ensure_init()) return rc;
-    if (!g_flush_buf) LSPK_CUDA(cudaMalloc(&g_flush_buf, kFlushBytes));
+    if (!g_flush_buf) LSPK_CUDA(device_malloc(&g_flush_buf, kFlushBytes));
     static int v = 0;
     LSPK_CUDA(cudaMemsetAsync(g_flush_buf, ++v & 0xff, kFlushBytes, g_stream));
     return LSPK_OK;

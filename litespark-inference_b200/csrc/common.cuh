@@ -23,6 +23,9 @@ int  ensure_init();                                 // bind to a GPU on first us
 // the MoE and Mamba blocks) grows by free + malloc, which moves it.  A CUDA graph captured earlier holds the
 // old addresses, so whoever moves scratch bumps this counter and every graph owner compares it with the value
 // it recorded at capture and re-captures when they differ.
+// cudaMalloc that gives parked memory (inference states kept for reuse, runtime.cu) back before it fails.
+cudaError_t device_malloc(void** p, size_t bytes);
+bool release_parked_states();                       // true if something was freed
 unsigned scratch_generation();
 void scratch_moved();
 

@@ -22,7 +22,7 @@ static void* slot(int i, size_t bytes) {
         if (g_slot[i]) cudaFree(g_slot[i]);
         g_slot[i] = nullptr;
         size_t want = bytes + bytes / 4 + 256;
-        if (cudaMalloc(&g_slot[i], want) != cudaSuccess) {
+        if (device_malloc((void**)&g_slot[i], want) != cudaSuccess) {
             g_slot_bytes[i] = 0;
             fail(LSPK_ERR_CUDA, "device scratch allocation of %zu bytes failed", want);
             return nullptr;
@@ -264,10 +264,10 @@ int lspk_register_embedding(int kind, const void* emb_host, const float* emb_sca
     LSPK_REQUIRE(kind == 0 || emb_scale_host, "lspk_register_embedding: int8/int4 need the scale vector");
     EmbEntry e = {};
     e.kind = kind; e.V = V; e.H = H;
-    LSPK_CUDA(cudaMalloc(&e.emb, emb_bytes(kind, V, H)));
+    LSPK_CUDA(device_malloc((void**)&e.emb, emb_bytes(kind, V, H)));
     LSPK_CUDA(cudaMemcpy(e.emb, emb_host, emb_bytes(kind, V, H), cudaMemcpyHostToDevice));
     if (kind != 0) {
-        LSPK_CUDA(cudaMalloc((void**)&e.scale, (size_t)V * 4));
+        LSPK_CUDA(device_malloc((void**)&e.scale, (size_t)V * 4));
         LSPK_CUDA(cudaMemcpy(e.scale, emb_scale_host, (size_t)V * 4, cudaMemcpyHostToDevice));
     }
     auto it = g_emb.find(emb_host);

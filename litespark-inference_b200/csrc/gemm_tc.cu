@@ -600,7 +600,7 @@ static int grow(void** p, size_t* cap, size_t need) {
     *p = nullptr;
     *cap = 0;
     scratch_moved();
-    LSPK_CUDA(cudaMalloc(p, need + need / 4 + 256));
+    LSPK_CUDA(device_malloc(p, need + need / 4 + 256));
     *cap = need + need / 4 + 256;
     return LSPK_OK;
 }

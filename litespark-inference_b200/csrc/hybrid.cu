@@ -149,9 +149,9 @@ int lspk_hybrid_set_embedding(lspk_hybrid_t hh, const uint16_t* emb_bf16_host, c
     const size_t eb = (size_t)h->V * h->H * 2;
     if (h->emb) cudaFree(h->emb);
     if (h->final_norm) cudaFree(h->final_norm);
-    LSPK_CUDA(cudaMalloc((void**)&h->emb, eb));
+    LSPK_CUDA(device_malloc((void**)&h->emb, eb));
     LSPK_CUDA(cudaMemcpy(h->emb, emb_bf16_host, eb, cudaMemcpyHostToDevice));
-    LSPK_CUDA(cudaMalloc((void**)&h->final_norm, (size_t)h->H * 2));
+    LSPK_CUDA(device_malloc((void**)&h->final_norm, (size_t)h->H * 2));
     LSPK_CUDA(cudaMemcpy(h->final_norm, final_norm_gamma, (size_t)h->H * 2, cudaMemcpyHostToDevice));
     h->bytes += eb + (size_t)h->H * 2;
     return LSPK_OK;
@@ -194,7 +194,7 @@ lspk_hybrid_state_t lspk_hybrid_state_create(lspk_hybrid_t hh, int batch, int ma
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** p, size_t bytes) {
         if (e != cudaSuccess) return;
-        e = cudaMalloc(p, bytes);
+        e = device_malloc(p, bytes);
         s->bytes += bytes;
     };
     for (auto& L : h->layers) {
@@ -288,7 +288,7 @@ int lspk_hybrid_prefill(lspk_hybrid_state_t sh, const int* tokens_host, int T, i
     // one graph replay per prompt position; the token ids of all positions are staged once
     std::vector<int> all(tokens_host, tokens_host + (size_t)T * B);
     int* d_tokens = nullptr;
-    LSPK_CUDA(cudaMalloc((void**)&d_tokens, (size_t)T * B * 4));
+    LSPK_CUDA(device_malloc((void**)&d_tokens, (size_t)T * B * 4));
     cudaError_t e = cudaMemcpyAsync(d_tokens, all.data(), (size_t)T * B * 4, cudaMemcpyHostToDevice, stream());
     for (int t = 0; t < T && e == cudaSuccess; ++t) {
         e = cudaMemcpyAsync(s->ctl + B, d_tokens + (size_t)t * B, (size_t)B * 4, cudaMemcpyDeviceToDevice, stream());

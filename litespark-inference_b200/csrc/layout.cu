@@ -100,8 +100,8 @@ lspk_weight_t lspk_upload_packed(const uint8_t* packed_host, int N, int K, float
     w->bytes = (size_t)w->groups * w->chunks * kRowsPerGroup * 16;
     w->dev = nullptr;
     uint8_t* staging = nullptr;
-    cudaError_t e = cudaMalloc(&w->dev, w->bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&staging, (size_t)N * Kb);
+    cudaError_t e = device_malloc((void**)&w->dev, w->bytes);
+    if (e == cudaSuccess) e = device_malloc((void**)&staging, (size_t)N * Kb);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(staging, packed_host, (size_t)N * Kb, cudaMemcpyHostToDevice, stream());
     if (e == cudaSuccess) {
@@ -142,9 +142,9 @@ lspk_weight_t lspk_upload_bf16_ternary(const uint16_t* w_bf16_host, int N, int K
     w->dev = nullptr;
     uint16_t* master = nullptr;
     uint8_t* staging = nullptr;
-    cudaError_t e = cudaMalloc(&w->dev, w->bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&master, (size_t)N * K * 2);
-    if (e == cudaSuccess) e = cudaMalloc(&staging, (size_t)N * Kb);
+    cudaError_t e = device_malloc((void**)&w->dev, w->bytes);
+    if (e == cudaSuccess) e = device_malloc((void**)&master, (size_t)N * K * 2);
+    if (e == cudaSuccess) e = device_malloc((void**)&staging, (size_t)N * Kb);
     if (e == cudaSuccess) e = cudaMemcpyAsync(master, w_bf16_host, (size_t)N * K * 2, cudaMemcpyHostToDevice, stream());
     if (e == cudaSuccess) {
         const long long n_bytes = (long long)N * Kb;
@@ -179,7 +179,7 @@ int lspk_download_packed(lspk_weight_t h, uint8_t* packed_host_out) {
     Weight* w = reinterpret_cast<Weight*>(h);
     const int Kb = w->K / 4;
     uint8_t* staging = nullptr;
-    LSPK_CUDA(cudaMalloc(&staging, (size_t)w->N * Kb));
+    LSPK_CUDA(device_malloc((void**)&staging, (size_t)w->N * Kb));
     const long long total = (long long)w->N * Kb;
     const int block = 256;
     const int grid = (int)((total + block - 1) / block < 65535 ? (total + block - 1) / block : 65535);

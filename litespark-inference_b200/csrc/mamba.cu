@@ -171,8 +171,8 @@ int mamba_reserve(Mamba* m, int B) {
     m->zx = m->v = nullptr;
     m->cap_B = 0;
     scratch_moved();
-    LSPK_CUDA(cudaMalloc((void**)&m->zx, (size_t)B * m->in_out * 4));
-    LSPK_CUDA(cudaMalloc((void**)&m->v, (size_t)B * m->d_inner * 4));
+    LSPK_CUDA(device_malloc((void**)&m->zx, (size_t)B * m->in_out * 4));
+    LSPK_CUDA(device_malloc((void**)&m->v, (size_t)B * m->d_inner * 4));
     m->bytes += (size_t)B * (m->in_out + m->d_inner) * 4;
     m->cap_B = B;
     return LSPK_OK;
@@ -248,7 +248,7 @@ lspk_mamba_t lspk_mamba_create(const lspk_mamba_config* cfg, const uint8_t* in_p
     cudaError_t e = (m->in_proj && m->out_proj) ? cudaSuccess : cudaErrorMemoryAllocation;
     auto up = [&](void** dst, const void* src, size_t bytes) {
         if (e != cudaSuccess) return;
-        e = cudaMalloc(dst, bytes);
+        e = device_malloc(dst, bytes);
         if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
         m->bytes += bytes;
     };

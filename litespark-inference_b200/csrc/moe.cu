@@ -187,7 +187,7 @@ __global__ void moe_combine_kernel(float* __restrict__ x, const float* __restric
 }
 
 static int moe_alloc(void** p, size_t bytes, Moe* m) {
-    LSPK_CUDA(cudaMalloc(p, bytes ? bytes : 16));
+    LSPK_CUDA(device_malloc(p, bytes ? bytes : 16));
     m->bytes += bytes;
     return LSPK_OK;
 }
@@ -386,8 +386,8 @@ lspk_moe_t lspk_moe_create(int n_experts, int hidden, int inter, const uint8_t* 
     m->mat_stride = gu_chunks > d_chunks ? gu_chunks : d_chunks;
     const size_t host_mat = (size_t)inter * hidden / 4;
     uint8_t* staging = nullptr;
-    cudaError_t e = cudaMalloc((void**)&m->w, (size_t)n_experts * 3 * m->mat_stride * 16);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&staging, host_mat);
+    cudaError_t e = device_malloc((void**)&m->w, (size_t)n_experts * 3 * m->mat_stride * 16);
+    if (e == cudaSuccess) e = device_malloc((void**)&staging, host_mat);
     for (int ex = 0; ex < n_experts && e == cudaSuccess; ++ex) {
         for (int which = 0; which < 3 && e == cudaSuccess; ++which) {
             const uint8_t* src = experts_packed_host + ((size_t)ex * 3 + which) * host_mat;
@@ -403,7 +403,7 @@ lspk_moe_t lspk_moe_create(int n_experts, int hidden, int inter, const uint8_t* 
     m->bytes = (size_t)n_experts * 3 * m->mat_stride * 16;
     auto up = [&](void** dst, const void* src, size_t bytes) {
         if (e != cudaSuccess) return;
-        e = cudaMalloc(dst, bytes);
+        e = device_malloc(dst, bytes);
         if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
         m->bytes += bytes;
     };

@@ -6,6 +6,8 @@
 // sequence of kernel launches; the per-op arithmetic lives in linear.cu / rows.cu /
 // attention.cu / lm_head.cu.
 #include <string.h>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "runtime_internal.cuh"
@@ -136,7 +138,7 @@ int launch_finish_step(int* ctl, unsigned long long* best, int* tokens_out, int 
 // ---- helpers -------------------------------------------------------------------------------
 
 static int dev_alloc(void** p, size_t bytes, size_t* tally) {
-    LSPK_CUDA(cudaMalloc(p, bytes ? bytes : 16));
+    LSPK_CUDA(device_malloc(p, bytes ? bytes : 16));
     if (tally) *tally += bytes;
     return LSPK_OK;
 }
@@ -165,9 +167,11 @@ static int upload_table(DevTable& t, int kind, const void* host, const float* sc
 // are 180 MB at that shape, allocated only for prompts that long.
 constexpr int kMaxPrefillRows = 2048;
 
-// Grows the row scratch of the layers.  Graphs captured before hold the old addresses and are dropped.
+// Grows the row scratch of the layers: 128 rows (or the batch) at first, then at once to the longest prompt the state
+// can take.  Graphs captured before hold the old addresses and are dropped.
 static int reserve_rows(State* s, int rows) {
     if (rows <= s->cap_rows) return LSPK_OK;
+    if (s->cap_rows > 0 && s->t_max > rows) rows = s->t_max < kMaxPrefillRows ? s->t_max : kMaxPrefillRows;
     const lspk_model_config& c = s->m->cfg;
     const size_t R = (size_t)((rows + 127) / 128) * 128, H = c.hidden_size, I = c.intermediate_size, kv = s->m->kv_dim();
     LSPK_CUDA(cudaStreamSynchronize(stream()));
@@ -187,11 +191,57 @@ static int reserve_rows(State* s, int rows) {
     }
     s->cap_rows = 0;
     for (const Buf& b : bufs) {
-        LSPK_CUDA(cudaMalloc(b.p, R * b.width * 4));
+        LSPK_CUDA(device_malloc(b.p, R * b.width * 4));
         s->bytes += R * b.width * 4;
     }
     s->cap_rows = (int)R;
     return LSPK_OK;
+}
+
+// Pinned staging for logits, made when a call first wants them (a greedy loop never does; pinning takes milliseconds).
+static int reserve_host_logits(State* s) {
+    if (!s->h_logits) LSPK_CUDA(cudaMallocHost((void**)&s->h_logits, (size_t)s->logits_rows * s->m->cfg.vocab_size * 4));
+    return LSPK_OK;
+}
+
+// Parked states.  A program that makes a state per request (the facade does) frees and makes the same one over and over;
+// its allocations, pinned buffers and instantiated graph cost several milliseconds.  A freed state is therefore kept, at
+// most one per live model and kMaxParkedBytes each, and handed out again, cleared, to a request for the same shape and
+// rope tables.  It is given back when its model is freed, when another state takes its place, and when an allocation
+// fails (device_malloc).
+constexpr size_t kMaxParkedBytes = (size_t)1 << 30;
+static std::mutex g_park_mu;
+static std::map<unsigned long long, State*> g_parked;      // one entry per live model; null: nothing parked
+static unsigned long long g_next_model_id = 0;
+
+static void destroy_state(State* s);
+
+// The model's tensors are about to change (or to go): the graphs of a parked state hold their addresses.
+static void drop_parked(Model* m, bool model_goes = false) {
+    State* parked = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_park_mu);
+        auto it = g_parked.find(m->id);
+        if (it != g_parked.end()) {
+            std::swap(parked, it->second);
+            if (model_goes) g_parked.erase(it);
+        }
+    }
+    if (parked) destroy_state(parked);
+}
+
+bool release_parked_states() {
+    std::vector<State*> gone;
+    {
+        std::lock_guard<std::mutex> lk(g_park_mu);
+        for (auto& kv : g_parked)
+            if (kv.second) {
+                gone.push_back(kv.second);
+                kv.second = nullptr;
+            }
+    }
+    for (State* s : gone) destroy_state(s);
+    return !gone.empty();
 }
 
 // One transformer layer for `rows` rows held in the state's scratch buffers.
@@ -298,15 +348,40 @@ static int enqueue_step(State* s, bool store_logits, bool host_io = false) {
         if (int rc = lm_head_launch(head.kind, head.data, head.scale, s->x, store_logits ? s->logits : nullptr, 1, V, H,
                                     m->final_norm.g, m->final_norm.is_bf16, c.rms_norm_eps, s->best)) return rc;
     } else {
-        // the greedy choice of every row comes out of the LM head itself (bf16 table) or of a row argmax it
-        // launches (int8 / int4 tables); logits are written only where something reads them
-        const bool need_logits = store_logits || head.kind != 0 || (H % 32) != 0;
+        // the greedy choice of every row comes out of the LM head itself (or, for odd hidden sizes, of a row argmax it
+        // launches); logits are written only where something reads them
+        const bool need_logits = store_logits || !lm_head_rows_on_tensor_cores(head.kind, H);
         if (int rc = lm_head_launch(head.kind, head.data, head.scale, s->x, need_logits ? s->logits : nullptr, B, V, H,
                                     m->final_norm.g, m->final_norm.is_bf16, c.rms_norm_eps, s->best)) return rc;
     }
     LSPK_CUDA(launch(finish_step_kernel, dim3(1), dim3(((B + 31) / 32) * 32), 0, true, s->ctl, s->best,
                      s->tokens_out, B, s->t_max, host_io ? s->io_pkt_dev : (unsigned long long*)nullptr,
                      host_io ? s->io_seq_dev : (unsigned*)nullptr));
+    return LSPK_OK;
+}
+
+static void destroy_state(State* s) {
+    cudaStreamSynchronize(stream());
+    for (auto& g : s->graph)
+        if (g) cudaGraphExecDestroy(g);
+    void* dev[] = {s->cache_k, s->cache_v, s->rope_cos, s->rope_sin, s->rope_cur, s->ctl, s->best, s->tokens_out, s->x, s->q, s->k,
+                   s->v, s->attn, s->inter, s->logits, s->tok_rows};
+    for (void* p : dev) cudaFree(p);
+    if (s->h_int) cudaFreeHost(s->h_int);
+    if (s->h_logits) cudaFreeHost(s->h_logits);
+    if (s->io_pkt) cudaFreeHost(s->io_pkt);
+    cudaFree(s->io_seq_dev);
+    delete s;
+}
+
+// A state as after creation: empty cache, position 0.  Ordered on the library stream.
+static int clear_state(State* s) {
+    const size_t cache_bytes = (size_t)s->batch * s->seq_stride() * s->kv_elem();
+    LSPK_CUDA(cudaMemsetAsync(s->cache_k, 0, cache_bytes, stream()));
+    LSPK_CUDA(cudaMemsetAsync(s->cache_v, 0, cache_bytes, stream()));
+    LSPK_CUDA(cudaMemsetAsync(s->ctl, 0, (size_t)(2 * s->batch + 1) * 4, stream()));
+    LSPK_CUDA(cudaMemsetAsync(s->best, 0, (size_t)s->batch * 8, stream()));
+    s->host_pos.assign(s->batch, 0);
     return LSPK_OK;
 }
 
@@ -320,18 +395,23 @@ static int build_graph(State* s, int variant) {
         cudaGraphExecDestroy(s->graph[variant]);
         s->graph[variant] = nullptr;
     }
-    // First run the step once outside capture: it sets the kernels' shared-memory attributes
-    // (not allowed while capturing) and surfaces launch errors directly.  The warm-up must not
+    // The first time a model takes a step of this shape, run it once outside capture: it sets the kernels'
+    // shared-memory attributes, sizes library scratch (neither is allowed while capturing) and surfaces launch errors
+    // directly.  Both outlive the state, so further states of the shape go straight to the capture.  The warm-up must not
     // change the state: save and restore the control block around it.
-    const int nctl = 2 * s->batch + 1;
-    std::vector<int> saved(nctl);
-    LSPK_CUDA(cudaMemcpyAsync(saved.data(), s->ctl, nctl * sizeof(int), cudaMemcpyDeviceToHost, stream()));
-    LSPK_CUDA(cudaStreamSynchronize(stream()));
-    if (int rc = enqueue_step(s, variant == 1, variant == 2)) return rc;
-    LSPK_CUDA(cudaStreamSynchronize(stream()));
-    LSPK_CUDA(cudaMemcpyAsync(s->ctl, saved.data(), nctl * sizeof(int), cudaMemcpyHostToDevice, stream()));
-    LSPK_CUDA(cudaStreamSynchronize(stream()));
-    if (variant == 2) s->io_seq += 1;          // the warm-up step counted itself on the device
+    const int shape = (s->batch * 2 + s->kv_fp16) * 4 + variant;
+    if (!s->m->warmed.count(shape)) {
+        const int nctl = 2 * s->batch + 1;
+        std::vector<int> saved(nctl);
+        LSPK_CUDA(cudaMemcpyAsync(saved.data(), s->ctl, nctl * sizeof(int), cudaMemcpyDeviceToHost, stream()));
+        LSPK_CUDA(cudaStreamSynchronize(stream()));
+        if (int rc = enqueue_step(s, variant == 1, variant == 2)) return rc;
+        LSPK_CUDA(cudaStreamSynchronize(stream()));
+        LSPK_CUDA(cudaMemcpyAsync(s->ctl, saved.data(), nctl * sizeof(int), cudaMemcpyHostToDevice, stream()));
+        LSPK_CUDA(cudaStreamSynchronize(stream()));
+        if (variant == 2) s->io_seq += 1;          // the warm-up step counted itself on the device
+        s->m->warmed.insert(shape);
+    }
 
     cudaGraph_t g = nullptr;
     LSPK_CUDA(cudaStreamBeginCapture(stream(), cudaStreamCaptureModeThreadLocal));
@@ -374,6 +454,9 @@ lspk_model_t lspk_model_create(const lspk_model_config* cfg) {
     Model* m = new Model();
     m->cfg = *cfg;
     m->layers.resize(cfg->num_layers);
+    std::lock_guard<std::mutex> lk(g_park_mu);
+    m->id = ++g_next_model_id;
+    g_parked[m->id] = nullptr;
     return reinterpret_cast<lspk_model_t>(m);
 }
 
@@ -391,6 +474,7 @@ int lspk_model_set_projection(lspk_model_t h, int layer, int which, const uint8_
     lspk_weight_t w = lspk_upload_packed(packed_host, N, K, scale);
     if (!w) return LSPK_ERR_CUDA;
     DevLayer& L = m->layers[layer];
+    drop_parked(m);
     if (L.proj[which]) lspk_weight_free(L.proj[which]);
     L.proj[which] = w;
     m->bytes += reinterpret_cast<Weight*>(w)->bytes;
@@ -411,6 +495,7 @@ int lspk_model_set_projection_bf16(lspk_model_t h, int layer, int which, const u
     lspk_weight_t w = lspk_upload_bf16_ternary(w_bf16_host, N, K, absmean);
     if (!w) return LSPK_ERR_CUDA;
     DevLayer& L = m->layers[layer];
+    drop_parked(m);
     if (L.proj[which]) lspk_weight_free(L.proj[which]);
     L.proj[which] = w;
     m->bytes += reinterpret_cast<Weight*>(w)->bytes;
@@ -430,6 +515,7 @@ int lspk_model_set_norm(lspk_model_t h, int layer, int which, const void* gamma_
     }
     const int want = which == LSPK_NORM_FFN_SUB ? m->cfg.intermediate_size : m->cfg.hidden_size;
     LSPK_REQUIRE(K == want, "lspk_model_set_norm: length %d, expected %d", K, want);
+    drop_parked(m);
     if (n->g) cudaFree(n->g);
     const size_t bytes = (size_t)K * (is_bf16 ? 2 : 4);
     if (int rc = dev_alloc(&n->g, bytes, &m->bytes)) return rc;
@@ -442,12 +528,14 @@ int lspk_model_set_norm(lspk_model_t h, int layer, int which, const void* gamma_
 int lspk_model_set_embedding(lspk_model_t h, int kind, const void* emb_host, const float* scale_host) {
     LSPK_REQUIRE(h, "lspk_model_set_embedding: null model");
     Model* m = reinterpret_cast<Model*>(h);
+    drop_parked(m);
     return upload_table(m->emb, kind, emb_host, scale_host, m->cfg.vocab_size, m->cfg.hidden_size, &m->bytes);
 }
 
 int lspk_model_set_lm_head(lspk_model_t h, int kind, const void* head_host, const float* scale_host) {
     LSPK_REQUIRE(h, "lspk_model_set_lm_head: null model");
     Model* m = reinterpret_cast<Model*>(h);
+    drop_parked(m);
     return upload_table(m->head, kind, head_host, scale_host, m->cfg.vocab_size, m->cfg.hidden_size, &m->bytes);
 }
 
@@ -483,6 +571,7 @@ int lspk_model_free(lspk_model_t h) {
     if (!h) return LSPK_OK;
     Model* m = reinterpret_cast<Model*>(h);
     cudaStreamSynchronize(stream());
+    drop_parked(m, true);
     for (auto& L : m->layers) {
         for (auto& w : L.proj) lspk_weight_free(w);
         for (auto& n : L.norm) cudaFree(n.g);
@@ -504,8 +593,30 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
         fail(LSPK_ERR_ARG, "lspk_state_create: bad arguments (model finalised? t_max=%d batch=%d)", t_max, batch);
         return nullptr;
     }
+    const size_t half_table = (size_t)t_max * (m->D() / 2);
+    {
+        State* again = nullptr;
+        {
+            std::lock_guard<std::mutex> lk(g_park_mu);
+            auto it = g_parked.find(m->id);
+            State* c = it != g_parked.end() ? it->second : nullptr;
+            if (c && c->t_max == t_max && c->batch == batch && c->kv_fp16 == (kv_fp16 ? 1 : 0) &&
+                memcmp(c->rope_host.data(), rope_cos, half_table * 4) == 0 &&
+                memcmp(c->rope_host.data() + half_table, rope_sin, half_table * 4) == 0) {
+                again = c;
+                it->second = nullptr;
+            }
+        }
+        if (again) {
+            if (clear_state(again) == LSPK_OK) return reinterpret_cast<lspk_state_t>(again);
+            destroy_state(again);
+        }
+    }
     State* s = new State();
     s->m = m;
+    s->model_id = m->id;
+    s->rope_host.assign(rope_cos, rope_cos + half_table);
+    s->rope_host.insert(s->rope_host.end(), rope_sin, rope_sin + half_table);
     s->t_max = t_max;
     s->batch = batch;
     s->kv_fp16 = kv_fp16 ? 1 : 0;
@@ -526,7 +637,6 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
     rc |= dev_alloc((void**)&s->logits, (size_t)s->logits_rows * V * 4, &s->bytes);
     rc |= reserve_rows(s, batch > 128 ? batch : 128);
     if (!rc && cudaMallocHost((void**)&s->h_int, (size_t)(t_max * batch + 2 * batch + 16) * 4) != cudaSuccess) rc = 1;
-    if (!rc && cudaMallocHost((void**)&s->h_logits, (size_t)s->logits_rows * V * 4) != cudaSuccess) rc = 1;
     if (!rc && batch == 1) {
         // the two words of the host-fed step (see State): mapped pinned memory and its device alias
         void *io = nullptr, *io_dev = nullptr;
@@ -541,22 +651,19 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
             s->io_pkt_dev = static_cast<unsigned long long*>(io_dev);
             s->io_tok_dev = reinterpret_cast<int*>(static_cast<char*>(io_dev) + 16);
             rc |= dev_alloc((void**)&s->io_seq_dev, 4, &s->bytes);
-            if (!rc && cudaMemset(s->io_seq_dev, 0, 4) != cudaSuccess) rc = 1;
+            if (!rc && cudaMemsetAsync(s->io_seq_dev, 0, 4, stream()) != cudaSuccess) rc = 1;
         }
     }
     if (!rc) {
-        cudaError_t e = cudaMemset(s->cache_k, 0, cache_bytes);
-        if (e == cudaSuccess) e = cudaMemset(s->cache_v, 0, cache_bytes);
-        if (e == cudaSuccess) e = cudaMemset(s->ctl, 0, (size_t)(2 * batch + 1) * 4);
-        if (e == cudaSuccess) e = cudaMemset(s->best, 0, (size_t)batch * 8);
-        if (e == cudaSuccess) e = cudaMemcpy(s->rope_cos, rope_cos, (size_t)t_max * (D / 2) * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(s->rope_sin, rope_sin, (size_t)t_max * (D / 2) * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaDeviceSynchronize();   // the memsets ran on the default stream
+        cudaError_t e = cudaMemcpyAsync(s->rope_cos, s->rope_host.data(), half_table * 4, cudaMemcpyHostToDevice, stream());
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->rope_sin, s->rope_host.data() + half_table, half_table * 4, cudaMemcpyHostToDevice, stream());
+        if (clear_state(s)) rc = 1;
         if (e != cudaSuccess) rc = 1;
     }
     if (rc) {
         fail(LSPK_ERR_CUDA, "lspk_state_create: allocation failed (%s)", cudaGetErrorString(cudaGetLastError()));
-        lspk_state_free(reinterpret_cast<lspk_state_t>(s));
+        destroy_state(s);
         return nullptr;
     }
     return reinterpret_cast<lspk_state_t>(s);
@@ -565,20 +672,14 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
 int lspk_state_free(lspk_state_t h) {
     if (!h) return LSPK_OK;
     State* s = reinterpret_cast<State*>(h);
-    cudaStreamSynchronize(stream());
-    for (auto& g : s->graph)
-        if (g) cudaGraphExecDestroy(g);
-    void* dev[] = {s->cache_k, s->cache_v, s->rope_cos, s->rope_sin, s->rope_cur, s->ctl, s->best, s->tokens_out, s->x, s->q, s->k,
-                   s->v, s->attn, s->inter, s->logits, s->tok_rows};
-    for (void* p : dev) cudaFree(p);
-    if (s->h_int) cudaFreeHost(s->h_int);
-    if (s->h_logits) cudaFreeHost(s->h_logits);
-    if (s->io_pkt) cudaFreeHost(s->io_pkt);
-    cudaFree(s->io_seq_dev);
-    delete s;
+    if (s->bytes <= kMaxParkedBytes) {
+        std::lock_guard<std::mutex> lk(g_park_mu);
+        auto it = g_parked.find(s->model_id);      // no entry: the model is gone
+        if (it != g_parked.end()) std::swap(it->second, s);
+    }
+    if (s) destroy_state(s);
     return LSPK_OK;
 }
-
 int lspk_state_get_pos(lspk_state_t h, int seq) {
     State* s = reinterpret_cast<State*>(h);
     if (!s || seq < 0 || seq >= s->batch) return -1;
@@ -655,6 +756,8 @@ int lspk_forward_step(lspk_state_t h, const int* tokens_host, float* logits_host
         return LSPK_OK;
     }
     const int variant = (logits_host || B > 1) ? 1 : 0;
+    if (logits_host)
+        if (int rc = reserve_host_logits(s)) return rc;
     if (int rc = build_graph(s, variant)) return rc;
     memcpy(s->h_int, tokens_host, (size_t)B * 4);
     LSPK_CUDA(cudaMemcpyAsync(s->ctl + B, s->h_int, (size_t)B * 4, cudaMemcpyHostToDevice, stream()));
@@ -703,6 +806,8 @@ int lspk_forward_prefill(lspk_state_t h, int seq, const int* tokens_host, int T,
     if (s->host_pos[seq] + T > s->t_max)
         return fail(LSPK_ERR_STATE, "prefill would exceed t_max: pos=%d T=%d t_max=%d", s->host_pos[seq], T, s->t_max);
     const DevTable& head = m->head.data ? m->head : m->emb;
+    if (last_logits_host || all_logits_host)
+        if (int rc = reserve_host_logits(s)) return rc;
     if (int rc = reserve_rows(s, T < kMaxPrefillRows ? T : kMaxPrefillRows)) return rc;
     for (int t0 = 0; t0 < T; t0 += s->cap_rows) {
         const int rows = (T - t0) < s->cap_rows ? (T - t0) : s->cap_rows;

@@ -1,6 +1,7 @@
 // Model and inference-state containers of the device-resident forward pass, shared between runtime.cu (which
 // owns them) and the measurement harnesses in bench_probes.cu.
 #pragma once
+#include <set>
 #include <vector>
 
 #include "internal.cuh"
@@ -32,12 +33,16 @@ struct Model {
     DevTable emb, head;
     bool finalized = false;
     size_t bytes = 0;
+    unsigned long long id = 0;        // never reused: states find their model's parking place by it
+    std::set<int> warmed;             // step shapes (batch, KV type, graph variant) that have run once outside capture
     int D() const { return cfg.hidden_size / cfg.num_heads; }
     int kv_dim() const { return cfg.num_kv_heads * D(); }
 };
 
 struct State {
     Model* m = nullptr;
+    unsigned long long model_id = 0;
+    std::vector<float> rope_host;     // the tables the state was created with (cos, then sin)
     int t_max = 0, batch = 1, kv_fp16 = 1;
     int cap_rows = 0;                 // rows the scratch buffers hold
     void *cache_k = nullptr, *cache_v = nullptr;

@@ -11,6 +11,7 @@ explicitly.  The host still owns tokens, positions and the speculative-decoding 
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -122,6 +123,12 @@ def default_kv_dtype() -> str:
     return os.environ.get("LITESPARK_KV_DTYPE", "fp16").lower()
 
 
+@functools.lru_cache(maxsize=8)
+def _rope_tables(head_dim: int, t_max: int, theta: float):
+    """``rope_tables`` of a shape, kept: computing them takes longer than making the state."""
+    return rope_tables(head_dim, t_max, theta)
+
+
 class InferState:
     """KV cache + RoPE tables + scratch of ``batch`` sequences, on the GPU
     (reference runtime.py:59-111)."""
@@ -136,7 +143,7 @@ class InferState:
         self.kv_dtype = (kv_dtype or default_kv_dtype()).lower()
         if self.kv_dtype not in ("fp16", "fp32"):
             raise ValueError("kv_dtype must be 'fp16' or 'fp32'")
-        cos, sin = rope_tables(D, self.t_max, c.rope_theta)
+        cos, sin = _rope_tables(D, self.t_max, c.rope_theta)
         self.handle = self.lib.lspk_state_create(self.model.handle, self.t_max, self.batch,
                                                  int(self.kv_dtype == "fp16"), _ptr(cos), _ptr(sin))
         if not self.handle:

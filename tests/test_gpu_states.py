@@ -1,0 +1,75 @@
+"""Inference states that are freed and made again, and the LM head's table formats."""
+import importlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+dev = importlib.import_module("litespark_inference_b200.torchless.device")
+K = importlib.import_module("litespark_inference_b200.torchless.kernel")
+rt = importlib.import_module("litespark_inference_b200.torchless.runtime")
+synthetic = importlib.import_module("litespark_inference_b200.torchless.synthetic")
+
+
+def test_a_state_made_again_is_a_new_state():
+    """A freed state may be handed out again: empty cache, position 0, the same tokens as a fresh one; with another
+    shape, after the model's tensors changed, and after the model has gone it is not."""
+    cfg = synthetic.toy_config()
+    m = synthetic.random_model(cfg, seed=3, norm_jitter=0.1)
+    dm = rt.DeviceModel(m)
+    prompt = [int(t) for t in np.random.default_rng(1).integers(0, cfg.vocab_size, 20)]
+    want = rt.generate(dm, prompt, 10, state=rt.init_state(dm, 64))      # freed here
+    for _ in range(3):
+        st = rt.init_state(dm, 64)
+        assert st.pos == 0
+        k, v = st.read_kv(0, 64)
+        assert not k.any() and not v.any()
+        assert rt.generate(dm, prompt, 10, state=st) == want
+        two = rt.init_state(dm, 64)                                      # while the first is in use
+        assert rt.generate(dm, prompt, 10, state=two) == want
+        st.close()
+        two.close()
+    other = rt.init_state(dm, 65, kv_dtype="fp32")
+    assert rt.generate(dm, prompt, 10, state=other)[0] == want[0]
+    other.close()
+    # new norm weights: the graph of the parked state must not survive them
+    g = np.ascontiguousarray(m.final_norm[::-1])
+    K.check(dm.lib.lspk_model_set_norm(dm.handle, -1, 4, g.ctypes.data, 1, g.shape[0]))
+    m2 = synthetic.random_model(cfg, seed=3, norm_jitter=0.1)
+    m2.final_norm = g
+    dm2 = rt.DeviceModel(m2)
+    assert rt.generate(dm, prompt, 10, state=rt.init_state(dm, 65, kv_dtype="fp32")) == \
+        rt.generate(dm2, prompt, 10, state=rt.init_state(dm2, 65, kv_dtype="fp32"))
+    late = rt.init_state(dm2, 64)
+    dm2.close()
+    late.close()                                                         # its model is gone
+    dm.close()
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+# one row (pairs of table rows per warp), the tensor-core tiles at 2, 8, 9, 17 rows; hidden sizes on and off its K step;
+# an odd vocabulary
+@pytest.mark.parametrize("T,H", [(1, 2560), (1, 96), (2, 128), (8, 2560), (9, 256), (17, 640), (3, 96)])
+def test_lm_head_formats(kind, T, H):
+    rng = np.random.default_rng(kind * 100 + T)
+    V = 1037
+    x = (rng.standard_normal((T, H)) * np.exp(rng.uniform(-3, 3, (T, 1)))).astype(np.float32)
+    sc = rng.uniform(0.5, 1.5, V).astype(np.float32)
+    if kind == 0:
+        table = (rng.standard_normal((V, H)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        vals = (table.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    elif kind == 1:
+        table = rng.integers(-128, 128, (V, H)).astype(np.int8)
+        vals = table.astype(np.float64) * sc[:, None]
+    else:
+        table = rng.integers(0, 256, (V, H // 2)).astype(np.uint8)
+        n = np.stack([table & 15, table >> 4], axis=-1).reshape(V, H).astype(np.int64)
+        vals = (n - 16 * (n > 7)).astype(np.float64) * sc[:, None]
+    de, ds, dx = dev.DeviceArray.from_numpy(table), dev.DeviceArray.from_numpy(sc), dev.DeviceArray.from_numpy(x)
+    dl = dev.DeviceArray((T, V), np.float32)
+    K.check(K.load_library().lspk_lm_head(kind, de.ptr, ds.ptr if kind else None, dx.ptr, dl.ptr, T, V, H))
+    want = x.astype(np.float64) @ vals.T
+    # fp32 sums of H products in any order: H * 2^-24 of the sum of their magnitudes at the very most
+    bound = H * 2.0**-24 * (np.abs(x).astype(np.float64) @ np.abs(vals).T) + 1e-30
+    assert (np.abs(dl.numpy() - want) <= bound).all()
