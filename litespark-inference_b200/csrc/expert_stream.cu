@@ -1,0 +1,340 @@
+// Expert-grouped ternary products of the MoE layer, several routed rows: every expert's matrix streamed once past
+// the rows routed to it, in ONE persistent launch per stage (gate / up pair, then down).
+//
+// What bounds it: the bytes of the expert matrices that have rows (71 MB of gate / up, 35 MB of down at eight experts
+// of 6912 x 2560).  One CTA per SM; the CTAs are dealt out evenly over the passes (an expert and up to eight of its
+// rows), and a CTA takes a contiguous run of the pass's 16-row groups.  Four warps request the run's stages in order
+// into a shared-memory ring (cp.async.bulk + mbarrier), across pass boundaries; each of twelve consumer warps
+// computes whole row groups alone: mma.sync.m16n8k32.u8.s8 on the masked 2-bit fields (operand mapping of
+// linear_mma.cu), no CTA-wide barrier and no cross-warp sum per row group.  (The eight-row kernel used here before
+// cut every row group along K over its eight warps: two barriers and a reduction through shared memory per 20 KB.)
+// A bulk copy is issued by an elected lane (elect.sync).  The row lists are made here from the router's choices, no
+// kernel of their own; the int8 rows come in the eight-row tile's layout, one bulk copy each.
+// Integer throughout, results equal to the one-row kernel's bit for bit.
+#include "internal.cuh"
+#include "ternary_core.cuh"
+
+namespace lspk {
+
+constexpr int kEConsumers = 12;
+constexpr int kEProducers = 4;
+constexpr int kEThreads = 32 * (kEConsumers + kEProducers);
+constexpr int kEStageChunks = 40;                                  // 16-row x 16-byte chunks per stage (all matrices)
+constexpr int kEStageBytes = kEStageChunks * kRowsPerGroup * 16;   // 10 KB
+constexpr int kESlotsMax = 20;
+constexpr int kET = 8;                                             // rows per pass: the MMA's N
+constexpr int kESmem = 225 * 1024;                                 // dynamic shared memory to share out
+constexpr long long kEBudgetCycles = 1ll << 31;                    // every wait of a CTA gives up after about a second
+
+__device__ __forceinline__ void e_consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEConsumers) : "memory"); }
+
+__device__ __forceinline__ bool e_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+__device__ __forceinline__ void e_mma(int c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <bool PAIR>
+__global__ void __launch_bounds__(kEThreads, 1)
+ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int rs = mma_row_stride(p.chunks * kWeightsPerChunk);
+    uint32_t* ring = reinterpret_cast<uint32_t*>(smem_raw);                                     // [slots][stage]
+    int8_t* xq = reinterpret_cast<int8_t*>(smem_raw + (size_t)p.slots * kEStageBytes);          // [kET][rs], permuted
+    __shared__ __align__(8) uint64_t full[kESlotsMax], empty[kESlotsMax], xbar;
+    __shared__ int s_seq[kESlotsMax];            // 1 + the number of the last stage requested into each slot (0: none yet)
+    __shared__ int s_count[32];
+    __shared__ int s_rows[kET], s_sumx[kET];
+    __shared__ float s_scale[kET];
+    __shared__ int s_abort;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    PhaseTrace tr;
+    tr.begin(p.trace, p.trace_cap, PAIR ? 11 : 12);
+    tr.mark();                                   // 0: entry
+    const long long deadline = clock64() + kEBudgetCycles;
+    auto expired = [&]() { return clock64() > deadline || *(volatile int*)&s_abort != 0; };
+    if (tid < p.slots) {
+        s_seq[tid] = 0;
+        mbar_init(&full[tid], 1);
+        mbar_init(&empty[tid], 1);
+        fence_mbar_init();
+    } else if (tid == 32) {
+        s_abort = 0;
+        mbar_init(&xbar, kET);
+        fence_mbar_init();
+    } else if (tid >= 64 && tid < 96) {
+        s_count[tid - 64] = 0;
+    }
+    __syncthreads();
+    grid_dependency_launch();
+    // sel_ready: the choices were made before the previous kernel's predecessor ended and the previous kernel let this
+    // one start only after that (its launch trigger stands behind its own dependency wait)
+    if (!p.sel_ready) grid_dependency_wait();
+    auto choice = [&](int r) -> int { return __ldcg(p.sel + r); };
+    for (int r = tid; r < p.R; r += kEThreads) {
+        const int e = choice(r);
+        if (e >= 0 && e < p.E) atomicAdd(&s_count[e], 1);
+    }
+    __syncthreads();
+    // passes: lane e of every warp holds expert e's number of passes and their running sum
+    const int my_tiles = (s_count[lane] + kET - 1) / kET;
+    int incl = my_tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int other = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += other;
+    }
+    const int n_pass = __shfl_sync(0xffffffffu, incl, 31);
+    const int per = max(1, (int)gridDim.x / max(1, n_pass));       // CTAs of a pass
+    const int pass_step = (int)gridDim.x / per;
+    const int part = (int)blockIdx.x % per;
+    const int g_lo = (int)((long long)p.groups * part / per), g_hi = (int)((long long)p.groups * (part + 1) / per);
+    // CTAs beyond per * pass_step have no share
+    const int pass0 = (int)blockIdx.x / per < pass_step ? (int)blockIdx.x / per : n_pass;
+    auto locate = [&](int pass, int& e, int& tile) {               // whole warps
+        const unsigned m = __ballot_sync(0xffffffffu, incl > pass);
+        e = __ffs(m) - 1;
+        tile = pass - __shfl_sync(0xffffffffu, incl - my_tiles, e);
+    };
+    const int sub = p.sub, cps = p.cps, chunks = p.chunks;
+
+    if (warp >= kEConsumers) {
+        // ---------------- producers: warp pw requests stages pw, pw + kEProducers, ... as slots come free ------------
+        const int pw = warp - kEConsumers;
+        uint64_t policy;
+        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+        int q = 0;
+        bool ok = true;
+        for (int pass = pass0; pass < n_pass && ok; pass += pass_step) {
+            int e, tile;
+            locate(pass, e, tile);
+            const size_t off = (size_t)e * p.w_stride + (size_t)g_lo * chunks * kRowsPerGroup;
+            const uint4* ua = p.w[0] + off;
+            const uint4* ub = p.w[PAIR ? 1 : 0] + off;
+            for (int g = g_lo; g < g_hi && ok; ++g) {
+                for (int s = 0; s < sub; ++s, ++q) {
+                    if (q % kEProducers != pw) continue;
+                    const int slot = q % p.slots;
+                    if (q >= p.slots) {          // the slot's previous occupant has to be consumed first
+                        const uint32_t parity = (uint32_t)(q / p.slots - 1) & 1u;
+                        bool freed = mbar_try_wait(&empty[slot], parity);
+                        while (!freed && !expired()) freed = mbar_try_wait(&empty[slot], parity);
+                        ok = __all_sync(0xffffffffu, freed);
+                        if (!ok) break;
+                    }
+                    const int c0 = s * cps, c1 = min(c0 + cps, chunks);
+                    const uint32_t bytes = (uint32_t)(c1 - c0) * kRowsPerGroup * 16u;
+                    unsigned char* dst = smem_raw + (size_t)slot * kEStageBytes;
+                    if (e_elect()) {
+                        mbar_expect_tx(&full[slot], bytes * (PAIR ? 2u : 1u));
+                        bulk_load_policy(dst, ua + (size_t)c0 * kRowsPerGroup, bytes, &full[slot], policy);
+                        if (PAIR) bulk_load_policy(dst + bytes, ub + (size_t)c0 * kRowsPerGroup, bytes, &full[slot], policy);
+                        // consumers test full[slot] only after they have seen the request: a phase test ahead of the
+                        // slot's previous use would succeed on the stale phase
+                        __threadfence_block();
+                        *(volatile int*)&s_seq[slot] = q + 1;
+                    }
+                    __syncwarp();
+                }
+                ua += (size_t)chunks * kRowsPerGroup;
+                ub += (size_t)chunks * kRowsPerGroup;
+            }
+        }
+        if (!ok && lane == 0 && !*(volatile int*)&s_abort) {       // a consumer did not free its slot in time
+            s_abort = 1;
+            if (p.error_flag) atomicExch(p.error_flag, LSPK_ERR_DEVICE_WAIT);
+        }
+        return;      // consumers wait for everything that was requested
+    }
+
+    // ---------------- consumers: warp w takes row groups g_lo + w, g_lo + w + 12, ... of each pass ----------------------
+    tr.mark();                                   // 1: passes known
+    if (p.sel_ready) grid_dependency_wait();
+    tr.mark();                                   // 2: predecessor finished
+    const int gid = lane >> 2, t4 = lane & 3;
+    bool dead = false;                           // a wait of this warp ran out: it leaves the ring alone from here on
+    bool skip = false;                           // another warp gave up: keep draining the ring, compute nothing
+    int q_base = 0;
+    uint32_t x_phase = 0;
+    for (int pass = pass0; pass < n_pass; pass += pass_step) {
+        int e, tile;
+        locate(pass, e, tile);
+        const int mt = min(kET, s_count[e] - tile * kET);
+        e_consumer_barrier();                    // the previous pass's rows are no longer read
+        if (warp == 0) {
+            // routed rows of rank tile * 8 .. tile * 8 + mt - 1 among the expert's, ascending
+            int base = -tile * kET;
+            for (int r0 = 0; r0 < p.R && base < kET; r0 += 32) {
+                const bool match = r0 + lane < p.R && choice(r0 + lane) == e;
+                const unsigned m = __ballot_sync(0xffffffffu, match);
+                const int rank = base + __popc(m & ((1u << lane) - 1u));
+                if (match && rank >= 0 && rank < kET) s_rows[rank] = r0 + lane;
+                base += __popc(m);
+            }
+        }
+        e_consumer_barrier();
+        if (p.x_sums) {
+            // rows already in the tile's layout: one bulk copy each, requested by as many warps
+            if (warp < kET) {
+                if (warp < mt) {
+                    const int row = s_rows[warp] >> p.in_shift;
+                    if (e_elect()) {
+                        const uint32_t bytes = (uint32_t)chunks * kWeightsPerChunk;
+                        mbar_expect_tx(&xbar, bytes);
+                        bulk_load(xq + (size_t)warp * rs, p.x + (size_t)row * rs, bytes, &xbar);
+                    }
+                    if (lane == 0) { s_scale[warp] = p.xs[row]; s_sumx[warp] = p.x_sums[row]; }
+                } else if (lane == 0) {
+                    mbar_arrive(&xbar);          // rows of the tile that do not exist are neither filled nor stored
+                }
+            }
+            bool there = mbar_try_wait(&xbar, x_phase);
+            while (!there && !(clock64() > deadline)) there = mbar_try_wait(&xbar, x_phase);
+            x_phase ^= 1u;
+            if (!there) {
+                s_abort = 1;
+                if (p.error_flag) atomicExch(p.error_flag, LSPK_ERR_DEVICE_WAIT);
+            }
+        } else if (warp < mt) {
+            // plain int8 rows, a warp per row: permuted 16-element blocks, their sum, their scale
+            const int nblk = chunks * 4;
+            int8_t* dst = xq + (size_t)warp * rs;
+            const int row = s_rows[warp] >> p.in_shift;
+            const int8_t* src = p.x + (size_t)row * p.K;
+            int sumx = 0;
+#pragma unroll 4
+            for (int b = lane; b < nblk; b += 32) {
+                uint32_t a[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (b * 16 + i * 4 < p.K) a[i] = __ldcg(reinterpret_cast<const uint32_t*>(src + b * 16 + i * 4));
+                uint32_t o0, o1, o2, o3;
+                transpose4x4_bytes(a[0], a[1], a[2], a[3], o0, o1, o2, o3);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sumx = __dp4a((int)a[i], 0x01010101, sumx);
+                *reinterpret_cast<uint4*>(dst + b * 16) = make_uint4(o0, o1, o2, o3);
+            }
+            sumx = __reduce_add_sync(0xffffffffu, sumx);
+            if (lane == 0) { s_scale[warp] = p.xs[row]; s_sumx[warp] = sumx; }
+        }
+        e_consumer_barrier();
+        if (*(volatile int*)&s_abort) skip = true;
+        tr.mark();                               // 3: rows staged
+        const float ws0 = p.scales[3 * e + p.scale_idx[0]], ws1 = p.scales[3 * e + p.scale_idx[PAIR ? 1 : 0]];
+        const int8_t* xrow = xq + (size_t)gid * rs + t4 * 16;       // B operand: token gid
+        for (int g = g_lo + warp; !dead && g < g_hi; g += kEConsumers) {
+            int acc_a[4][4], acc_b[PAIR ? 4 : 1][4];
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    acc_a[f][c] = 0;
+                    if (PAIR) acc_b[f][c] = 0;
+                }
+            for (int s = 0; s < sub; ++s) {
+                const int q = q_base + (g - g_lo) * sub + s;
+                const int slot = q % p.slots;
+                const uint32_t parity = (uint32_t)(q / p.slots) & 1u;
+                bool arrived = *(volatile int*)&s_seq[slot] > q;       // first the request (see the producer), then the data
+                while (!arrived && !(clock64() > deadline)) arrived = *(volatile int*)&s_seq[slot] > q;
+                if (arrived) {
+                    arrived = mbar_try_wait(&full[slot], parity);
+                    while (!arrived && !(clock64() > deadline)) arrived = mbar_try_wait(&full[slot], parity);
+                }
+                if (!__all_sync(0xffffffffu, arrived)) {
+                    dead = true;
+                    if (lane == 0) {
+                        s_abort = 1;
+                        if (p.error_flag) atomicExch(p.error_flag, LSPK_ERR_DEVICE_WAIT);
+                    }
+                    break;
+                }
+                tr.mark();                       // 4+: a stage is there
+                const int c0 = s * cps, nc = skip ? 0 : min(cps, chunks - c0);
+                const uint32_t* sa = ring + (size_t)slot * (kEStageBytes / 4) + lane;
+                const uint32_t* sb = sa + (size_t)nc * 64;
+                const int8_t* xs = xrow + (size_t)c0 * 64;
+                auto pair_step = [&](int c, bool two) {
+                    const uint4 x0 = *reinterpret_cast<const uint4*>(xs + (size_t)c * 64);
+                    uint4 x1 = make_uint4(0, 0, 0, 0);
+                    if (two) x1 = *reinterpret_cast<const uint4*>(xs + (size_t)c * 64 + 64);
+                    const uint32_t b0[4] = {x0.x, x0.y, x0.z, x0.w}, b1[4] = {x1.x, x1.y, x1.z, x1.w};
+                    const uint32_t a0 = sa[c * 64], a1 = sa[c * 64 + 32];
+                    const uint32_t a2 = two ? sa[c * 64 + 64] : 0x55555555u, a3 = two ? sa[c * 64 + 96] : 0x55555555u;
+                    uint32_t u0 = 0, u1 = 0, u2 = 0, u3 = 0;
+                    if (PAIR) {
+                        u0 = sb[c * 64];
+                        u1 = sb[c * 64 + 32];
+                        u2 = two ? sb[c * 64 + 64] : 0x55555555u;
+                        u3 = two ? sb[c * 64 + 96] : 0x55555555u;
+                    }
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) {
+                        const uint32_t mask = 0x03030303u << (2 * f);
+                        e_mma(acc_a[f], a0 & mask, a1 & mask, a2 & mask, a3 & mask, b0[f], b1[f]);
+                        if (PAIR) e_mma(acc_b[f], u0 & mask, u1 & mask, u2 & mask, u3 & mask, b0[f], b1[f]);
+                    }
+                };
+                int c = 0;
+#pragma unroll(PAIR ? 2 : 4)
+                for (; c + 1 < nc; c += 2) pair_step(c, true);
+                if (c < nc) pair_step(c, false);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[slot]);               // every lane has read the slot
+            }
+            if (dead || skip) continue;
+            // C fragment: c0, c1 = (row gid, tokens 2 t4, 2 t4 + 1), c2, c3 = (row gid + 8, same); masks combined by exact shifts
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int tok = 2 * t4 + (c & 1);
+                const int n = g * kRowsPerGroup + gid + ((c >> 1) << 3);
+                if (tok < mt && n < p.N) {
+                    const int sx = s_sumx[tok];
+                    const float xsc = s_scale[tok];
+                    const size_t o = (size_t)s_rows[tok] * p.N + n;
+                    const int va = acc_a[0][c] + (acc_a[1][c] >> 2) + (acc_a[2][c] >> 4) + (acc_a[3][c] >> 6) - sx;
+                    if (p.acc[0]) p.acc[0][o] = va;
+                    const float ya = __fmul_rn((float)va, __fmul_rn(xsc, ws0));
+                    if (PAIR) {
+                        const int vb = acc_b[0][c] + (acc_b[1][c] >> 2) + (acc_b[2][c] >> 4) + (acc_b[3][c] >> 6) - sx;
+                        if (p.acc[1]) p.acc[1][o] = vb;
+                        const float yb = __fmul_rn((float)vb, __fmul_rn(xsc, ws1));
+                        const float gpos = fmaxf(ya, 0.0f);
+                        p.out[o] = __fmul_rn(__fmul_rn(gpos, gpos), yb);
+                    } else {
+                        p.out[o] = ya;
+                    }
+                }
+            }
+        }
+        q_base += (g_hi - g_lo) * sub;
+    }
+    tr.end();
+}
+
+int expert_stream_launch(ExpertStreamParams p, bool pair) {
+    const size_t rows = (size_t)kET * mma_row_stride(p.chunks * kWeightsPerChunk);
+    int slots = rows < (size_t)kESmem ? (int)((kESmem - rows) / kEStageBytes) : 0;
+    // three slots keep the ring turning at the longest rows (K of about 24000); the model shapes have 17 to 20
+    LSPK_REQUIRE(slots >= 3, "expert products: K=%d too large for eight rows in shared memory (limit about 24000)", p.K);
+    p.slots = slots < kESlotsMax ? slots : kESlotsMax;
+    p.cps = kEStageChunks / (pair ? 2 : 1);
+    p.sub = (p.chunks + p.cps - 1) / p.cps;
+    p.error_flag = device_wait_flag();
+    p.trace = trace_buffer();
+    p.trace_cap = trace_capacity();
+    const size_t smem = (size_t)p.slots * kEStageBytes + rows;
+    auto kern = pair ? ternary_expert_stream_kernel<true> : ternary_expert_stream_kernel<false>;
+    LSPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kESmem));
+    LSPK_CUDA(launch(kern, dim3(sm_count()), dim3(kEThreads), smem, true, p));
+    return LSPK_OK;
+}
+
+}  // namespace lspk

@@ -7,8 +7,7 @@ namespace lspk {
 // layout.cu: reference byte layout (device copy) -> device chunk layout, on the library stream.
 cudaError_t retile_to_device_launch(const uint8_t* src_dev, uint4* dst_dev, int N, int Kb, int groups, int chunks);
 
-// linear.cu: kernel parameters (filled by linear_cuda_core, or directly by the MoE layer for its
-// expert-grouped launches).
+// linear.cu: kernel parameters (filled by linear_cuda_core).
 struct LinearSeg {
     const uint4* w;
     float* out;
@@ -16,7 +15,6 @@ struct LinearSeg {
     int N;
     int groups;
     float w_scale;
-    int scale_idx;         // grouped mode: index of this matrix inside an expert's scale triple
 };
 
 // Internal prologue of the eight-row kernel: int8 rows already in its shared-memory layout (permuted 16-element
@@ -42,20 +40,12 @@ struct LinearParams {
     int8_t* xq_out;
     float* xscale_out;
     int stream_weights;    // 1: weights are read once by this launch -> evict-first loads
-    int bulk_stages;       // > 0 (expert-grouped launches of the eight-row kernel): weight ring of this many stages
     int* error_flag;       // set to LSPK_ERR_DEVICE_WAIT when a bounded wait of that variant runs out
     unsigned long long* trace;
     int trace_cap;
-    // ---- expert-grouped mode (blockIdx.z = expert): rows and their count come from device arrays ----
-    const int* grp_counts;     // [experts] rows routed to each expert
-    const int* grp_rows;       // [experts][grp_rows_stride] output row of each routed row
-    int grp_rows_stride;
-    int grp_in_shift;          // input row = output row >> shift (1: two routed rows share one input row)
-    size_t grp_w_stride;       // uint4 units between consecutive experts' copies of a matrix
-    const float* grp_scales;   // [experts][3] weight scales
 };
 
-// linear_mma.cu: the eight-row tile kernel (mma.sync int8), also used for expert-grouped launches.
+// linear_mma.cu: the eight-row tile kernel (mma.sync int8).
 // Quantise (and normalise) M > 1 rows once into caller scratch and turn the call into an int8-prologue one.
 int split_row_prologue(lspk_linear_args* a, int K, int8_t* q_scratch, float* scale_scratch);
 // Library-owned scratch for that (grown with cudaMalloc: size it once outside stream capture).
@@ -64,14 +54,15 @@ int quant_scratch(size_t M, size_t K, int8_t** q, float** s, int** sums = nullpt
 // quantise + permute); *done = 0 when the shape / alignment does not allow it.
 int quantize_rows_permuted(const lspk_linear_args* a, int K, int Kp, int8_t* out_perm, float* scales, int* done,
                            int stride = 0, int* sums = nullptr);
-// rows.cu: RMSNorm + quantiser of T rows, row t with the gamma_sel[t]-th bf16 weight vector.
+// rows.cu: RMSNorm + quantiser of T rows, row t with the gamma_sel[t]-th bf16 weight vector.  tiled_sums (K % 8 == 0):
+// rows in the eight-row tile's layout, and the sum of each.
 int norm_quant_rows_selected(const float* x, const void* gamma_bf16, const int* gamma_sel, int8_t* out, float* scales,
-                             int T, int K, float eps);
-int linear_mma_launch(const LinearParams& p, bool pair, bool grouped, int grid_x, int grid_y, int grid_z);
+                             int T, int K, float eps, int* tiled_sums = nullptr);
+int linear_mma_launch(const LinearParams& p, bool pair, int grid_x, int grid_y);
 __host__ __device__ inline int mma_row_stride(int Kp) { return (Kp % 128 == 0) ? Kp + 64 : Kp; }
 
 // Launch the CUDA-core kernel with fully prepared parameters.  mt: rows per CTA tile (1, 2, 4 or 8).
-int linear_launch_params(const LinearParams& p, int mt, bool pair, bool grouped, int grid_x, int grid_y, int grid_z);
+int linear_launch_params(const LinearParams& p, int mt, bool pair, int grid_x, int grid_y);
 
 // linear.cu: validate + launch the CUDA-core ternary linear kernel on the library stream.
 int linear_cuda_core(const lspk_linear_args* a);
@@ -156,9 +147,36 @@ struct StreamParams {
     int n;
     int total_units;
     int* error_flag;
+    int sel_ready;              // caller: the experts chosen by sel are final when the kernel starts (moe.cu)
     int wait_for_predecessor;   // the requesting warps may not start before the previous kernel has finished (sel)
 };
 // Launch the streamed batch described by p->it[0 .. p->n) on the library stream.
 int stream_launch(StreamParams* p);
+
+// Expert-grouped products of several routed rows (expert_stream.cu).  Routed row r (of R) belongs to expert sel[r], reads
+// input row r >> in_shift and writes row r of `out`; expert e's matrices are w[m] + e * w_stride, its scales
+// scales[3 * e + scale_idx[m]].  pair: out = relu(w0 x)^2 * (w1 x), else w0 x.
+struct ExpertStreamParams {
+    const uint4* w[2];
+    size_t w_stride;       // uint4 units
+    const float* scales;
+    int scale_idx[2];
+    const int8_t* x;       // x_sums: rows in the eight-row tile's layout (kProInt8Tiled), mma_row_stride apart; else natural
+    const float* xs;
+    const int* x_sums;     // with the tile layout: sum of each row's int8 values
+    int in_shift;
+    const int* sel;
+    int R, E;              // E <= 32
+    int sel_ready;         // sel is final when the kernel starts (see moe.cu)
+    float* out;
+    int32_t* acc[2];       // optional
+    int N, K, chunks, groups;
+    // ---- filled by expert_stream_launch ----
+    int slots, cps, sub;
+    int* error_flag;
+    unsigned long long* trace;
+    int trace_cap;
+};
+int expert_stream_launch(ExpertStreamParams p, bool pair);
 
 }  // namespace lspk

@@ -2,7 +2,7 @@
 // with the activation quantiser (and optionally the RMSNorm in front of it) fused in as a prologue and
 // the residual add / ReLU^2 gate fused as epilogue.  The kernel is written for MT token rows per CTA
 // tile; only MT = 1 (the decode GEMV) is instantiated: two and more rows go to the tensor-core kernels
-// (linear_mma.cu, gemm_tc.cu), expert-grouped launches to linear_mma.cu.
+// (linear_mma.cu, gemm_tc.cu).
 //
 // Replaces matmul_lut_avx512_m1 / _mT (matmul_lut_avx512_extern_c.cpp:150-236, 258-339) and,
 // through the prologue / epilogue switches, quantize_activation (:425-466),
@@ -49,9 +49,7 @@ __device__ __forceinline__ float cta8_max_nonneg(float v, float* slot) {
 // NI      16-byte weight loads per lane per batch (covers K <= 4096 at 4, K <= 8192 at 8 in one batch)
 // NB      16-element activation blocks a thread owns in the fp32 prologue (K <= 4096 * NB)
 // PAIR    gate/up pairing (two weight streams, gated epilogue)
-// GROUPED expert-grouped launch: blockIdx.z is the expert; its row list and row count are read from
-//         device arrays, its weights and scales are found by stride (packed-expert MoE GEMV)
-template <int MT, int NI, int NB, bool PAIR, bool GROUPED>
+template <int MT, int NI, int NB, bool PAIR>
 #ifdef LSPK_LINEAR_MIN_BLOCKS
 __global__ void __launch_bounds__(kThreads, LSPK_LINEAR_MIN_BLOCKS)
 #else
@@ -69,8 +67,6 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
     float* redf = reinterpret_cast<float*>(part + kPartInts);          // [32] reduction scratch
     float* s_scale = redf + 32;                                        // [MT]
     int* s_sumx = reinterpret_cast<int*>(s_scale + MT);                // [MT][warps] partial sums of x
-    const int z = GROUPED ? blockIdx.z : 0;
-    const size_t w_off = GROUPED ? (size_t)z * p.grp_w_stride : 0;
 
     // ---- row groups of this CTA: blockIdx.x, blockIdx.x + gridDim.x, ... (flat over the segments) ----
     auto locate = [&](int flat, int& seg_i, int& grp) {
@@ -84,8 +80,8 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
         }
     };
     auto load_batch = [&](int seg_i, int grp, int base, uint4* dst_a, uint4* dst_b) {
-        const uint4* wa_base = p.seg[seg_i].w + w_off + (size_t)grp * p.chunks * kRowsPerGroup + r;
-        const uint4* wb_base = PAIR ? (p.seg[1].w + w_off + (size_t)grp * p.chunks * kRowsPerGroup + r) : nullptr;
+        const uint4* wa_base = p.seg[seg_i].w + (size_t)grp * p.chunks * kRowsPerGroup + r;
+        const uint4* wb_base = PAIR ? (p.seg[1].w + (size_t)grp * p.chunks * kRowsPerGroup + r) : nullptr;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
             const int j = 2 * (warp + kWarps * (base + i)) + h;
@@ -114,11 +110,10 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
     locate(flat0, s0, g0);
 
     // ---- everything that does not depend on the previous kernel is requested first: the first
-    //      batch of packed weights and the norm weights (neither is written by the forward pass).
-    //      An expert-grouped launch cannot: whether this expert has any row is device data. ----
+    //      batch of packed weights and the norm weights (neither is written by the forward pass). ----
     uint4 wa[NI], wb[PAIR ? NI : 1];
     uint4 na[NI], nb_[PAIR ? NI : 1];                // the next row group's first batch
-    if (!GROUPED) load_batch(s0, g0, 0, wa, wb);
+    load_batch(s0, g0, 0, wa, wb);
     float gm[NB][16];
     if (normed) {
 #pragma unroll
@@ -150,30 +145,21 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
     grid_dependency_wait();
     tr.mark();                                   // 1: predecessor finished
 
-    const int M_eff = GROUPED ? p.grp_counts[z] : p.M;
-    const int* rows = GROUPED ? p.grp_rows + (size_t)z * p.grp_rows_stride : nullptr;
     const int out_m = tid >> 4, out_r = tid & 15;
     const int tail_start = p.K & ~15;      // the reference's scalar-tail rounding rule applies from here
-    bool first_tile = true;
 
-    // Plain launches give every row tile its own CTA (grid.y), so this loop runs once for them (and the
-    // compiler is told so: register lifetimes end with the single pass); expert-grouped launches, whose
-    // row count is device data, walk their tiles here.
-    for (int m0 = blockIdx.y * MT; m0 < M_eff; m0 += gridDim.y * MT) {
-        const int mt = min(MT, M_eff - m0);
-        auto out_row = [&](int m) -> int { return GROUPED ? rows[m0 + m] : m0 + m; };
-        auto in_row = [&](int m) -> int { return GROUPED ? (rows[m0 + m] >> p.grp_in_shift) : m0 + m; };
+    {
+        const int m0 = blockIdx.y * MT;            // the grid covers every tile of rows
+        const int mt = min(MT, p.M - m0);
         int flat = flat0, s = s0, g = g0;
         // residual value of this thread's output element (ADD epilogue), requested as early as possible
         auto residual_of = [&](int seg_i, int grp) -> float {
             if (p.epilogue != LSPK_EPI_ADD || tid >= MT * 16 || out_m >= mt) return 0.0f;
             const int n = grp * kRowsPerGroup + out_r;
             if (n >= p.seg[seg_i].N) return 0.0f;
-            return p.seg[seg_i].out[(size_t)out_row(out_m) * p.seg[seg_i].N + n];
+            return p.seg[seg_i].out[(size_t)(m0 + out_m) * p.seg[seg_i].N + n];
         };
         float resid = residual_of(s, g);
-        if (GROUPED || !first_tile) load_batch(s, g, 0, wa, wb);
-        first_tile = false;
 
         // ---- prologue: this tile's activations -> permuted int8 rows in shared memory ---------------
         for (int m = 0; m < mt; ++m) {
@@ -181,7 +167,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
             int sumx = 0;
             float scale = 1.0f;
             if (!fp32_in) {
-                const int8_t* src = p.x_i8 + (size_t)in_row(m) * p.K;
+                const int8_t* src = p.x_i8 + (size_t)(m0 + m) * p.K;
                 for (int b = tid; b < Kp / 16; b += kThreads) {
                     uint32_t a[4];
 #pragma unroll
@@ -194,10 +180,10 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                     transpose4x4_bytes(a[0], a[1], a[2], a[3], o0, o1, o2, o3);
                     *reinterpret_cast<uint4*>(xq_row + b * 16) = make_uint4(o0, o1, o2, o3);
                 }
-                scale = p.x_scales[in_row(m)];
+                scale = p.x_scales[(m0 + m)];
             } else {
                 // every thread keeps its 16-element blocks in registers through all three passes
-                const float* src = p.x_f32 + (size_t)in_row(m) * p.K;
+                const float* src = p.x_f32 + (size_t)(m0 + m) * p.K;
                 float v[NB][16];
                 float ssq = 0.0f;
 #pragma unroll
@@ -215,7 +201,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                 }
                 if (p.prologue == LSPK_PRO_GATED_RMSNORM_QUANT) {
                     // v = x * SiLU(gate), SiLU(g) = g / (1 + exp(-g)); each step a single rounding
-                    const float* gsrc = p.gate_f32 + (size_t)in_row(m) * p.K;
+                    const float* gsrc = p.gate_f32 + (size_t)(m0 + m) * p.K;
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb) {
                         const int k0 = (tid + nb * kThreads) * 16;
@@ -282,7 +268,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                             if (tap) {
 #pragma unroll
                                 for (int q = 0; q < 4; ++q)
-                                    *reinterpret_cast<uint32_t*>(p.xq_out + (size_t)out_row(m) * p.K + k0 + q * 4) =
+                                    *reinterpret_cast<uint32_t*>(p.xq_out + (size_t)(m0 + m) * p.K + k0 + q * 4) =
                                         pack4_bytes(t[q * 4], t[q * 4 + 1], t[q * 4 + 2], t[q * 4 + 3]);
                             }
                         } else {
@@ -305,7 +291,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                                 }
                                 a[q] = word;
                                 if (tap && k0 + q * 4 < p.K)
-                                    *reinterpret_cast<uint32_t*>(p.xq_out + (size_t)out_row(m) * p.K + k0 + q * 4) = word;
+                                    *reinterpret_cast<uint32_t*>(p.xq_out + (size_t)(m0 + m) * p.K + k0 + q * 4) = word;
                             }
                             transpose4x4_bytes(a[0], a[1], a[2], a[3], o0, o1, o2, o3);
                         }
@@ -322,7 +308,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
             if (lane == 0) s_sumx[m * kWarps + warp] = sumx;
             if (tid == 0) {
                 s_scale[m] = scale;
-                if (p.xscale_out && blockIdx.x == 0) p.xscale_out[out_row(m)] = scale;
+                if (p.xscale_out && blockIdx.x == 0) p.xscale_out[m0 + m] = scale;
             }
         }
         tr.mark();                                   // 6: quantised rows written
@@ -396,14 +382,14 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                         sx += s_sumx[out_m * kWarps + w];
                     }
                     va -= sx;
-                    const size_t o = (size_t)out_row(out_m) * sg.N + n;
+                    const size_t o = (size_t)(m0 + out_m) * sg.N + n;
                     if (sg.acc_out) sg.acc_out[o] = va;
-                    const float wsa = GROUPED ? p.grp_scales[z * 3 + sg.scale_idx] : sg.w_scale;
+                    const float wsa = sg.w_scale;
                     const float ya = __fmul_rn((float)va, __fmul_rn(s_scale[out_m], wsa));
                     if (PAIR) {
                         vb -= sx;
                         if (p.seg[1].acc_out) p.seg[1].acc_out[o] = vb;
-                        const float wsb = GROUPED ? p.grp_scales[z * 3 + p.seg[1].scale_idx] : p.seg[1].w_scale;
+                        const float wsb = p.seg[1].w_scale;
                         const float yb = __fmul_rn((float)vb, __fmul_rn(s_scale[out_m], wsb));
                         if (p.epilogue == LSPK_EPI_SILU_MUL) {
                             // the reference's Falcon gate (runtime.py:726-732): g / (1 + exp(-g)) * u
@@ -436,7 +422,6 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                 load_batch(s, g, 0, wa, wb);
             }
         }
-        if (!GROUPED) break;
     }
     tr.end();
 }
@@ -447,10 +432,10 @@ static size_t linear_smem_bytes(int MT, int Kp, bool pair) {
     b += 32 * 4 + MT * 4 + MT * kWarps * 4;
     return b;
 }
-template <int MT, int NI, int NB, bool PAIR, bool GROUPED>
+template <int MT, int NI, int NB, bool PAIR>
 static cudaError_t launch_linear(const LinearParams& p, dim3 grid, size_t smem) {
     static bool attr_set = false;
-    auto kern = ternary_linear_kernel<MT, NI, NB, PAIR, GROUPED>;
+    auto kern = ternary_linear_kernel<MT, NI, NB, PAIR>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
@@ -462,19 +447,19 @@ static cudaError_t launch_linear(const LinearParams& p, dim3 grid, size_t smem) 
 template <int MT>
 static cudaError_t launch_linear_mt(const LinearParams& p, dim3 grid, bool pair, size_t smem) {
     if (p.chunks <= 64)
-        return pair ? launch_linear<MT, 4, 1, true, false>(p, grid, smem) : launch_linear<MT, 4, 1, false, false>(p, grid, smem);
+        return pair ? launch_linear<MT, 4, 1, true>(p, grid, smem) : launch_linear<MT, 4, 1, false>(p, grid, smem);
     if (p.chunks <= 128)
-        return pair ? launch_linear<MT, 8, 2, true, false>(p, grid, smem) : launch_linear<MT, 8, 2, false, false>(p, grid, smem);
-    return pair ? launch_linear<MT, 8, 8, true, false>(p, grid, smem) : launch_linear<MT, 8, 8, false, false>(p, grid, smem);
+        return pair ? launch_linear<MT, 8, 2, true>(p, grid, smem) : launch_linear<MT, 8, 2, false>(p, grid, smem);
+    return pair ? launch_linear<MT, 8, 8, true>(p, grid, smem) : launch_linear<MT, 8, 8, false>(p, grid, smem);
 }
 
-int linear_launch_params(const LinearParams& p, int mt, bool pair, bool grouped, int grid_x, int grid_y, int grid_z) {
-    // more than one token row per tile (and every expert-grouped launch): the eight-row mma kernel
-    if (mt > 1 || grouped) return linear_mma_launch(p, pair, grouped, grid_x, grid_y, grid_z);
+int linear_launch_params(const LinearParams& p, int mt, bool pair, int grid_x, int grid_y) {
+    // more than one token row per tile: the eight-row mma kernel
+    if (mt > 1) return linear_mma_launch(p, pair, grid_x, grid_y);
     const int Kp = p.chunks * kWeightsPerChunk;
     const size_t smem = linear_smem_bytes(1, Kp, pair);
     LSPK_REQUIRE(smem <= 200 * 1024 && p.chunks <= 512, "linear: K=%d too large (limit 32768)", p.K);
-    const dim3 grid(grid_x, grid_y, grid_z);
+    const dim3 grid(grid_x, grid_y);
     const cudaError_t e = launch_linear_mt<1>(p, grid, pair, smem);
     if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "linear launch failed: %s", cudaGetErrorString(e));
     return LSPK_OK;
@@ -538,7 +523,7 @@ int linear_cuda_core(const lspk_linear_args* a) {
         LSPK_REQUIRE(w && w->K == p.K, "linear: matrices must share K");
         LSPK_REQUIRE(pair ? (i == 1 || a->out[i] != nullptr) : a->out[i] != nullptr, "linear: null output");
         LSPK_REQUIRE(!pair || w->N == w0->N, "linear: gate and up must have the same N");
-        p.seg[i] = LinearSeg{w->dev, a->out[i], a->acc_out[i], w->N, w->groups, w->scale, i};
+        p.seg[i] = LinearSeg{w->dev, a->out[i], a->acc_out[i], w->N, w->groups, w->scale};
         groups += w->groups;
     }
     if (pair) groups = w0->groups;
@@ -589,7 +574,7 @@ int linear_cuda_core(const lspk_linear_args* a) {
     int ctas = groups;
     const int per_wave = tiles == 1 ? 2 * sm_count() : (2 * sm_count() + tiles - 1) / tiles;
     if (ctas > per_wave) ctas = per_wave > 0 ? per_wave : 1;
-    return linear_launch_params(p, MT, pair, false, ctas, tiles, 1);
+    return linear_launch_params(p, MT, pair, ctas, tiles);
 }
 
 }  // namespace lspk

@@ -4,7 +4,7 @@
 // count the one-token kernel spends on one.  Same contract and epilogues as
 // ternary_linear_kernel in linear.cu (matmul_lut_avx512_mT, matmul_lut_avx512_extern_c.cpp:258-339,
 // plus the fused helpers); this is the path of the small batches: speculative validation, several
-// sequences decoded in lock step, the rows an expert receives in the MoE layer.
+// sequences decoded in lock step.  (The rows an expert receives in the MoE layer: expert_stream.cu.)
 //
 // Operand mapping (no re-layout: the device chunk layout is read as is).  The 256-byte tile of
 // "16 rows x one 64-weight chunk" is 64 words; lane l of a warp loads word l (row l/4, the
@@ -40,13 +40,6 @@ __device__ __forceinline__ void mma_u8s8(int c[4], uint32_t a0, uint32_t a1, uin
 // consecutive rows start 64 bytes apart modulo 128, which makes the quarter-warp 16-byte loads (two tokens x
 // four words) conflict-free.
 
-// BULK: the packed weights of the CTA's row groups arrive in a shared-memory ring by bulk asynchronous copies
-// (one thread requests up to p.bulk_stages groups ahead, each a contiguous block of the device layout) instead of
-// per-lane register loads.  For launches that stream tens of megabytes (the expert-grouped MoE products): the
-// bytes in flight per SM then do not depend on registers or on where the CTA is in its reduction.
-constexpr int kMBulkStages = 4;
-constexpr int kMIssuers = 4;                          // warps whose lane 0 requests a quarter of each stage
-constexpr unsigned kMBulkSpinLimit = 1u << 22;
 // Pre-tiled int8 rows (the row quantiser's output, already in the tile's layout) arrive by bulk copies in
 // segments of 16 chunks along K, one mbarrier per segment, so the MMAs of the first segment start while the
 // later ones are still on their way; every wait on a segment ends at a clock deadline.
@@ -55,7 +48,7 @@ constexpr int kMXSegMax = 24;                        // covers K up to 24576
 constexpr long long kMXWaitCycles = 1ll << 31;
 static_assert(kMWarps == kMT && kMXSegMax <= 32, "row staging maps warp -> row and lane -> segment");
 
-template <bool PAIR, bool GROUPED, bool BULK>
+template <bool PAIR>
 __global__ void __launch_bounds__(kMThreads)
 ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -69,15 +62,6 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     constexpr int kPartInts = kMWarps * kMT * 16 * (PAIR ? 2 : 1);
     float* s_scale = reinterpret_cast<float*>(part + kPartInts);               // [kMT]
     int* s_sumx = reinterpret_cast<int*>(s_scale + kMT);                       // [kMT]
-    unsigned char* ring_base = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(s_sumx + kMT) + 127) & ~uintptr_t(127));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(ring_base);                   // [kMBulkStages]
-    uint32_t* ring = reinterpret_cast<uint32_t*>(ring_base + 128);             // [stages][PAIR?2:1][chunks*64 words]
-    const int grp_words = p.chunks * 64;
-    const int stage_words = grp_words * (PAIR ? 2 : 1);
-
-    const int z = GROUPED ? blockIdx.z : 0;
-    const size_t w_off = GROUPED ? (size_t)z * p.grp_w_stride : 0;
     const int pairs = (p.chunks + 1) / 2;
 
     auto locate = [&](int flat, int& seg_i, int& grp) {
@@ -93,8 +77,8 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     // weights of chunk pair (warp + 8*(base+i)) of a row group: for each of the two chunks the words of
     // row gid and of row gid+8 -> 4 words per pair (8 with the gate/up pairing)
     auto load_batch = [&](int seg_i, int grp, int base, uint32_t (*dst_a)[4], uint32_t (*dst_b)[4]) {
-        const uint32_t* wa = reinterpret_cast<const uint32_t*>(p.seg[seg_i].w + w_off + (size_t)grp * p.chunks * kRowsPerGroup);
-        const uint32_t* wb = PAIR ? reinterpret_cast<const uint32_t*>(p.seg[1].w + w_off + (size_t)grp * p.chunks * kRowsPerGroup)
+        const uint32_t* wa = reinterpret_cast<const uint32_t*>(p.seg[seg_i].w + (size_t)grp * p.chunks * kRowsPerGroup);
+        const uint32_t* wb = PAIR ? reinterpret_cast<const uint32_t*>(p.seg[1].w + (size_t)grp * p.chunks * kRowsPerGroup)
                                   : nullptr;
 #pragma unroll
         for (int i = 0; i < kMNI; ++i) {
@@ -131,11 +115,11 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     PhaseTrace tr;
     tr.begin(p.trace, p.trace_cap, 3);
     tr.mark();                                          // 0: entry
-    if (!GROUPED && !BULK) load_batch(s0, g0, 0, wa, wb);       // weights never depend on the previous kernel
+    load_batch(s0, g0, 0, wa, wb);                      // weights never depend on the previous kernel
     __shared__ __align__(8) uint64_t xbars[kMXSegMax];
     const int nxseg = (p.chunks + kMXSegChunks - 1) / kMXSegChunks;
     // CTA-uniform: a full tile of pre-tiled rows, one token tile per CTA
-    const bool x_async = !GROUPED && !BULK && p.prologue == kProInt8Tiled && nxseg <= kMXSegMax &&
+    const bool x_async = p.prologue == kProInt8Tiled && nxseg <= kMXSegMax &&
                          p.M - (int)blockIdx.y * kMT >= kMT;
     if (x_async) {
         if (tid < nxseg) {
@@ -148,60 +132,20 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     grid_dependency_wait();
     tr.mark();                                          // 1: predecessor finished
 
-    const int M_eff = GROUPED ? p.grp_counts[z] : p.M;
-    const int* rows = GROUPED ? p.grp_rows + (size_t)z * p.grp_rows_stride : nullptr;
     const int out_m = tid >> 4, out_r = tid & 15;
-    bool first_tile = true;
-
-    // BULK: the CTA's work as one sequence: for every token tile, every row group of this CTA
-    const int ngrp_cta = (int)blockIdx.x < p.total_groups ? (p.total_groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const int tile_step = (int)gridDim.y * kMT;
-    const int ntile_cta = M_eff > (int)blockIdx.y * kMT ? (M_eff - 1 - (int)blockIdx.y * kMT) / tile_step + 1 : 0;
-    const int total_it = BULK ? ngrp_cta * ntile_cta : 0;
-    // Request part `part` (of kMIssuers equal pieces) of sequence element it_ into its stage.  The pieces of a stage
-    // are requested by different warps: one thread gets a bulk copy out only every few hundred cycles, which would
-    // otherwise sit on the CTA's critical path once per row group.
-    auto issue_it = [&](int it_, int part) {
-        int ss, gg;
-        locate((int)blockIdx.x + (it_ % ngrp_cta) * (int)gridDim.x, ss, gg);
-        const int st = it_ % p.bulk_stages;
-        const uint32_t bytes = (uint32_t)grp_words * 4u / kMIssuers;             // chunks * 64: a multiple of 16
-        uint32_t* dst = ring + (size_t)st * stage_words + (size_t)part * (bytes / 4u);
-        mbar_expect_tx(&bars[st], bytes * (PAIR ? 2u : 1u));
-        const uint4* src_a = p.seg[ss].w + w_off + (size_t)gg * p.chunks * kRowsPerGroup + (size_t)part * (bytes / 16u);
-        bulk_load_stream(dst, src_a, bytes, &bars[st]);
-        if (PAIR)
-            bulk_load_stream(dst + grp_words,
-                             p.seg[1].w + w_off + (size_t)gg * p.chunks * kRowsPerGroup + (size_t)part * (bytes / 16u), bytes,
-                             &bars[st]);
-    };
-    int it = 0;
     int wait_failed = 0;
     bool give_up = false;                              // CTA-uniform: a bounded wait ran out somewhere in the CTA
-    if (BULK) {
-        if (tid == 0) {
-            for (int st = 0; st < p.bulk_stages; ++st) mbar_init(&bars[st], kMIssuers);
-            fence_mbar_init();
-            for (int i = 0; i < p.bulk_stages && i < total_it; ++i)
-                for (int part = 0; part < kMIssuers; ++part) issue_it(i, part);
-        }
-        // the barriers are used after the __syncthreads that follows the prologue of the first tile
-    }
-
-    for (int m0 = blockIdx.y * kMT; m0 < M_eff; m0 += gridDim.y * kMT) {
-        const int mt = min(kMT, M_eff - m0);
-        auto out_row = [&](int m) -> int { return GROUPED ? rows[m0 + m] : m0 + m; };
-        auto in_row = [&](int m) -> int { return GROUPED ? (rows[m0 + m] >> p.grp_in_shift) : m0 + m; };
+    {
+        const int m0 = blockIdx.y * kMT;                // the grid covers every tile of rows
+        const int mt = min(kMT, p.M - m0);
         int flat = flat0, s = s0, g = g0;
         auto residual_of = [&](int seg_i, int grp) -> float {
             if (p.epilogue != LSPK_EPI_ADD || tid >= kMT * 16 || out_m >= mt) return 0.0f;
             const int n = grp * kRowsPerGroup + out_r;
             if (n >= p.seg[seg_i].N) return 0.0f;
-            return p.seg[seg_i].out[(size_t)out_row(out_m) * p.seg[seg_i].N + n];
+            return p.seg[seg_i].out[(size_t)(m0 + out_m) * p.seg[seg_i].N + n];
         };
-        float resid = BULK ? 0.0f : residual_of(s, g);
-        if (!BULK && (GROUPED || !first_tile)) load_batch(s, g, 0, wa, wb);
-        first_tile = false;
+        float resid = residual_of(s, g);
 
         // ---- prologue: the tile's rows -> permuted int8 rows in shared memory ------------------------------
         if (x_async) {
@@ -238,7 +182,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                 for (int b = lane; b < nblk; b += 32) *reinterpret_cast<uint4*>(xq_row + b * 16) = make_uint4(0, 0, 0, 0);
                 if (lane == 0) { s_scale[m] = 0.0f; s_sumx[m] = 0; }
             } else {
-                const int8_t* src = p.x_i8 + (size_t)in_row(m) * p.K;
+                const int8_t* src = p.x_i8 + (size_t)(m0 + m) * p.K;
                 int sumx = 0;
                 if ((p.K & 15) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
                     // whole 16-element blocks, 16-byte aligned: one load per block, four blocks in flight per lane
@@ -272,7 +216,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                     }
                 }
                 sumx = warp_sum(sumx);
-                if (lane == 0) { s_scale[m] = p.x_scales[in_row(m)]; s_sumx[m] = sumx; }
+                if (lane == 0) { s_scale[m] = p.x_scales[m0 + m]; s_sumx[m] = sumx; }
             }
         }
         tr.mark();                                                 // 2: rows staged (or requested)
@@ -300,39 +244,6 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                     if (PAIR) acc_b[f][c] = 0;
                 }
             const int8_t* xrow = xq + (size_t)gid * rs;            // B operand: token gid
-            if (BULK) {
-                const int st = it % p.bulk_stages;
-                const uint32_t parity = (uint32_t)(it / p.bulk_stages) & 1u;
-                bool arrived = false;
-                for (unsigned i = 0; i < kMBulkSpinLimit && !arrived; ++i) arrived = mbar_try_wait(&bars[st], parity);
-                wait_failed |= arrived ? 0 : 1;
-                const uint32_t* sa = ring + (size_t)st * stage_words + lane;
-#pragma unroll 2
-                for (int pr = warp; pr < pairs; pr += kMWarps) {
-                    const int j0 = 2 * pr;
-                    const bool two = j0 + 1 < p.chunks;
-                    const uint4 x0 = *reinterpret_cast<const uint4*>(xrow + (size_t)(4 * j0 + t4) * 16);
-                    uint4 x1 = make_uint4(0, 0, 0, 0);
-                    if (two) x1 = *reinterpret_cast<const uint4*>(xrow + (size_t)(4 * (j0 + 1) + t4) * 16);
-                    const uint32_t xb0[4] = {x0.x, x0.y, x0.z, x0.w};
-                    const uint32_t xb1[4] = {x1.x, x1.y, x1.z, x1.w};
-                    const uint32_t a0 = sa[j0 * 64], a1 = sa[j0 * 64 + 32];
-                    const uint32_t a2 = two ? sa[(j0 + 1) * 64] : 0x55555555u, a3 = two ? sa[(j0 + 1) * 64 + 32] : 0x55555555u;
-                    uint32_t b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-                    if (PAIR) {
-                        b0 = sa[grp_words + j0 * 64];
-                        b1 = sa[grp_words + j0 * 64 + 32];
-                        b2 = two ? sa[grp_words + (j0 + 1) * 64] : 0x55555555u;
-                        b3 = two ? sa[grp_words + (j0 + 1) * 64 + 32] : 0x55555555u;
-                    }
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) {
-                        const uint32_t mask = 0x03030303u << (2 * f);
-                        mma_u8s8(acc_a[f], a0 & mask, a1 & mask, a2 & mask, a3 & mask, xb0[f], xb1[f]);
-                        if (PAIR) mma_u8s8(acc_b[f], b0 & mask, b1 & mask, b2 & mask, b3 & mask, xb0[f], xb1[f]);
-                    }
-                }
-            } else
             for (int base = 0;; ) {
 #pragma unroll
                 for (int i = 0; i < kMNI; ++i) {
@@ -369,7 +280,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                 load_batch(s, g, base, wa, wb);
             }
             tr.mark();                                             // 4+: MMAs of a row group done
-            if (!BULK && has_next) load_batch(ns, ng, 0, wa, wb);  // in flight during the reduction below
+            if (has_next) load_batch(ns, ng, 0, wa, wb);  // in flight during the reduction below
 
             // masks -> one int; C fragment: c0,c1 = (row gid, tokens 2*t4, 2*t4+1), c2,c3 = (row gid+8, same)
 #pragma unroll
@@ -383,24 +294,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                     part[kMWarps * kMT * 16 + (warp * kMT + tok) * 16 + row] = u;
                 }
             }
-            if (BULK) {
-                // every warp is done with this stage: request the element bulk_stages ahead into it.  A wait that
-                // ran out ends the CTA once its outstanding copies (bounded wait again) have landed.
-                if (__syncthreads_or(wait_failed)) {
-                    if (tid == 0) {
-                        if (p.error_flag) atomicExch(p.error_flag, LSPK_ERR_DEVICE_WAIT);
-                        for (int k = it + 1; k < it + p.bulk_stages && k < total_it; ++k) {
-                            bool done = false;
-                            for (unsigned i = 0; i < kMBulkSpinLimit && !done; ++i)
-                                done = mbar_try_wait(&bars[k % p.bulk_stages], (uint32_t)(k / p.bulk_stages) & 1u);
-                        }
-                    }
-                    give_up = true;
-                } else {
-                    if (lane == 0 && warp < kMIssuers && it + p.bulk_stages < total_it) issue_it(it + p.bulk_stages, warp);
-                    ++it;
-                }
-            } else if (x_pending) {
+            if (x_pending) {
                 x_pending = false;
                 if (__syncthreads_or(wait_failed)) {
                     // a segment never arrived: report, give the copies in flight one more bounded wait, leave
@@ -429,14 +323,14 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                     }
                     const int sx = s_sumx[out_m];
                     va -= sx;
-                    const size_t o = (size_t)out_row(out_m) * sg.N + n;
+                    const size_t o = (size_t)(m0 + out_m) * sg.N + n;
                     if (sg.acc_out) sg.acc_out[o] = va;
-                    const float wsa = GROUPED ? p.grp_scales[z * 3 + sg.scale_idx] : sg.w_scale;
+                    const float wsa = sg.w_scale;
                     const float ya = __fmul_rn((float)va, __fmul_rn(s_scale[out_m], wsa));
                     if (PAIR) {
                         vb -= sx;
                         if (p.seg[1].acc_out) p.seg[1].acc_out[o] = vb;
-                        const float wsb = GROUPED ? p.grp_scales[z * 3 + p.seg[1].scale_idx] : p.seg[1].w_scale;
+                        const float wsb = p.seg[1].w_scale;
                         const float yb = __fmul_rn((float)vb, __fmul_rn(s_scale[out_m], wsb));
                         if (p.epilogue == LSPK_EPI_SILU_MUL) {
                             sg.out[o] = __fmul_rn(__fdiv_rn(ya, __fadd_rn(expf(-ya), 1.0f)), yb);
@@ -445,7 +339,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                             sg.out[o] = __fmul_rn(__fmul_rn(gpos, gpos), yb);
                         }
                     } else if (p.epilogue == LSPK_EPI_ADD) {
-                        sg.out[o] = __fadd_rn(BULK ? sg.out[o] : resid, ya);
+                        sg.out[o] = __fadd_rn(resid, ya);
                     } else {
                         sg.out[o] = ya;
                     }
@@ -459,16 +353,14 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
             g = ng;
             resid = next_resid;
         }
-        if (give_up) break;
-        if (!GROUPED) break;
     }
     tr.end();
 }
 
-template <bool PAIR, bool GROUPED, bool BULK = false>
+template <bool PAIR>
 static cudaError_t launch_mma(const LinearParams& p, dim3 grid, size_t smem) {
     static bool attr_set = false;
-    auto kern = ternary_linear_mma_kernel<PAIR, GROUPED, BULK>;
+    auto kern = ternary_linear_mma_kernel<PAIR>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
@@ -479,24 +371,14 @@ static cudaError_t launch_mma(const LinearParams& p, dim3 grid, size_t smem) {
 
 // Launch the eight-row kernel.  K is limited by the shared-memory activation tile (8 rows of K bytes).
 // Rows arrive quantised (INT8 prologue); fp32 rows are quantised once by the row kernel beforehand.
-int linear_mma_launch(const LinearParams& p, bool pair, bool grouped, int grid_x, int grid_y, int grid_z) {
-    LSPK_REQUIRE(p.prologue == LSPK_PRO_INT8 || (p.prologue == kProInt8Tiled && !grouped),
+int linear_mma_launch(const LinearParams& p, bool pair, int grid_x, int grid_y) {
+    LSPK_REQUIRE(p.prologue == LSPK_PRO_INT8 || p.prologue == kProInt8Tiled,
                  "linear: the eight-row kernel takes int8 rows (prologue %d)", p.prologue);
     const int Kp = p.chunks * kWeightsPerChunk;
     size_t smem = (size_t)kMT * mma_row_stride(Kp) + (size_t)kMWarps * kMT * 16 * (pair ? 2 : 1) * 4 + kMT * 8 + 64;
     LSPK_REQUIRE(smem <= 200 * 1024, "linear: K=%d too large for the 8-row activation tile (limit about 24000)", p.K);
-    const dim3 grid(grid_x, grid_y, grid_z);
-    if (p.bulk_stages > 0) {
-        // expert-grouped launches only (set by the MoE layer): ring behind the tile
-        LSPK_REQUIRE(grouped && p.bulk_stages <= kMBulkStages, "linear (mma): bulk ring is for expert-grouped launches");
-        smem += 256 + (size_t)p.bulk_stages * p.chunks * 256 * (pair ? 2 : 1);
-        LSPK_REQUIRE(smem <= 200 * 1024, "linear (mma): bulk ring too large");
-        cudaError_t e = pair ? launch_mma<true, true, true>(p, grid, smem) : launch_mma<false, true, true>(p, grid, smem);
-        if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "linear (mma, bulk) launch failed: %s", cudaGetErrorString(e));
-        return LSPK_OK;
-    }
-    cudaError_t e = grouped ? (pair ? launch_mma<true, true>(p, grid, smem) : launch_mma<false, true>(p, grid, smem))
-                            : (pair ? launch_mma<true, false>(p, grid, smem) : launch_mma<false, false>(p, grid, smem));
+    const dim3 grid(grid_x, grid_y);
+    cudaError_t e = pair ? launch_mma<true>(p, grid, smem) : launch_mma<false>(p, grid, smem);
     if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "linear (mma) launch failed: %s", cudaGetErrorString(e));
     return LSPK_OK;
 }

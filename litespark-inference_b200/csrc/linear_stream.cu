@@ -304,7 +304,7 @@ int stream_launch(StreamParams* p) {
         it.sub = (it.chunks + it.cps - 1) / it.cps;
         unit0 += it.groups;
         q0 += it.groups * it.sub;
-        if (it.sel) p->wait_for_predecessor = 1;
+        if (it.sel && !p->sel_ready) p->wait_for_predecessor = 1;
     }
     p->total_units = unit0;
     static bool attr_set = false;

@@ -7,11 +7,10 @@
 //
 // Kernel sequence (all on the library stream, no host synchronisation):
 //   moe_router_kernel        one CTA per token: norm, quantise, router logits, softmax, top-2
-//   moe_group_kernel         rows (token, slot) listed per expert, ascending (more than one token;
-//                            the router kernel lists a single token's two rows itself)
-//   ternary_linear_mma_kernel expert-grouped launch, gate/up pair, ReLU^2 epilogue  (grid.z = expert)
+//   gate / up pair, ReLU^2   every chosen expert's matrices streamed past its rows: expert_stream.cu
+//                            (a single token: the streamed batch of linear_stream.cu)
 //   row_norm_quant_kernel    per routed row: RMSNorm with the row's expert's weights + quantiser
-//   ternary_linear_mma_kernel expert-grouped launch, down projection
+//   down                     as gate / up; its weights are requested under the quantiser
 //   moe_combine_kernel       x += w_0 y_0 + w_1 y_1
 // The expert matrices live in one device buffer [expert][gate|up|down] in the device chunk layout;
 // an expert with no routed row costs no weight traffic.
@@ -40,20 +39,21 @@ struct Moe {
     int cap_B = 0;
     int8_t *xq = nullptr, *xq2 = nullptr;
     float *xs = nullptr, *xs2 = nullptr, *selw = nullptr, *inter = nullptr, *ydown = nullptr;
-    int *sel = nullptr, *counts = nullptr, *rows = nullptr;
+    int *sel = nullptr, *sums = nullptr, *sums2 = nullptr;
     size_t bytes = 0;
 };
 
 // One CTA per token row: RMSNorm, quantiser, router logits (one warp per expert, round-robin), softmax
-// and top-2 inside warp 0.  With a single token (gridDim.x == 1) the per-expert row lists are written
-// here as well, which saves the grouping kernel.  H is a multiple of 4 (checked at creation).
+// and top-2 inside warp 0.  TILED (several tokens): int8 rows in the eight-row tile's layout, with their sums.  H is a multiple of 4 (checked at creation).
+template <bool TILED>
 __global__ void __launch_bounds__(kMoeThreads)
 moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamma, const float* __restrict__ router,
                   int8_t* __restrict__ xq, float* __restrict__ xs, int* __restrict__ sel, float* __restrict__ selw,
-                  int* __restrict__ counts, int* __restrict__ rows, int rows_stride, int H, int E, float eps) {
+                  int* __restrict__ sums, int H, int E, float eps) {
     extern __shared__ __align__(16) float hs[];           // [H] normalised row
     __shared__ __align__(16) float red[16];
     __shared__ float s_logit[kMaxExperts];
+    __shared__ int s_sum[kMoeThreads / 32];
     grid_dependency_launch();
     grid_dependency_wait();
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -98,8 +98,7 @@ moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamm
     const float scale = quant_scale_from_absmax(amax);
     const float inv = rcp_rn(scale);
     const int tail_start = H & ~15;
-    uint32_t* xq4 = reinterpret_cast<uint32_t*>(xq + (size_t)t * H);
-    for (int i = tid; i < H4; i += kMoeThreads) {
+    auto quant4 = [&](int i) -> uint32_t {
         const float4 v = hs4[i];
         const float f[4] = {v.x, v.y, v.z, v.w};
         uint32_t word = 0;
@@ -110,7 +109,30 @@ moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamm
             else q = max(-127, min(127, (int)roundf(__fmul_rn(f[e], inv))));
             word |= ((uint32_t)q & 0xffu) << (8 * e);
         }
-        xq4[i] = word;
+        return word;
+    };
+    if (TILED) {
+        // the eight-row tile's layout: the four lanes of a 16-element block exchange their words, lane q assembles output
+        // word q from byte q of the four
+        const int Kp = (H + kWeightsPerChunk - 1) / kWeightsPerChunk * kWeightsPerChunk, P4 = Kp >> 2;
+        uint32_t* dst = reinterpret_cast<uint32_t*>(xq + (size_t)t * mma_row_stride(Kp));
+        const int q = lane & 3, base = lane & ~3;
+        int sumx = 0;
+        for (int i0 = 0; i0 < P4; i0 += kMoeThreads) {              // uniform trip count: shuffles need whole warps
+            const int i = i0 + tid;
+            const uint32_t mine = i < H4 ? quant4(i) : 0u;
+            sumx = __dp4a((int)mine, 0x01010101, sumx);
+            const uint32_t w0 = __shfl_sync(0xffffffffu, mine, base + 0), w1 = __shfl_sync(0xffffffffu, mine, base + 1);
+            const uint32_t w2 = __shfl_sync(0xffffffffu, mine, base + 2), w3 = __shfl_sync(0xffffffffu, mine, base + 3);
+            const uint32_t pick = 0x4440u + 0x1111u * (uint32_t)q;     // byte q of the first operand, byte q of the second
+            const uint32_t lo = __byte_perm(w0, w1, pick & 0x00ffu), hi = __byte_perm(w2, w3, pick & 0x00ffu);
+            if (i < P4) dst[i] = __byte_perm(lo, hi, 0x5410);
+        }
+        sumx = __reduce_add_sync(0xffffffffu, sumx);
+        if (lane == 0) s_sum[warp] = sumx;
+    } else {
+        uint32_t* xq4 = reinterpret_cast<uint32_t*>(xq + (size_t)t * H);
+        for (int i = tid; i < H4; i += kMoeThreads) xq4[i] = quant4(i);
     }
     if (tid == 0) xs[t] = scale;
     // router logits: warp w takes experts w, w + 8, ...
@@ -128,6 +150,11 @@ moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamm
         if (lane == 0) s_logit[e] = acc;
     }
     __syncthreads();
+    if (TILED && tid == 32) {
+        int total = 0;
+        for (int w = 0; w < kMoeThreads / 32; ++w) total += s_sum[w];
+        sums[t] = total;
+    }
     if (warp == 0) {
         // softmax over the experts (E <= 32: one lane each), then the two largest (ties to the lower index)
         const bool valid = lane < E;
@@ -151,26 +178,6 @@ moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamm
             selw[2 * t] = __fdiv_rn(p0, den);
             selw[2 * t + 1] = __fdiv_rn(p1, den);
         }
-        if (gridDim.x == 1 && valid) {
-            // single token: routed row 0 goes to expert i0, routed row 1 to expert i1
-            counts[lane] = (lane == i0 || lane == i1) ? 1 : 0;
-            if (lane == i0) rows[(size_t)lane * rows_stride] = 0;
-            if (lane == i1) rows[(size_t)lane * rows_stride] = 1;
-        }
-    }
-}
-
-// rows[e][0..counts[e]) = the routed rows (2*token + slot) of expert e, ascending.
-__global__ void moe_group_kernel(const int* __restrict__ sel, int n_rows, int E, int* __restrict__ counts,
-                                 int* __restrict__ rows, int rows_stride) {
-    grid_dependency_launch();
-    grid_dependency_wait();
-    const int e = threadIdx.x;
-    if (e < E) {
-        int c = 0;
-        for (int r = 0; r < n_rows; ++r)
-            if (sel[r] == e) rows[(size_t)e * rows_stride + c++] = r;
-        counts[e] = c;
     }
 }
 
@@ -196,7 +203,7 @@ static int moe_alloc(void** p, size_t bytes, Moe* m) {
 int moe_reserve(Moe* m, int B) {
     if (B <= m->cap_B) return LSPK_OK;
     void** old[] = {(void**)&m->xq, (void**)&m->xq2, (void**)&m->xs, (void**)&m->xs2, (void**)&m->selw,
-                    (void**)&m->inter, (void**)&m->ydown, (void**)&m->sel, (void**)&m->counts, (void**)&m->rows};
+                    (void**)&m->inter, (void**)&m->ydown, (void**)&m->sel, (void**)&m->sums, (void**)&m->sums2};
     for (void** p : old) {
         cudaFree(*p);
         *p = nullptr;
@@ -205,14 +212,15 @@ int moe_reserve(Moe* m, int B) {
     scratch_moved();
     const size_t R = 2 * (size_t)B;
     int rc = 0;
-    rc |= moe_alloc((void**)&m->xq, (size_t)B * m->H, m);
+    const size_t row_gu = mma_row_stride(m->chunks_gu * kWeightsPerChunk), row_d = mma_row_stride(m->chunks_d * kWeightsPerChunk);
+    rc |= moe_alloc((void**)&m->xq, (size_t)B * row_gu, m);
+    rc |= moe_alloc((void**)&m->sums, (size_t)B * 4, m);
+    rc |= moe_alloc((void**)&m->sums2, R * 4, m);
     rc |= moe_alloc((void**)&m->xs, (size_t)B * 4, m);
     rc |= moe_alloc((void**)&m->sel, R * 4, m);
     rc |= moe_alloc((void**)&m->selw, R * 4, m);
-    rc |= moe_alloc((void**)&m->counts, (size_t)m->E * 4, m);
-    rc |= moe_alloc((void**)&m->rows, (size_t)m->E * R * 4, m);
     rc |= moe_alloc((void**)&m->inter, R * m->I * 4, m);
-    rc |= moe_alloc((void**)&m->xq2, R * m->I, m);
+    rc |= moe_alloc((void**)&m->xq2, R * row_d, m);
     rc |= moe_alloc((void**)&m->xs2, R * 4, m);
     rc |= moe_alloc((void**)&m->ydown, R * m->H * 4, m);
     if (rc) return rc;
@@ -227,21 +235,20 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
     const int H = m->H, I = m->I, E = m->E, R = 2 * B;
     static bool attr_set = false;
     if (!attr_set) {
-        LSPK_CUDA(cudaFuncSetAttribute(moe_router_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        LSPK_CUDA(cudaFuncSetAttribute(moe_router_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        LSPK_CUDA(cudaFuncSetAttribute(moe_router_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set = true;
     }
-    LSPK_CUDA(launch(moe_router_kernel, dim3(B), dim3(kMoeThreads), (size_t)H * 4, true, (const float*)x,
-                     (const uint16_t*)m->norm, (const float*)m->router, m->xq, m->xs, m->sel, m->selw, m->counts, m->rows, R,
-                     H, E, m->eps));
-    if (B > 1)      // a single token's two rows are listed by the router kernel itself
-        LSPK_CUDA(launch(moe_group_kernel, dim3(1), dim3(32), 0, true, (const int*)m->sel, R, E, m->counts, m->rows, R));
-
+    LSPK_CUDA(launch(B > 1 ? moe_router_kernel<true> : moe_router_kernel<false>, dim3(B), dim3(kMoeThreads), (size_t)H * 4, true, (const float*)x,
+                     (const uint16_t*)m->norm, (const float*)m->router, m->xq, m->xs, m->sel, m->selw,
+                     m->sums, H, E, m->eps));
     if (B == 1) {
         // A single token: its two experts' products are one-row products whose matrices the router has just chosen.
         // Both experts of a stage go through ONE launch of the streamed batch (linear_stream.cu), which reads the
         // expert indices on the device; same integer arithmetic as the eight-row kernel, so the same bits.
         static StreamParams sp;
         sp.n = 2;
+        sp.sel_ready = 0;
         for (int slot = 0; slot < 2; ++slot) {
             StreamItem& it = sp.it[slot];
             it = StreamItem{};
@@ -286,6 +293,7 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
             it.nm = 1;
             it.epilogue = LSPK_EPI_STORE;
         }
+        sp.sel_ready = 1;              // as for several tokens below: requested under the quantiser
         if (int rc = stream_launch(&sp)) return rc;
         LSPK_CUDA(launch(moe_combine_kernel, dim3(B), dim3(256), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
         if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, m->sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
@@ -293,64 +301,50 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
         return LSPK_OK;
     }
 
-    // At most min(E, R) experts have rows; CTAs of the others leave at once.  Two resident CTAs per SM
-    // over the experts that can be active keeps enough weight bytes in flight.
-    const int active = E < R ? E : R;
-    int ctas = (2 * sm_count() + active - 1) / active;
-    // The expert products stream tens of megabytes per launch: the weights go through the bulk-copy ring of the
-    // eight-row kernel, three stages deep where they fit.  CTAs per SM follow from the ring's size.
-    const int knob_bulk = 3;
-    auto bulk_ctas = [&](int chunks, bool pair, int Kp, int* stages) -> int {
-        int st = knob_bulk > 4 ? 4 : knob_bulk;
-        const size_t stage = (size_t)chunks * 256 * (pair ? 2 : 1);
-        const size_t base = (size_t)8 * mma_row_stride(Kp) + (size_t)8 * 8 * 16 * (pair ? 2 : 1) * 4 + 8 * 8 + 64 + 256;
-        while (st > 1 && base + st * stage > 110 * 1024) --st;
-        *stages = st;
-        const size_t smem = base + st * stage + 1024;
-        int per_sm = (int)((227 * 1024) / smem);
-        if (per_sm < 1) per_sm = 1;
-        if (per_sm > 3) per_sm = 3;
-        return (per_sm * sm_count() + active - 1) / active;
-    };
-    LinearParams p = {};
-    p.error_flag = device_wait_flag();
-    p.trace = trace_buffer();
-    p.trace_cap = trace_capacity();
-    p.prologue = LSPK_PRO_INT8;
-    p.stream_weights = 0;
-    p.grp_counts = m->counts;
-    p.grp_rows = m->rows;
-    p.grp_rows_stride = R;
-    p.grp_w_stride = 3 * m->mat_stride;
-    p.grp_scales = m->scales;
-    p.M = R;
-    // gate / up
+    // several tokens: every expert's matrices streamed once past the rows routed to it (expert_stream.cu)
+    ExpertStreamParams p = {};
+    p.w_stride = 3 * m->mat_stride;
+    p.scales = m->scales;
+    p.sel = m->sel;
+    p.R = R;
+    p.E = E;
+    p.w[0] = m->w;
+    p.w[1] = m->w + m->mat_stride;
+    p.scale_idx[0] = 0;
+    p.scale_idx[1] = 1;
+    p.x = m->xq;
+    p.xs = m->xs;
+    p.x_sums = m->sums;
+    p.in_shift = 1;                    // routed row 2*token + slot reads token's activations
+    p.out = m->inter;
+    p.acc[0] = acc_gate;
+    p.acc[1] = acc_up;
+    p.N = I;
     p.K = H;
     p.chunks = m->chunks_gu;
-    p.n_seg = 2;
-    p.total_groups = m->groups_gu;
-    p.epilogue = LSPK_EPI_RELU2_MUL;
-    p.seg[0] = LinearSeg{m->w, m->inter, acc_gate, I, m->groups_gu, 1.0f, 0};
-    p.seg[1] = LinearSeg{m->w + m->mat_stride, nullptr, acc_up, I, m->groups_gu, 1.0f, 1};
-    p.x_i8 = m->xq;
-    p.x_scales = m->xs;
-    p.grp_in_shift = 1;                // routed row 2*token + slot reads token's activations
-    if (knob_bulk > 0) ctas = bulk_ctas(p.chunks, true, p.chunks * kWeightsPerChunk, &p.bulk_stages);
-    if (int rc = linear_launch_params(p, 8, true, true, ctas < m->groups_gu ? ctas : m->groups_gu, 1, E)) return rc;
+    p.groups = m->groups_gu;
+    if (int rc = expert_stream_launch(p, true)) return rc;
     // SubLN + quantiser per routed row, with the row's expert's norm weights
-    if (int rc = norm_quant_rows_selected(m->inter, m->sub_norm, m->sel, m->xq2, m->xs2, R, I, m->eps)) return rc;
-    // down
+    int* const sums2 = I % 8 == 0 ? m->sums2 : nullptr;      // else natural rows: an expert's norm weights are not 16-byte aligned
+    if (int rc = norm_quant_rows_selected(m->inter, m->sub_norm, m->sel, m->xq2, m->xs2, R, I, m->eps, sums2)) return rc;
+    // The quantiser lets its successor start only once gate / up has ended (norm_quant_rows_selected), the router long
+    // before: the down matrices are requested under the quantiser.
+    p.sel_ready = 1;
+    p.w[0] = m->w + 2 * m->mat_stride;
+    p.w[1] = nullptr;
+    p.scale_idx[0] = 2;
+    p.x = m->xq2;
+    p.xs = m->xs2;
+    p.x_sums = sums2;
+    p.in_shift = 0;
+    p.out = m->ydown;
+    p.acc[0] = acc_down;
+    p.acc[1] = nullptr;
+    p.N = H;
     p.K = I;
     p.chunks = m->chunks_d;
-    p.n_seg = 1;
-    p.total_groups = m->groups_d;
-    p.epilogue = LSPK_EPI_STORE;
-    p.seg[0] = LinearSeg{m->w + 2 * m->mat_stride, m->ydown, acc_down, H, m->groups_d, 1.0f, 2};
-    p.x_i8 = m->xq2;
-    p.x_scales = m->xs2;
-    p.grp_in_shift = 0;
-    if (knob_bulk > 0) ctas = bulk_ctas(p.chunks, false, p.chunks * kWeightsPerChunk, &p.bulk_stages);
-    if (int rc = linear_launch_params(p, 8, false, true, ctas < m->groups_d ? ctas : m->groups_d, 1, E)) return rc;
+    p.groups = m->groups_d;
+    if (int rc = expert_stream_launch(p, false)) return rc;
     LSPK_CUDA(launch(moe_combine_kernel, dim3(B), dim3(256), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
     if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, m->sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
     if (selw_out) LSPK_CUDA(cudaMemcpyAsync(selw_out, m->selw, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
@@ -424,7 +418,7 @@ int lspk_moe_free(lspk_moe_t h) {
     Moe* m = reinterpret_cast<Moe*>(h);
     cudaStreamSynchronize(stream());
     void* dev[] = {m->w, m->scales, m->router, m->norm, m->sub_norm, m->xq, m->xq2, m->xs, m->xs2, m->selw,
-                   m->inter, m->ydown, m->sel, m->counts, m->rows};
+                   m->inter, m->ydown, m->sel, m->sums, m->sums2};
     for (void* p : dev) cudaFree(p);
     delete m;
     return LSPK_OK;

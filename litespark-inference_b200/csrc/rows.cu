@@ -47,8 +47,9 @@ row_norm_quant_kernel(const float* __restrict__ x, const float* __restrict__ gat
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* xs = reinterpret_cast<float*>(smem_raw);
     __shared__ float red[32];
-    grid_dependency_launch();
+    if (!gamma_sel) grid_dependency_launch();
     grid_dependency_wait();
+    if (gamma_sel) grid_dependency_launch();     // not earlier: see norm_quant_rows_selected
     const int t = blockIdx.x, tid = threadIdx.x;
     const float* src = x + (size_t)t * K;
     const float* gsrc = gate ? gate + (size_t)t * K : nullptr;
@@ -239,8 +240,9 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
         }
     };
     if (norm && !gamma_sel) load_gamma(gamma_base);
-    grid_dependency_launch();
+    if (!gamma_sel) grid_dependency_launch();
     grid_dependency_wait();
+    if (gamma_sel) grid_dependency_launch();     // not earlier: see norm_quant_rows_selected
     if (norm && gamma_sel)
         load_gamma(reinterpret_cast<const char*>(gamma_base) + (size_t)gamma_sel[t] * K * (gamma_is_bf16 ? 2 : 4));
 
@@ -420,9 +422,13 @@ int split_row_prologue(lspk_linear_args* a, int K, int8_t* q_scratch, float* sca
 }
 
 // RMSNorm + quantiser of T rows where row t takes the gamma_sel[t]-th weight vector (bf16, K each).
+// The kernel lets its successor start only after its own dependency wait: whatever ran before its predecessor's end --
+// gamma_sel among it -- is then final when the successor starts, which may so read gamma_sel ahead of its wait.
 int norm_quant_rows_selected(const float* x, const void* gamma_bf16, const int* gamma_sel, int8_t* out, float* scales,
-                             int T, int K, float eps) {
-    return launch_rows(x, gamma_bf16, 1, nullptr, out, scales, T, K, eps, 3, nullptr, gamma_sel);
+                             int T, int K, float eps, int* tiled_sums) {
+    const int Kp = (K + kWeightsPerChunk - 1) / kWeightsPerChunk * kWeightsPerChunk;
+    return launch_rows(x, gamma_bf16, 1, nullptr, out, scales, T, K, eps, 3, nullptr, gamma_sel, tiled_sums ? Kp : 0,
+                       tiled_sums ? mma_row_stride(Kp) : 0, tiled_sums);
 }
 
 // Quantise fp32 rows (QUANT, RMSNORM_QUANT or GATED_RMSNORM_QUANT prologue of `a`) straight into the permuted,
