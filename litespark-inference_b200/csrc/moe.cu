@@ -49,15 +49,25 @@ template <bool TILED>
 __global__ void __launch_bounds__(kMoeThreads)
 moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamma, const float* __restrict__ router,
                   int8_t* __restrict__ xq, float* __restrict__ xs, int* __restrict__ sel, float* __restrict__ selw,
-                  int* __restrict__ sums, int H, int E, float eps) {
-    extern __shared__ __align__(16) float hs[];           // [H] normalised row
+                  int* __restrict__ sums, int H, int E, float eps, int staged) {
+    extern __shared__ __align__(16) float hs[];           // [H] normalised row; staged: [E][H] router, [H] bf16 norm weights
     __shared__ __align__(16) float red[16];
     __shared__ float s_logit[kMaxExperts];
     __shared__ int s_sum[kMoeThreads / 32];
-    grid_dependency_launch();
-    grid_dependency_wait();
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int H4 = H >> 2;
+    grid_dependency_launch();
+    // The router matrix and the norm weights (85 KB at eight experts of 2560) do not depend on the previous kernel: they
+    // come into shared memory under it, instead of from HBM in the middle of this kernel's chain.
+    float4* const wr_s = reinterpret_cast<float4*>(hs) + H4;
+    uint2* const gamma_s = reinterpret_cast<uint2*>(wr_s + (size_t)E * H4);
+    if (staged) {
+        const float4* wr4 = reinterpret_cast<const float4*>(router);
+        for (int i = tid; i < E * H4; i += kMoeThreads)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(wr_s + i)), "l"(wr4 + i) : "memory");
+        for (int i = tid; i < H4; i += kMoeThreads) gamma_s[i] = __ldg(reinterpret_cast<const uint2*>(gamma) + i);
+    }
+    grid_dependency_wait();
     const float4* src4 = reinterpret_cast<const float4*>(x + (size_t)t * H);
     float4* hs4 = reinterpret_cast<float4*>(hs);
     float ssq = 0.0f;
@@ -80,7 +90,7 @@ moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamm
     float amax = 0.0f;
     for (int i = tid; i < H4; i += kMoeThreads) {
         float4 v = hs4[i];
-        const uint2 gb = *reinterpret_cast<const uint2*>(gamma + 4 * i);
+        const uint2 gb = staged ? gamma_s[i] : __ldg(reinterpret_cast<const uint2*>(gamma) + i);      // staged: this thread's own store
         v.x = __fmul_rn(__fmul_rn(v.x, rrms), __uint_as_float(gb.x << 16));
         v.y = __fmul_rn(__fmul_rn(v.y, rrms), __uint_as_float(gb.x & 0xffff0000u));
         v.z = __fmul_rn(__fmul_rn(v.z, rrms), __uint_as_float(gb.y << 16));
@@ -91,7 +101,8 @@ moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamm
     {
         const uint32_t u = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
         if (lane == 0) red[8 + warp] = __uint_as_float(u);
-        __syncthreads();                                   // also publishes the normalised row
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();                                   // also publishes the normalised row and the router matrix
         const float4 a = *reinterpret_cast<const float4*>(red + 8), b = *reinterpret_cast<const float4*>(red + 12);
         amax = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
     }
@@ -138,13 +149,19 @@ moe_router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ gamm
     // router logits: warp w takes experts w, w + 8, ...
     for (int e = warp; e < E; e += kMoeThreads / 32) {
         const float4* wr4 = reinterpret_cast<const float4*>(router + (size_t)e * H);
+        const float4* ws4 = wr_s + (size_t)e * H4;
         float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-        for (int i = lane; i < H4; i += 32) {
-            const float4 h = hs4[i], w = __ldg(wr4 + i);
+        auto add = [&](const float4& h, const float4& w) {
             a0 = fmaf(h.x, w.x, a0);
             a1 = fmaf(h.y, w.y, a1);
             a2 = fmaf(h.z, w.z, a2);
             a3 = fmaf(h.w, w.w, a3);
+        };
+        if (staged) {
+#pragma unroll 4
+            for (int i = lane; i < H4; i += 32) add(hs4[i], ws4[i]);
+        } else {
+            for (int i = lane; i < H4; i += 32) add(hs4[i], __ldg(wr4 + i));
         }
         const float acc = warp_sum((a0 + a1) + (a2 + a3));
         if (lane == 0) s_logit[e] = acc;
@@ -185,12 +202,18 @@ __global__ void moe_combine_kernel(float* __restrict__ x, const float* __restric
                                    int H) {
     grid_dependency_launch();
     grid_dependency_wait();
-    const int t = blockIdx.x;
-    const float w0 = selw[2 * t], w1 = selw[2 * t + 1];
-    const float* y0 = y + (size_t)(2 * t) * H;
-    const float* y1 = y0 + H;
-    for (int k = threadIdx.x; k < H; k += blockDim.x)
-        x[(size_t)t * H + k] = __fadd_rn(x[(size_t)t * H + k], __fadd_rn(__fmul_rn(w0, y0[k]), __fmul_rn(w1, y1[k])));
+    // a thread takes four elements of a token: one trip to memory, whatever H is
+    const int t = blockIdx.x, k = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (k >= H) return;
+    const float2 w = *reinterpret_cast<const float2*>(selw + 2 * t);
+    const float4 a = *reinterpret_cast<const float4*>(y + (size_t)(2 * t) * H + k);
+    const float4 b = *reinterpret_cast<const float4*>(y + (size_t)(2 * t + 1) * H + k);
+    float4 v = *reinterpret_cast<const float4*>(x + (size_t)t * H + k);
+    v.x = __fadd_rn(v.x, __fadd_rn(__fmul_rn(w.x, a.x), __fmul_rn(w.y, b.x)));
+    v.y = __fadd_rn(v.y, __fadd_rn(__fmul_rn(w.x, a.y), __fmul_rn(w.y, b.y)));
+    v.z = __fadd_rn(v.z, __fadd_rn(__fmul_rn(w.x, a.z), __fmul_rn(w.y, b.z)));
+    v.w = __fadd_rn(v.w, __fadd_rn(__fmul_rn(w.x, a.w), __fmul_rn(w.y, b.w)));
+    *reinterpret_cast<float4*>(x + (size_t)t * H + k) = v;
 }
 
 static int moe_alloc(void** p, size_t bytes, Moe* m) {
@@ -239,9 +262,12 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
         LSPK_CUDA(cudaFuncSetAttribute(moe_router_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set = true;
     }
-    LSPK_CUDA(launch(B > 1 ? moe_router_kernel<true> : moe_router_kernel<false>, dim3(B), dim3(kMoeThreads), (size_t)H * 4, true, (const float*)x,
+    const size_t extra = (size_t)E * H * 4 + (size_t)H * 2;
+    const int staged = (size_t)H * 4 + extra <= 200 * 1024;     // else the router matrix is read where it lies
+    LSPK_CUDA(launch(B > 1 ? moe_router_kernel<true> : moe_router_kernel<false>, dim3(B), dim3(kMoeThreads),
+                     (size_t)H * 4 + (staged ? extra : 0), true, (const float*)x,
                      (const uint16_t*)m->norm, (const float*)m->router, m->xq, m->xs, m->sel, m->selw,
-                     m->sums, H, E, m->eps));
+                     m->sums, H, E, m->eps, staged));
     if (B == 1) {
         // A single token: its two experts' products are one-row products whose matrices the router has just chosen.
         // Both experts of a stage go through ONE launch of the streamed batch (linear_stream.cu), which reads the
@@ -295,7 +321,7 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
         }
         sp.sel_ready = 1;              // as for several tokens below: requested under the quantiser
         if (int rc = stream_launch(&sp)) return rc;
-        LSPK_CUDA(launch(moe_combine_kernel, dim3(B), dim3(256), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
+        LSPK_CUDA(launch(moe_combine_kernel, dim3(B, (H + 511) / 512), dim3(128), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
         if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, m->sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
         if (selw_out) LSPK_CUDA(cudaMemcpyAsync(selw_out, m->selw, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
         return LSPK_OK;
@@ -345,7 +371,7 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
     p.chunks = m->chunks_d;
     p.groups = m->groups_d;
     if (int rc = expert_stream_launch(p, false)) return rc;
-    LSPK_CUDA(launch(moe_combine_kernel, dim3(B), dim3(256), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
+    LSPK_CUDA(launch(moe_combine_kernel, dim3(B, (H + 511) / 512), dim3(128), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
     if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, m->sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
     if (selw_out) LSPK_CUDA(cudaMemcpyAsync(selw_out, m->selw, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
     return LSPK_OK;
