@@ -684,6 +684,276 @@ __global__ void __launch_bounds__(NT, MINB) attention_split_kernel(const AttnPar
     tr.end();
 }
 
+// The split form for several sequences with long caches: a CTA takes HG query heads of one KV head at once.  One CTA per
+// query head pulls every cache row through the L2 once per head of the group (four times at 20 / 5 heads: 80 MB a layer
+// at two sequences of 2000 fp32 positions, 17.9 us; the 20 MB once are 3.1 us of HBM time), four rows in flight per
+// thread.  Two heads and eight rows measured best there: decode of two sequences behind 1989 positions 1.63 -> 1.54 ms
+// per step; four heads with sixteen rows 1.61 (80 CTAs, and the exchange of dot products grows with the heads).
+// Every sum is formed in the order of the kernel above (defined for 256 threads), so each head's result is the same to
+// the bit whichever kernel computes it.
+// SB: keys per group in flight (each of K and V); MINB: CTAs per SM the register budget is held to.
+template <typename KVT, int D, int HG, int SB, int MINB>
+__global__ void __launch_bounds__(kAttnThreads, MINB) attention_group_kernel(const AttnParams p) {
+    namespace cg = cooperative_groups;
+    constexpr int VEC = KvVec<KVT>::N;
+    constexpr int TPK = D / VEC;                // lanes per key: one 16-byte load of a cache row each
+    constexpr int NG = kAttnThreads / TPK;      // key groups
+    constexpr int KPB = NG * SB;                // local keys per batch
+    constexpr int SX = 4;                       // keys whose dot products are reduced together
+    static_assert(TPK <= 32 && TPK >= SX && SB % SX == 0 && HG <= kSplit && D <= kAttnThreads, "attention_group_kernel");
+    extern __shared__ __align__(16) float at_smem[];
+    float* qs = at_smem;                  // [HG][D] rotated queries
+    float* ks = qs + HG * D;              // [D] rotated current key
+    float* vs = ks + D;                   // [D] current value
+    float* raw = vs + D;                  // [HG + 1][D] raw q and k before rotation
+    float* part = raw + (HG + 1) * D;     // [HG][NG][D] value partial sums of this CTA
+    float* fin = part + HG * NG * D;      // [kSplit][D] the cluster's partials of head `rank`
+    float* sc = fin + kSplit * D;         // [HG][local] scores / exponentials
+    __shared__ __align__(16) float cl_max[kSplit], cl_sum[kSplit];
+    __shared__ __align__(16) float red[2][HG][8];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int r = (int)cluster.block_rank();
+    // announced here, waited for in front of the first remote store (as above)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    grid_dependency_launch();
+    grid_dependency_wait();
+
+    const int t = blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int G = p.Q / p.KV, h0 = blockIdx.x * HG, kvh = h0 / G;         // HG divides G
+    const int half = D / 2;
+    const int kd = p.KV * D;
+    const int local = (p.t_max + kSplit - 1) / kSplit + 1;
+    KVT* ck = reinterpret_cast<KVT*>(p.cache_k) + (size_t)t * p.cache_seq_stride + (size_t)kvh * D;
+    KVT* cv = reinterpret_cast<KVT*>(p.cache_v) + (size_t)t * p.cache_seq_stride + (size_t)kvh * D;
+    const float* qrow = p.q + (size_t)t * p.Q * D + (size_t)h0 * D;
+    const int g = tid / TPK, c = tid % TPK;
+    const int pos = p.pos_per_row ? p.pos_ptr[t] : p.pos_ptr[0] + t;
+
+    // requests that do not need the position
+    constexpr int NQ = ((HG + 1) * D + kAttnThreads - 1) / kAttnThreads;
+    float q_raw[NQ], vr = 0.0f;
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+        const int i = tid + u * kAttnThreads;
+        q_raw[u] = i < HG * D ? qrow[i] : i < (HG + 1) * D ? p.k_cur[(size_t)t * kd + (size_t)kvh * D + i - HG * D] : 0.0f;
+    }
+    if (tid < D) vr = p.v_cur[(size_t)t * kd + (size_t)kvh * D + tid];
+    uint4 kbuf[SB], vbuf[SB];
+    auto request = [&](uint4* buf, const KVT* base_ptr, int base, int limit) {
+#pragma unroll
+        for (int j = 0; j < SB; ++j) {
+            const int i = r + kSplit * (base + g + j * NG);
+            if (i < limit) buf[j] = *(reinterpret_cast<const uint4*>(base_ptr + (size_t)i * kd) + c);
+        }
+    };
+    request(kbuf, ck, 0, p.t_max);               // rows past the position are allocated and never used
+    request(vbuf, cv, 0, p.t_max);
+
+    const int n = pos + 1;
+    const int n_local = n > r ? (n - r + kSplit - 1) / kSplit : 0;     // keys r, r + kSplit, ... below n
+    const bool owner = (pos % kSplit) == r;
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+        const int i = tid + u * kAttnThreads;
+        if (i < (HG + 1) * D) raw[i] = q_raw[u];
+    }
+    __syncthreads();                             // the rotation pairs element i with i + half
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+        const int e = tid + u * kAttnThreads;
+        if (e < (HG + 1) * D) {
+            const int d = e % D, i = d < half ? d : d - half;
+            const float* row = raw + (e - d);
+            const float cr = p.rope_cur ? p.rope_cur[(size_t)t * D + i] : p.rope_cos[(size_t)pos * half + i];
+            const float sr = p.rope_cur ? p.rope_cur[(size_t)t * D + half + i] : p.rope_sin[(size_t)pos * half + i];
+            const float x1 = row[i], x2 = row[half + i];
+            const float y = d < half ? __fsub_rn(__fmul_rn(x1, cr), __fmul_rn(x2, sr))
+                                     : __fadd_rn(__fmul_rn(x1, sr), __fmul_rn(x2, cr));
+            if (e < HG * D) {
+                qs[e] = y;
+            } else {
+                ks[d] = kv_round<KVT>(y);
+                if (owner && h0 % G == 0) ck[(size_t)pos * kd + d] = kv_make<KVT>(y);
+            }
+        }
+    }
+    if (tid < D) {
+        vs[tid] = kv_round<KVT>(vr);
+        if (owner && h0 % G == 0) cv[(size_t)pos * kd + tid] = kv_make<KVT>(vr);
+    }
+    __syncthreads();
+
+    // ---- scores of this CTA's keys: a key row is unpacked once for the HG heads ------------------------------
+    const float inv_sqrt_d = 1.0f / sqrtf((float)D);
+    float mx[HG];
+    {
+        float qreg[HG][VEC];
+#pragma unroll
+        for (int hd = 0; hd < HG; ++hd) {
+            mx[hd] = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) qreg[hd][e] = qs[hd * D + c * VEC + e];
+        }
+        for (int base = 0; base < n_local; base += KPB) {
+            if (base > 0) request(kbuf, ck, base, pos);
+#pragma unroll
+            for (int j0 = 0; j0 < SB; j0 += SX) {
+                float dotp[HG][SX];
+#pragma unroll
+                for (int j = 0; j < SX; ++j) {
+                    const int i = r + kSplit * (base + g + (j0 + j) * NG);
+                    float f[VEC];
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) f[e] = 0.0f;
+                    if (i == pos) {
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e) f[e] = ks[c * VEC + e];
+                    } else if (i < n) {
+                        KvVec<KVT>::unpack(kbuf[j0 + j], f);
+                    }
+#pragma unroll
+                    for (int hd = 0; hd < HG; ++hd) {
+                        float d = 0.0f;
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e) d = fmaf(qreg[hd][e], f[e], d);
+                        dotp[hd][j] = d;
+                    }
+                }
+                const int jl = base + g + (j0 + c) * NG;             // lane c < SX ends up with key j0 + c of its group
+#pragma unroll
+                for (int hd = 0; hd < HG; ++hd) {
+#pragma unroll
+                    for (int o = TPK / 2; o >= 1; o >>= 1) {
+                        if (o >= SX) {
+#pragma unroll
+                            for (int j = 0; j < SX; ++j) dotp[hd][j] += __shfl_xor_sync(0xffffffffu, dotp[hd][j], o);
+                        } else {
+                            const bool upper = (c & o) != 0;
+#pragma unroll
+                            for (int k = 0; k < o; ++k) {
+                                const float send = upper ? dotp[hd][k] : dotp[hd][k + o];
+                                const float keep = upper ? dotp[hd][k + o] : dotp[hd][k];
+                                dotp[hd][k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                            }
+                        }
+                    }
+                    if (c < SX && r + kSplit * jl < n) {
+                        const float sv = __fmul_rn(dotp[hd][0], inv_sqrt_d);
+                        sc[hd * local + jl] = sv;
+                        mx[hd] = fmaxf(mx[hd], sv);
+                    }
+                }
+            }
+        }
+    }
+
+    // ---- each head's maximum, exponentials relative to it, and their sum -------------------------------------
+#pragma unroll
+    for (int hd = 0; hd < HG; ++hd) {
+        const uint32_t u = __reduce_max_sync(0xffffffffu, float_to_ordered(mx[hd]));
+        if (lane == 0) red[0][hd][warp] = ordered_to_float(u);
+    }
+    __syncthreads();
+    float sum[HG];
+#pragma unroll
+    for (int hd = 0; hd < HG; ++hd) {
+        const float4 a = *reinterpret_cast<const float4*>(red[0][hd]), b = *reinterpret_cast<const float4*>(red[0][hd] + 4);
+        mx[hd] = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+        sum[hd] = 0.0f;
+        for (int j = tid; j < n_local; j += kAttnThreads) {
+            const float e = expf(sc[hd * local + j] - mx[hd]);
+            sc[hd * local + j] = e;
+            sum[hd] += e;
+        }
+        sum[hd] = warp_sum(sum[hd]);
+        if (lane == 0) red[1][hd][warp] = sum[hd];
+    }
+    __syncthreads();                              // also publishes sc[] to the value phase
+#pragma unroll
+    for (int hd = 0; hd < HG; ++hd) {
+        const float4 a = *reinterpret_cast<const float4*>(red[1][hd]), b = *reinterpret_cast<const float4*>(red[1][hd] + 4);
+        sum[hd] = ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+    }
+
+    // ---- unnormalised weighted sums of this CTA's values ------------------------------------------------------
+    float o[HG][VEC];
+#pragma unroll
+    for (int hd = 0; hd < HG; ++hd)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) o[hd][e] = 0.0f;
+    for (int base = 0; base < n_local; base += KPB) {
+        if (base > 0) request(vbuf, cv, base, pos);
+#pragma unroll
+        for (int j = 0; j < SB; ++j) {
+            const int jl = base + g + j * NG;
+            const int i = r + kSplit * jl;
+            if (i < n) {
+                float f[VEC];
+                if (i == pos) {
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) f[e] = vs[c * VEC + e];
+                } else {
+                    KvVec<KVT>::unpack(vbuf[j], f);
+                }
+#pragma unroll
+                for (int hd = 0; hd < HG; ++hd) {
+                    const float pi = sc[hd * local + jl];
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) o[hd][e] = fmaf(pi, f[e], o[hd][e]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int hd = 0; hd < HG; ++hd)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) part[(hd * NG + g) * D + c * VEC + e] = o[hd][e];
+    __syncthreads();
+    // ---- hand (maximum, sum, partial output) of head hd to rank hd, which merges the kSplit softmax pieces ---
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // every CTA of the cluster is running
+    for (int e = tid; e < HG * D; e += kAttnThreads) {
+        const int hd = e / D, d = e % D;
+        float acc = 0.0f;
+#pragma unroll
+        for (int w = 0; w < NG; ++w) acc += part[(hd * NG + w) * D + d];
+        cluster.map_shared_rank(fin, hd)[r * D + d] = acc;
+    }
+    if (tid == 0) {
+#pragma unroll
+        for (int hd = 0; hd < HG; ++hd) {
+            cluster.map_shared_rank(cl_max, hd)[r] = mx[hd];
+            cluster.map_shared_rank(cl_sum, hd)[r] = sum[hd];
+        }
+    }
+    cluster.sync();
+    if (r < HG && tid < D) {
+        float M = cl_max[0];
+#pragma unroll
+        for (int w = 1; w < kSplit; ++w) M = fmaxf(M, cl_max[w]);
+        float L = 0.0f, acc = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kSplit; ++w) {
+            const float wgt = expf(cl_max[w] - M);               // 0 for a piece without keys (maximum -inf)
+            L = fmaf(cl_sum[w], wgt, L);
+            acc = fmaf(fin[w * D + tid], wgt, acc);
+        }
+        p.out[(size_t)t * p.Q * D + (size_t)(h0 + r) * D + tid] = __fdiv_rn(acc, L);
+    }
+}
+
+template <typename KVT, int D, int HG, int SB, int MINB>
+static cudaError_t launch_attention_group(const AttnParams& p, size_t sm) {
+    static bool attr_set = false;
+    auto kern = attention_group_kernel<KVT, D, HG, SB, MINB>;
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return e;
+        attr_set = true;
+    }
+    return launch_cluster(kern, dim3(p.Q / HG, p.T, kSplit), dim3(kAttnThreads), sm, true, dim3(1, 1, kSplit), p);
+}
+
 // Prefill form: kRows consecutive query rows of one head per CTA (rows of one sequence, already rotated,
 // keys and values already in the cache).  Every key / value row is fetched once for the kRows queries
 // instead of once per query; row r attends keys 0 .. pos0 + t0 + r.  Same lane layout as the one-row
@@ -939,6 +1209,17 @@ static int attention_launch_t(const AttnParams& p) {
             split_attr_set = true;
         }
         LSPK_REQUIRE(sm <= 200 * 1024, "attention: t_max=%d too large for the shared score buffer", p.t_max);
+        // Several sequences with long caches, and query heads that share a KV head: cache rows fetched once for two heads.
+        // Long: a CTA may hold more keys than two of the other kernel's batches.  Shorter caches are bound by latency and
+        // want the CTAs: eight sequences behind 128 to 205 positions took 1.35 ms per step in the other kernel, 1.46 in
+        // this one (four heads).  One sequence stays there for the same reason.
+        const int ng = kAttnThreads / tpk;
+        const size_t gsm = (size_t)((2 * 2 + 3) * D + 2 * ng * D + kSplit * D + 2 * local_keys) * sizeof(float);
+        if (p.T > 1 && (p.Q / p.KV) % 2 == 0 && D <= 128 && gsm <= 200 * 1024 && local_keys > 8 * ng) {
+            const cudaError_t ge = D == 128 ? launch_attention_group<KVT, 128, 2, 8, 2>(p, gsm) : launch_attention_group<KVT, 64, 2, 8, 2>(p, gsm);
+            if (ge != cudaSuccess) return fail(LSPK_ERR_CUDA, "attention (grouped heads) launch failed: %s", cudaGetErrorString(ge));
+            return LSPK_OK;
+        }
         const dim3 sgrid(p.Q, p.T, kSplit), cl(1, 1, kSplit);
         cudaError_t se;
         if (D == 64) se = launch_cluster(attention_split_kernel<KVT, 64>, sgrid, dim3(kAttnThreads), sm, true, cl, p);
