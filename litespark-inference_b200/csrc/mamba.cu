@@ -8,7 +8,8 @@
 //   out = out_proj(quant(RMSNorm(y * SiLU(z))));  x += out      ternary linear, residual epilogue
 // The state update is the HBM-bound part: the fp32 state [heads, head_dim, d_state] (2.6 MB per
 // sequence and layer at 80 x 64 x 128) is read and written once per step.  One CTA owns half a head (32 rows of
-// 128 states, 16 KB in and out; grid = 2 * heads x sequences) or, for four and more sequences, a whole head.
+// 128 states, 16 KB in and out; grid = 2 * heads x sequences); for four and more sequences the states are a stream through one CTA
+// per SM.
 #include "internal.cuh"
 #include "../../include/lspk_hybrid.h"
 
@@ -28,26 +29,51 @@ struct Mamba {
 
 __device__ __forceinline__ float silu_f(float v) { return __fdiv_rn(v, __fadd_rn(expf(-v), 1.0f)); }
 
-// P = head_dim = 64, N = d_state = 128.  A CTA of 256 threads owns ROWS rows of one head (32: half a head, grid
-// 2 * heads x sequences; 64: a whole head, grid heads x sequences); 8 threads share a row, a thread holds 16 state
-// values of each of its ROWS / 32 rows.  Whole-head CTAs keep twice the state bytes in flight per thread and run
-// the B / C convolution once per head instead of twice: the form for several sequences, where the launch is bound
-// by HBM; with one sequence the half-head form covers more SMs.  Same arithmetic per element in both.
-template <int ROWS>
-__global__ void __launch_bounds__(256, ROWS == 64 ? 4 : 1)
+// depthwise conv step of one channel (ring of the last four inputs, width 4) + SiLU
+__device__ __forceinline__ float conv_silu(float bias, const float4& taps, const float4& hist, float newv, int pos) {
+    const float h4[4] = {hist.x, hist.y, hist.z, hist.w};
+    const float w4[4] = {taps.x, taps.y, taps.z, taps.w};
+    float acc = bias;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const int sl = (pos - 3 + j) & 3;
+        const float hv = sl == 0 ? h4[0] : sl == 1 ? h4[1] : sl == 2 ? h4[2] : h4[3];
+        acc = __fadd_rn(acc, __fmul_rn(w4[j], hv));
+    }
+    return silu_f(__fadd_rn(acc, __fmul_rn(w4[3], newv)));
+}
+// four states of a row: state * dA + dtx * B, and their part of the row's output
+__device__ __forceinline__ void ssu_update(float4& s4, float dA, float dtx, const float4& Bv, const float4& Cv, float& ysum) {
+    s4.x = __fadd_rn(__fmul_rn(s4.x, dA), __fmul_rn(dtx, Bv.x));
+    s4.y = __fadd_rn(__fmul_rn(s4.y, dA), __fmul_rn(dtx, Bv.y));
+    s4.z = __fadd_rn(__fmul_rn(s4.z, dA), __fmul_rn(dtx, Bv.z));
+    s4.w = __fadd_rn(__fmul_rn(s4.w, dA), __fmul_rn(dtx, Bv.w));
+    ysum = fmaf(s4.x, Cv.x, ysum);
+    ysum = fmaf(s4.y, Cv.y, ysum);
+    ysum = fmaf(s4.z, Cv.z, ysum);
+    ysum = fmaf(s4.w, Cv.w, ysum);
+}
+// over the eight lanes of a row
+__device__ __forceinline__ float ssu_row_sum(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return v + __shfl_xor_sync(0xffffffffu, v, 1);
+}
+
+// P = head_dim = 64, N = d_state = 128.  A CTA of 256 threads owns half a head (grid 2 * heads x sequences): the form for
+// one to three sequences, where covering the SMs counts.  8 threads share a row; thread `seg` of a row holds the four
+// 16-byte pieces seg, seg + 8, ... of its 128 states.
+constexpr int ROWS = 32;
+__global__ void __launch_bounds__(256)
 mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr,
                   const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ A,
                   const float* __restrict__ dt_bias, const float* __restrict__ Dskip, float* __restrict__ vout,
                   int d_inner, int conv_dim, int in_out, size_t state_floats) {
-    constexpr int P = 64, N = 128, RS = ROWS / 32;       // RS: rows per thread
-    static_assert(ROWS == 32 || ROWS == 64, "a CTA owns half a head or a whole one");
+    constexpr int P = 64, N = 128;
     __shared__ float xs_s[ROWS];
-    // B and C with four floats of padding after every 16: the eight threads of a row read 16-byte pieces 80 bytes
-    // apart, which fall into eight different bank groups (64 bytes apart they collide four ways)
-    constexpr int NPAD = N + N / 16 * 4;
-    __shared__ __align__(16) float B_s[NPAD];
-    __shared__ __align__(16) float C_s[NPAD];
-    const int b = blockIdx.y, hh = blockIdx.x, head = ROWS == 64 ? hh : hh >> 1, p0 = ROWS == 64 ? 0 : (hh & 1) * ROWS;
+    __shared__ __align__(16) float B_s[N];
+    __shared__ __align__(16) float C_s[N];
+    const int b = blockIdx.y, hh = blockIdx.x, head = hh >> 1, p0 = (hh & 1) * ROWS;
     const int tid = threadIdx.x;
     grid_dependency_launch();
     grid_dependency_wait();
@@ -56,17 +82,11 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     // convolution.  Not before the wait: the state was written by this kernel one decode step ago, and with
     // programmatic launch nothing orders code in front of the wait after a kernel that is not the direct
     // predecessor (in a short chain -- a single layer stepped in a loop -- that kernel may still be running).
-    float4 st[RS][4];
-    float4* srow[RS];
-    {
-        float* ssm0 = state + (size_t)b * state_floats + (size_t)conv_dim * 4;
+    float4 st[4];
+    float4* const srow = reinterpret_cast<float4*>(state + (size_t)b * state_floats + (size_t)conv_dim * 4 +
+                                                   (size_t)(head * P + p0 + (tid >> 3)) * N) + (tid & 7);
 #pragma unroll
-        for (int rr = 0; rr < RS; ++rr) {
-            srow[rr] = reinterpret_cast<float4*>(ssm0 + ((size_t)(head * P + p0 + 32 * rr + (tid >> 3)) * N + (tid & 7) * 16));
-#pragma unroll
-            for (int q = 0; q < 4; ++q) st[rr][q] = srow[rr][q];
-        }
-    }
+    for (int q = 0; q < 4; ++q) st[q] = srow[8 * q];
     const float* zrow = zx + (size_t)b * in_out;
     const float* xbc_raw = zrow + d_inner;
     const float* dt_raw = zrow + d_inner + conv_dim;
@@ -77,9 +97,7 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     // per-head scalars and this thread's gate inputs: requested here so that their round trip overlaps the
     // convolution's (they are used after the barrier below)
     const float dt_in = dt_raw[head], dt_b = dt_bias[head], a_head = A[head], d_head = Dskip[head];
-    float z_gate[RS];
-#pragma unroll
-    for (int rr = 0; rr < RS; ++rr) z_gate[rr] = (tid & 7) == 0 ? zrow[head * P + p0 + 32 * rr + (tid >> 3)] : 0.0f;
+    const float z_gate = (tid & 7) == 0 ? zrow[head * P + p0 + (tid >> 3)] : 0.0f;
 
     // depthwise conv step + SiLU for the channels this CTA needs: its ROWS x-channels, all of B and C.  A thread
     // takes channel index tid and, the first ROWS + 2 N - 256 threads, a second one; everything both need (the
@@ -106,20 +124,10 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     for (int k = 0; k < 2; ++k) {
         if (k == 0 || second) {
             const int idx = tid + 256 * k;
-            const float h4[4] = {hist[k].x, hist[k].y, hist[k].z, hist[k].w};
-            const float w4[4] = {taps[k].x, taps[k].y, taps[k].z, taps[k].w};
-            float acc = bias[k];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const int sl = (pos - 3 + j) & 3;
-                const float hv = sl == 0 ? h4[0] : sl == 1 ? h4[1] : sl == 2 ? h4[2] : h4[3];
-                acc = __fadd_rn(acc, __fmul_rn(w4[j], hv));
-            }
-            acc = __fadd_rn(acc, __fmul_rn(w4[3], newv[k]));
-            const float act = silu_f(acc);
+            const float act = conv_silu(bias[k], taps[k], hist[k], newv[k], pos);
             if (idx < ROWS) xs_s[idx] = act;
-            else if (idx < ROWS + N) B_s[(idx - ROWS) + ((idx - ROWS) >> 4) * 4] = act;
-            else C_s[(idx - ROWS - N) + ((idx - ROWS - N) >> 4) * 4] = act;
+            else if (idx < ROWS + N) B_s[idx - ROWS] = act;
+            else C_s[idx - ROWS - N] = act;
             // the newest input replaces the oldest slot; nobody reads that slot during this step
             if (idx < ROWS || hh == 0) ring[(size_t)cch[k] * 4 + slot] = newv[k];
         }
@@ -129,36 +137,169 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     const float dv = __fadd_rn(dt_in, dt_b);
     const float dt = dv > 20.0f ? dv : log1pf(expf(dv));
     const float dA = expf(__fmul_rn(dt, a_head));
-    const int seg = tid & 7;
+    const int seg = tid & 7, p = tid >> 3;
+    const float xv = xs_s[p];
+    const float dtx = __fmul_rn(dt, xv);
+    float ysum = 0.0f;
 #pragma unroll
-    for (int rr = 0; rr < RS; ++rr) {
-        const int p = 32 * rr + (tid >> 3);
-        const float xv = xs_s[p];
-        const float dtx = __fmul_rn(dt, xv);
-        float ysum = 0.0f;
+    for (int q = 0; q < 4; ++q) {
+        const float4 Bv = reinterpret_cast<const float4*>(B_s)[8 * q + seg];
+        const float4 Cv = reinterpret_cast<const float4*>(C_s)[8 * q + seg];
+        ssu_update(st[q], dA, dtx, Bv, Cv, ysum);
+        srow[8 * q] = st[q];
+    }
+    ysum = ssu_row_sum(ysum);
+    if (seg == 0) {
+        const float y = __fadd_rn(ysum, __fmul_rn(d_head, xv));
+        vout[(size_t)b * d_inner + head * P + p0 + p] = __fmul_rn(y, silu_f(z_gate));
+    }
+}
+
+// Four and more sequences: the launch is bound by the state's trip through the SMs (84 MB in and out at sixteen sequences
+// of 80 heads; 12.9 us at the measured copy rate).  A CTA per half or whole head kept too little of it in flight: the
+// convolution in front of each head's update waits for memory with the SM's registers holding the loads, and 1280
+// CTAs are 2.2 waves of four per SM (20.9 us).  Here one CTA per SM takes a contiguous run of (sequence, head) pairs: a warp
+// brings their 32 KB state matrices into a ring of five slots by bulk copies and sends each back by a bulk copy once
+// sixteen warps have updated it in place; the convolution, the gate and the step sizes of up to kSsuChunk heads are
+// formed together, ahead of the updates, while the ring fills: 19.0 us cold at sixteen sequences, of which about 4 are
+// the launch and the first tile's trip.  Taken from four sequences (two tiles and more per SM): with it a hybrid step of
+// four took 973 us (1249 with the CTA-per-head form and the slower MoE of that time), below that the SMs are not covered.
+// Same arithmetic and sums as the kernel above.
+constexpr int kSsuSlots = 5, kSsuChunk = 12, kSsuWarps = 16;
+constexpr int kSsuThreads = 32 * (kSsuWarps + 1);
+constexpr uint32_t kSsuTileBytes = 64 * 128 * 4;
+constexpr long long kSsuBudgetCycles = 1ll << 31;              // every wait of a CTA gives up after about a second
+
+__global__ void __launch_bounds__(kSsuThreads, 1)
+mamba2_ssu_stream_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr,
+                         const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ A,
+                         const float* __restrict__ dt_bias, const float* __restrict__ Dskip, float* __restrict__ vout,
+                         int d_inner, int conv_dim, int in_out, size_t state_floats, int nheads, int items, int* error_flag) {
+    constexpr int P = 64, N = 128;
+    extern __shared__ __align__(128) unsigned char ring[];
+    __shared__ __align__(8) uint64_t full[kSsuSlots], done[kSsuSlots];
+    __shared__ __align__(16) float B_s[N], C_s[N];
+    __shared__ float xs_s[kSsuChunk * P], zs_s[kSsuChunk * P];
+    __shared__ float dt_s[kSsuChunk], dA_s[kSsuChunk], D_s[kSsuChunk];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int lo = (int)((long long)items * blockIdx.x / gridDim.x), hi = (int)((long long)items * (blockIdx.x + 1) / gridDim.x);
+    const long long deadline = clock64() + kSsuBudgetCycles;
+    if (tid < kSsuSlots) {
+        mbar_init(&full[tid], 1);
+        mbar_init(&done[tid], kSsuWarps);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    grid_dependency_launch();
+    grid_dependency_wait();                  // also orders this launch after the one that wrote the state a step ago
+    auto tile_of = [&](int it) -> float* {
+        return state + (size_t)(it / nheads) * state_floats + (size_t)conv_dim * 4 + (size_t)(it % nheads) * P * N;
+    };
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+        bool ok = mbar_try_wait(bar, parity);
+        while (!ok && !(clock64() > deadline)) ok = mbar_try_wait(bar, parity);
+        return ok;
+    };
+
+    if (warp == kSsuWarps) {
+        // ---------------- the ring: one lane requests, and sends back, tile after tile ------------------------------
+        if (lane == 0) {
+            auto request = [&](int it) {
+                const int slot = (it - lo) % kSsuSlots;
+                mbar_expect_tx(&full[slot], kSsuTileBytes);
+                bulk_load(ring + (size_t)slot * kSsuTileBytes, tile_of(it), kSsuTileBytes, &full[slot]);
+            };
+            int requested = lo;
+            for (; requested < hi && requested < lo + kSsuSlots; ++requested) request(requested);
+            for (int it = lo; it < hi; ++it) {
+                const int slot = (it - lo) % kSsuSlots;
+                if (!wait(&done[slot], (uint32_t)((it - lo) / kSsuSlots) & 1u)) {
+                    // the updating warps gave up: let the copies in flight land, then leave
+                    if (error_flag) atomicExch(error_flag, LSPK_ERR_DEVICE_WAIT);
+                    const long long until = clock64() + kSsuBudgetCycles;
+                    for (int k = it; k < requested; ++k)
+                        while (!mbar_try_wait(&full[(k - lo) % kSsuSlots], (uint32_t)((k - lo) / kSsuSlots) & 1u) && clock64() <= until) {}
+                    break;
+                }
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(tile_of(it)),
+                             "r"(smem_u32(ring + (size_t)slot * kSsuTileBytes)), "r"(kSsuTileBytes)
+                             : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                // the tile before this one has left its slot: refill it
+                if (it > lo && requested < hi) {
+                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    request(requested++);
+                }
+            }
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        }
+        return;
+    }
+
+    const int seg = tid & 7, p = tid >> 3;
+    bool ok = true;
+    for (int i0 = lo; i0 < hi;) {
+        // up to kSsuChunk heads of one sequence: convolution step + SiLU of their x channels and of B and C, gates, step sizes
+        const int b = i0 / nheads, h0 = i0 % nheads;
+        const int n = min(min(hi - i0, kSsuChunk), nheads - h0), nx = n * P;
+        const float* zrow = zx + (size_t)b * in_out;
+        float* conv_ring = state + (size_t)b * state_floats;            // [conv_dim][4]
+        const int pos = pos_ptr[b];
+#pragma unroll 2
+        for (int idx = tid; idx < nx + 2 * N; idx += 32 * kSsuWarps) {
+            const int ch = idx < nx ? h0 * P + idx : d_inner + (idx - nx);
+            const float newv = zrow[d_inner + ch];
+            const float4 taps = *reinterpret_cast<const float4*>(conv_w + (size_t)ch * 4);
+            const float4 hist = *reinterpret_cast<const float4*>(conv_ring + (size_t)ch * 4);
+            const float z = idx < nx ? zrow[h0 * P + idx] : 0.0f;
+            const float act = conv_silu(conv_b[ch], taps, hist, newv, pos);
+            if (idx < nx) {
+                xs_s[idx] = act;
+                zs_s[idx] = silu_f(z);
+            } else if (idx < nx + N) {
+                B_s[idx - nx] = act;
+            } else {
+                C_s[idx - nx - N] = act;
+            }
+            // the newest input replaces the oldest slot; nobody reads that slot during this step
+            if (idx < nx || h0 == 0) conv_ring[(size_t)ch * 4 + (pos & 3)] = newv;
+        }
+        if (tid < n) {
+            const float dv = __fadd_rn(zrow[d_inner + conv_dim + h0 + tid], dt_bias[h0 + tid]);
+            const float dt = dv > 20.0f ? dv : log1pf(expf(dv));
+            dt_s[tid] = dt;
+            dA_s[tid] = expf(__fmul_rn(dt, A[h0 + tid]));
+            D_s[tid] = Dskip[h0 + tid];
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kSsuWarps) : "memory");
+        float4 Bv[4], Cv[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const float4 Bv = *reinterpret_cast<const float4*>(B_s + seg * 20 + q * 4);
-            const float4 Cv = *reinterpret_cast<const float4*>(C_s + seg * 20 + q * 4);
-            float4 s4 = st[rr][q];
-            s4.x = __fadd_rn(__fmul_rn(s4.x, dA), __fmul_rn(dtx, Bv.x));
-            s4.y = __fadd_rn(__fmul_rn(s4.y, dA), __fmul_rn(dtx, Bv.y));
-            s4.z = __fadd_rn(__fmul_rn(s4.z, dA), __fmul_rn(dtx, Bv.z));
-            s4.w = __fadd_rn(__fmul_rn(s4.w, dA), __fmul_rn(dtx, Bv.w));
-            ysum = fmaf(s4.x, Cv.x, ysum);
-            ysum = fmaf(s4.y, Cv.y, ysum);
-            ysum = fmaf(s4.z, Cv.z, ysum);
-            ysum = fmaf(s4.w, Cv.w, ysum);
-            srow[rr][q] = s4;
+            Bv[q] = reinterpret_cast<const float4*>(B_s)[8 * q + seg];
+            Cv[q] = reinterpret_cast<const float4*>(C_s)[8 * q + seg];
         }
-        ysum += __shfl_xor_sync(0xffffffffu, ysum, 4);
-        ysum += __shfl_xor_sync(0xffffffffu, ysum, 2);
-        ysum += __shfl_xor_sync(0xffffffffu, ysum, 1);
-        if (seg == 0) {
-            const int ch = head * P + p0 + p;
-            const float y = __fadd_rn(ysum, __fmul_rn(d_head, xv));
-            vout[(size_t)b * d_inner + ch] = __fmul_rn(y, silu_f(z_gate[rr]));
+        for (int k = 0; k < n && ok; ++k) {
+            const int it = i0 + k - lo, slot = it % kSsuSlots;
+            ok = __all_sync(0xffffffffu, wait(&full[slot], (uint32_t)(it / kSsuSlots) & 1u));
+            if (!ok) break;
+            float4* srow = reinterpret_cast<float4*>(ring + (size_t)slot * kSsuTileBytes) + p * (N / 4) + seg;
+            const float dA = dA_s[k], xv = xs_s[k * P + p], dtx = __fmul_rn(dt_s[k], xv);
+            float ysum = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float4 st = srow[8 * q];
+                ssu_update(st, dA, dtx, Bv[q], Cv[q], ysum);
+                srow[8 * q] = st;
+            }
+            fence_async_smem();                  // the copy back reads what this thread wrote
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&done[slot]);
+            ysum = ssu_row_sum(ysum);
+            if (seg == 0)
+                vout[(size_t)b * d_inner + (h0 + k) * P + p] = __fmul_rn(__fadd_rn(ysum, __fmul_rn(D_s[k], xv)), zs_s[k * P + p]);
         }
+        i0 += n;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kSsuWarps) : "memory");      // the chunk's arrays are rewritten next
     }
 }
 
@@ -195,14 +336,23 @@ int mamba_step(Mamba* m, float* x, float* state, const int* pos, int B) {
     a.eps = m->cfg.eps;
     // several rows: linear_cuda_core quantises them once, straight into the eight-row kernel's tile layout
     if (int rc = linear_cuda_core(&a)) return rc;
-    if (B >= 4)
-        LSPK_CUDA(launch(mamba2_ssu_kernel<64>, dim3(m->cfg.nheads, B), dim3(256), 0, true, (const float*)m->zx, state, pos,
+    const int items = m->cfg.nheads * B;
+    if (B >= 4) {
+        static bool attr_set = false;
+        const size_t smem = (size_t)kSsuSlots * kSsuTileBytes;
+        if (!attr_set) {
+            LSPK_CUDA(cudaFuncSetAttribute(mamba2_ssu_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            attr_set = true;
+        }
+        LSPK_CUDA(launch(mamba2_ssu_stream_kernel, dim3(items < sm_count() ? items : sm_count()), dim3(kSsuThreads), smem, true,
+                         (const float*)m->zx, state, pos, (const float*)m->conv_w, (const float*)m->conv_b, (const float*)m->A,
+                         (const float*)m->dt_bias, (const float*)m->D, m->v, m->d_inner, m->conv_dim, m->in_out,
+                         m->state_floats(), m->cfg.nheads, items, device_wait_flag()));
+    } else {
+        LSPK_CUDA(launch(mamba2_ssu_kernel, dim3(m->cfg.nheads * 2, B), dim3(256), 0, true, (const float*)m->zx, state, pos,
                          (const float*)m->conv_w, (const float*)m->conv_b, (const float*)m->A, (const float*)m->dt_bias,
                          (const float*)m->D, m->v, m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
-    else
-        LSPK_CUDA(launch(mamba2_ssu_kernel<32>, dim3(m->cfg.nheads * 2, B), dim3(256), 0, true, (const float*)m->zx, state, pos,
-                         (const float*)m->conv_w, (const float*)m->conv_b, (const float*)m->A, (const float*)m->dt_bias,
-                         (const float*)m->D, m->v, m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
+    }
     lspk_linear_args o = {};
     o.w[0] = m->out_proj;
     o.out[0] = x;
