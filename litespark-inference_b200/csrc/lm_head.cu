@@ -199,6 +199,11 @@ lm_head_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_scal
 //   int8, int4   the integers become fp16 in registers (bits | 0x6400 is 1024 + value) and x is cut into fp16 terms (11
 //                bits each) after an exact scaling by a power of two
 constexpr int kLmmStepsInFlight = 6;      // K steps of table data in flight per lane (12 x 16 bytes)
+// One CTA per SM (its rows of x fill the shared memory), bound by the table bytes it keeps in flight: a bf16 table takes
+// sixteen warps (two blocks of eight rows, 657 MB: 226 -> 180 us cold).  The integer tables have half and a quarter of
+// the bytes per row, and their decode does not fit the 128 registers of sixteen warps (decode of two sequences with an
+// int8 table: 1.53 ms per step with eight warps, 1.57 with sixteen).
+__host__ __device__ constexpr int lmm_warps(int kind) { return kind == 0 ? 16 : 8; }
 
 template <bool F16>
 __device__ __forceinline__ void lm_mma_16816(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -280,14 +285,15 @@ __device__ __forceinline__ void lmm_operand(const uint4& c, int i, uint32_t a[2]
 // and the table tiles of position b / passes, so the CTAs that need the same table rows run next to each other
 // and the table comes from HBM once (the second reader finds it in L2).
 template <int KIND, int NT>
-__global__ void __launch_bounds__(kLmThreads)
+__global__ void __launch_bounds__(32 * lmm_warps(KIND))
 lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_scale, const float* __restrict__ x,
                    float* __restrict__ logits, int T_all, int V, int H, const void* __restrict__ norm_gamma, int gamma_is_bf16,
                    float eps, unsigned long long* __restrict__ best_keys, int passes) {
     using TR = LmmTraits<KIND>;
+    constexpr int kLmmWarps = lmm_warps(KIND);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* xs = reinterpret_cast<uint16_t*>(smem_raw);
-    __shared__ unsigned long long s_best[kLmWarps][8 * NT];
+    __shared__ unsigned long long s_best[kLmmWarps][8 * NT];
     __shared__ float s_unscale[8 * NT];
     unsigned long long best[NT][2];                          // greedy argmax keys of tokens 8 n + 2 t4 + {0, 1}
 #pragma unroll
@@ -305,7 +311,7 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_
     const size_t row_chunks = (size_t)H / TR::KPL;
 
     // table rows of this warp's first tile can be requested before the activations exist
-    auto tile_of = [&](int i) { return (cta * kLmWarps + warp) + i * ncta * kLmWarps; };
+    auto tile_of = [&](int i) { return (cta * kLmmWarps + warp) + i * ncta * kLmmWarps; };
     uint4 buf[kLmmStepsInFlight][2];
     auto request = [&](int v0, int s0) {
 #pragma unroll
@@ -331,7 +337,7 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_
                              : reinterpret_cast<const float*>(norm_gamma)[k];
     };
     // rows of x (optionally RMS-normalised) -> three 16-bit terms in shared memory, a row per warp (no barrier)
-    for (int r = warp; r < R; r += kLmWarps) {
+    for (int r = warp; r < R; r += kLmmWarps) {
         const float* xr = x + (size_t)r * H;
         float rrms = 1.0f, scale = 1.0f;
         if (r < T && (norm_gamma || TR::kF16)) {
@@ -457,7 +463,7 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_
         if (tid < 8 * NT && tid < T) {
             unsigned long long k = s_best[0][tid];
 #pragma unroll
-            for (int w = 1; w < kLmWarps; ++w) k = s_best[w][tid] > k ? s_best[w][tid] : k;
+            for (int w = 1; w < kLmmWarps; ++w) k = s_best[w][tid] > k ? s_best[w][tid] : k;
             atomicMax(best_keys + tid, k);
         }
     }
@@ -474,7 +480,7 @@ static cudaError_t launch_lm_mma(dim3 grid, size_t smem, const uint4* emb, const
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
-    return launch(kern, grid, dim3(kLmThreads), smem, true, emb, emb_scale, x, logits, T, V, H, norm_gamma, gamma_is_bf16, eps,
+    return launch(kern, grid, dim3(32 * lmm_warps(KIND)), smem, true, emb, emb_scale, x, logits, T, V, H, norm_gamma, gamma_is_bf16, eps,
                   best_key, passes);
 }
 
@@ -509,7 +515,7 @@ int lm_head_launch(int kind, const void* emb, const float* emb_scale, const floa
         const size_t smem = (size_t)3 * rows_per_cta * (H + 32) * 2;
         LSPK_REQUIRE(smem <= 200 * 1024, "lm_head: H=%d too large for %d rows", H, rows_per_cta);
         LSPK_REQUIRE(passes <= sm_count(), "lm_head: too many rows (%d) for one launch", T);
-        int per_pass = (V + 16 * kLmWarps - 1) / (16 * kLmWarps);
+        int per_pass = (V + 16 * lmm_warps(kind) - 1) / (16 * lmm_warps(kind));
         if (per_pass > sm_count() / passes) per_pass = sm_count() / passes;
         const dim3 mgrid(per_pass * passes);
         cudaError_t e;
