@@ -1,0 +1,41 @@
+"""The Mamba-2 state update of four and more sequences (state matrices as a stream through one CTA per SM) at the edges of
+its split: fewer heads than CTAs, sequences shorter than a chunk of heads, runs that cross a sequence, full slot rings."""
+import importlib
+import sys
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+sys.path.insert(0, str(Path(__file__).resolve().parent.parent / "oracle"))
+import oracle_blocks as ob  # noqa: E402
+
+hyb = importlib.import_module("litespark_inference_b200.torchless.hybrid")
+dev = importlib.import_module("litespark_inference_b200.torchless.device")
+
+
+@pytest.mark.parametrize("nheads,B", [(1, 4), (4, 5), (20, 40), (80, 4), (13, 150)])
+def test_streamed_state_update_matches_oracle(port, nheads, B):
+    cfg = hyb.HybridConfig(hidden_size=256, num_layers=2, vocab_size=64, num_experts=2, intermediate_size=64, nheads=nheads,
+                           headdim=64, d_state=128)
+    layer = next(L for L in hyb.random_hybrid(cfg, seed=nheads, norm_jitter=0.1).layers if L.kind == "mamba")
+    dmb = hyb.DeviceMamba(layer, cfg.hidden_size, cfg.rms_norm_eps)
+    state = dev.DeviceArray((B, dmb.state_floats), np.float32)
+    state.fill_bytes(0)
+    picked = sorted({0, 1, B // 2, B - 1})
+    ost = {b: ob.MambaState(layer) for b in picked}
+    rng = np.random.default_rng(B)
+    for step in range(5):                  # more steps than the conv ring has slots
+        x = rng.standard_normal((B, cfg.hidden_size)).astype(np.float32)
+        dx = dev.DeviceArray.from_numpy(x)
+        dmb.step(dx, state, dev.DeviceArray.from_numpy(np.full(B, step, np.int32)), B)
+        got, st = dx.numpy(), state.numpy()
+        for b in picked:
+            want = ob.mamba_layer_step(port, layer, ost[b], x[b], cfg.rms_norm_eps)
+            # the tolerances of test_gpu_hybrid.py: one of 127 quantiser steps on the output, fp32 sums on the state
+            assert np.abs(got[b] - want).max() <= 5e-3 * np.abs(want - x[b]).max(), (step, b)
+            ssm = st[b, layer.conv_dim * 4:].reshape(nheads, 64, 128)
+            assert np.allclose(ssm, ost[b].ssm, rtol=1e-4, atol=1e-4 * np.abs(ost[b].ssm).max()), (step, b)
+    dmb.free()
