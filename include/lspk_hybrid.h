@@ -40,6 +40,10 @@ size_t lspk_moe_device_bytes(lspk_moe_t m);
 int lspk_moe_forward(lspk_moe_t m, float* x_dev, int B, int32_t* sel_out, float* selw_out,
                      int32_t* acc_gate_out, int32_t* acc_up_out, int32_t* acc_down_out);
 
+/* The ring of the expert products of several tokens, for tests (host code only): the slot that the stage-th stage of a CTA
+ * goes through at rows of K values, and the requesting warp that fills it.  A slot has one such warp. */
+int lspk_debug_expert_stage(int K, int stage, int* slot_out, int* producer_out);
+
 /* ---- Mamba-2 decode step ------------------------------------------------------------------- */
 typedef struct lspk_mamba_s* lspk_mamba_t;
 

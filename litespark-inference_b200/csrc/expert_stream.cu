@@ -4,7 +4,7 @@
 // What bounds it: the bytes of the expert matrices that have rows (71 MB of gate / up, 35 MB of down at eight experts
 // of 6912 x 2560).  One CTA per SM; the CTAs are dealt out evenly over the passes (an expert and up to eight of its
 // rows), and a CTA takes a contiguous run of the pass's 16-row groups.  Four warps request the run's stages in order
-// into a shared-memory ring (cp.async.bulk + mbarrier), across pass boundaries; each of twelve consumer warps
+// into a shared-memory ring (cp.async.bulk + mbarrier; a slot always by the same warp), across pass boundaries; each of twelve consumer warps
 // computes whole row groups alone: mma.sync.m16n8k32.u8.s8 on the masked 2-bit fields (operand mapping of
 // linear_mma.cu), no CTA-wide barrier and no cross-warp sum per row group.  (The eight-row kernel used here before
 // cut every row group along K over its eight warps: two barriers and a reduction through shared memory per 20 KB.)
@@ -24,6 +24,12 @@ constexpr int kEStageBytes = kEStageChunks * kRowsPerGroup * 16;   // 10 KB
 constexpr int kESlotsMax = 20;
 constexpr int kET = 8;                                             // rows per pass: the MMA's N
 constexpr int kESmem = 225 * 1024;                                 // dynamic shared memory to share out
+// The requesting warp of a stage follows from its slot.  A slot is then filled by one warp from first to last, which the
+// phase test in front of a refill needs: the warp has itself seen the release before the one it waits for, so the
+// barrier is at most one phase away from the tested parity.  (Dealt out by stage number, with a slot count that is no
+// multiple of the warps -- K = 6912 leaves 17 -- a warp two releases ahead of a slow reader takes an old phase for its own
+// and overwrites the stage being read.)
+__host__ __device__ constexpr int e_producer_of_slot(int slot) { return slot % kEProducers; }
 constexpr long long kEBudgetCycles = 1ll << 31;                    // every wait of a CTA gives up after about a second
 
 __device__ __forceinline__ void e_consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEConsumers) : "memory"); }
@@ -106,7 +112,7 @@ ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
     const int sub = p.sub, cps = p.cps, chunks = p.chunks;
 
     if (warp >= kEConsumers) {
-        // ---------------- producers: warp pw requests stages pw, pw + kEProducers, ... as slots come free ------------
+        // ---------------- producers: warp pw requests the stages of its slots in order, as the slots come free -------
         const int pw = warp - kEConsumers;
         uint64_t policy;
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
@@ -120,8 +126,8 @@ ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
             const uint4* ub = p.w[PAIR ? 1 : 0] + off;
             for (int g = g_lo; g < g_hi && ok; ++g) {
                 for (int s = 0; s < sub; ++s, ++q) {
-                    if (q % kEProducers != pw) continue;
                     const int slot = q % p.slots;
+                    if (e_producer_of_slot(slot) != pw) continue;
                     if (q >= p.slots) {          // the slot's previous occupant has to be consumed first
                         const uint32_t parity = (uint32_t)(q / p.slots - 1) & 1u;
                         bool freed = mbar_try_wait(&empty[slot], parity);
@@ -319,12 +325,17 @@ ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
     tr.end();
 }
 
+static int expert_slots(int chunks) {
+    const size_t rows = (size_t)kET * mma_row_stride(chunks * kWeightsPerChunk);
+    const int slots = rows < (size_t)kESmem ? (int)((kESmem - rows) / kEStageBytes) : 0;
+    return slots < kESlotsMax ? slots : kESlotsMax;
+}
+
 int expert_stream_launch(ExpertStreamParams p, bool pair) {
     const size_t rows = (size_t)kET * mma_row_stride(p.chunks * kWeightsPerChunk);
-    int slots = rows < (size_t)kESmem ? (int)((kESmem - rows) / kEStageBytes) : 0;
+    p.slots = expert_slots(p.chunks);
     // three slots keep the ring turning at the longest rows (K of about 24000); the model shapes have 17 to 20
-    LSPK_REQUIRE(slots >= 3, "expert products: K=%d too large for eight rows in shared memory (limit about 24000)", p.K);
-    p.slots = slots < kESlotsMax ? slots : kESlotsMax;
+    LSPK_REQUIRE(p.slots >= 3, "expert products: K=%d too large for eight rows in shared memory (limit about 24000)", p.K);
     p.cps = kEStageChunks / (pair ? 2 : 1);
     p.sub = (p.chunks + p.cps - 1) / p.cps;
     p.error_flag = device_wait_flag();
@@ -338,3 +349,13 @@ int expert_stream_launch(ExpertStreamParams p, bool pair) {
 }
 
 }  // namespace lspk
+
+extern "C" int lspk_debug_expert_stage(int K, int stage, int* slot_out, int* producer_out) {
+    using namespace lspk;
+    LSPK_REQUIRE(K >= 4 && stage >= 0 && slot_out && producer_out, "lspk_debug_expert_stage: bad arguments");
+    const int slots = expert_slots((K + kWeightsPerChunk - 1) / kWeightsPerChunk);
+    LSPK_REQUIRE(slots >= 3, "lspk_debug_expert_stage: K=%d has no ring", K);
+    *slot_out = stage % slots;
+    *producer_out = e_producer_of_slot(*slot_out);
+    return LSPK_OK;
+}

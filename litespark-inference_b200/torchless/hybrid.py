@@ -34,6 +34,7 @@ SIGNATURES = {
     "lspk_moe_free": ([_vp], _ci),
     "lspk_moe_device_bytes": ([_vp], _sz),
     "lspk_moe_forward": ([_vp, _vp, _ci, _vp, _vp, _vp, _vp, _vp], _ci),
+    "lspk_debug_expert_stage": ([_ci, _ci, _vp, _vp], _ci),
     "lspk_mamba_create": ([ctypes.POINTER(MambaConfigC), _vp, _cf, _vp, _cf, _vp, _vp, _vp, _vp, _vp, _vp, _vp], _vp),
     "lspk_mamba_free": ([_vp], _ci),
     "lspk_mamba_device_bytes": ([_vp], _sz),

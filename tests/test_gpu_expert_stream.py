@@ -54,3 +54,26 @@ def test_expert_products_match_oracle(port, hidden, inter, experts, B):
         # one of 127 steps of the second quantiser, on an output that sums sqrt(inter) of them: below 5e-3 of its peak
         assert np.abs(got[t] - want).max() <= 5e-3 * np.abs(want - x[t]).max()
     assert exact > 0
+
+
+def test_many_passes_equal_single_tokens():
+    """The model's matrices and enough rows that a CTA's share turns the ring of the down stage (17 slots at K = 6912)
+    several times, where every slot has to keep its requesting warp: each row as the one-token kernels compute it, which
+    are other code and share its integer sums and roundings, so equal to the bit; and the same again on every run."""
+    cfg = hyb.HybridConfig(hidden_size=2560, num_layers=2, vocab_size=64, num_experts=8, intermediate_size=6912, nheads=2,
+                           headdim=64, d_state=128)
+    layer = next(L for L in hyb.random_hybrid(cfg, seed=8, norm_jitter=0.1).layers if L.kind == "moe")
+    dm = hyb.DeviceMoE(layer, cfg.rms_norm_eps)
+    B = 64
+    x = np.random.default_rng(64).standard_normal((B, 2560)).astype(np.float32)
+    runs = []
+    for _ in range(6):
+        dx = dev.DeviceArray.from_numpy(x)
+        dm.forward(dx, B)
+        runs.append(dx.numpy())
+    assert all(np.array_equal(r, runs[0]) for r in runs)
+    for t in range(B):
+        one = dev.DeviceArray.from_numpy(x[t:t + 1])
+        dm.forward(one, 1)
+        assert np.array_equal(one.numpy()[0], runs[0][t]), t
+    dm.free()
