@@ -467,28 +467,53 @@ int linear_launch_params(const LinearParams& p, int mt, bool pair, int grid_x, i
     return LSPK_OK;
 }
 
-// Host-side validation + launch of the CUDA-core kernel.  Used by lspk_linear and by the
-// forward pass.
-int linear_cuda_core(const lspk_linear_args* a) {
+// What a call has to bring, whichever kernel takes it.
+static int check_linear_args(const lspk_linear_args* a) {
     LSPK_REQUIRE(a, "linear: null args");
     LSPK_REQUIRE(a->n_mats >= 1 && a->n_mats <= 3, "linear: n_mats must be 1..3 (got %d)", a->n_mats);
     LSPK_REQUIRE(a->M >= 1, "linear: M must be >= 1 (got %d)", a->M);
+    LSPK_REQUIRE(a->epilogue >= LSPK_EPI_STORE && a->epilogue <= LSPK_EPI_SILU_MUL, "linear: unknown epilogue %d", a->epilogue);
     const bool pair = a->epilogue == LSPK_EPI_RELU2_MUL || a->epilogue == LSPK_EPI_SILU_MUL;
     LSPK_REQUIRE(!pair || a->n_mats == 2, "linear: the gated epilogues take exactly two matrices (gate, up)");
-    LinearParams p = {};
     const Weight* w0 = reinterpret_cast<const Weight*>(a->w[0]);
     LSPK_REQUIRE(w0, "linear: null weight");
+    for (int i = 0; i < a->n_mats; ++i) {
+        const Weight* w = reinterpret_cast<const Weight*>(a->w[i]);
+        LSPK_REQUIRE(w && w->K == w0->K, "linear: matrices must share K");
+        LSPK_REQUIRE(a->out[i] || (pair && i == 1), "linear: null output");
+        LSPK_REQUIRE(!pair || w->N == w0->N, "linear: gate and up must have the same N");
+    }
+    switch (a->prologue) {
+        case LSPK_PRO_INT8:
+            LSPK_REQUIRE(a->x_i8 && a->x_scales, "linear: INT8 prologue needs x_i8 and x_scales");
+            break;
+        case LSPK_PRO_GATED_RMSNORM_QUANT:
+            LSPK_REQUIRE(a->gate_f32, "linear: GATED_RMSNORM_QUANT prologue needs gate_f32");
+            /* fallthrough */
+        case LSPK_PRO_RMSNORM_QUANT:
+            LSPK_REQUIRE(a->gamma, "linear: RMSNORM_QUANT prologue needs gamma");
+            /* fallthrough */
+        case LSPK_PRO_QUANT:
+            LSPK_REQUIRE(a->x_f32, "linear: fp32 prologue needs x_f32");
+            break;
+        default:
+            return fail(LSPK_ERR_ARG, "linear: unknown prologue %d", a->prologue);
+    }
+    return LSPK_OK;
+}
+
+// Host-side validation + launch of the CUDA-core kernel.  Used by lspk_linear and by the
+// forward pass.
+int linear_cuda_core(const lspk_linear_args* a) {
+    if (int rc = check_linear_args(a)) return rc;
+    const bool pair = a->epilogue == LSPK_EPI_RELU2_MUL || a->epilogue == LSPK_EPI_SILU_MUL;
+    LinearParams p = {};
+    const Weight* w0 = reinterpret_cast<const Weight*>(a->w[0]);
     // Several rows of fp32 input: normalise + quantise them once in their own kernel (fused into the
     // product, every CTA would repeat that work for all rows) and continue with the int8 prologue.
     lspk_linear_args split;
     const int* tiled_sums = nullptr;
     if (a->M > 1 && a->prologue != LSPK_PRO_INT8) {
-        LSPK_REQUIRE(a->prologue >= LSPK_PRO_QUANT && a->prologue <= LSPK_PRO_GATED_RMSNORM_QUANT,
-                     "linear: unknown prologue %d", a->prologue);
-        LSPK_REQUIRE(a->x_f32, "linear: fp32 prologue needs x_f32");
-        LSPK_REQUIRE(a->prologue == LSPK_PRO_QUANT || a->gamma, "linear: RMSNORM_QUANT prologue needs gamma");
-        LSPK_REQUIRE(a->prologue != LSPK_PRO_GATED_RMSNORM_QUANT || a->gate_f32,
-                     "linear: GATED_RMSNORM_QUANT prologue needs gate_f32");
         split = *a;
         int8_t* q = nullptr;
         float* sc = nullptr;
@@ -522,9 +547,6 @@ int linear_cuda_core(const lspk_linear_args* a) {
     int groups = 0;
     for (int i = 0; i < a->n_mats; ++i) {
         const Weight* w = reinterpret_cast<const Weight*>(a->w[i]);
-        LSPK_REQUIRE(w && w->K == p.K, "linear: matrices must share K");
-        LSPK_REQUIRE(pair ? (i == 1 || a->out[i] != nullptr) : a->out[i] != nullptr, "linear: null output");
-        LSPK_REQUIRE(!pair || w->N == w0->N, "linear: gate and up must have the same N");
         p.seg[i] = LinearSeg{w->dev, a->out[i], a->acc_out[i], w->N, w->groups, w->scale};
         groups += w->groups;
     }
@@ -547,26 +569,6 @@ int linear_cuda_core(const lspk_linear_args* a) {
     p.trace = trace_buffer();
     p.trace_cap = trace_capacity();
     p.error_flag = device_wait_flag();
-    switch (a->prologue) {
-        case kProInt8Tiled:                      // set above, never by a caller
-            LSPK_REQUIRE(tiled_sums != nullptr, "linear: unknown prologue %d", a->prologue);
-            break;
-        case LSPK_PRO_INT8:
-            LSPK_REQUIRE(a->x_i8 && a->x_scales, "linear: INT8 prologue needs x_i8 and x_scales");
-            break;
-        case LSPK_PRO_GATED_RMSNORM_QUANT:
-            LSPK_REQUIRE(a->gate_f32, "linear: GATED_RMSNORM_QUANT prologue needs gate_f32");
-            /* fallthrough */
-        case LSPK_PRO_RMSNORM_QUANT:
-            LSPK_REQUIRE(a->gamma, "linear: RMSNORM_QUANT prologue needs gamma");
-            /* fallthrough */
-        case LSPK_PRO_QUANT:
-            LSPK_REQUIRE(a->x_f32, "linear: fp32 prologue needs x_f32");
-            break;
-        default:
-            return fail(LSPK_ERR_ARG, "linear: unknown prologue %d", a->prologue);
-    }
-    LSPK_REQUIRE(a->epilogue >= 0 && a->epilogue <= 3, "linear: unknown epilogue %d", a->epilogue);
     const int MT = a->M == 1 ? 1 : 8;
     // At most two CTAs per SM when there is a single token tile (measured best on B200: the prologue
     // runs once per CTA, which then loops over its row groups).  With several token tiles the grid's
@@ -593,7 +595,7 @@ extern "C" int lspk_linear_force_path(int path) {
 
 extern "C" int lspk_linear(const lspk_linear_args* a) {
     if (int rc = ensure_init()) return rc;
-    LSPK_REQUIRE(a, "lspk_linear: null args");
+    if (int rc = check_linear_args(a)) return rc;
     if (a->prologue != LSPK_PRO_INT8) {
         LSPK_REQUIRE(((uintptr_t)a->x_f32 & 15) == 0 && ((uintptr_t)a->gate_f32 & 15) == 0,
                      "lspk_linear: x_f32 / gate_f32 must be 16-byte aligned");
