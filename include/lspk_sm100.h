@@ -48,7 +48,7 @@ int lspk_sm_count(void);
 const char* lspk_last_error(void);      /* last recorded message ("" if none)            */
 int lspk_error_count(void);             /* number of failures recorded so far            */
 void lspk_clear_error(void);
-int lspk_set_pdl(int enabled);          /* programmatic dependent launch between kernels */
+int lspk_set_pdl(int enabled);          /* programmatic dependent launch between kernels, from the next launch or capture on */
 int lspk_sync(void);                    /* wait for everything queued on the stream      */
 
 void* lspk_malloc(size_t bytes);        /* device memory; NULL on failure                */
@@ -69,8 +69,9 @@ int lspk_timer_stop(float* ms_out);
 /* In-kernel phase trace (measurement aid): after lspk_trace_begin, CTA 0 of each traced kernel
  * appends a record of 16 uint64 words [kernel id, globaltimer ns at entry, SM clock at phase marks
  * ..., globaltimer ns at exit]; lspk_trace_read copies the records out and clears the counter.
- * Kernels captured into a CUDA graph before lspk_trace_begin do not record; a later call with the same or a
- * smaller max_records keeps the buffer (graphs captured in between stay valid), a larger one replaces it. */
+ * A state's CUDA graph captured before the first lspk_trace_begin does not record; a later call with the same or a
+ * smaller max_records keeps the buffer (graphs captured in between stay valid), a larger one replaces it (the library
+ * captures its graphs again before their next launch). */
 int lspk_trace_begin(int max_records);
 int lspk_trace_read(unsigned long long* host_out, int max_records, int* n_out);
 

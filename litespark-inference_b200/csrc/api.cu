@@ -151,6 +151,8 @@ void lspk_clear_error(void) {
 }
 
 int lspk_set_pdl(int enabled) {
+    // a parked state's graph holds the launch attributes of its capture: the next state captures anew
+    if (g_pdl != (enabled != 0)) release_parked_states();
     g_pdl = enabled != 0;
     return LSPK_OK;
 }
@@ -235,16 +237,19 @@ int lspk_trace_begin(int max_records) {
     if (int rc = ensure_init()) return rc;
     LSPK_REQUIRE(max_records >= 1, "lspk_trace_begin: max_records must be positive");
     // A buffer that is large enough is kept (only its counter is cleared): graphs captured while it was
-    // installed hold its address.  A larger one replaces it; such graphs must then be rebuilt by their owner.
+    // installed hold its address.  A larger one replaces it, and such graphs are captured again before their next
+    // launch.  The graphs of parked states go in either case: a state made from here on records.
     if (g_trace && max_records <= g_trace_cap) {
         LSPK_CUDA(cudaDeviceSynchronize());
         LSPK_CUDA(cudaMemset(g_trace, 0, 8));
         LSPK_CUDA(cudaDeviceSynchronize());
         return LSPK_OK;
     }
+    release_parked_states();
     if (g_trace) {
         LSPK_CUDA(cudaDeviceSynchronize());
         cudaFree(g_trace);
+        scratch_moved();
     }
     g_trace = nullptr;
     g_trace_cap = 0;

@@ -1,5 +1,8 @@
 """Inference states that are freed and made again, and the LM head's table formats."""
 import importlib
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -45,6 +48,70 @@ def test_a_state_made_again_is_a_new_state():
     dm2.close()
     late.close()                                                         # its model is gone
     dm.close()
+
+
+_TRACE_AND_LAUNCH_MODE = """
+import ctypes, importlib
+import numpy as np
+import __graft_entry__ as entry
+entry.load_package()
+K = importlib.import_module("litespark_inference_b200.torchless.kernel")
+rt = importlib.import_module("litespark_inference_b200.torchless.runtime")
+synthetic = importlib.import_module("litespark_inference_b200.torchless.synthetic")
+dm = rt.DeviceModel(synthetic.random_model(synthetic.toy_config(), seed=3))
+lib = dm.lib
+
+def records():
+    n, out = ctypes.c_int(), np.zeros((4096, 16), np.uint64)
+    K.check(lib.lspk_trace_read(out.ctypes.data, 4096, ctypes.byref(n)))
+    return n.value
+
+def free_bytes():
+    f = ctypes.c_size_t()
+    K.check(lib.lspk_mem_info(ctypes.byref(f), None))
+    return f.value
+
+def one_step(st):
+    return rt.forward_one(dm, st, 5)
+
+st = rt.init_state(dm, 64)
+want = one_step(st)
+st.close()                                   # its graph was captured without a trace
+K.check(lib.lspk_trace_begin(64))
+st = rt.init_state(dm, 64)
+assert np.array_equal(one_step(st), want)
+per_step = records()
+assert per_step > 0
+st.close()
+K.check(lib.lspk_trace_begin(32))            # fits the buffer: a state made again keeps its graph and records
+st = rt.init_state(dm, 64)
+assert np.array_equal(one_step(st), want) and records() == per_step
+K.check(lib.lspk_trace_begin(2048))          # replaces the buffer under a live state ...
+assert rt.forward_one(dm, st, 7).shape == want.shape and records() > 0
+st.close()
+K.check(lib.lspk_trace_begin(4096))          # ... and under a freed one
+st = rt.init_state(dm, 64)
+assert np.array_equal(one_step(st), want) and records() > 0
+st.close()
+st = rt.init_state(dm, 8192, batch=8, kv_dtype="fp32")     # large enough to show in the free memory; parked in its place
+held = st.device_bytes
+assert held > 50e6
+st.close()
+before = free_bytes()
+K.check(lib.lspk_set_pdl(1))                 # no change: the freed state stays
+assert free_bytes() == before
+K.check(lib.lspk_set_pdl(0))
+assert free_bytes() >= before + held // 2
+st = rt.init_state(dm, 64)
+assert np.array_equal(one_step(st), want)
+"""
+
+
+def test_a_state_made_after_a_trace_or_launch_mode_change_uses_it():
+    """In a process of its own: the trace buffer stays installed."""
+    r = subprocess.run([sys.executable, "-c", _TRACE_AND_LAUNCH_MODE], cwd=Path(__file__).resolve().parent.parent,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("kind", [0, 1, 2])
