@@ -60,7 +60,7 @@ static int enqueue_hybrid_step(HybridState* s) {
     } else {
         // several sequences: the LM head returns each row's greedy choice itself (logits only where its
         // tensor-core form does not apply and a row argmax has to read them)
-        if (int rc = lm_head_launch(0, m->emb, nullptr, s->x, (m->H % 32) ? s->logits : nullptr, B, m->V, m->H,
+        if (int rc = lm_head_launch(0, m->emb, nullptr, s->x, lm_head_rows_on_tensor_cores(0, B, m->H) ? nullptr : s->logits, B, m->V, m->H,
                                     m->final_norm, 1, m->eps, s->best))
             return rc;
     }

@@ -76,7 +76,7 @@ int lm_head_launch(int kind, const void* emb, const float* emb_scale, const floa
                    int T, int V, int H, const void* norm_gamma, int gamma_is_bf16, float eps,
                    unsigned long long* best_key);
 
-bool lm_head_rows_on_tensor_cores(int kind, int H);      // several rows: argmax without a logits buffer
+bool lm_head_rows_on_tensor_cores(int kind, int T, int H);   // several rows: argmax without a logits buffer
 
 // runtime.cu: small kernels of a decode step, shared with the hybrid runtime.
 //   ctl layout: pos[batch], token[batch], step counter.

@@ -484,8 +484,19 @@ static cudaError_t launch_lm_mma(dim3 grid, size_t smem, const uint4* emb, const
                   best_key, passes);
 }
 
-// Whether several rows go to the tensor-core kernel (a K step of it is 32, 64 or 128 wide).
-bool lm_head_rows_on_tensor_cores(int kind, int H) { return H % (kind == 0 ? 32 : kind == 1 ? 64 : 128) == 0; }
+// Rows of x that a CTA of the tensor-core kernel holds: sixteen where their three 16-bit terms fit the shared memory
+// (H <= 2101) and there are as many, else eight (H <= 4234), else none.
+static int lmm_rows_per_cta(int T, int H) {
+    auto fits = [&](int rows) { return (size_t)3 * rows * (H + 32) * 2 <= 200 * 1024; };
+    return T > 8 && fits(16) ? 16 : fits(8) ? 8 : 0;
+}
+
+// Whether T rows go to the tensor-core kernel: a K step of it is 32, 64 or 128 wide, its rows have to fit the shared
+// memory, and every block of rows needs a CTA.
+bool lm_head_rows_on_tensor_cores(int kind, int T, int H) {
+    const int rows = lmm_rows_per_cta(T, H);
+    return T > 1 && H % (kind == 0 ? 32 : kind == 1 ? 64 : 128) == 0 && rows && (T + rows - 1) / rows <= sm_count();
+}
 
 // norm_gamma / best_key may be null; best_key points at T keys (one greedy argmax per row of x, combined with
 // atomicMax: the caller clears them).  Larger T is tiled here.
@@ -505,16 +516,12 @@ int lm_head_launch(int kind, const void* emb, const float* emb_scale, const floa
     const int cap = sm_count() * 4;
     if (grid > cap) grid = cap;
     const uint4* e4 = reinterpret_cast<const uint4*>(emb);
-    if (T > 1 && lm_head_rows_on_tensor_cores(kind, H) && (logits || best_key) && ((uintptr_t)x & 15) == 0) {
-        // several rows: tensor-core kernel.  A CTA holds sixteen rows where their three 16-bit
-        // terms fit the shared memory (H <= 2100), else eight; more rows than that are row blocks served side by
+    if (lm_head_rows_on_tensor_cores(kind, T, H) && (logits || best_key) && ((uintptr_t)x & 15) == 0) {
+        // several rows: tensor-core kernel.  More rows than a CTA holds are row blocks served side by
         // side in one launch (the kernel's `passes`), so the table is read from HBM once
-        const int nt = ((size_t)3 * 16 * (H + 32) * 2 <= 200 * 1024 && T > 8) ? 2 : 1;
-        const int rows_per_cta = 8 * nt;
+        const int rows_per_cta = lmm_rows_per_cta(T, H), nt = rows_per_cta / 8;
         const int passes = (T + rows_per_cta - 1) / rows_per_cta;
         const size_t smem = (size_t)3 * rows_per_cta * (H + 32) * 2;
-        LSPK_REQUIRE(smem <= 200 * 1024, "lm_head: H=%d too large for %d rows", H, rows_per_cta);
-        LSPK_REQUIRE(passes <= sm_count(), "lm_head: too many rows (%d) for one launch", T);
         int per_pass = (V + 16 * lmm_warps(kind) - 1) / (16 * lmm_warps(kind));
         if (per_pass > sm_count() / passes) per_pass = sm_count() / passes;
         const dim3 mgrid(per_pass * passes);

@@ -348,9 +348,9 @@ static int enqueue_step(State* s, bool store_logits, bool host_io = false) {
         if (int rc = lm_head_launch(head.kind, head.data, head.scale, s->x, store_logits ? s->logits : nullptr, 1, V, H,
                                     m->final_norm.g, m->final_norm.is_bf16, c.rms_norm_eps, s->best)) return rc;
     } else {
-        // the greedy choice of every row comes out of the LM head itself (or, for odd hidden sizes, of a row argmax it
-        // launches); logits are written only where something reads them
-        const bool need_logits = store_logits || !lm_head_rows_on_tensor_cores(head.kind, H);
+        // the greedy choice of every row comes out of the LM head itself (or, for odd and for long rows, of a row argmax
+        // it launches); logits are written only where something reads them
+        const bool need_logits = store_logits || !lm_head_rows_on_tensor_cores(head.kind, B, H);
         if (int rc = lm_head_launch(head.kind, head.data, head.scale, s->x, need_logits ? s->logits : nullptr, B, V, H,
                                     m->final_norm.g, m->final_norm.is_bf16, c.rms_norm_eps, s->best)) return rc;
     }

@@ -140,3 +140,55 @@ def test_lm_head_formats(kind, T, H):
     # fp32 sums of H products in any order: H * 2^-24 of the sum of their magnitudes at the very most
     bound = H * 2.0**-24 * (np.abs(x).astype(np.float64) @ np.abs(vals).T) + 1e-30
     assert (np.abs(dl.numpy() - want) <= bound).all()
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+# rows whose three 16-bit terms are the longest that fit the tensor-core kernel and the next longer, a wide model's hidden
+# size, the widest that the eight rows of the other kernel fit; more rows than its CTAs take
+@pytest.mark.parametrize("T,H", [(8, 4224), (2, 4352), (2, 5120), (8, 5120), (9, 5120), (2, 25600), (8, 6400), (1190, 128)])
+def test_lm_head_rows_of_any_width(kind, T, H):
+    rng = np.random.default_rng(H + T)
+    V = 67
+    x = rng.standard_normal((T, H)).astype(np.float32)
+    sc = rng.uniform(0.5, 1.5, V).astype(np.float32)
+    if kind == 0:
+        table = (rng.standard_normal((V, H)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        vals = (table.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    elif kind == 1:
+        table = rng.integers(-128, 128, (V, H)).astype(np.int8)
+        vals = table * sc.astype(np.float64)[:, None]
+    else:
+        table = rng.integers(0, 256, (V, H // 2)).astype(np.uint8)
+        n = np.stack([table & 15, table >> 4], axis=-1).reshape(V, H).astype(np.int64)
+        vals = (n - 16 * (n > 7)) * sc.astype(np.float64)[:, None]
+    de, ds, dx = dev.DeviceArray.from_numpy(table), dev.DeviceArray.from_numpy(sc), dev.DeviceArray.from_numpy(x)
+    dl = dev.DeviceArray((T, V), np.float32)
+    K.check(K.load_library().lspk_lm_head(kind, de.ptr, ds.ptr if kind else None, dx.ptr, dl.ptr, T, V, H))
+    # as in test_lm_head_formats
+    bound = H * 2.0**-24 * (np.abs(x).astype(np.float64) @ np.abs(vals).T)
+    assert (np.abs(dl.numpy() - x.astype(np.float64) @ vals.T) <= bound).all()
+
+
+@pytest.mark.parametrize("table", ["bf16", "int8", "int4"])
+def test_batched_decode_of_a_wide_model(table):
+    """A hidden size beyond the tensor-core LM head: the greedy choice of several sequences comes from a row argmax."""
+    cfg = synthetic.toy_config(hidden=5120, layers=1, heads=40, kv_heads=8, inter=256, vocab=256)
+    m = synthetic.random_model(cfg, seed=2, norm_jitter=0.1)
+    loader = importlib.import_module("litespark_inference_b200.torchless.loader")
+    if table != "bf16":
+        q, m.embed_scale = loader.quantize_embedding(m.embed_tokens, 127 if table == "int8" else 7)
+        setattr(m, "embed_" + table, q)
+        m.embed_tokens = None
+    dm = rt.DeviceModel(m)
+    st = rt.init_state(dm, 32, batch=2)
+    toks = np.array([3, 77], np.int32)
+    for _ in range(4):
+        nxt, logits = rt.forward_step(st, toks, want_logits=True)
+        assert list(nxt) == [int(np.argmax(r)) for r in logits]
+        toks = nxt
+    ids = np.empty((3, 2), np.int32)
+    K.check(dm.lib.lspk_decode_greedy(st.handle, toks.ctypes.data, 3, ids.ctypes.data))
+    st.close()
+    rows = rt.forward_prefill_all_logits(dm, rt.init_state(dm, 32), [1, 2, 3, 4, 5])
+    assert np.isfinite(rows).all()
+    dm.close()
