@@ -193,11 +193,14 @@ lm_head_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_scal
 // the N side (one or two tiles of eight), and the table bytes go from global memory straight into A
 // fragments: lane (g, t) loads 16 bytes of row g and of row g + 8 per K step; which k's a
 // lane holds is a permutation of K that the x fragments repeat, so no shuffle is needed.
-// x stays fp32-exact: it is split into three 16-bit terms, each product is exact in the fp32 accumulator, so the
-// result differs from the fp32 dot product only in summation order, like every other reduction here.
-//   bf16 table   bf16 terms (8 bits each, the range of fp32)
+// x stays fp32-exact: it is split into three 16-bit terms, and each product is exact in the fp32 accumulator.
+//   bf16 table   bf16 terms (8 bits each, the range of fp32).  The whole dot product is one chain through the MMA's
+//                accumulator, which truncates: 8.7e-6 of the 2-norm of the products at H = 2560 (one row, in the kernel
+//                above: 1.7e-7).  Its sixteen warps already use all of their 128 registers; fresh sums are untried there.
 //   int8, int4   the integers become fp16 in registers (bits | 0x6400 is 1024 + value) and x is cut into fp16 terms (11
-//                bits each) after an exact scaling by a power of two
+//                bits each) after an exact scaling by a power of two.  The three products of 16 values start from zero
+//                and are added up in fp32, first within a batch of loads: 1.1e-7 (chained it was 5.7e-6), at no cost (eight
+//                rows, 128256 x 2560: int8 94 us, int4 96; chained 96 and 100)
 constexpr int kLmmStepsInFlight = 6;      // K steps of table data in flight per lane (12 x 16 bytes)
 // One CTA per SM (its rows of x fill the shared memory), bound by the table bytes it keeps in flight: a bf16 table takes
 // sixteen warps (two blocks of eight rows, 657 MB: 226 -> 180 us cold).  The integer tables have half and a quarter of
@@ -401,6 +404,11 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_
                 const int nt = tile_of(it + 1);
                 if (nt * 16 < V) request(nt * 16, 0);
             }
+            float part[NT][4];                                       // this batch's sums (integer tables)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) part[n][c] = 0.0f;
 #pragma unroll
             for (int u = 0; u < kLmmStepsInFlight; ++u) {
                 const int sidx = s0 + u;
@@ -415,17 +423,31 @@ lm_head_mma_kernel(const uint4* __restrict__ emb, const float* __restrict__ emb_
                         const int piece = KIND == 2 ? j ^ (t4 >> 1) : j;
 #pragma unroll
                         for (int n = 0; n < NT; ++n) {
+                            float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+                            float* const d0 = TR::kF16 ? c0 : acc[n];
+                            float* const d1 = TR::kF16 ? c1 : acc[n];
 #pragma unroll
-                            for (int term = 0; term < 3; ++term) {
+                            for (int i = 0; i < 3; ++i) {
+                                const int term = TR::kF16 ? 2 - i : i;      // smallest first into a fresh sum
                                 // this lane's B data: token row 8 n + g, the k's of its table load
                                 const uint4 b = *reinterpret_cast<const uint4*>(
                                     xs + (size_t)(term * R + 8 * n + g) * ld + (size_t)sidx * TR::kStep + t4 * TR::KPL + piece * 8);
-                                lm_mma_16816<TR::kF16>(acc[n], lo0[0], hi0[0], lo0[1], hi0[1], b.x, b.y);
-                                lm_mma_16816<TR::kF16>(acc[n], lo1[0], hi1[0], lo1[1], hi1[1], b.z, b.w);
+                                lm_mma_16816<TR::kF16>(d0, lo0[0], hi0[0], lo0[1], hi0[1], b.x, b.y);
+                                lm_mma_16816<TR::kF16>(d1, lo1[0], hi1[0], lo1[1], hi1[1], b.z, b.w);
+                            }
+                            if (TR::kF16) {
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) part[n][c] += c0[c] + c1[c];
                             }
                         }
                     }
                 }
+            }
+            if (TR::kF16) {
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[n][c] += part[n][c];
             }
         }
         // C fragment: c0, c1 = (table row g, tokens 2 t4, 2 t4 + 1), c2, c3 = (table row g + 8, same tokens)

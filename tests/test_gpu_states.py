@@ -192,3 +192,34 @@ def test_batched_decode_of_a_wide_model(table):
     rows = rt.forward_prefill_all_logits(dm, rt.init_state(dm, 32), [1, 2, 3, 4, 5])
     assert np.isfinite(rows).all()
     dm.close()
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("T,H", [(2, 256), (8, 2560), (9, 640), (16, 2560), (2, 4096)])
+def test_lm_head_rows_as_accurate_as_one_row(kind, T, H):
+    """The tensor-core form for several rows against the one-row kernel (fp32 multiply-adds): as close to float64."""
+    rng = np.random.default_rng(kind * 10 + H)
+    V = 2003
+    x = rng.standard_normal((T, H)).astype(np.float32)
+    if kind == 1:
+        table = rng.integers(-128, 128, (V, H)).astype(np.int8)
+        vals = table.astype(np.float64)
+    else:
+        table = rng.integers(0, 256, (V, H // 2)).astype(np.uint8)
+        n = np.stack([table & 15, table >> 4], axis=-1).reshape(V, H).astype(np.int64)
+        vals = (n - 16 * (n > 7)).astype(np.float64)
+    de, ds = dev.DeviceArray.from_numpy(table), dev.DeviceArray.from_numpy(np.ones(V, np.float32))
+
+    def logits(rows):
+        dx, dl = dev.DeviceArray.from_numpy(rows), dev.DeviceArray((rows.shape[0], V), np.float32)
+        K.check(K.load_library().lspk_lm_head(kind, de.ptr, ds.ptr, dx.ptr, dl.ptr, rows.shape[0], V, H))
+        return dl.numpy()
+
+    want = x.astype(np.float64) @ vals.T
+    norm = np.sqrt(x.astype(np.float64) ** 2 @ (vals ** 2).T)
+    err = [np.sqrt(np.mean(((got - want) / norm) ** 2)) for got in (logits(x), np.concatenate([logits(r[None]) for r in x]))]
+    # the one-row sums round H / 32 times per lane and five times across lanes; tensor-core sums of 48 products truncate
+    # once each, and some dozens of them are added: no more, up to the scatter of two rounding patterns
+    assert err[0] <= 1.15 * err[1], err
+    # an fp32 sum of products of these magnitudes, within a few units in the last place of its norm
+    assert err[0] <= 4 * 2.0**-24
