@@ -52,6 +52,7 @@ cudaStream_t stream() { return g_stream_override ? g_stream_override : g_stream;
 cudaStream_t main_stream() { return g_stream; }
 void set_stream_override(cudaStream_t s) { g_stream_override = s; }
 bool pdl_enabled() { return g_pdl; }
+void set_pdl_enabled(bool on) { g_pdl = on; }
 int sm_count() { return g_sm_count; }
 
 // Word that kernels with bounded waits set when a wait runs out.  It is part of the library image (zero when

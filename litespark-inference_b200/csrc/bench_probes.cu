@@ -566,13 +566,13 @@ int lspk_bench_linear_copies_independent(const lspk_weight_t* w, const lspk_weig
         cudaEventRecord(fork, main_stream());
         for (int s = 0; s < n_streams; ++s) cudaStreamWaitEvent(side[s], fork, 0);
         const bool pdl_was = pdl_enabled();
-        lspk_set_pdl(0);                                  // no programmatic edges: plain independent nodes
+        set_pdl_enabled(false);                           // no programmatic edges: plain independent nodes
         for (int i = 0; i < n_w * passes && rc == LSPK_OK; ++i) {
             set_stream_override(side[i % n_streams]);
             rc = one(i % n_w, y + (size_t)(i % n_streams) * y_stride);
         }
         set_stream_override(nullptr);
-        lspk_set_pdl(pdl_was ? 1 : 0);
+        set_pdl_enabled(pdl_was);
         for (int s = 0; s < n_streams; ++s) {
             cudaEventRecord(join[s], side[s]);
             cudaStreamWaitEvent(main_stream(), join[s], 0);

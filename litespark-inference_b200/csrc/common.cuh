@@ -17,6 +17,7 @@ cudaStream_t stream();                              // the library's launch stre
 cudaStream_t main_stream();                         // the same, ignoring a measurement override
 void set_stream_override(cudaStream_t s);           // measurement aid: route launches to another stream (nullptr: off)
 bool pdl_enabled();                                 // programmatic dependent launch on/off
+void set_pdl_enabled(bool on);                      // for launches of one's own, also while capturing (lspk_set_pdl frees memory)
 int  sm_count();
 int  ensure_init();                                 // bind to a GPU on first use
 // Library-owned device scratch (the row quantiser's buffers, the K-split workspace, the per-layer buffers of

@@ -104,6 +104,15 @@ K.check(lib.lspk_set_pdl(0))
 assert free_bytes() >= before + held // 2
 st = rt.init_state(dm, 64)
 assert np.array_equal(one_step(st), want)
+st.close()                                   # a timing harness that turns programmatic launch off while it captures
+dev = importlib.import_module("litespark_inference_b200.torchless.device")
+w = dev.DeviceWeight(np.full((64, 64), 0x55, np.uint8), 1.0)
+x, y, ms = dev.DeviceArray.from_numpy(np.ones(256, np.float32)), dev.DeviceArray((2, 64), np.float32), ctypes.c_float()
+K.check(lib.lspk_set_pdl(1))
+st = rt.init_state(dm, 64)
+one_step(st)
+st.close()
+K.check(lib.lspk_bench_linear_copies_independent((ctypes.c_void_p * 1)(w.handle), None, 1, x.ptr, y.ptr, 1, 1, 2, 1, ctypes.byref(ms)))
 """
 
 
