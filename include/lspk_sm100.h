@@ -131,8 +131,8 @@ typedef struct {
 #define LSPK_MAX_GEMV_M 8
 /* Replaces matmul_lut_{tag}_m1 / _mT (matmul_lut_avx512_extern_c.cpp:150-236, 258-339) plus
  * the helpers fused around them.  Any M >= 1.  One row: the dp4a GEMV with the prologue fused in.
- * 2..8 rows: one tile of LSPK_MAX_GEMV_M rows on the warp-level int8 tensor cores (mma.sync).  More
- * rows: the TMA + tcgen05 GEMM (all four epilogues; the gated prologue stays on the tile kernel).
+ * 2..8 rows (2..16 that come as int8): tiles of LSPK_MAX_GEMV_M rows on the warp-level int8 tensor cores (mma.sync).
+ * More rows: the TMA + tcgen05 GEMM (all four epilogues; the gated prologue stays on the tile kernel).
  * With more than one row of fp32 input the rows are normalised + quantised once, by a separate kernel,
  * into library scratch that grows with cudaMalloc: make the first call of a new size outside stream
  * capture.  The kernels request the packed weights and gamma before they wait for the work queued ahead of them

@@ -35,6 +35,7 @@
 #include <stdlib.h>
 
 #include "internal.cuh"
+#include "ternary_core.cuh"
 
 namespace lspk {
 
@@ -548,7 +549,9 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_
 }
 
 // int8 rows [M, K] in natural order -> [M, Kp] with the 4x4 transpose inside every 16-element block
-// (Kp = K rounded up to 64, zero padded), the order the expanded weights come out in, and the sum of each row.
+// (Kp = K rounded up to 64, zero padded), the order the expanded weights come out in, and the sum of each row.  A CTA per
+// row, a block per thread and trip (K is a multiple of 4, rows are 4-byte aligned): with the GEMM behind it 8.9 us for 32 rows
+// of 6912 -> 2560, 14.3 a byte at a time.
 __global__ void __launch_bounds__(256)
 permute_rows_kernel(const int8_t* __restrict__ src, int8_t* __restrict__ dst, int* __restrict__ sums, int K, int Kp) {
     __shared__ int part[32];
@@ -556,11 +559,17 @@ permute_rows_kernel(const int8_t* __restrict__ src, int8_t* __restrict__ dst, in
     grid_dependency_wait();
     const size_t t = blockIdx.x;
     int sum = 0;
-    for (int kp = threadIdx.x; kp < Kp; kp += blockDim.x) {
-        const int k = perm_index(kp);                      // the transpose is its own inverse
-        const int8_t v = k < K ? src[t * K + k] : (int8_t)0;
-        dst[t * Kp + kp] = v;
-        sum += v;
+    for (int b = threadIdx.x; b < Kp / 16; b += blockDim.x) {
+        uint32_t a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = b * 16 + i * 4;
+            a[i] = k < K ? *reinterpret_cast<const uint32_t*>(src + t * K + k) : 0u;
+            sum = __dp4a((int)a[i], 0x01010101, sum);
+        }
+        uint32_t o0, o1, o2, o3;
+        transpose4x4_bytes(a[0], a[1], a[2], a[3], o0, o1, o2, o3);
+        *reinterpret_cast<uint4*>(dst + t * Kp + b * 16) = make_uint4(o0, o1, o2, o3);
     }
     sum = block_sum(sum, part);
     if (threadIdx.x == 0) sums[t] = sum;
@@ -715,9 +724,13 @@ static TcPlan plan_tiles(int tiles, bool pair, int M, int k_blocks) {
 // Fewest rows this kernel takes: with one eight-row tile the mma.sync kernel (linear_mma.cu) is level with it (33 us for
 // the four products of a layer at 8 rows, here 35), with two it is behind (16 rows: 38 and 34 us; 31 rows: 55 and 36).
 constexpr int kTcMinRows = 9;
+// Rows that come as int8 pay one launch more here (permute_rows_kernel) and none there: at 9 to 16 rows the four products
+// of a layer take 29.6 us here and 27.7 there, at 17 to 24 rows 29.5 and 38.9.
+constexpr int kTcMinRowsInt8 = 17;
 
 // Tensor-core path: one launch for all matrices of the call (plus the row quantiser in front of it).
-int linear_tensor_core(const lspk_linear_args* a, int* handled) {
+// forced: as few rows as it can, whatever is faster.
+int linear_tensor_core(const lspk_linear_args* a, int* handled, bool forced) {
     *handled = 0;
     if (a->M < kTcMinRows) return LSPK_OK;
     const bool pair = a->epilogue == LSPK_EPI_RELU2_MUL || a->epilogue == LSPK_EPI_SILU_MUL;
@@ -728,6 +741,8 @@ int linear_tensor_core(const lspk_linear_args* a, int* handled) {
     if (!enc) return LSPK_OK;
     const Weight* w0 = reinterpret_cast<const Weight*>(a->w[0]);
     if (!w0) return LSPK_OK;
+    // (rows too long for the other kernel's shared memory, about 24000, stay here)
+    if (a->M < kTcMinRowsInt8 && a->prologue == LSPK_PRO_INT8 && !forced && w0->K <= 16384) return LSPK_OK;
     const int M = a->M, K = w0->K, Kp = w0->chunks * kWeightsPerChunk;
 
     // ---- activations: int8 rows + scales, then the permuted, padded copy the tensor map reads ----

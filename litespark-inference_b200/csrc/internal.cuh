@@ -69,7 +69,7 @@ int linear_cuda_core(const lspk_linear_args* a);
 
 // gemm_tc.cu: tcgen05 tensor-core path for large M.  Returns LSPK_OK and sets *handled = 1 when it
 // ran; leaves *handled = 0 when the shape is outside what it supports.
-int linear_tensor_core(const lspk_linear_args* a, int* handled);
+int linear_tensor_core(const lspk_linear_args* a, int* handled, bool forced);
 
 // lm_head.cu
 int lm_head_launch(int kind, const void* emb, const float* emb_scale, const float* x, float* logits,

@@ -607,7 +607,7 @@ extern "C" int lspk_linear(const lspk_linear_args* a) {
     }
     if (g_force_path != 1) {
         int handled = 0;
-        if (int rc = linear_tensor_core(a, &handled)) return rc;
+        if (int rc = linear_tensor_core(a, &handled, g_force_path == 2)) return rc;
         if (handled) return LSPK_OK;
         if (g_force_path == 2) return fail(LSPK_ERR_ARG, "lspk_linear: shape not supported by the tensor-core path");
     }

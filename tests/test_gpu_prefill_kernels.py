@@ -45,6 +45,21 @@ def test_gemm_tiles_bit_exact(M, N, Kd, epilogue):
     assert np.array_equal(out.numpy(), want)      # the same roundings in the same order
 
 
+@pytest.mark.parametrize("M", [8, 9, 16, 17, 24])
+@pytest.mark.parametrize("Kd", [4, 68, 2560, 4100])          # rows of one word, off the 16-element block, of several trips
+def test_int8_rows_on_either_side_of_the_choice_of_a_kernel(M, Kd):
+    rng = np.random.default_rng(M + Kd)
+    N = 130
+    w, xq = rng.integers(-1, 2, (N, Kd), dtype=np.int8), rng.integers(-127, 128, (M, Kd), dtype=np.int8)
+    xs = rng.uniform(0.01, 0.02, M).astype(np.float32)
+    W = dev.DeviceWeight(pack.pack_ternary_4_per_byte(w), 0.75)
+    out, acc = dev.DeviceArray((M, N), np.float32), dev.DeviceArray((M, N), np.int32)
+    dev.linear([W], [out], M, x_i8=dev.DeviceArray.from_numpy(xq), x_scales=dev.DeviceArray.from_numpy(xs), acc_outs=[acc])
+    want = xq.astype(np.int32) @ w.T.astype(np.int32)
+    assert np.array_equal(acc.numpy(), want)
+    assert np.array_equal(out.numpy(), want.astype(np.float32) * (xs * np.float32(0.75))[:, None])
+
+
 @pytest.mark.parametrize("kv", ["fp16", "fp32"])
 # head sizes 64 and 128; 1, 2, 4, 5 query heads per KV head (heads that share a CTA); rows around the 16-row tile; the
 # key-split form (few rows) and the shared form (many rows x heads); a context in front of the rows
