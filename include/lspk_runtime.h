@@ -87,6 +87,10 @@ int lspk_state_step_kernel_count(lspk_state_t s);
  * `polls` times (1..65536), gives up, and raises the library's wait flag; the next lspk_tc_check_error then
  * returns LSPK_ERR_DEVICE_WAIT once and clears it.  Nothing faults and the context stays usable. */
 int lspk_debug_expire_wait(int polls);
+
+/* Test aid for running out of memory: device allocations of more than `bytes` made by the library fail from here on as if
+ * the GPU had none left (0: back to normal). */
+int lspk_debug_allocation_limit(size_t bytes);
 #ifdef __cplusplus
 }
 #endif

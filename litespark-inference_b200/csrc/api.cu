@@ -62,11 +62,14 @@ static int* g_wait_flag = nullptr;
 int* device_wait_flag() { return g_wait_flag; }
 int bound_device() { return g_device; }
 
+static size_t g_alloc_limit = 0;                    // test aid: device allocations above it fail (0: none do)
+
 cudaError_t device_malloc(void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
+    auto attempt = [&]() { return g_alloc_limit && bytes > g_alloc_limit ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes); };
+    cudaError_t e = attempt();
     if (e == cudaErrorMemoryAllocation && release_parked_states()) {
         cudaGetLastError();
-        e = cudaMalloc(p, bytes);
+        e = attempt();
     }
     return e;
 }
@@ -155,6 +158,11 @@ int lspk_set_pdl(int enabled) {
     // a parked state's graph holds the launch attributes of its capture: the next state captures anew
     if (g_pdl != (enabled != 0)) release_parked_states();
     g_pdl = enabled != 0;
+    return LSPK_OK;
+}
+
+int lspk_debug_allocation_limit(size_t bytes) {
+    g_alloc_limit = bytes;
     return LSPK_OK;
 }
 

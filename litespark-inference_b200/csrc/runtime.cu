@@ -216,8 +216,10 @@ static unsigned long long g_next_model_id = 0;
 
 static void destroy_state(State* s);
 
-// The model's tensors are about to change (or to go): the graphs of a parked state hold their addresses.
+// The model's tensors are about to change (or to go): the graphs of a parked state hold their addresses, and a step may
+// take other kernels than the warmed one.
 static void drop_parked(Model* m, bool model_goes = false) {
+    m->warmed.clear();
     State* parked = nullptr;
     {
         std::lock_guard<std::mutex> lk(g_park_mu);
@@ -395,12 +397,13 @@ static int build_graph(State* s, int variant) {
         cudaGraphExecDestroy(s->graph[variant]);
         s->graph[variant] = nullptr;
     }
-    // The first time a model takes a step of this shape, run it once outside capture: it sets the kernels'
-    // shared-memory attributes, sizes library scratch (neither is allowed while capturing) and surfaces launch errors
-    // directly.  Both outlive the state, so further states of the shape go straight to the capture.  The warm-up must not
-    // change the state: save and restore the control block around it.
-    const int shape = (s->batch * 2 + s->kv_fp16) * 4 + variant;
-    if (!s->m->warmed.count(shape)) {
+    // The first time a model takes a step of this shape, run it once outside capture: it sizes library scratch (which may
+    // not grow while capturing), loads the kernels and surfaces launch errors directly.  All of that outlives the state, so
+    // further states of the shape go straight to the capture, as long as the model's tensors (table formats choose
+    // kernels) and the library's scratch are still those of the warm-up; the shape holds what else chooses a kernel.  The
+    // warm-up must not change the state: save and restore the control block around it.
+    unsigned& warm_gen = s->m->warmed[std::make_tuple(s->batch, s->kv_fp16, s->t_max, variant)];      // 0: never
+    if (warm_gen != scratch_generation()) {
         const int nctl = 2 * s->batch + 1;
         std::vector<int> saved(nctl);
         LSPK_CUDA(cudaMemcpyAsync(saved.data(), s->ctl, nctl * sizeof(int), cudaMemcpyDeviceToHost, stream()));
@@ -410,7 +413,7 @@ static int build_graph(State* s, int variant) {
         LSPK_CUDA(cudaMemcpyAsync(s->ctl, saved.data(), nctl * sizeof(int), cudaMemcpyHostToDevice, stream()));
         LSPK_CUDA(cudaStreamSynchronize(stream()));
         if (variant == 2) s->io_seq += 1;          // the warm-up step counted itself on the device
-        s->m->warmed.insert(shape);
+        warm_gen = scratch_generation();
     }
 
     cudaGraph_t g = nullptr;

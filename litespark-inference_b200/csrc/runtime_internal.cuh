@@ -1,7 +1,8 @@
 // Model and inference-state containers of the device-resident forward pass, shared between runtime.cu (which
 // owns them) and the measurement harnesses in bench_probes.cu.
 #pragma once
-#include <set>
+#include <map>
+#include <tuple>
 #include <vector>
 
 #include "internal.cuh"
@@ -34,7 +35,9 @@ struct Model {
     bool finalized = false;
     size_t bytes = 0;
     unsigned long long id = 0;        // never reused: states find their model's parking place by it
-    std::set<int> warmed;             // step shapes (batch, KV type, graph variant) that have run once outside capture
+    // step shapes (batch, KV type, t_max, graph variant) that have run once outside capture, and the scratch generation
+    // they left; emptied when a tensor of the model changes
+    std::map<std::tuple<int, int, int, int>, unsigned> warmed;
     int D() const { return cfg.hidden_size / cfg.num_heads; }
     int kv_dim() const { return cfg.num_kv_heads * D(); }
 };

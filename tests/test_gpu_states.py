@@ -118,9 +118,60 @@ K.check(lib.lspk_bench_linear_copies_independent((ctypes.c_void_p * 1)(w.handle)
 
 def test_a_state_made_after_a_trace_or_launch_mode_change_uses_it():
     """In a process of its own: the trace buffer stays installed."""
-    r = subprocess.run([sys.executable, "-c", _TRACE_AND_LAUNCH_MODE], cwd=Path(__file__).resolve().parent.parent,
-                       capture_output=True, text=True, timeout=300)
+    _in_own_process(_TRACE_AND_LAUNCH_MODE)
+
+
+_SCRATCH_LOST = """
+import ctypes, importlib
+import numpy as np
+import __graft_entry__ as entry
+entry.load_package()
+name = "litespark_inference_b200.torchless."
+K, rt, dev, synthetic, loader = (importlib.import_module(name + n) for n in ("kernel", "runtime", "device", "synthetic", "loader"))
+m = synthetic.random_model(synthetic.toy_config(), seed=3)
+dm = rt.DeviceModel(m)
+lib = dm.lib
+toks = np.array([1, 2, 3, 4], np.int32)
+
+def two_steps(t_max=64):
+    st = rt.init_state(dm, t_max, batch=4)
+    rt.forward_step(st, toks)
+    logits = rt.forward_step(st, toks + 9, want_logits=True)[1]
+    st.close()
+    return logits
+
+want = two_steps()
+# a product of many rows that finds no memory: the library's int8 rows are gone, the next step has to make them again
+M, Kd = 4096, 1024
+w = dev.DeviceWeight(np.full((64, Kd // 4), 0x55, np.uint8), 1.0)
+x, y, q = dev.DeviceArray((M, Kd), np.float32), dev.DeviceArray((M, 64), np.float32), dev.DeviceArray((M, Kd), np.int8)
+x.fill_bytes(0)
+a = K.LinearArgs()
+a.w[0], a.out[0], a.n_mats, a.M, a.prologue, a.x_f32, a.xq_out = w.handle, y.ptr, 1, M, K.PRO_QUANT, x.ptr, q.ptr
+K.check(lib.lspk_linear_force_path(1))
+K.check(lib.lspk_debug_allocation_limit(1 << 20))
+assert lib.lspk_linear(ctypes.byref(a)) == 2
+K.check(lib.lspk_debug_allocation_limit(0))
+K.check(lib.lspk_linear_force_path(0))
+assert np.array_equal(two_steps(), want)
+# a long cache takes another attention kernel, another table another LM head
+assert np.array_equal(two_steps(4000), want)
+q8, s8 = loader.quantize_embedding(m.embed_tokens, 127)
+K.check(lib.lspk_model_set_lm_head(dm.handle, 1, q8.ctypes.data, s8.ctypes.data))
+int8 = two_steps()
+assert 0 < np.abs(int8 - want).max() < 0.1 * np.abs(want).max()
+"""
+
+
+def _in_own_process(code):
+    r = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True,
+                       timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_a_step_shape_is_warmed_again_after_scratch_or_tables_changed():
+    """In a process of its own, whose scratch no other test has grown."""
+    _in_own_process(_SCRATCH_LOST)
 
 
 @pytest.mark.parametrize("kind", [0, 1, 2])
