@@ -91,6 +91,13 @@ int lspk_debug_expire_wait(int polls);
 /* Test aid for running out of memory: device allocations of more than `bytes` made by the library fail from here on as if
  * the GPU had none left (0: back to normal). */
 int lspk_debug_allocation_limit(size_t bytes);
+
+/* Test aid: the attention section of one prefill layer on device arrays.  T consecutive rows of one sequence, the first at
+ * position *pos (pos + T <= t_max): q [T, Q * D] is rotated in place, the rows' keys (rotated) and values [T, KV * D] are
+ * written to the caches [t_max, KV, D] (fp16 or fp32), out [T, Q * D] receives the attention.  rope_cos / rope_sin [t_max, D / 2]. */
+int lspk_debug_prefill_attention(float* q, const float* k_cur, const float* v_cur, void* cache_k, void* cache_v,
+                                 const float* rope_cos, const float* rope_sin, const int* pos, float* out, int T, int Q,
+                                 int KV, int D, int t_max, int kv_fp16);
 #ifdef __cplusplus
 }
 #endif

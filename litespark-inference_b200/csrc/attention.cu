@@ -1253,3 +1253,28 @@ int attention_launch(const AttnParams& p_in, int kv_is_fp16) {
 }
 
 }  // namespace lspk
+
+extern "C" int lspk_debug_prefill_attention(float* q, const float* k_cur, const float* v_cur, void* cache_k, void* cache_v,
+                                            const float* rope_cos, const float* rope_sin, const int* pos, float* out, int T,
+                                            int Q, int KV, int D, int t_max, int kv_fp16) {
+    using namespace lspk;
+    if (int rc = ensure_init()) return rc;
+    LSPK_REQUIRE(q && k_cur && v_cur && cache_k && cache_v && rope_cos && rope_sin && pos && out && T >= 1 && T <= t_max &&
+                 Q >= 1 && KV >= 1, "lspk_debug_prefill_attention: bad arguments");
+    AttnParams p = {};
+    p.q = q;
+    p.k_cur = k_cur;
+    p.v_cur = v_cur;
+    p.out = out;
+    p.cache_k = cache_k;
+    p.cache_v = cache_v;
+    p.rope_cos = rope_cos;
+    p.rope_sin = rope_sin;
+    p.pos_ptr = pos;
+    p.T = T;
+    p.Q = Q;
+    p.KV = KV;
+    p.D = D;
+    p.t_max = t_max;
+    return attention_launch(p, kv_fp16);
+}

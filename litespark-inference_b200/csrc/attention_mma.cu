@@ -2,14 +2,17 @@
 // already in the cache) against the cached keys, causal, grouped queries, streaming softmax.  Replaces the scores ->
 // softmax -> weighted-sum section of the reference's prefill (runtime.py:381-407) for 16 and more rows.
 //
-// fp32 in, fp32 out, with the products formed by mma.sync on 16-bit operands that represent every fp32 input exactly:
+// fp32 in, fp32 out, with the products formed by mma.sync on 16-bit operands:
 //   fp16 cache   keys and values are fp16 as they stand; a query row (scaled by a power of two so that its largest
-//                element is near 2^14) and the probabilities (scaled by 2^14) are cut into three fp16 terms of 11 bits
+//                element is near 2^14) and the probabilities (scaled by 2^14) are cut into three fp16 terms of 11 bits.
+//                The terms end at 2^-24, which is 2^-38 of the largest: elements below 2^-15 of it lose bits there
 //   fp32 cache   everything is cut into three bf16 terms of 8 bits (the range of fp32, so no scaling); of the nine
-//                products the six above 2^-24 of the largest are formed
-// The products of 16 elements form one tensor-core sum started from zero, which a rounded fp32 addition then adds to the
-// running one (the tensor core truncates: chained through its accumulator the scores of a saturated softmax, near 10^3,
-// came out several times less accurate).  The softmax uses expf and a running maximum.
+//                products the six down to 2^-18 of the largest are formed, the others are below 2^-26
+// The products of 16 elements form one tensor-core sum started from zero, two of which meet in a rounded fp32 addition
+// before another adds them to the running sum (the tensor core truncates: chained through its accumulator the scores of a
+// saturated softmax, near 10^3, came out several times less accurate).  The softmax uses expf and a running maximum.
+// Error against float64, 2-norm, 1531 rows x 20 heads of 128: 3.5e-7 where scores have a spread of 4, and 3.7e-7 in
+// fp32 multiply-adds (attention_rows_kernel); over 16 to 1531 rows and spreads of 1 to 12 it is 0.85 to 1.0 of theirs.
 //
 // One warp owns 16 query rows of one head.  Two splits of the four warps of a CTA:
 //   WK = 1   four row tiles (heads of one KV head first, then positions) share every key / value tile: the form for
@@ -96,6 +99,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
     using L = PfLayout<KVT, D, WK>;
     constexpr int KT = L::KT, KI = L::KI, RB = L::kRowBytes, kCombos = PfTraits<KVT>::kCombos;
     constexpr int kSet = sizeof(KVT) == 2 ? 0 : 1;
+    constexpr int kQkUnroll = kSet == 0 ? 1 : 2;
     constexpr int kChunkMask = 7;                          // 16-byte chunks of a row are permuted by row & 7
     extern __shared__ __align__(128) unsigned char pf_smem[];
     grid_dependency_launch();
@@ -264,35 +268,44 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
             for (int i = 0; i < KT / 8; ++i)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
+            // unrolled as far as the registers of a thread go (D = 128, shared form: whole, 10.16 and 15.40 ms for a prompt of
+            // 1531 rows with an fp16 and an fp32 cache; as here, 10.01 and 14.95)
+#pragma unroll kQkUnroll
+            for (int kp = 0; kp < D / 32; ++kp) {                      // two k steps: their sums meet before the running one
+                uint32_t qa[2][3][4];
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
-                uint32_t qa[3][4];
+                for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
-                for (int pl = 0; pl < 3; ++pl) {
-                    // lanes 0-15: rows 0-15 at chunk 2 ks; lanes 16-31: the same rows at chunk 2 ks + 1
-                    const int r = lane & 15, c = ks * 2 + (lane >> 4);
-                    ldsm4(qa[pl], q_base + pl * 16 * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
-                }
+                    for (int pl = 0; pl < 3; ++pl) {
+                        // lanes 0-15: rows 0-15 at chunk 2 ks; lanes 16-31: the same rows at chunk 2 ks + 1
+                        const int r = lane & 15, c = (kp * 2 + kk) * 2 + (lane >> 4);
+                        ldsm4(qa[kk][pl], q_base + pl * 16 * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
+                    }
 #pragma unroll
                 for (int nt = 0; nt < KT / 16; ++nt) {
-                    uint32_t kb[L::kPlanes][4];
+                    float c0[2][4], c1[2][4];
 #pragma unroll
-                    for (int pl = 0; pl < L::kPlanes; ++pl) {
-                        // matrices: keys 0-7 / chunk 0, keys 0-7 / chunk 1, keys 8-15 / chunk 0, keys 8-15 / chunk 1
-                        const int r = nt * 16 + (lane & 7) + ((lane >> 4) << 3), c = ks * 2 + ((lane >> 3) & 1);
-                        ldsm4(kb[pl], kbase + pl * KI * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
-                    }
-                    float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+                    for (int kk = 0; kk < 2; ++kk) {
+                        uint32_t kb[L::kPlanes][4];
 #pragma unroll
-                    for (int cb = 0; cb < kCombos; ++cb) {
-                        const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
-                        mma16816<KVT>(c0, qa[a], kb[b][0], kb[b][1]);
-                        mma16816<KVT>(c1, qa[a], kb[b][2], kb[b][3]);
+                        for (int pl = 0; pl < L::kPlanes; ++pl) {
+                            // matrices: keys 0-7 / chunk 0, keys 0-7 / chunk 1, keys 8-15 / chunk 0, keys 8-15 / chunk 1
+                            const int r = nt * 16 + (lane & 7) + ((lane >> 4) << 3), c = (kp * 2 + kk) * 2 + ((lane >> 3) & 1);
+                            ldsm4(kb[pl], kbase + pl * KI * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) c0[kk][e] = c1[kk][e] = 0.0f;
+#pragma unroll
+                        for (int cb = 0; cb < kCombos; ++cb) {
+                            const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
+                            mma16816<KVT>(c0[kk], qa[kk][a], kb[b][0], kb[b][1]);
+                            mma16816<KVT>(c1[kk], qa[kk][a], kb[b][2], kb[b][3]);
+                        }
                     }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        s[nt * 2][e] += c0[e];
-                        s[nt * 2 + 1][e] += c1[e];
+                        s[nt * 2][e] += c0[0][e] + c0[1][e];
+                        s[nt * 2 + 1][e] += c1[0][e] + c1[1][e];
                     }
                 }
             }
@@ -317,13 +330,26 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
                 mx[h] = nm[h];
                 sum[h] *= corr[h];
             }
+            // The tile's terms are summed apart: added to the running sums one by one, those of 1531 keys round 383 times in
+            // every lane.  Pairs first where a tile has 64 keys; where it has 32, one by one as they come (pairs: 1.5 % more
+            // time for a prompt of 1024 rows, no less error).
+            float tile_sum[2] = {0.0f, 0.0f};
 #pragma unroll
             for (int i = 0; i < KT / 8; ++i)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     s[i][e] = expf(s[i][e] - base[e >> 1]);
-                    sum[e >> 1] += s[i][e];
+                    if (kSet == 1) tile_sum[e >> 1] += s[i][e];
                 }
+            if (kSet == 0) {
+#pragma unroll
+                for (int i = 0; i < KT / 8; ++i) {
+                    tile_sum[0] += s[i][0] + s[i][1];
+                    tile_sum[1] += s[i][2] + s[i][3];
+                }
+            }
+            sum[0] += tile_sum[0];
+            sum[1] += tile_sum[1];
             if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
 #pragma unroll
                 for (int i = 0; i < D / 8; ++i) {
@@ -333,40 +359,48 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
                     o[i][3] *= corr[1];
                 }
             }
-            // o += P V: the score accumulators of 16 keys are the A operand of one k step
+            // o += P V: the score accumulators of 16 keys are the A operand of one k step, two steps where the tile has them
+            constexpr int PP = KT >= 32 ? 2 : 1;
 #pragma unroll
-            for (int ks = 0; ks < KT / 16; ++ks) {
+            for (int kp = 0; kp < KT / 16 / PP; ++kp) {
                 constexpr float ps = kSet == 0 ? kProbScale : 1.0f;
-                uint32_t pa[3][4];
+                uint32_t pa[PP][3][4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float* sv = s[ks * 2 + (j >> 1)];
-                    uint32_t t3[3];
-                    split3<KVT>(sv[(j & 1) * 2] * ps, sv[(j & 1) * 2 + 1] * ps, t3);
-                    pa[0][j] = t3[0];
-                    pa[1][j] = t3[1];
-                    pa[2][j] = t3[2];
-                }
+                for (int kk = 0; kk < PP; ++kk)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float* sv = s[(kp * PP + kk) * 2 + (j >> 1)];
+                        uint32_t t3[3];
+                        split3<KVT>(sv[(j & 1) * 2] * ps, sv[(j & 1) * 2 + 1] * ps, t3);
+                        pa[kk][0][j] = t3[0];
+                        pa[kk][1][j] = t3[1];
+                        pa[kk][2][j] = t3[2];
+                    }
 #pragma unroll
                 for (int nt = 0; nt < D / 16; ++nt) {
-                    uint32_t vb[L::kPlanes][4];
+                    float c0[PP][4], c1[PP][4];
 #pragma unroll
-                    for (int pl = 0; pl < L::kPlanes; ++pl) {
-                        // matrices (transposed): keys 0-7 / chunk 0, keys 8-15 / chunk 0, keys 0-7 / chunk 1, keys 8-15 / chunk 1
-                        const int r = ks * 16 + (lane & 15), c = nt * 2 + (lane >> 4);
-                        ldsm4_t(vb[pl], vbase + pl * KI * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
-                    }
-                    float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+                    for (int kk = 0; kk < PP; ++kk) {
+                        uint32_t vb[L::kPlanes][4];
 #pragma unroll
-                    for (int cb = 0; cb < kCombos; ++cb) {
-                        const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
-                        mma16816<KVT>(c0, pa[a], vb[b][0], vb[b][1]);
-                        mma16816<KVT>(c1, pa[a], vb[b][2], vb[b][3]);
+                        for (int pl = 0; pl < L::kPlanes; ++pl) {
+                            // matrices (transposed): keys 0-7 / chunk 0, keys 8-15 / chunk 0, keys 0-7 / chunk 1, keys 8-15 / chunk 1
+                            const int r = (kp * PP + kk) * 16 + (lane & 15), c = nt * 2 + (lane >> 4);
+                            ldsm4_t(vb[pl], vbase + pl * KI * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) c0[kk][e] = c1[kk][e] = 0.0f;
+#pragma unroll
+                        for (int cb = 0; cb < kCombos; ++cb) {
+                            const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
+                            mma16816<KVT>(c0[kk], pa[kk][a], vb[b][0], vb[b][1]);
+                            mma16816<KVT>(c1[kk], pa[kk][a], vb[b][2], vb[b][3]);
+                        }
                     }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        o[nt * 2][e] += c0[e];
-                        o[nt * 2 + 1][e] += c1[e];
+                        o[nt * 2][e] += PP == 2 ? c0[0][e] + c0[PP - 1][e] : c0[0][e];
+                        o[nt * 2 + 1][e] += PP == 2 ? c1[0][e] + c1[PP - 1][e] : c1[0][e];
                     }
                 }
             }
