@@ -80,6 +80,39 @@ __device__ __forceinline__ void ldsm4_t(uint32_t r[4], uint32_t addr) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
+// One query row of one head by a whole warp, keys 0 .. n - 1: plain fp32 multiply-adds, probabilities normalised in front
+// of the values.  The slow way for rows whose result is not finite.  A tile product touches more than a row's own keys, and
+// a split operand more than its own value: a masked key has probability 0, and 0 times an infinite value is NaN; an infinity
+// leaves NaN in the lower terms of its split, where a score of -inf would only have switched its key off.
+template <typename KVT, int D>
+__device__ __noinline__ void attend_row_plain(const float* q, const KVT* k, const KVT* v, float* out, int n, int kd) {
+    constexpr int EL = D / 32;
+    const int lane = threadIdx.x & 31;
+    float qv[EL], o[EL];
+#pragma unroll
+    for (int e = 0; e < EL; ++e) {
+        qv[e] = q[lane + 32 * e];
+        o[e] = 0.0f;
+    }
+    const float inv_sqrt_d = 1.0f / sqrtf((float)D);
+    auto score = [&](int i) -> float {
+        float d = 0.0f;
+#pragma unroll
+        for (int e = 0; e < EL; ++e) d = fmaf(qv[e], (float)k[(size_t)i * kd + lane + 32 * e], d);
+        return __fmul_rn(warp_sum(d), inv_sqrt_d);
+    };
+    float mx = -INFINITY, sum = 0.0f;
+    for (int i = 0; i < n; ++i) mx = fmaxf(mx, score(i));
+    for (int i = 0; i < n; ++i) sum += expf(score(i) - mx);
+    for (int i = 0; i < n; ++i) {
+        const float pi = __fdiv_rn(expf(score(i) - mx), sum);
+#pragma unroll
+        for (int e = 0; e < EL; ++e) o[e] = fmaf(pi, (float)v[(size_t)i * kd + lane + 32 * e], o[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < EL; ++e) out[lane + 32 * e] = o[e];
+}
+
 template <typename KVT, int D, int WK>
 struct PfLayout {
     static constexpr int kPlanes = PfTraits<KVT>::kPlanes;
@@ -413,17 +446,31 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
         sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
     }
     constexpr float unp = kSet == 0 ? 1.0f / kProbScale : 1.0f;
+    auto redo_row = [&](int t) {
+        const size_t at = (size_t)t * p.Q * D + (size_t)head * D;
+        attend_row_plain<KVT, D>(p.q + at, ck, cv, p.out + at, pos0 + t + 1, kd);
+    };
     if (WK == 1) {
+        unsigned redo[2];                                  // lanes that hold part of a row that is not finite
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int t = row0 + (lane >> 2) + 8 * h;
+            bool finite = true;
             if (t < p.T) {
                 float* dst = p.out + (size_t)t * p.Q * D + (size_t)head * D + (lane & 3) * 2;
 #pragma unroll
-                for (int i = 0; i < D / 8; ++i)
-                    *reinterpret_cast<float2*>(dst + i * 8) =
-                        make_float2(__fdiv_rn(o[i][h * 2] * unp, sum[h]), __fdiv_rn(o[i][h * 2 + 1] * unp, sum[h]));
+                for (int i = 0; i < D / 8; ++i) {
+                    const float2 y = make_float2(__fdiv_rn(o[i][h * 2] * unp, sum[h]), __fdiv_rn(o[i][h * 2 + 1] * unp, sum[h]));
+                    *reinterpret_cast<float2*>(dst + i * 8) = y;
+                    finite = finite && fabsf(y.x) < INFINITY && fabsf(y.y) < INFINITY;
+                }
             }
+            redo[h] = __ballot_sync(0xffffffffu, !finite);
+        }
+        if (redo[0] | redo[1]) {
+            __syncwarp();                                  // the stores above, by other lanes, come first
+            for (int r = 0; r < 16; ++r)
+                if ((redo[r >> 3] >> (4 * (r & 7))) & 15u) redo_row(row0 + r);
         }
         return;
     }
@@ -443,6 +490,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
         }
     }
     __syncthreads();
+    unsigned redo = 0;                                     // rows that are not finite
     for (int i = tid; i < 16 * D; i += kPfThreads) {
         const int r = i / D, d = i % D, t = row0 + r;
         if (t >= p.T) continue;
@@ -456,7 +504,18 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
             den = fmaf(fm[64 + w * 16 + r], wgt, den);
             acc = fmaf(fo[(size_t)(w * 16 + r) * D + d], wgt, acc);
         }
-        p.out[(size_t)t * p.Q * D + (size_t)head * D + d] = __fdiv_rn(acc, den);
+        const float y = __fdiv_rn(acc, den);
+        p.out[(size_t)t * p.Q * D + (size_t)head * D + d] = y;
+        redo |= (fabsf(y) < INFINITY ? 0u : 1u) << r;
+    }
+    if (__syncthreads_or((int)redo)) {
+        __shared__ unsigned s_redo;
+        if (tid == 0) s_redo = 0;
+        __syncthreads();
+        if (redo) atomicOr(&s_redo, redo);
+        __syncthreads();
+        for (int r = warp; r < 16; r += 4)
+            if ((s_redo >> r) & 1u) redo_row(row0 + r);
     }
 }
 

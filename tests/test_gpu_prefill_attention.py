@@ -69,3 +69,43 @@ def test_no_less_accurate_than_fp32_multiply_adds(Q, KV, D, T, ctx, kv, spread):
     assert err <= 2.0**-20
     # two roundings of the same sums: equal up to their scatter
     assert err <= 1.1 * ref + 2e-8
+
+
+@pytest.mark.parametrize("kv", ["fp16", "fp32"])
+# the key-split form and the shared form; 40 rows: a last tile that is not full
+@pytest.mark.parametrize("Q,KV,D,T,ctx", [(4, 2, 128, 40, 9), (5, 1, 64, 33, 0), (20, 5, 128, 520, 0), (12, 6, 64, 640, 20)])
+@pytest.mark.parametrize("what", ["value", "nan value", "key", "query", "context value", "huge values"])
+def test_values_that_are_not_finite_stay_where_they_belong(Q, KV, D, T, ctx, kv, what):
+    """An infinite or missing value, key or query element reaches the rows that attend to it and no other, as in the kernel
+    for fewer rows, which never touches a masked key."""
+    a = Attention(Q, KV, D, T, ctx, kv, spread=1.0)
+    at = T - 7                                     # a row of the last tiles: masked for the rows in front of it
+    if what == "value":
+        a.v[at, 0, 3] = 1e6 if kv == "fp16" else np.inf            # an fp16 cache overflows at 65504
+    elif what == "nan value":
+        a.v[at, KV - 1, D - 1] = np.nan
+    elif what == "key":                            # scores of -inf switch the key off, of +inf and NaN spoil the row
+        a.k[at, 0, 5] = np.inf
+    elif what == "query":
+        a.q[at, Q - 1, 0] = -np.inf
+    elif what == "context value":
+        if not ctx:
+            pytest.skip("no context")
+        a.cv[2, 0, 1] = np.inf                     # for every row
+    else:
+        if kv == "fp16":
+            pytest.skip("fp16 values do not reach the end of fp32")
+        a.v[:, 0, 0] = 2e38                        # sums of unnormalised probabilities would leave fp32
+        a.cv[:, 0, 0] = 2e38
+    got, _, ck, cv = a.run(T)
+    want, _, ck2, cv2 = a.run(8)
+    assert np.array_equal(ck, ck2, equal_nan=True) and np.array_equal(cv, cv2, equal_nan=True)
+    if what != "huge values":
+        assert not np.isfinite(want).all()
+    assert np.isfinite(want[:at]).all() or what == "context value"
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+    ok = np.isfinite(want)
+    assert np.array_equal(np.sign(got[np.isinf(got)]), np.sign(want[np.isinf(want)]))
+    scale = np.abs(want[ok]).max() if what == "huge values" else 1.0
+    # two roundings of the same sums of values of order 1 (of the largest)
+    assert np.abs(got[ok] / scale - want[ok] / scale).max() <= 2.0**-18
