@@ -23,10 +23,11 @@ template <> struct EmbTraits<0> { static constexpr int E = 8;  };   // bf16: 8 v
 template <> struct EmbTraits<1> { static constexpr int E = 16; };   // int8
 template <> struct EmbTraits<2> { static constexpr int E = 32; };   // int4, low nibble first
 
-// The s-th group of four consecutive values of a 16-byte chunk.  The integer formats go through the mantissa of 2^23
-// (bits | 0x4b000000, then minus the bias: exact) because integer-to-float conversions issue at a fraction of the add
-// rate (int4, 128256 x 2560: 115 us with them, and the table's 164 MB take 25).  int4 nibbles stay at their bit offset:
-// value e of a group comes out times 16^e, and x is staged divided by it (int4_unscale), so every product is the same.
+// The s-th group of four consecutive values of a 16-byte chunk.  int4 goes through the mantissa of 2^23 (bits | 0x4b000000,
+// then minus the bias: exact) because integer-to-float conversions issue at a fraction of the add rate (a decode step of
+// one sequence 721 us with them, 686 without; the table's 164 MB take 25).  Its nibbles stay at their bit offset:
+// value e of a group comes out times 16^e, and x is staged divided by it (staged_x), so every product is the same.  int8
+// has half the values per byte and keeps the conversions (128256 x 2560: 69 us with them, 81 through the mantissa).
 template <int KIND>
 __device__ __forceinline__ void decode4(const uint4& c, int s, float f[4]) {
     const uint32_t w[4] = {c.x, c.y, c.z, c.w};
@@ -37,9 +38,9 @@ __device__ __forceinline__ void decode4(const uint4& c, int s, float f[4]) {
         f[2] = __uint_as_float(b << 16);
         f[3] = __uint_as_float(b & 0xffff0000u);
     } else if (KIND == 1) {
-        const uint32_t a = w[s & 3] ^ 0x80808080u;                          // value + 128
+        const uint32_t a = w[s & 3];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) f[e] = __uint_as_float(__byte_perm(a, 0x4b000000u, 0x7440 + e)) - 8388736.0f;
+        for (int e = 0; e < 4; ++e) f[e] = (float)((int)(a << (24 - 8 * e)) >> 24);
     } else {
         const uint32_t a = w[(s >> 1) & 3] >> ((s & 1) * 16);               // two bytes = four nibbles
 #pragma unroll
@@ -586,10 +587,10 @@ int lm_head_launch(int kind, const void* emb, const float* emb_scale, const floa
                            norm_gamma, gamma_is_bf16, eps, bk);                                             \
         } while (0)
         if (tt == 1) {
-            // integer formats: a value of x fetched from shared memory serves two table rows (one row at a time the
-            // reads of x, 4 bytes per half a byte of int4 table, would take longer than the table)
+            // int4: a value of x fetched from shared memory serves two table rows (one row at a time the reads of x, 4 bytes
+            // per half a byte of table, would take longer than the table).  int8: one (two: 86 us and not 69)
             if (kind == 0) LSPK_LM_LAUNCH(0, 1, 10, 1);
-            else if (kind == 1) LSPK_LM_LAUNCH(1, 1, 5, 2);
+            else if (kind == 1) LSPK_LM_LAUNCH(1, 1, 5, 1);
             else LSPK_LM_LAUNCH(2, 1, 3, 2);
         } else {
             // measured at V = 128256, H = 2560, 8 rows (loads in flight, table rows per warp): (4,1) 396 us,
