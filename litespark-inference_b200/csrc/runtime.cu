@@ -164,16 +164,21 @@ static int upload_table(DevTable& t, int kind, const void* host, const float* sc
 
 // Most prompt rows that go through the layers at once.  The products' cost per row falls with the rows of a launch (a
 // layer's four at 2560 / 6912: 45 us for 128 rows, 74 for 512, 175 for 1531) and levels off there; 2048 rows of scratch
-// are 180 MB at that shape, allocated only for prompts that long.
+// are 130 MB at that shape.
 constexpr int kMaxPrefillRows = 2048;
+constexpr int kMinRows = 128;
 
-// Grows the row scratch of the layers: 128 rows (or the batch) at first, then at once to the longest prompt the state
-// can take.  Graphs captured before hold the old addresses and are dropped.
+// Grows the row scratch of the layers: 128 rows (or the batch) at first, then to the prompt, at least to twice what there
+// was (up to the longest prompt a state can take), so that a state of many prompts moves it a few times only.  Where
+// memory is short it settles for less: a prompt then goes through the layers in more pieces.  Graphs captured before hold
+// the old addresses and are dropped.
 static int reserve_rows(State* s, int rows) {
     if (rows <= s->cap_rows) return LSPK_OK;
-    if (s->cap_rows > 0 && s->t_max > rows) rows = s->t_max < kMaxPrefillRows ? s->t_max : kMaxPrefillRows;
+    const int least = s->batch > kMinRows ? s->batch : kMinRows;
+    const int longest = s->t_max < kMaxPrefillRows ? s->t_max : kMaxPrefillRows;
+    if (rows < 2 * s->cap_rows) rows = 2 * s->cap_rows < longest ? 2 * s->cap_rows : (rows > longest ? rows : longest);
     const lspk_model_config& c = s->m->cfg;
-    const size_t R = (size_t)((rows + 127) / 128) * 128, H = c.hidden_size, I = c.intermediate_size, kv = s->m->kv_dim();
+    const size_t H = c.hidden_size, I = c.intermediate_size, kv = s->m->kv_dim();
     LSPK_CUDA(cudaStreamSynchronize(stream()));
     for (auto& g : s->graph) {
         if (g) cudaGraphExecDestroy(g);
@@ -182,20 +187,32 @@ static int reserve_rows(State* s, int rows) {
     struct Buf { void** p; size_t width; };
     const Buf bufs[] = {{(void**)&s->x, H}, {(void**)&s->q, H}, {(void**)&s->k, kv}, {(void**)&s->v, kv}, {(void**)&s->attn, H},
                         {(void**)&s->inter, I}, {(void**)&s->tok_rows, 1}};
-    for (const Buf& b : bufs) {
-        if (*b.p) {
+    size_t width = 0;
+    for (const Buf& b : bufs) width += b.width;
+    auto release = [&]() {
+        for (const Buf& b : bufs) {
             cudaFree(*b.p);
-            s->bytes -= (size_t)s->cap_rows * b.width * 4;
+            *b.p = nullptr;
         }
-        *b.p = nullptr;
-    }
+    };
+    release();
+    s->bytes -= (size_t)s->cap_rows * width * 4;
     s->cap_rows = 0;
-    for (const Buf& b : bufs) {
-        LSPK_CUDA(device_malloc(b.p, R * b.width * 4));
-        s->bytes += R * b.width * 4;
+    for (size_t R = (size_t)((rows + 127) / 128) * 128;; R = (R / 2 + 127) / 128 * 128) {
+        if (R < (size_t)least) R = (size_t)((least + 127) / 128) * 128;
+        cudaError_t e = cudaSuccess;
+        for (const Buf& b : bufs)
+            if (e == cudaSuccess) e = device_malloc(b.p, R * b.width * 4);
+        if (e == cudaSuccess) {
+            s->cap_rows = (int)R;
+            s->bytes += R * width * 4;
+            return LSPK_OK;
+        }
+        release();
+        cudaGetLastError();
+        if (e != cudaErrorMemoryAllocation || R <= (size_t)((least + 127) / 128) * 128)
+            return fail(LSPK_ERR_CUDA, "scratch of %zu rows: %s", R, cudaGetErrorString(e));
     }
-    s->cap_rows = (int)R;
-    return LSPK_OK;
 }
 
 // Pinned staging for logits, made when a call first wants them (a greedy loop never does; pinning takes milliseconds).

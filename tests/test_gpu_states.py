@@ -163,6 +163,44 @@ assert 0 < np.abs(int8 - want).max() < 0.1 * np.abs(want).max()
 """
 
 
+_SHORT_OF_MEMORY = """
+import importlib
+import numpy as np
+import __graft_entry__ as entry
+entry.load_package()
+name = "litespark_inference_b200.torchless."
+K, rt, synthetic = (importlib.import_module(name + n) for n in ("kernel", "runtime", "synthetic"))
+dm = rt.DeviceModel(synthetic.random_model(synthetic.toy_config(), seed=3, norm_jitter=0.1))
+lib = dm.lib
+toks = [int(t) for t in np.random.default_rng(1).integers(0, 1024, 1000)]
+row = 4 * (3 * 256 + 2 * 128 + 512 + 1)
+a, b = rt.init_state(dm, 2048), rt.init_state(dm, 2048)
+small = a.device_bytes
+want = rt.forward_prefill(dm, a, toks)
+assert a.device_bytes == small + (1024 - 128) * row          # as many rows as the prompt, not as the cache could take
+K.check(lib.lspk_debug_allocation_limit(1200000))            # the widest buffer finds room for 512 rows
+got = rt.forward_prefill(dm, b, toks)
+assert b.pos == 1000 and b.device_bytes == small + (512 - 128) * row
+# pieces of 512 rows: other attention sums, so as for a prompt given in pieces (test_gpu_prefill_kernels.py)
+assert np.abs(got - want).max() <= 5e-3 * (want.max() - want.min())
+K.check(lib.lspk_debug_allocation_limit(1000))               # nothing at all: an error, and the state is still good for use
+b.pos = 0
+try:
+    rt.forward_prefill(dm, b, toks)
+    raise SystemExit("a prefill without memory went through")
+except K.KernelError:
+    pass
+K.check(lib.lspk_debug_allocation_limit(0))
+b.pos = 0
+assert np.abs(rt.forward_prefill(dm, b, toks) - want).max() <= 5e-3 * (want.max() - want.min())
+assert b.device_bytes == a.device_bytes
+"""
+
+
+def test_a_long_prompt_makes_do_with_less_memory():
+    _in_own_process(_SHORT_OF_MEMORY)
+
+
 def _in_own_process(code):
     r = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True,
                        timeout=300)
