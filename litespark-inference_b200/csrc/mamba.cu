@@ -8,8 +8,7 @@
 //   out = out_proj(quant(RMSNorm(y * SiLU(z))));  x += out      ternary linear, residual epilogue
 // The state update is the HBM-bound part: the fp32 state [heads, head_dim, d_state] (2.6 MB per
 // sequence and layer at 80 x 64 x 128) is read and written once per step.  One CTA owns half a head (32 rows of
-// 128 states, 16 KB in and out; grid = 2 * heads x sequences); for four and more sequences the states are a stream through one CTA
-// per SM.
+// 128 states, 16 KB in and out; grid = 2 * heads x sequences).
 #include "internal.cuh"
 #include "../../include/lspk_hybrid.h"
 
@@ -60,9 +59,11 @@ __device__ __forceinline__ float ssu_row_sum(float v) {
     return v + __shfl_xor_sync(0xffffffffu, v, 1);
 }
 
-// P = head_dim = 64, N = d_state = 128.  A CTA of 256 threads owns half a head (grid 2 * heads x sequences): the form for
-// one to three sequences, where covering the SMs counts.  8 threads share a row; thread `seg` of a row holds the four
-// 16-byte pieces seg, seg + 8, ... of its 128 states.
+// P = head_dim = 64, N = d_state = 128.  A CTA of 256 threads owns half a head (grid 2 * heads x sequences).  8 threads
+// share a row; thread `seg` of a row holds the four 16-byte pieces seg, seg + 8, ... of its 128 states.
+// One form for any number of sequences.  A persistent one (a CTA per SM, whole heads through a ring of bulk copies) was
+// faster by itself at sixteen sequences with a cold cache (19.0 us against 20.9) and slower in a hybrid step at every
+// number: 1006 us against 987 for four sequences, 1088 against 1061 for eight, 1420 against 1401 for sixteen.
 constexpr int ROWS = 32;
 __global__ void __launch_bounds__(256)
 mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr,
@@ -155,154 +156,6 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     }
 }
 
-// Four and more sequences: the launch is bound by the state's trip through the SMs (84 MB in and out at sixteen sequences
-// of 80 heads; 12.9 us at the measured copy rate).  A CTA per half or whole head kept too little of it in flight: the
-// convolution in front of each head's update waits for memory with the SM's registers holding the loads, and 1280
-// CTAs are 2.2 waves of four per SM (20.9 us).  Here one CTA per SM takes a contiguous run of (sequence, head) pairs: a warp
-// brings their 32 KB state matrices into a ring of five slots by bulk copies and sends each back by a bulk copy once
-// sixteen warps have updated it in place; the convolution, the gate and the step sizes of up to kSsuChunk heads are
-// formed together, ahead of the updates, while the ring fills: 19.0 us cold at sixteen sequences, of which about 4 are
-// the launch and the first tile's trip.  Taken from four sequences (two tiles and more per SM): with it a hybrid step of
-// four took 973 us (1249 with the CTA-per-head form and the slower MoE of that time), below that the SMs are not covered.
-// Same arithmetic and sums as the kernel above.
-constexpr int kSsuSlots = 5, kSsuChunk = 12, kSsuWarps = 16;
-constexpr int kSsuThreads = 32 * (kSsuWarps + 1);
-constexpr uint32_t kSsuTileBytes = 64 * 128 * 4;
-constexpr long long kSsuBudgetCycles = 1ll << 31;              // every wait of a CTA gives up after about a second
-
-__global__ void __launch_bounds__(kSsuThreads, 1)
-mamba2_ssu_stream_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr,
-                         const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ A,
-                         const float* __restrict__ dt_bias, const float* __restrict__ Dskip, float* __restrict__ vout,
-                         int d_inner, int conv_dim, int in_out, size_t state_floats, int nheads, int items, int* error_flag) {
-    constexpr int P = 64, N = 128;
-    extern __shared__ __align__(128) unsigned char ring[];
-    __shared__ __align__(8) uint64_t full[kSsuSlots], done[kSsuSlots];
-    __shared__ __align__(16) float B_s[N], C_s[N];
-    __shared__ float xs_s[kSsuChunk * P], zs_s[kSsuChunk * P];
-    __shared__ float dt_s[kSsuChunk], dA_s[kSsuChunk], D_s[kSsuChunk];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int lo = (int)((long long)items * blockIdx.x / gridDim.x), hi = (int)((long long)items * (blockIdx.x + 1) / gridDim.x);
-    const long long deadline = clock64() + kSsuBudgetCycles;
-    if (tid < kSsuSlots) {
-        mbar_init(&full[tid], 1);
-        mbar_init(&done[tid], kSsuWarps);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    grid_dependency_launch();
-    grid_dependency_wait();                  // also orders this launch after the one that wrote the state a step ago
-    auto tile_of = [&](int it) -> float* {
-        return state + (size_t)(it / nheads) * state_floats + (size_t)conv_dim * 4 + (size_t)(it % nheads) * P * N;
-    };
-    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-        bool ok = mbar_try_wait(bar, parity);
-        while (!ok && !(clock64() > deadline)) ok = mbar_try_wait(bar, parity);
-        return ok;
-    };
-
-    if (warp == kSsuWarps) {
-        // ---------------- the ring: one lane requests, and sends back, tile after tile ------------------------------
-        if (lane == 0) {
-            auto request = [&](int it) {
-                const int slot = (it - lo) % kSsuSlots;
-                mbar_expect_tx(&full[slot], kSsuTileBytes);
-                bulk_load(ring + (size_t)slot * kSsuTileBytes, tile_of(it), kSsuTileBytes, &full[slot]);
-            };
-            int requested = lo;
-            for (; requested < hi && requested < lo + kSsuSlots; ++requested) request(requested);
-            for (int it = lo; it < hi; ++it) {
-                const int slot = (it - lo) % kSsuSlots;
-                if (!wait(&done[slot], (uint32_t)((it - lo) / kSsuSlots) & 1u)) {
-                    // the updating warps gave up: let the copies in flight land, then leave
-                    if (error_flag) atomicExch(error_flag, LSPK_ERR_DEVICE_WAIT);
-                    const long long until = clock64() + kSsuBudgetCycles;
-                    for (int k = it; k < requested; ++k)
-                        while (!mbar_try_wait(&full[(k - lo) % kSsuSlots], (uint32_t)((k - lo) / kSsuSlots) & 1u) && clock64() <= until) {}
-                    break;
-                }
-                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(tile_of(it)),
-                             "r"(smem_u32(ring + (size_t)slot * kSsuTileBytes)), "r"(kSsuTileBytes)
-                             : "memory");
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                // the tile before this one has left its slot: refill it
-                if (it > lo && requested < hi) {
-                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    request(requested++);
-                }
-            }
-            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-        }
-        return;
-    }
-
-    const int seg = tid & 7, p = tid >> 3;
-    bool ok = true;
-    for (int i0 = lo; i0 < hi;) {
-        // up to kSsuChunk heads of one sequence: convolution step + SiLU of their x channels and of B and C, gates, step sizes
-        const int b = i0 / nheads, h0 = i0 % nheads;
-        const int n = min(min(hi - i0, kSsuChunk), nheads - h0), nx = n * P;
-        const float* zrow = zx + (size_t)b * in_out;
-        float* conv_ring = state + (size_t)b * state_floats;            // [conv_dim][4]
-        const int pos = pos_ptr[b];
-#pragma unroll 2
-        for (int idx = tid; idx < nx + 2 * N; idx += 32 * kSsuWarps) {
-            const int ch = idx < nx ? h0 * P + idx : d_inner + (idx - nx);
-            const float newv = zrow[d_inner + ch];
-            const float4 taps = *reinterpret_cast<const float4*>(conv_w + (size_t)ch * 4);
-            const float4 hist = *reinterpret_cast<const float4*>(conv_ring + (size_t)ch * 4);
-            const float z = idx < nx ? zrow[h0 * P + idx] : 0.0f;
-            const float act = conv_silu(conv_b[ch], taps, hist, newv, pos);
-            if (idx < nx) {
-                xs_s[idx] = act;
-                zs_s[idx] = silu_f(z);
-            } else if (idx < nx + N) {
-                B_s[idx - nx] = act;
-            } else {
-                C_s[idx - nx - N] = act;
-            }
-            // the newest input replaces the oldest slot; nobody reads that slot during this step
-            if (idx < nx || h0 == 0) conv_ring[(size_t)ch * 4 + (pos & 3)] = newv;
-        }
-        if (tid < n) {
-            const float dv = __fadd_rn(zrow[d_inner + conv_dim + h0 + tid], dt_bias[h0 + tid]);
-            const float dt = dv > 20.0f ? dv : log1pf(expf(dv));
-            dt_s[tid] = dt;
-            dA_s[tid] = expf(__fmul_rn(dt, A[h0 + tid]));
-            D_s[tid] = Dskip[h0 + tid];
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * kSsuWarps) : "memory");
-        float4 Bv[4], Cv[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            Bv[q] = reinterpret_cast<const float4*>(B_s)[8 * q + seg];
-            Cv[q] = reinterpret_cast<const float4*>(C_s)[8 * q + seg];
-        }
-        for (int k = 0; k < n && ok; ++k) {
-            const int it = i0 + k - lo, slot = it % kSsuSlots;
-            ok = __all_sync(0xffffffffu, wait(&full[slot], (uint32_t)(it / kSsuSlots) & 1u));
-            if (!ok) break;
-            float4* srow = reinterpret_cast<float4*>(ring + (size_t)slot * kSsuTileBytes) + p * (N / 4) + seg;
-            const float dA = dA_s[k], xv = xs_s[k * P + p], dtx = __fmul_rn(dt_s[k], xv);
-            float ysum = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float4 st = srow[8 * q];
-                ssu_update(st, dA, dtx, Bv[q], Cv[q], ysum);
-                srow[8 * q] = st;
-            }
-            fence_async_smem();                  // the copy back reads what this thread wrote
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&done[slot]);
-            ysum = ssu_row_sum(ysum);
-            if (seg == 0)
-                vout[(size_t)b * d_inner + (h0 + k) * P + p] = __fmul_rn(__fadd_rn(ysum, __fmul_rn(D_s[k], xv)), zs_s[k * P + p]);
-        }
-        i0 += n;
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * kSsuWarps) : "memory");      // the chunk's arrays are rewritten next
-    }
-}
-
 size_t mamba_state_floats(const Mamba* m) { return m->state_floats(); }
 
 int mamba_reserve(Mamba* m, int B) {
@@ -336,23 +189,9 @@ int mamba_step(Mamba* m, float* x, float* state, const int* pos, int B) {
     a.eps = m->cfg.eps;
     // several rows: linear_cuda_core quantises them once, straight into the eight-row kernel's tile layout
     if (int rc = linear_cuda_core(&a)) return rc;
-    const int items = m->cfg.nheads * B;
-    if (B >= 4) {
-        static bool attr_set = false;
-        const size_t smem = (size_t)kSsuSlots * kSsuTileBytes;
-        if (!attr_set) {
-            LSPK_CUDA(cudaFuncSetAttribute(mamba2_ssu_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            attr_set = true;
-        }
-        LSPK_CUDA(launch(mamba2_ssu_stream_kernel, dim3(items < sm_count() ? items : sm_count()), dim3(kSsuThreads), smem, true,
-                         (const float*)m->zx, state, pos, (const float*)m->conv_w, (const float*)m->conv_b, (const float*)m->A,
-                         (const float*)m->dt_bias, (const float*)m->D, m->v, m->d_inner, m->conv_dim, m->in_out,
-                         m->state_floats(), m->cfg.nheads, items, device_wait_flag()));
-    } else {
-        LSPK_CUDA(launch(mamba2_ssu_kernel, dim3(m->cfg.nheads * 2, B), dim3(256), 0, true, (const float*)m->zx, state, pos,
-                         (const float*)m->conv_w, (const float*)m->conv_b, (const float*)m->A, (const float*)m->dt_bias,
-                         (const float*)m->D, m->v, m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
-    }
+    LSPK_CUDA(launch(mamba2_ssu_kernel, dim3(m->cfg.nheads * 2, B), dim3(256), 0, true, (const float*)m->zx, state, pos,
+                     (const float*)m->conv_w, (const float*)m->conv_b, (const float*)m->A, (const float*)m->dt_bias,
+                     (const float*)m->D, m->v, m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
     lspk_linear_args o = {};
     o.w[0] = m->out_proj;
     o.out[0] = x;

@@ -1,5 +1,4 @@
-"""The Mamba-2 state update of four and more sequences (state matrices as a stream through one CTA per SM) at the edges of
-its split: fewer heads than CTAs, sequences shorter than a chunk of heads, runs that cross a sequence, full slot rings."""
+"""The Mamba-2 state update of four and more sequences: one head and many, few sequences and more than a hundred."""
 import importlib
 import sys
 from pathlib import Path
@@ -17,7 +16,7 @@ dev = importlib.import_module("litespark_inference_b200.torchless.device")
 
 
 @pytest.mark.parametrize("nheads,B", [(1, 4), (4, 5), (20, 40), (80, 4), (13, 150)])
-def test_streamed_state_update_matches_oracle(port, nheads, B):
+def test_batched_state_update_matches_oracle(port, nheads, B):
     cfg = hyb.HybridConfig(hidden_size=256, num_layers=2, vocab_size=64, num_experts=2, intermediate_size=64, nheads=nheads,
                            headdim=64, d_state=128)
     layer = next(L for L in hyb.random_hybrid(cfg, seed=nheads, norm_jitter=0.1).layers if L.kind == "mamba")
