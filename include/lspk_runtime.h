@@ -55,7 +55,11 @@ int lspk_model_free(lspk_model_t m);
  * rope_tables (ops.py:40-50) so that the rotation uses bit-identical tables. */
 lspk_state_t lspk_state_create(lspk_model_t m, int t_max, int batch, int kv_fp16,
                                const float* rope_cos, const float* rope_sin);
+/* A freed state is kept for the next lspk_state_create of the same model, shape and tables: one per model, 1 GiB together.
+ * The library takes that memory back when one of its own allocations fails; other allocators of the process cannot, so a
+ * program that shares the GPU with one calls lspk_release_parked_states when it is done with states for a while. */
 int lspk_state_free(lspk_state_t s);
+int lspk_release_parked_states(void);
 int lspk_state_get_pos(lspk_state_t s, int seq);
 int lspk_state_set_pos(lspk_state_t s, int seq, int pos);    /* rollback / reuse (runtime.py:629) */
 size_t lspk_state_device_bytes(lspk_state_t s);

@@ -74,6 +74,15 @@ cudaError_t device_malloc(void** p, size_t bytes) {
     return e;
 }
 
+cudaError_t pinned_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMallocHost(p, bytes);
+    if (e == cudaErrorMemoryAllocation && release_parked_states()) {
+        cudaGetLastError();
+        e = cudaMallocHost(p, bytes);
+    }
+    return e;
+}
+
 // Lazily bind to a device the first time any entry point needs one.
 
 int ensure_init() {
@@ -192,7 +201,7 @@ int lspk_free(void* dev) {
 void* lspk_host_alloc(size_t bytes) {
     if (ensure_init()) return nullptr;
     void* p = nullptr;
-    cudaError_t e = cudaMallocHost(&p, bytes ? bytes : 16);
+    cudaError_t e = pinned_malloc(&p, bytes ? bytes : 16);
     if (e != cudaSuccess) {
         fail(LSPK_ERR_CUDA, "cudaMallocHost(%zu) failed: %s", bytes, cudaGetErrorString(e));
         return nullptr;

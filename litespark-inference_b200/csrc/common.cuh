@@ -20,13 +20,14 @@ bool pdl_enabled();                                 // programmatic dependent la
 void set_pdl_enabled(bool on);                      // for launches of one's own, also while capturing (lspk_set_pdl frees memory)
 int  sm_count();
 int  ensure_init();                                 // bind to a GPU on first use
-// Library-owned device scratch (the row quantiser's buffers, the K-split workspace, the per-layer buffers of
+// cudaMalloc / cudaMallocHost that give parked memory (inference states kept for reuse, runtime.cu) back before they fail.
+cudaError_t device_malloc(void** p, size_t bytes);
+cudaError_t pinned_malloc(void** p, size_t bytes);
+bool release_parked_states();                       // true if something was freed
+// Library-owned device scratch (the row quantiser's buffers, the per-layer buffers of
 // the MoE and Mamba blocks) grows by free + malloc, which moves it.  A CUDA graph captured earlier holds the
 // old addresses, so whoever moves scratch bumps this counter and every graph owner compares it with the value
 // it recorded at capture and re-captures when they differ.
-// cudaMalloc that gives parked memory (inference states kept for reuse, runtime.cu) back before it fails.
-cudaError_t device_malloc(void** p, size_t bytes);
-bool release_parked_states();                       // true if something was freed
 unsigned scratch_generation();
 void scratch_moved();
 

@@ -211,8 +211,8 @@ lspk_hybrid_state_t lspk_hybrid_state_create(lspk_hybrid_t hh, int batch, int ma
     alloc((void**)&s->tokens_out, (size_t)max_steps * batch * 4);
     alloc((void**)&s->x, (size_t)batch * h->H * 4);
     alloc((void**)&s->logits, (size_t)lrows * h->V * 4);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&s->h_int, (size_t)(max_steps * batch + 2 * batch + 16) * 4);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&s->h_logits, (size_t)batch * h->V * 4);
+    if (e == cudaSuccess) e = pinned_malloc((void**)&s->h_int, (size_t)(max_steps * batch + 2 * batch + 16) * 4);
+    if (e == cudaSuccess) e = pinned_malloc((void**)&s->h_logits, (size_t)batch * h->V * 4);
     if (e != cudaSuccess || lspk_hybrid_state_reset(reinterpret_cast<lspk_hybrid_state_t>(s)) != LSPK_OK) {
         fail(LSPK_ERR_CUDA, "lspk_hybrid_state_create: %s", cudaGetErrorString(e));
         lspk_hybrid_state_free(reinterpret_cast<lspk_hybrid_state_t>(s));

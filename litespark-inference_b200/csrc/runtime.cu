@@ -217,15 +217,16 @@ static int reserve_rows(State* s, int rows) {
 
 // Pinned staging for logits, made when a call first wants them (a greedy loop never does; pinning takes milliseconds).
 static int reserve_host_logits(State* s) {
-    if (!s->h_logits) LSPK_CUDA(cudaMallocHost((void**)&s->h_logits, (size_t)s->logits_rows * s->m->cfg.vocab_size * 4));
+    if (!s->h_logits) LSPK_CUDA(pinned_malloc((void**)&s->h_logits, (size_t)s->logits_rows * s->m->cfg.vocab_size * 4));
     return LSPK_OK;
 }
 
 // Parked states.  A program that makes a state per request (the facade does) frees and makes the same one over and over;
 // its allocations, pinned buffers and instantiated graph cost several milliseconds.  A freed state is therefore kept, at
-// most one per live model and kMaxParkedBytes each, and handed out again, cleared, to a request for the same shape and
-// rope tables.  It is given back when its model is freed, when another state takes its place, and when an allocation
-// fails (device_malloc).
+// most one per live model and kMaxParkedBytes together, and handed out again, cleared, to a request for the same shape and
+// rope tables.  It is given back when its model is freed, when another state takes its place, when an allocation of this
+// library fails (device_malloc, pinned_malloc), and on request (lspk_release_parked_states): another allocator in the
+// process cannot see that the memory is to be had.
 constexpr size_t kMaxParkedBytes = (size_t)1 << 30;
 static std::mutex g_park_mu;
 static std::map<unsigned long long, State*> g_parked;      // one entry per live model; null: nothing parked
@@ -656,7 +657,7 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
     rc |= dev_alloc((void**)&s->tokens_out, (size_t)t_max * batch * 4, &s->bytes);
     rc |= dev_alloc((void**)&s->logits, (size_t)s->logits_rows * V * 4, &s->bytes);
     rc |= reserve_rows(s, batch > 128 ? batch : 128);
-    if (!rc && cudaMallocHost((void**)&s->h_int, (size_t)(t_max * batch + 2 * batch + 16) * 4) != cudaSuccess) rc = 1;
+    if (!rc && pinned_malloc((void**)&s->h_int, (size_t)(t_max * batch + 2 * batch + 16) * 4) != cudaSuccess) rc = 1;
     if (!rc && batch == 1) {
         // the two words of the host-fed step (see State): mapped pinned memory and its device alias
         void *io = nullptr, *io_dev = nullptr;
@@ -692,14 +693,25 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
 int lspk_state_free(lspk_state_t h) {
     if (!h) return LSPK_OK;
     State* s = reinterpret_cast<State*>(h);
-    if (s->bytes <= kMaxParkedBytes) {
+    {
         std::lock_guard<std::mutex> lk(g_park_mu);
         auto it = g_parked.find(s->model_id);      // no entry: the model is gone
-        if (it != g_parked.end()) std::swap(it->second, s);
+        if (it != g_parked.end()) {
+            size_t others = 0;
+            for (const auto& kv : g_parked)
+                if (kv.second && kv.second != it->second) others += kv.second->bytes;
+            if (s->bytes + others <= kMaxParkedBytes) std::swap(it->second, s);
+        }
     }
     if (s) destroy_state(s);
     return LSPK_OK;
 }
+
+int lspk_release_parked_states(void) {
+    release_parked_states();
+    return LSPK_OK;
+}
+
 int lspk_state_get_pos(lspk_state_t h, int seq) {
     State* s = reinterpret_cast<State*>(h);
     if (!s || seq < 0 || seq >= s->batch) return -1;

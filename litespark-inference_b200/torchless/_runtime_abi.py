@@ -31,6 +31,7 @@ SIGNATURES = {
     "lspk_forward_prefill": ([_vp, _ci, _vp, _ci, _vp, _vp, _vp], _ci),
     "lspk_decode_greedy": ([_vp, _vp, _ci, _vp], _ci),
     "lspk_state_step_kernel_count": ([_vp], _ci),
+    "lspk_release_parked_states": ([], _ci),
     "lspk_debug_expire_wait": ([_ci], _ci),
     "lspk_debug_prefill_attention": ([_vp] * 9 + [_ci] * 6, _ci),
     "lspk_debug_allocation_limit": ([_sz], _ci),

@@ -199,6 +199,12 @@ def init_state(model, t_max: int, batch: int = 1, kv_dtype: Optional[str] = None
     return InferState(model, t_max, batch=batch, kv_dtype=kv_dtype)
 
 
+def release_parked_states() -> None:
+    """Give back the GPU memory of closed states that the library keeps for the next state of the same shape (one per
+    model, 1 GiB together), for a program that shares the GPU with another allocator."""
+    _k.check(_k.load_library(True).lspk_release_parked_states())
+
+
 def _raise_state(lib, rc: int):
     msg = lib.lspk_last_error().decode()
     if rc == 4:      # LSPK_ERR_STATE: the reference raises RuntimeError for an exhausted cache

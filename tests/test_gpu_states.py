@@ -121,6 +121,48 @@ def test_a_state_made_after_a_trace_or_launch_mode_change_uses_it():
     _in_own_process(_TRACE_AND_LAUNCH_MODE)
 
 
+_GIVEN_BACK = """
+import ctypes, importlib
+import numpy as np
+import __graft_entry__ as entry
+entry.load_package()
+name = "litespark_inference_b200.torchless."
+K, rt, synthetic = (importlib.import_module(name + n) for n in ("kernel", "runtime", "synthetic"))
+dms = [rt.DeviceModel(synthetic.random_model(synthetic.toy_config(), seed=3)) for _ in range(4)]
+lib = dms[0].lib
+
+def free_bytes():
+    f = ctypes.c_size_t()
+    K.check(lib.lspk_mem_info(ctypes.byref(f), None))
+    return f.value
+
+big = dict(t_max=8192, batch=24, kv_dtype="fp32")            # 400 MB: two of them are kept, a third is not
+held = []
+for dm in dms:
+    st = rt.init_state(dm, **big)
+    size = st.device_bytes
+    rt.forward_step(st, np.arange(24, dtype=np.int32))
+    before = free_bytes()
+    st.close()
+    held.append(free_bytes() - before < size // 2)
+assert 3.9e8 < size < 4.4e8 and held == [True, True, False, False], (size, held)
+before = free_bytes()
+rt.release_parked_states()
+assert free_bytes() - before > 1.9 * size
+rt.release_parked_states()                                   # nothing left: no effect
+st = rt.init_state(dms[0], **big)
+st.close()
+K.check(lib.lspk_debug_allocation_limit(1 << 30))            # an allocation of this library that fails takes it back
+before = free_bytes()
+assert not lib.lspk_malloc(2 << 30)
+assert free_bytes() - before > 0.9 * size
+"""
+
+
+def test_memory_of_parked_states_is_bounded_and_given_back():
+    _in_own_process(_GIVEN_BACK)
+
+
 _SCRATCH_LOST = """
 import ctypes, importlib
 import numpy as np
