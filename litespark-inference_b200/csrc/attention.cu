@@ -1147,6 +1147,31 @@ __global__ void __launch_bounds__(kAttnThreads) attention_rows_kernel(const Attn
     }
 }
 
+// Shared memory of attention_group_kernel with two heads.
+static size_t attention_group_smem(int D, int t_max, int kv_bytes) {
+    const int groups = kAttnThreads / (D * kv_bytes / 16), local_keys = (t_max + kSplit - 1) / kSplit + 1;
+    return (size_t)((2 * 2 + 3) * D + 2 * groups * D + kSplit * D + 2 * local_keys) * sizeof(float);
+}
+
+// When the grouped form pays, by the positions a step attends to (not by the room in the cache: a serving state has a long
+// one and mostly short contexts).  It halves the reads of the cache and takes half the CTAs, of the 256-thread kind.  Measured
+// at 20 / 5 heads of 128, ms per step of the whole decoder, other kernel -> this one:
+//   2 sequences, fp16   1.261 -> 1.237 at 30 keys each, 1.388 -> 1.246 at 1000; fp32 1.168 -> 1.202 at 30, 1.214 -> 1.202 at 300
+//   3                   1.297 -> 1.245 and 1.264 -> 1.208 at 30 keys: always (the other kernel's 480 CTAs are 1.1 waves)
+//   8, fp16             1.245 -> 1.492 at 200 keys, 1.455 -> 1.521 at 700, 1.578 -> 1.546 at 1000, 2.034 -> 1.833 at 2000
+//   8, fp32             1.297 -> 1.404 at 200, 1.393 -> 1.407 at 300, 1.487 -> 1.414 at 400, 2.747 -> 2.126 at 2000
+//   8, one of them long, the others 20 keys: fp16 1.278 -> 1.479 at 1000, 1.508 -> 1.485 at 2000; fp32 1.456 -> 1.389 at 1000
+// The middle between the longest and the mean sequence orders both kinds of batch; with the lines below no batch of 2 to
+// 32 sequences up to 4000 keys is more than 6 % behind the better kernel (by the room in the cache: 40 %).
+bool attention_group_heads(int T, int Q, int KV, int D, int t_max, int kv_is_fp16, long long longest, long long total) {
+    if (T < 2 || Q % KV || (Q / KV) % 2 || (D != 64 && D != 128) || attention_group_smem(D, t_max, kv_is_fp16 ? 2 : 4) > 200 * 1024)
+        return false;
+    const long long depth = (longest + total / T) / 2;
+    if (T == 3) return true;
+    if (T == 2) return kv_is_fp16 || depth >= 275;
+    return depth >= (kv_is_fp16 ? 900 : 275);
+}
+
 template <typename KVT>
 static int attention_launch_t(const AttnParams& p) {
     const int D = p.D;
@@ -1209,13 +1234,9 @@ static int attention_launch_t(const AttnParams& p) {
             split_attr_set = true;
         }
         LSPK_REQUIRE(sm <= 200 * 1024, "attention: t_max=%d too large for the shared score buffer", p.t_max);
-        // Several sequences with long caches, and query heads that share a KV head: cache rows fetched once for two heads.
-        // Long: a CTA may hold more keys than two of the other kernel's batches.  Shorter caches are bound by latency and
-        // want the CTAs: eight sequences behind 128 to 205 positions took 1.35 ms per step in the other kernel, 1.46 in
-        // this one (four heads).  One sequence stays there for the same reason.
-        const int ng = kAttnThreads / tpk;
-        const size_t gsm = (size_t)((2 * 2 + 3) * D + 2 * ng * D + kSplit * D + 2 * local_keys) * sizeof(float);
-        if (p.T > 1 && (p.Q / p.KV) % 2 == 0 && D <= 128 && gsm <= 200 * 1024 && local_keys > 8 * ng) {
+        if (p.group_heads) {
+            const size_t gsm = attention_group_smem(D, p.t_max, (int)sizeof(KVT));
+            LSPK_REQUIRE((p.Q / p.KV) % 2 == 0 && D <= 128 && gsm <= 200 * 1024, "attention: this shape has no grouped-heads form");
             const cudaError_t ge = D == 128 ? launch_attention_group<KVT, 128, 2, 8, 2>(p, gsm) : launch_attention_group<KVT, 64, 2, 8, 2>(p, gsm);
             if (ge != cudaSuccess) return fail(LSPK_ERR_CUDA, "attention (grouped heads) launch failed: %s", cudaGetErrorString(ge));
             return LSPK_OK;

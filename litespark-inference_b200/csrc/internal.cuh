@@ -110,10 +110,13 @@ struct AttnParams {
     size_t cache_seq_stride;  // elements between the caches of consecutive sequences (pos_per_row)
     int T, Q, KV, D, t_max;
     int fused;             // 1: rotate + cache write inside the attention kernel (independent rows)
+    int group_heads;       // fused: two query heads of a KV head per CTA (attention_group_heads said so)
     unsigned long long* trace;
     int trace_cap;
 };
 int attention_launch(const AttnParams& p, int kv_is_fp16);
+// Whether a decode step of T sequences, the longest and all together so many positions long, wants AttnParams::group_heads.
+bool attention_group_heads(int T, int Q, int KV, int D, int t_max, int kv_is_fp16, long long longest, long long total);
 // attention_mma.cu: tensor-core form for 16 and more consecutive rows of one sequence (rope_store_kernel has run).
 int attention_prefill_mma(const AttnParams& p, int kv_is_fp16, int* handled);
 

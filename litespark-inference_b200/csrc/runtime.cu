@@ -325,6 +325,7 @@ int run_layer(State* s, int li, int rows, bool per_row_seq, int seq, bool skip_a
         p.D = m->D();
         p.t_max = s->t_max;
         p.fused = (per_row_seq || rows == 1) ? 1 : 0;
+        p.group_heads = s->group_heads ? 1 : 0;
         if (int rc = attention_launch(p, s->kv_fp16)) return rc;
     }
     {
@@ -405,8 +406,26 @@ static int clear_state(State* s) {
     return LSPK_OK;
 }
 
+// The kind of graph (State::graph) that a step of several sequences `ahead` steps from now takes.
+static int batch_variant(const State* s, int ahead) {
+    const lspk_model_config& c = s->m->cfg;
+    long long longest = 0, total = 0;
+    for (int pos : s->host_pos) {
+        const long long n = (long long)pos + ahead + 1;
+        longest = n > longest ? n : longest;
+        total += n;
+    }
+    return attention_group_heads(s->batch, c.num_heads, c.num_kv_heads, s->m->D(), s->t_max, s->kv_fp16, longest, total) ? 3 : 1;
+}
+
 static int build_graph(State* s, int variant) {
     if (int rc = reserve_rows(s, s->batch)) return rc;
+    auto enqueue_variant = [&]() {
+        s->group_heads = variant == 3;
+        const int rc = enqueue_step(s, variant == 1 || variant == 3, variant == 2);
+        s->group_heads = false;
+        return rc;
+    };
     if (s->graph[variant] && s->graph_gen[variant] == scratch_generation()) return LSPK_OK;
     if (s->graph[variant]) {
         // library scratch whose addresses the graph holds was moved by a later call (a larger prefill, a
@@ -426,7 +445,7 @@ static int build_graph(State* s, int variant) {
         std::vector<int> saved(nctl);
         LSPK_CUDA(cudaMemcpyAsync(saved.data(), s->ctl, nctl * sizeof(int), cudaMemcpyDeviceToHost, stream()));
         LSPK_CUDA(cudaStreamSynchronize(stream()));
-        if (int rc = enqueue_step(s, variant == 1, variant == 2)) return rc;
+        if (int rc = enqueue_variant()) return rc;
         LSPK_CUDA(cudaStreamSynchronize(stream()));
         LSPK_CUDA(cudaMemcpyAsync(s->ctl, saved.data(), nctl * sizeof(int), cudaMemcpyHostToDevice, stream()));
         LSPK_CUDA(cudaStreamSynchronize(stream()));
@@ -436,7 +455,7 @@ static int build_graph(State* s, int variant) {
 
     cudaGraph_t g = nullptr;
     LSPK_CUDA(cudaStreamBeginCapture(stream(), cudaStreamCaptureModeThreadLocal));
-    int rc = enqueue_step(s, variant == 1, variant == 2);
+    int rc = enqueue_variant();
     cudaError_t e = cudaStreamEndCapture(stream(), &g);
     if (rc) {
         if (g) cudaGraphDestroy(g);
@@ -787,7 +806,7 @@ int lspk_forward_step(lspk_state_t h, const int* tokens_host, float* logits_host
         s->host_pos[0] += 1;
         return LSPK_OK;
     }
-    const int variant = (logits_host || B > 1) ? 1 : 0;
+    const int variant = B > 1 ? batch_variant(s, 0) : logits_host ? 1 : 0;
     if (logits_host)
         if (int rc = reserve_host_logits(s)) return rc;
     if (int rc = build_graph(s, variant)) return rc;
@@ -814,12 +833,15 @@ int lspk_decode_greedy(lspk_state_t h, const int* first_tokens_host, int n_steps
         if (s->host_pos[b] + n_steps > s->t_max)
             return fail(LSPK_ERR_STATE, "inference state exhausted: pos=%d + %d steps > t_max=%d", s->host_pos[b],
                         n_steps, s->t_max);
-    const int variant = B > 1 ? 1 : 0;
-    if (int rc = build_graph(s, variant)) return rc;
+    // several sequences: positions only grow, so there is one change of kind at most
+    auto variant_at = [&](int i) { return B > 1 ? batch_variant(s, i) : 0; };
+    if (int rc = build_graph(s, variant_at(0))) return rc;
+    if (variant_at(n_steps - 1) != variant_at(0))
+        if (int rc = build_graph(s, variant_at(n_steps - 1))) return rc;
     memcpy(s->h_int, first_tokens_host, (size_t)B * 4);
     s->h_int[B] = 0;   // step counter
     LSPK_CUDA(cudaMemcpyAsync(s->ctl + B, s->h_int, (size_t)(B + 1) * 4, cudaMemcpyHostToDevice, stream()));
-    for (int i = 0; i < n_steps; ++i) LSPK_CUDA(cudaGraphLaunch(s->graph[variant], stream()));
+    for (int i = 0; i < n_steps; ++i) LSPK_CUDA(cudaGraphLaunch(s->graph[variant_at(i)], stream()));
     LSPK_CUDA(cudaMemcpyAsync(s->h_int, s->tokens_out, (size_t)n_steps * B * 4, cudaMemcpyDeviceToHost, stream()));
     LSPK_CUDA(cudaStreamSynchronize(stream()));
     memcpy(tokens_out_host, s->h_int, (size_t)n_steps * B * 4);

@@ -71,8 +71,11 @@ struct State {
     unsigned long long* io_pkt_dev = nullptr;
     unsigned* io_seq_dev = nullptr;        // device: steps of this kind finished so far
     unsigned io_seq = 0;                   // host: the same count
-    cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};   // [0] no logits store, [1] with logits, [2] host-fed step
-    unsigned graph_gen[3] = {0, 0, 0};   // scratch_generation() at capture: a later move of library scratch voids the graph
+    // [0] no logits store, [1] with logits, [2] host-fed step, [3] several long sequences: as [1], the attention of two query
+    // heads per CTA
+    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
+    unsigned graph_gen[4] = {0, 0, 0, 0};   // scratch_generation() at capture: a later move of library scratch voids the graph
+    bool group_heads = false;            // while the kernels of a step of kind [3] are being enqueued
     int graph_nodes = 0;
     size_t bytes = 0;
     size_t kv_elem() const { return kv_fp16 ? 2 : 4; }

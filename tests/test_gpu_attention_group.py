@@ -45,3 +45,54 @@ def test_grouped_heads_equal_single_sequence(heads, kv_heads, head_dim, lens, t_
             assert np.array_equal(k1, together[b][li][0]) and np.array_equal(v1, together[b][li][1]), (b, li)
         s1.close()
     dm.close()
+
+
+@pytest.mark.parametrize("kv,lens,t_max", [
+    ("fp32", (270, 268, 271, 266), 2048),            # in the middle of the steps below the two forms change
+    ("fp16", (896, 890, 893, 898, 881), 1000),
+    ("fp32", (100, 440), 500),                       # two sequences, uneven
+    ("fp16", (5, 9), 4000),                          # a long cache with short sequences
+])
+def test_steps_across_the_change_of_form(kv, lens, t_max):
+    """The form follows the positions, step by step: host-driven steps, a greedy loop over the change, and each sequence
+    alone give the same cache rows to the bit (the first two the same tokens)."""
+    cfg = synthetic.toy_config(hidden=8 * 128, layers=2, heads=8, kv_heads=2)
+    dm = rt.to_device(synthetic.random_model(cfg, seed=6, norm_jitter=0.1))
+    rng = np.random.default_rng(len(lens))
+    steps, B = 14, len(lens)
+    prompts = [np.ascontiguousarray(rng.integers(0, cfg.vocab_size, n), dtype=np.int32) for n in lens]
+    first = rng.integers(0, cfg.vocab_size, B).astype(np.int32)
+
+    def state():
+        st = rt.init_state(dm, t_max, batch=B, kv_dtype=kv)
+        for b, p in enumerate(prompts):
+            assert st.lib.lspk_forward_prefill(st.handle, b, p.ctypes.data, int(p.size), None, None, None) == 0
+        return st
+
+    one, two = state(), state()
+    toks, fed = first, []
+    for _ in range(steps):
+        fed.append(toks)
+        toks = rt.forward_step(one, toks)
+    ids = np.empty((steps, B), np.int32)
+    assert two.lib.lspk_decode_greedy(two.handle, first.ctypes.data, steps, ids.ctypes.data) == 0
+    assert np.array_equal(ids[:-1], np.array(fed[1:])) and np.array_equal(ids[-1], toks)
+    for b, p in enumerate(prompts):
+        alone = rt.init_state(dm, t_max, kv_dtype=kv)
+        rt.forward_prefill(dm, alone, [int(t) for t in p])
+        for i in range(steps):
+            rt.forward_one(dm, alone, int(fed[i][b]))
+        for li in range(cfg.num_layers):
+            want = alone.read_kv(li, lens[b] + steps)
+            for st in (one, two):
+                got = st.read_kv(li, lens[b] + steps, seq=b)
+                assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (b, li)
+        alone.close()
+    # going back to short positions goes back to the other form
+    for b in range(B):
+        two.set_pos(b, 3)
+        one.set_pos(b, 3)
+    assert np.array_equal(rt.forward_step(one, first), rt.forward_step(two, first))
+    one.close()
+    two.close()
+    dm.close()
