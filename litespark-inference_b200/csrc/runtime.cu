@@ -223,14 +223,14 @@ static int reserve_host_logits(State* s) {
 
 // Parked states.  A program that makes a state per request (the facade does) frees and makes the same one over and over;
 // its allocations, pinned buffers and instantiated graph cost several milliseconds.  A freed state is therefore kept, at
-// most one per live model and kMaxParkedBytes together, and handed out again, cleared, to a request for the same shape and
-// rope tables.  It is given back when its model is freed, when another state takes its place, when an allocation of this
+// most one per live model and kMaxParkedBytes together (the longest parked go first), and handed out again, cleared, to a
+// request for the same shape and rope tables.  It is given back when its model is freed, when another state takes its place, when an allocation of this
 // library fails (device_malloc, pinned_malloc), and on request (lspk_release_parked_states): another allocator in the
 // process cannot see that the memory is to be had.
 constexpr size_t kMaxParkedBytes = (size_t)1 << 30;
 static std::mutex g_park_mu;
 static std::map<unsigned long long, State*> g_parked;      // one entry per live model; null: nothing parked
-static unsigned long long g_next_model_id = 0;
+static unsigned long long g_next_model_id = 0, g_parkings = 0;
 
 static void destroy_state(State* s);
 
@@ -712,17 +712,29 @@ lspk_state_t lspk_state_create(lspk_model_t h, int t_max, int batch, int kv_fp16
 int lspk_state_free(lspk_state_t h) {
     if (!h) return LSPK_OK;
     State* s = reinterpret_cast<State*>(h);
-    {
+    std::vector<State*> gone;
+    if (s->bytes <= kMaxParkedBytes) {
         std::lock_guard<std::mutex> lk(g_park_mu);
         auto it = g_parked.find(s->model_id);      // no entry: the model is gone
         if (it != g_parked.end()) {
-            size_t others = 0;
-            for (const auto& kv : g_parked)
-                if (kv.second && kv.second != it->second) others += kv.second->bytes;
-            if (s->bytes + others <= kMaxParkedBytes) std::swap(it->second, s);
+            s->parked_at = ++g_parkings;
+            std::swap(it->second, s);
+            for (;;) {                             // the longest parked ones make room
+                size_t total = 0;
+                State** oldest = nullptr;
+                for (auto& kv : g_parked)
+                    if (kv.second) {
+                        total += kv.second->bytes;
+                        if (&kv.second != &it->second && (!oldest || kv.second->parked_at < (*oldest)->parked_at)) oldest = &kv.second;
+                    }
+                if (total <= kMaxParkedBytes || !oldest) break;
+                gone.push_back(*oldest);
+                *oldest = nullptr;
+            }
         }
     }
     if (s) destroy_state(s);
+    for (State* g : gone) destroy_state(g);
     return LSPK_OK;
 }
 

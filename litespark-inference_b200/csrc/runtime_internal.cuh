@@ -44,7 +44,7 @@ struct Model {
 
 struct State {
     Model* m = nullptr;
-    unsigned long long model_id = 0;
+    unsigned long long model_id = 0, parked_at = 0;
     std::vector<float> rope_host;     // the tables the state was created with (cos, then sin)
     int t_max = 0, batch = 1, kv_fp16 = 1;
     int cap_rows = 0;                 // rows the scratch buffers hold

@@ -136,7 +136,7 @@ def free_bytes():
     K.check(lib.lspk_mem_info(ctypes.byref(f), None))
     return f.value
 
-big = dict(t_max=8192, batch=24, kv_dtype="fp32")            # 400 MB: two of them are kept, a third is not
+big = dict(t_max=8192, batch=24, kv_dtype="fp32")            # 400 MB: two of them are kept, a third takes the first one's place
 held = []
 for dm in dms:
     st = rt.init_state(dm, **big)
@@ -147,6 +147,9 @@ for dm in dms:
     held.append(free_bytes() - before < size // 2)
 assert 3.9e8 < size < 4.4e8 and held == [True, True, False, False], (size, held)
 before = free_bytes()
+st = rt.init_state(dms[3], **big)                            # the last one is among those kept
+assert free_bytes() == before
+st.close()
 rt.release_parked_states()
 assert free_bytes() - before > 1.9 * size
 rt.release_parked_states()                                   # nothing left: no effect
