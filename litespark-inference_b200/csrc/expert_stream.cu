@@ -31,6 +31,7 @@ constexpr int kESmem = 225 * 1024;                                 // dynamic sh
 // and overwrites the stage being read.)
 __host__ __device__ constexpr int e_producer_of_slot(int slot) { return slot % kEProducers; }
 constexpr long long kEBudgetCycles = 1ll << 31;                    // every wait of a CTA gives up after about a second
+constexpr unsigned kEDrainPolls = 1u << 20;
 
 __device__ __forceinline__ void e_consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEConsumers) : "memory"); }
 
@@ -321,6 +322,13 @@ ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
             }
         }
         q_base += (g_hi - g_lo) * sub;
+    }
+    if (dead) {
+        // this warp's stages may still be on their way: the CTA does not end before they have landed (bounded as well)
+        for (int slot = 0; slot < p.slots; ++slot) {
+            const int q = *(volatile int*)&s_seq[slot] - 1;
+            for (unsigned i = 0; q >= 0 && i < kEDrainPolls && !mbar_try_wait(&full[slot], (uint32_t)(q / p.slots) & 1u); ++i) {}
+        }
     }
     tr.end();
 }
