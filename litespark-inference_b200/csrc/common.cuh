@@ -182,6 +182,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// True in exactly one lane of a converged warp.  Single-thread instructions (bulk copies, MMAs, commits) take
+// uniform operands: behind this predicate the compiler knows that one lane runs them.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // Non-blocking test of a phase (try_wait may park the thread for a while before it answers).
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;

@@ -35,12 +35,6 @@ constexpr unsigned kEDrainPolls = 1u << 20;
 
 __device__ __forceinline__ void e_consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEConsumers) : "memory"); }
 
-__device__ __forceinline__ bool e_elect() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
-
 __device__ __forceinline__ void e_mma(int c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
@@ -63,7 +57,7 @@ ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     PhaseTrace tr;
-    tr.begin(p.trace, p.trace_cap, PAIR ? 11 : 12);
+    tr.begin(p.trace, p.trace_cap, PAIR ? 13 : 14);
     tr.mark();                                   // 0: entry
     const long long deadline = clock64() + kEBudgetCycles;
     auto expired = [&]() { return clock64() > deadline || *(volatile int*)&s_abort != 0; };
@@ -139,7 +133,7 @@ ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
                     const int c0 = s * cps, c1 = min(c0 + cps, chunks);
                     const uint32_t bytes = (uint32_t)(c1 - c0) * kRowsPerGroup * 16u;
                     unsigned char* dst = smem_raw + (size_t)slot * kEStageBytes;
-                    if (e_elect()) {
+                    if (elect_one()) {
                         mbar_expect_tx(&full[slot], bytes * (PAIR ? 2u : 1u));
                         bulk_load_policy(dst, ua + (size_t)c0 * kRowsPerGroup, bytes, &full[slot], policy);
                         if (PAIR) bulk_load_policy(dst + bytes, ub + (size_t)c0 * kRowsPerGroup, bytes, &full[slot], policy);
@@ -192,7 +186,7 @@ ternary_expert_stream_kernel(const __grid_constant__ ExpertStreamParams p) {
             if (warp < kET) {
                 if (warp < mt) {
                     const int row = s_rows[warp] >> p.in_shift;
-                    if (e_elect()) {
+                    if (elect_one()) {
                         const uint32_t bytes = (uint32_t)chunks * kWeightsPerChunk;
                         mbar_expect_tx(&xbar, bytes);
                         bulk_load(xq + (size_t)warp * rs, p.x + (size_t)row * rs, bytes, &xbar);
