@@ -380,7 +380,7 @@ def measure_shape(lib, dev, K, synthetic, rng, peak, name, Ms, copies_mb=300.0):
         ops = 2.0 * M * N * Kd
         row = {"shape": name, "N": N, "K": Kd, "M": M, "us": us, "GBps": nbytes / us / 1e3,
                "frac_hbm": nbytes / us / 1e3 / peak, "TOPS": ops / us / 1e6,
-               "path": "tcgen05" if M >= 32 else ("mma.sync" if M > 1 else "dp4a")}
+               "path": "tcgen05" if M >= 9 else ("mma.sync" if M > 1 else "dp4a")}
         if M == 1:
             # the same launches as independent graph nodes (forked streams): the kernel's amortised
             # throughput when it is not a link of a dependency chain.  Fused quantiser, then the reference
