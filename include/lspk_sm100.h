@@ -139,7 +139,7 @@ typedef struct {
  * on the library stream: both must be complete in memory when the call is made (the upload functions of this
  * header synchronise); activations, residuals and outputs are ordered after everything queued before. */
 int lspk_linear(const lspk_linear_args* a);
-int lspk_linear_force_path(int path);   /* 0 auto, 1 CUDA-core kernel only, 2 tcgen05 only */
+int lspk_linear_force_path(int path);   /* 0 auto, 1 no tcgen05, 2 tcgen05 only; from the next launch or capture on */
 /* n independent one-row products in ONE launch: product i is args[i], which must have M == 1 and the int8
  * prologue (x_i8 + x_scales: the contract of the reference's matmul_lut_{tag}_m1, matmul_lut_avx512_extern_c.cpp:
  * 150-236; quantise fp32 rows first with lspk_quantize_rows / lspk_rmsnorm_quantize_rows), one matrix with the

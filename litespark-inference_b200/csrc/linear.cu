@@ -589,6 +589,7 @@ static int g_force_path = 0;   // 0 auto, 1 CUDA-core only, 2 tensor-core only
 
 extern "C" int lspk_linear_force_path(int path) {
     LSPK_REQUIRE(path >= 0 && path <= 2, "lspk_linear_force_path: path must be 0, 1 or 2");
+    if (path != g_force_path) release_parked_states();     // their graphs hold the kernels of the path they were captured on
     g_force_path = path;
     return LSPK_OK;
 }

@@ -847,9 +847,9 @@ int lspk_decode_greedy(lspk_state_t h, const int* first_tokens_host, int n_steps
                         n_steps, s->t_max);
     // several sequences: positions only grow, so there is one change of kind at most
     auto variant_at = [&](int i) { return B > 1 ? batch_variant(s, i) : 0; };
-    if (int rc = build_graph(s, variant_at(0))) return rc;
-    if (variant_at(n_steps - 1) != variant_at(0))
-        if (int rc = build_graph(s, variant_at(n_steps - 1))) return rc;
+    const int kinds[3] = {variant_at(n_steps - 1), variant_at(0), variant_at(n_steps - 1)};
+    for (int kind : kinds)      // the last again, should the first have moved scratch
+        if (int rc = build_graph(s, kind)) return rc;
     memcpy(s->h_int, first_tokens_host, (size_t)B * 4);
     s->h_int[B] = 0;   // step counter
     LSPK_CUDA(cudaMemcpyAsync(s->ctl + B, s->h_int, (size_t)(B + 1) * 4, cudaMemcpyHostToDevice, stream()));

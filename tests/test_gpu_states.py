@@ -102,6 +102,12 @@ K.check(lib.lspk_set_pdl(1))                 # no change: the freed state stays
 assert free_bytes() == before
 K.check(lib.lspk_set_pdl(0))
 assert free_bytes() >= before + held // 2
+st = rt.init_state(dm, 8192, batch=8, kv_dtype="fp32")
+st.close()
+before = free_bytes()
+K.check(lib.lspk_linear_force_path(1))       # the kernels of the products are in the graph too
+assert free_bytes() >= before + held // 2
+K.check(lib.lspk_linear_force_path(0))
 st = rt.init_state(dm, 64)
 assert np.array_equal(one_step(st), want)
 st.close()                                   # a timing harness that turns programmatic launch off while it captures
