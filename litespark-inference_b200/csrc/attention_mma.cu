@@ -102,8 +102,12 @@ __device__ __noinline__ void attend_row_plain(const float* q, const KVT* k, cons
         return __fmul_rn(warp_sum(d), inv_sqrt_d);
     };
     float mx = -INFINITY, sum = 0.0f;
+    // several keys on their way at once: a chain of one key's trips to memory after the other's takes four times as long
+#pragma unroll 4
     for (int i = 0; i < n; ++i) mx = fmaxf(mx, score(i));
+#pragma unroll 4
     for (int i = 0; i < n; ++i) sum += expf(score(i) - mx);
+#pragma unroll 4
     for (int i = 0; i < n; ++i) {
         const float pi = __fdiv_rn(expf(score(i) - mx), sum);
 #pragma unroll
