@@ -32,6 +32,7 @@ constexpr int kSConsumers = 12;                  // warps that compute
 constexpr int kSProducers = 6;
 constexpr int kSThreads = 32 * (kSConsumers + kSProducers);
 constexpr int kSSlots = 18;                      // stages of the CTA's ring (shared by all consumer warps)
+static_assert(kSSlots % kSProducers == 0, "a slot has to keep its requesting warp: the phase test in front of a refill knows one phase back");
 constexpr int kSStageChunks = 40;                // 16-row x 16-byte chunks per stage (all matrices of a unit)
 constexpr int kSStageBytes = kSStageChunks * kRowsPerGroup * 16;   // 10240: 180 KB of ring per SM
 constexpr int kSMaxItems = kStreamMaxItems;
