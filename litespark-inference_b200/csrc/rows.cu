@@ -196,6 +196,15 @@ row_norm_quant_kernel(const float* __restrict__ x, const float* __restrict__ gat
     if (tid == 0) scales[t] = scale;
 }
 
+// v * inv to the nearest int8.  |v * inv| <= 127 by construction of inv, so round-to-nearest-even can be taken from the adder:
+// v * inv + 1.5 * 2^23 leaves the integer in the low mantissa byte (conversions issue at a quarter of its rate).  Not so for the
+// elements behind the last multiple of 16 (the reference's scalar tail: round half away from zero, clamp to +-127; zeros beyond
+// K) and for those that are not a number (0).
+constexpr float kRoundMagic = 12582912.0f;
+__device__ __forceinline__ uint32_t quant_exact(float v, float inv, int k, int K) {
+    return k < (K & ~15) ? (uint32_t)quant_one(v, inv) : k < K ? (uint32_t)max(-127, min(127, (int)roundf(__fmul_rn(v, inv)))) : 0u;
+}
+
 // Row quantiser for rows of up to 4096 * NB elements, everything in registers: a thread owns the 16-element blocks
 // tid, tid + 256 (the lanes of the canonical sum-of-squares order), loads them once, and -- having whole blocks --
 // writes the permuted layout of the tensor-core kernels without any exchange between lanes.  The norm weights
@@ -204,11 +213,15 @@ row_norm_quant_kernel(const float* __restrict__ x, const float* __restrict__ gat
 //   norm      apply RMSNorm (gamma, eps) before the quantiser
 //   perm_kp   > 0: write perm_kp bytes per row (K rounded up to 64, zero padded) in the permuted layout, rows
 //             perm_stride bytes apart, and optionally the sum of the row's int8 values; 0: natural order [T, K]
+// Bound by the latency of the row's arrival and of the serial steps behind it at few rows, by their instructions at many:
+// library divisions, two-barrier reductions and a conversion per element took 6 % of the MLP block of 512 rows (49.9 -> 46.9 us)
+// and 7 % of a decode step of eight sequences (1.26 -> 1.16 ms).  A row spread over 640 or 1024 threads, four elements each,
+// is no faster at 8 rows (both 1.18 ms) and slower at 512 (53 us).
 template <int NB>
 __global__ void __launch_bounds__(kRowThreads)
 row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gate, const void* __restrict__ gamma_base,
                       const int* __restrict__ gamma_sel, int gamma_is_bf16, int8_t* __restrict__ out_i8,
-                      float* __restrict__ scales, int K, float eps, int norm, int perm_kp, int perm_stride,
+                      float* __restrict__ scales, int K, float eps, float rcp_K, int norm, int perm_kp, int perm_stride,
                       int* __restrict__ sums) {
     __shared__ __align__(16) float red[32];
     const int t = blockIdx.x, tid = threadIdx.x;
@@ -283,8 +296,12 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
         for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
             for (int e = 0; e < 16; ++e) ss[e & 3] = fmaf(v[nb][e], v[nb][e], ss[e & 3]);
-        const float ssq = row_ssq_combine((ss[0] + ss[1]) + (ss[2] + ss[3]), red);
-        const float rrms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ssq, (float)K), eps)));
+        const float warp_ssq = warp_sum((ss[0] + ss[1]) + (ss[2] + ss[3]));
+        if ((tid & 31) == 0) red[tid >> 5] = warp_ssq;
+        __syncthreads();
+        const float ssq = canonical_ssq_combine(red);
+        const float mean = rcp_K != 0.0f ? div_const_rn(ssq, (float)K, rcp_K) : __fdiv_rn(ssq, (float)K);
+        const float rrms = rcp_rn(__fsqrt_rn(__fadd_rn(mean, eps)));
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
@@ -295,9 +312,14 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
     for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
         for (int e = 0; e < 16; ++e) amax = fmaxf(amax, fabsf(v[nb][e]));
-    amax = block_max(amax, red);
+    // non-negative floats order like their bit patterns; a slot of its own for every reduction, so one barrier each
+    const uint32_t warp_amax = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+    if ((tid & 31) == 0) red[8 + (tid >> 5)] = __uint_as_float(warp_amax);
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) amax = fmaxf(amax, red[8 + w]);
     const float scale = quant_scale_from_absmax(amax);
-    const float inv = __fdiv_rn(1.0f, scale);
+    const float inv = rcp_rn(scale);
     const int tail_start = K & ~15;
     const int limit = perm_kp > 0 ? perm_kp : K;
     int sumx = 0;
@@ -305,38 +327,38 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
     for (int nb = 0; nb < NB; ++nb) {
         const int k0 = (tid + nb * kRowThreads) * 16;
         if (k0 < limit) {
-            uint32_t a[4];
+            uint32_t w[16];
+            float all[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                uint32_t word = 0;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int k = k0 + q * 4 + e;
-                    int qv = 0;
-                    if (k < tail_start) {
-                        qv = quant_one(v[nb][q * 4 + e], inv);
-                    } else if (k < K) {
-                        qv = max(-127, min(127, (int)roundf(__fmul_rn(v[nb][q * 4 + e], inv))));
-                    }
-                    word |= ((uint32_t)qv & 0xffu) << (8 * e);
-                }
-                a[q] = word;
-                sumx = __dp4a((int)word, 0x01010101, sumx);
+            for (int e = 0; e < 16; ++e) {
+                const float f = __fmul_rn(v[nb][e], inv);
+                w[e] = __float_as_uint(__fadd_rn(f, kRoundMagic));
+                all[e & 3] += f;
             }
-            if (perm_kp > 0) {
-                uint32_t o0, o1, o2, o3;
-                transpose4x4_bytes(a[0], a[1], a[2], a[3], o0, o1, o2, o3);
-                *reinterpret_cast<uint4*>(out_i8 + (size_t)t * perm_stride + k0) = make_uint4(o0, o1, o2, o3);
+            const float any = (all[0] + all[1]) + (all[2] + all[3]);
+            if (k0 + 16 > tail_start || !(any == any)) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) w[e] = quant_exact(v[nb][e], inv, k0 + e, K);
+            }
+            uint32_t a[4];
+            if (perm_kp > 0) {      // packed in the transposed order
+#pragma unroll
+                for (int q = 0; q < 4; ++q) a[q] = pack4_bytes(w[q], w[4 + q], w[8 + q], w[12 + q]);
+                *reinterpret_cast<uint4*>(out_i8 + (size_t)t * perm_stride + k0) = make_uint4(a[0], a[1], a[2], a[3]);
             } else {
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
+                for (int q = 0; q < 4; ++q) {
+                    a[q] = pack4_bytes(w[q * 4], w[q * 4 + 1], w[q * 4 + 2], w[q * 4 + 3]);
                     if (k0 + q * 4 < K) *reinterpret_cast<uint32_t*>(out_i8 + (size_t)t * K + k0 + q * 4) = a[q];
+                }
             }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sumx = __dp4a((int)a[q], 0x01010101, sumx);
         }
     }
     if (sums) {                                        // uniform branch
         sumx = __reduce_add_sync(0xffffffffu, sumx);
-        int* redi = reinterpret_cast<int*>(red);
+        int* redi = reinterpret_cast<int*>(red + 16);
         if ((tid & 31) == 0) redi[tid >> 5] = sumx;
         __syncthreads();
         if (tid == 0) {
@@ -385,11 +407,12 @@ static int launch_rows(const float* x, const void* gamma, int gamma_is_bf16, flo
     // quantising rows of up to 8192 elements: the register-resident kernel
     if (vec && (mode & 2) && K <= 8192 && (perm_kp == 0 || perm_kp <= 8192)) {
         const int pstride = perm_stride > 0 ? perm_stride : perm_kp;
+        const float rcp_K = fma_division_ok((float)K) ? 1.0f / (float)K : 0.0f;
         const cudaError_t e = K <= 4096 && perm_kp <= 4096
             ? launch(row_quant_regs_kernel<1>, dim3(T), dim3(kRowThreads), 0, true, x, gate, gamma, gamma_sel, gamma_is_bf16,
-                     out_i8, scales, K, eps, mode & 1, perm_kp, pstride, sums)
+                     out_i8, scales, K, eps, rcp_K, mode & 1, perm_kp, pstride, sums)
             : launch(row_quant_regs_kernel<2>, dim3(T), dim3(kRowThreads), 0, true, x, gate, gamma, gamma_sel, gamma_is_bf16,
-                     out_i8, scales, K, eps, mode & 1, perm_kp, pstride, sums);
+                     out_i8, scales, K, eps, rcp_K, mode & 1, perm_kp, pstride, sums);
         if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "row quantiser launch failed: %s", cudaGetErrorString(e));
         return LSPK_OK;
     }
