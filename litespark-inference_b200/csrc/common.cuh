@@ -123,7 +123,14 @@ unsigned long long* trace_buffer();       // device pointer or nullptr
 int trace_capacity();                     // records
 
 #ifdef __CUDACC__
-struct PhaseTrace {
+// Every mark is a test, a clock read and a barrier to the compiler's scheduling: kernels whose code is read from L2 at each
+// launch (a decode step runs through more code than an SM caches) have an instantiation without.
+template <bool ON> struct PhaseTraceOf {
+    __device__ __forceinline__ void begin(unsigned long long*, int, int, int = 0) {}
+    __device__ __forceinline__ void mark() {}
+    __device__ __forceinline__ void end() {}
+};
+template <> struct PhaseTraceOf<true> {
     unsigned long long* rec;
     int n;
     // the recording thread is thread `thread` of block (0, 0, 0)
@@ -154,6 +161,7 @@ struct PhaseTrace {
         }
     }
 };
+using PhaseTrace = PhaseTraceOf<true>;
 #endif
 
 #ifdef __CUDACC__

@@ -25,6 +25,7 @@ namespace lspk {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr int kAnyPrologue = -1;
 
 // Reductions over the eight warps of a CTA.  One barrier each: the result is read back from `slot`
 // (8 floats, 16-byte aligned) by every thread, so two consecutive reductions need two slots.
@@ -49,14 +50,16 @@ __device__ __forceinline__ float cta8_max_nonneg(float v, float* slot) {
 // NI      16-byte weight loads per lane per batch (covers K <= 4096 at 4, K <= 8192 at 8 in one batch)
 // NB      16-element activation blocks a thread owns in the fp32 prologue (K <= 4096 * NB)
 // PAIR    gate/up pairing (two weight streams, gated epilogue)
-template <int MT, int NI, int NB, bool PAIR>
-#ifdef LSPK_LINEAR_MIN_BLOCKS
-__global__ void __launch_bounds__(kThreads, LSPK_LINEAR_MIN_BLOCKS)
-#else
+// PRO     LSPK_PRO_* of a plain call (K % 16 == 0, no trace, no int8 rows, scales or accumulators to hand out), or
+//         kAnyPrologue: every form, taken from the call
+// A decode step walks through five kernels a layer, together more code than an SM's instruction cache holds, so what a launch
+// does not execute costs as well: with the plain forms apart and one set of weight loads the code of q/k/v and o went from 39
+// to 17 KB, of gate/up from 43 to 20 KB, of down from 62 to 24 KB, a decode step at context 128 from 758 to 682 us.
+template <int MT, int NI, int NB, bool PAIR, int PRO>
 __global__ void __launch_bounds__(kThreads)
-#endif
 ternary_linear_kernel(const __grid_constant__ LinearParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool kPlain = PRO != kAnyPrologue;
     const int Kp = p.chunks * kWeightsPerChunk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r = lane & 15, h = lane >> 4;
@@ -79,6 +82,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
             }
         }
     };
+    const uint64_t policy = weight_policy(p.stream_weights);
     auto load_batch = [&](int seg_i, int grp, int base, uint4* dst_a, uint4* dst_b) {
         const uint4* wa_base = p.seg[seg_i].w + (size_t)grp * p.chunks * kRowsPerGroup + r;
         const uint4* wb_base = PAIR ? (p.seg[1].w + (size_t)grp * p.chunks * kRowsPerGroup + r) : nullptr;
@@ -86,25 +90,19 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
         for (int i = 0; i < NI; ++i) {
             const int j = 2 * (warp + kWarps * (base + i)) + h;
             if (j < p.chunks) {
-                // read-once weights bypass the L2 replacement queue so that the KV cache, the
-                // activations and the norm weights stay resident from token to token
-                if (p.stream_weights) {
-                    dst_a[i] = __ldcs(wa_base + (size_t)j * kRowsPerGroup);
-                    if (PAIR) dst_b[i] = __ldcs(wb_base + (size_t)j * kRowsPerGroup);
-                } else {
-                    dst_a[i] = __ldg(wa_base + (size_t)j * kRowsPerGroup);
-                    if (PAIR) dst_b[i] = __ldg(wb_base + (size_t)j * kRowsPerGroup);
-                }
+                dst_a[i] = ldg_policy(wa_base + (size_t)j * kRowsPerGroup, policy);
+                if (PAIR) dst_b[i] = ldg_policy(wb_base + (size_t)j * kRowsPerGroup, policy);
             }
         }
     };
-    PhaseTrace tr;
+    PhaseTraceOf<!kPlain> tr;
     tr.begin(p.trace, p.trace_cap, 1);
     tr.mark();                                   // 0: entry
     const int pairs = (p.chunks + 1) / 2;
-    const bool one_batch = kWarps * NI >= pairs;     // a row group's weights fit one register batch
-    const bool fp32_in = p.prologue != LSPK_PRO_INT8;
-    const bool normed = p.prologue == LSPK_PRO_RMSNORM_QUANT || p.prologue == LSPK_PRO_GATED_RMSNORM_QUANT;
+    const bool one_batch = NB <= 2 || kWarps * NI >= pairs;      // a row group's weights fit one register batch
+    const int pro = kPlain ? PRO : p.prologue;
+    const bool fp32_in = pro != LSPK_PRO_INT8;
+    const bool normed = pro == LSPK_PRO_RMSNORM_QUANT || pro == LSPK_PRO_GATED_RMSNORM_QUANT;
 
     int flat0 = blockIdx.x, s0, g0;
     locate(flat0, s0, g0);
@@ -123,7 +121,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
             for (int q = 0; q < 4; ++q) {
                 const int k = k0 + q * 4;
                 float4 gv = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (k < p.K) {
+                if ((kPlain ? k0 : k) < p.K) {
                     if (p.gamma_is_bf16) {
                         const uint2 gb = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.gamma) + k));
                         gv.x = __uint_as_float(gb.x << 16);
@@ -193,14 +191,14 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (k0 + q * 4 < p.K) t4 = *reinterpret_cast<const float4*>(src + k0 + q * 4);
+                        if ((kPlain ? k0 : k0 + q * 4) < p.K) t4 = *reinterpret_cast<const float4*>(src + k0 + q * 4);
                         v[nb][q * 4 + 0] = t4.x;
                         v[nb][q * 4 + 1] = t4.y;
                         v[nb][q * 4 + 2] = t4.z;
                         v[nb][q * 4 + 3] = t4.w;
                     }
                 }
-                if (p.prologue == LSPK_PRO_GATED_RMSNORM_QUANT) {
+                if (pro == LSPK_PRO_GATED_RMSNORM_QUANT) {
                     // v = x * SiLU(gate), SiLU(g) = g / (1 + exp(-g)); each step a single rounding
                     const float* gsrc = p.gate_f32 + (size_t)(m0 + m) * p.K;
 #pragma unroll
@@ -209,7 +207,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (k0 + q * 4 < p.K) t4 = *reinterpret_cast<const float4*>(gsrc + k0 + q * 4);
+                            if ((kPlain ? k0 : k0 + q * 4) < p.K) t4 = *reinterpret_cast<const float4*>(gsrc + k0 + q * 4);
                             const float gg[4] = {t4.x, t4.y, t4.z, t4.w};
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
@@ -246,55 +244,40 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                 tr.mark();                           // 5: absmax reduced
                 scale = quant_scale_from_absmax(amax);
                 const float inv = rcp_rn(scale);
-                const bool tap = (p.xq_out != nullptr) && blockIdx.x == 0;
+                const bool tap = !kPlain && (p.xq_out != nullptr) && blockIdx.x == 0;
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
                     const int b = tid + nb * kThreads;
                     const int k0 = b * 16;
                     if (k0 < Kp) {
-                        uint32_t o0, o1, o2, o3;
-                        if (k0 + 16 <= tail_start) {
-                            // |v * inv| <= 127 by construction of inv, so the saturation of the reference's
-                            // conversion never acts and round-to-nearest-even can be taken from the adder:
-                            // v + 1.5 * 2^23 leaves the integer in the low mantissa byte.  The words are
-                            // packed directly in the transposed order the dot products read.
-                            uint32_t t[16];
+                        // |v * inv| <= 127 by construction of inv, so the saturation of the reference's
+                        // conversion never acts and round-to-nearest-even can be taken from the adder:
+                        // v + 1.5 * 2^23 leaves the integer in the low mantissa byte.  The words are
+                        // packed directly in the transposed order the dot products read.
+                        uint32_t t[16];
 #pragma unroll
-                            for (int e = 0; e < 16; ++e)
-                                t[e] = __float_as_uint(__fadd_rn(__fmul_rn(v[nb][e], inv), 12582912.0f));
-                            o0 = pack4_bytes(t[0], t[4], t[8], t[12]);
-                            o1 = pack4_bytes(t[1], t[5], t[9], t[13]);
-                            o2 = pack4_bytes(t[2], t[6], t[10], t[14]);
-                            o3 = pack4_bytes(t[3], t[7], t[11], t[15]);
-                            if (tap) {
+                        for (int e = 0; e < 16; ++e)
+                            t[e] = __float_as_uint(__fadd_rn(__fmul_rn(v[nb][e], inv), 12582912.0f));
+                        if (!kPlain && k0 + 16 > tail_start) {
+                            // block past the last multiple of 16: the reference's scalar tail rounds halves
+                            // away from zero.  The rest of the nearest-even form is exact, so a half that went
+                            // towards zero is told by it; a NaN becomes 0.  Zeros beyond K.
 #pragma unroll
-                                for (int q = 0; q < 4; ++q)
+                            for (int e = 0; e < 16; ++e) {
+                                const float x = __fmul_rn(v[nb][e], inv);
+                                const float rest = __fsub_rn(x, __fsub_rn(__uint_as_float(t[e]), 12582912.0f));
+                                if (rest == copysignf(0.5f, x)) t[e] += rest > 0.0f ? 1u : 0xffffffffu;
+                                if (x != x) t[e] = 0u;
+                            }
+                        }
+                        const uint32_t o0 = pack4_bytes(t[0], t[4], t[8], t[12]), o1 = pack4_bytes(t[1], t[5], t[9], t[13]);
+                        const uint32_t o2 = pack4_bytes(t[2], t[6], t[10], t[14]), o3 = pack4_bytes(t[3], t[7], t[11], t[15]);
+                        if (tap) {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                if (k0 + q * 4 < p.K)
                                     *reinterpret_cast<uint32_t*>(p.xq_out + (size_t)(m0 + m) * p.K + k0 + q * 4) =
                                         pack4_bytes(t[q * 4], t[q * 4 + 1], t[q * 4 + 2], t[q * 4 + 3]);
-                            }
-                        } else {
-                            // block that reaches past the last multiple of 16: the reference's scalar tail
-                            // (round half away from zero, clamp to +-127), zeros beyond K
-                            uint32_t a[4];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                uint32_t word = 0;
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const int k = k0 + q * 4 + e;
-                                    int qv = 0;
-                                    if (k < tail_start) {
-                                        qv = (int)quant_rne_sat(__fmul_rn(v[nb][q * 4 + e], inv));
-                                    } else if (k < p.K) {
-                                        qv = max(-127, min(127, (int)roundf(__fmul_rn(v[nb][q * 4 + e], inv))));
-                                    }
-                                    word |= ((uint32_t)qv & 0xffu) << (8 * e);
-                                }
-                                a[q] = word;
-                                if (tap && k0 + q * 4 < p.K)
-                                    *reinterpret_cast<uint32_t*>(p.xq_out + (size_t)(m0 + m) * p.K + k0 + q * 4) = word;
-                            }
-                            transpose4x4_bytes(a[0], a[1], a[2], a[3], o0, o1, o2, o3);
                         }
                         sumx = __dp4a((int)o0, 0x01010101, sumx);
                         sumx = __dp4a((int)o1, 0x01010101, sumx);
@@ -309,7 +292,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
             if (lane == 0) s_sumx[m * kWarps + warp] = sumx;
             if (tid == 0) {
                 s_scale[m] = scale;
-                if (p.xscale_out && blockIdx.x == 0) p.xscale_out[m0 + m] = scale;
+                if (!kPlain && p.xscale_out && blockIdx.x == 0) p.xscale_out[m0 + m] = scale;
             }
         }
         tr.mark();                                   // 6: quantised rows written
@@ -384,12 +367,12 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                     }
                     va -= sx;
                     const size_t o = (size_t)(m0 + out_m) * sg.N + n;
-                    if (sg.acc_out) sg.acc_out[o] = va;
+                    if (!kPlain && sg.acc_out) sg.acc_out[o] = va;
                     const float wsa = sg.w_scale;
                     const float ya = __fmul_rn((float)va, __fmul_rn(s_scale[out_m], wsa));
                     if (PAIR) {
                         vb -= sx;
-                        if (p.seg[1].acc_out) p.seg[1].acc_out[o] = vb;
+                        if (!kPlain && p.seg[1].acc_out) p.seg[1].acc_out[o] = vb;
                         const float wsb = p.seg[1].w_scale;
                         const float yb = __fmul_rn((float)vb, __fmul_rn(s_scale[out_m], wsb));
                         if (p.epilogue == LSPK_EPI_SILU_MUL) {
@@ -434,10 +417,10 @@ static size_t linear_smem_bytes(int MT, int Kp, bool pair) {
     b += 32 * 4 + MT * 4 + MT * kWarps * 4;
     return b;
 }
-template <int MT, int NI, int NB, bool PAIR>
+template <int NI, int NB, bool PAIR, int PRO>
 static cudaError_t launch_linear(const LinearParams& p, dim3 grid, size_t smem) {
     static bool attr_set = false;
-    auto kern = ternary_linear_kernel<MT, NI, NB, PAIR>;
+    auto kern = ternary_linear_kernel<1, NI, NB, PAIR, PRO>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
@@ -445,14 +428,27 @@ static cudaError_t launch_linear(const LinearParams& p, dim3 grid, size_t smem) 
     }
     return launch(kern, grid, dim3(kThreads), smem, true, p);
 }
-
-template <int MT>
-static cudaError_t launch_linear_mt(const LinearParams& p, dim3 grid, bool pair, size_t smem) {
+// The plain forms up to K = 8192 have an instantiation each (see the kernel); longer rows are not launch-bound.
+template <int NI, int NB, bool PAIR>
+static cudaError_t launch_linear_pro(const LinearParams& p, dim3 grid, size_t smem) {
+    if constexpr (NB <= 2) {
+        bool plain = p.K % 16 == 0 && !p.trace && !p.xq_out && !p.xscale_out;
+        for (int i = 0; i < p.n_seg; ++i) plain = plain && !p.seg[i].acc_out;
+        if (plain) switch (p.prologue) {
+            case LSPK_PRO_INT8: return launch_linear<NI, NB, PAIR, LSPK_PRO_INT8>(p, grid, smem);
+            case LSPK_PRO_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_QUANT>(p, grid, smem);
+            case LSPK_PRO_RMSNORM_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_RMSNORM_QUANT>(p, grid, smem);
+            case LSPK_PRO_GATED_RMSNORM_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_GATED_RMSNORM_QUANT>(p, grid, smem);
+        }
+    }
+    return launch_linear<NI, NB, PAIR, kAnyPrologue>(p, grid, smem);
+}
+static cudaError_t launch_linear_row(const LinearParams& p, dim3 grid, bool pair, size_t smem) {
     if (p.chunks <= 64)
-        return pair ? launch_linear<MT, 4, 1, true>(p, grid, smem) : launch_linear<MT, 4, 1, false>(p, grid, smem);
+        return pair ? launch_linear_pro<4, 1, true>(p, grid, smem) : launch_linear_pro<4, 1, false>(p, grid, smem);
     if (p.chunks <= 128)
-        return pair ? launch_linear<MT, 8, 2, true>(p, grid, smem) : launch_linear<MT, 8, 2, false>(p, grid, smem);
-    return pair ? launch_linear<MT, 8, 8, true>(p, grid, smem) : launch_linear<MT, 8, 8, false>(p, grid, smem);
+        return pair ? launch_linear_pro<8, 2, true>(p, grid, smem) : launch_linear_pro<8, 2, false>(p, grid, smem);
+    return pair ? launch_linear_pro<8, 8, true>(p, grid, smem) : launch_linear_pro<8, 8, false>(p, grid, smem);
 }
 
 int linear_launch_params(const LinearParams& p, int mt, bool pair, int grid_x, int grid_y) {
@@ -462,7 +458,7 @@ int linear_launch_params(const LinearParams& p, int mt, bool pair, int grid_x, i
     const size_t smem = linear_smem_bytes(1, Kp, pair);
     LSPK_REQUIRE(smem <= 200 * 1024 && p.chunks <= 512, "linear: K=%d too large (limit 32768)", p.K);
     const dim3 grid(grid_x, grid_y);
-    const cudaError_t e = launch_linear_mt<1>(p, grid, pair, smem);
+    const cudaError_t e = launch_linear_row(p, grid, pair, smem);
     if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "linear launch failed: %s", cudaGetErrorString(e));
     return LSPK_OK;
 }

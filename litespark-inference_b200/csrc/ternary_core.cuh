@@ -15,6 +15,21 @@ __device__ __forceinline__ void transpose4x4_bytes(uint32_t a0, uint32_t a1, uin
     o3 = __byte_perm(t2, t3, 0x7632);
 }
 
+// Weight loads.  Weights that a launch reads once are marked evict-first in L2, so that the KV cache, the activations and the
+// norm weights stay resident from token to token; as a policy of one load instruction, not as two sets of loads.
+__device__ __forceinline__ uint64_t weight_policy(int read_once) {
+    uint64_t policy;
+    if (read_once) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+    return policy;
+}
+__device__ __forceinline__ uint4 ldg_policy(const uint4* p, uint64_t policy) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy));
+    return v;
+}
+
 // Accumulate one 16-byte weight chunk (64 weights) against the matching 64 permuted activations.
 __device__ __forceinline__ void chunk_dot(const uint4& wv, const int4* __restrict__ xp, int acc[4]) {
     const uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
