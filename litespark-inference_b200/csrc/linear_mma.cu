@@ -48,7 +48,12 @@ constexpr int kMXSegMax = 24;                        // covers K up to 24576
 constexpr long long kMXWaitCycles = 1ll << 31;
 static_assert(kMWarps == kMT && kMXSegMax <= 32, "row staging maps warp -> row and lane -> segment");
 
-template <bool PAIR>
+// FORM    kMmaTiled: pre-tiled rows, no trace, no accumulators to hand out; kMmaOneBatch: such rows with chunks for one batch of
+//         weights; kMmaAny: every form, taken from the call.
+// The plain forms are apart because their launches are short and their code cold: 16 and 19 KB (single, paired) of one batch, 18
+// and 22 KB of more, where the general form has 31 and 36; a decode step of eight sequences 1.26 -> 1.20 ms.
+enum { kMmaAny, kMmaTiled, kMmaOneBatch };
+template <bool PAIR, int FORM>
 __global__ void __launch_bounds__(kMThreads)
 ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -57,6 +62,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gid = lane >> 2, t4 = lane & 3;
 
+    constexpr bool kPlain = FORM != kMmaAny;
     int8_t* xq = reinterpret_cast<int8_t*>(smem_raw);                         // [kMT][rs] permuted int8
     int* part = reinterpret_cast<int*>(xq + (size_t)kMT * rs);                 // [PAIR?2:1][warps][kMT][16]
     constexpr int kPartInts = kMWarps * kMT * 16 * (PAIR ? 2 : 1);
@@ -74,6 +80,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
             }
         }
     };
+    const uint64_t policy = weight_policy(p.stream_weights);
     // weights of chunk pair (warp + 8*(base+i)) of a row group: for each of the two chunks the words of
     // row gid and of row gid+8 -> 4 words per pair (8 with the gate/up pairing)
     auto load_batch = [&](int seg_i, int grp, int base, uint32_t (*dst_a)[4], uint32_t (*dst_b)[4]) {
@@ -89,14 +96,11 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                 uint32_t a_lo = 0x55555555u, a_hi = 0x55555555u, b_lo = 0x55555555u, b_hi = 0x55555555u;
                 if (j < p.chunks) {
                     const size_t o = (size_t)j * 64 + lane;           // 64 words per 16-row chunk tile
-                    if (p.stream_weights) {
-                        a_lo = __ldcs(wa + o);
-                        a_hi = __ldcs(wa + o + 32);
-                        if (PAIR) { b_lo = __ldcs(wb + o); b_hi = __ldcs(wb + o + 32); }
-                    } else {
-                        a_lo = __ldg(wa + o);
-                        a_hi = __ldg(wa + o + 32);
-                        if (PAIR) { b_lo = __ldg(wb + o); b_hi = __ldg(wb + o + 32); }
+                    a_lo = ldg_policy(wa + o, policy);
+                    a_hi = ldg_policy(wa + o + 32, policy);
+                    if (PAIR) {
+                        b_lo = ldg_policy(wb + o, policy);
+                        b_hi = ldg_policy(wb + o + 32, policy);
                     }
                 }
                 dst_a[i][c * 2] = a_lo;
@@ -112,14 +116,14 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     int flat0 = blockIdx.x, s0, g0;
     locate(flat0, s0, g0);
     uint32_t wa[kMNI][4], wb[PAIR ? kMNI : 1][4];
-    PhaseTrace tr;
+    PhaseTraceOf<!kPlain> tr;
     tr.begin(p.trace, p.trace_cap, 3);
     tr.mark();                                          // 0: entry
     load_batch(s0, g0, 0, wa, wb);                      // weights never depend on the previous kernel
     __shared__ __align__(8) uint64_t xbars[kMXSegMax];
     const int nxseg = (p.chunks + kMXSegChunks - 1) / kMXSegChunks;
     // CTA-uniform: a full tile of pre-tiled rows, one token tile per CTA
-    const bool x_async = p.prologue == kProInt8Tiled && nxseg <= kMXSegMax &&
+    const bool x_async = (kPlain || p.prologue == kProInt8Tiled) && nxseg <= kMXSegMax &&
                          p.M - (int)blockIdx.y * kMT >= kMT;
     if (x_async) {
         if (tid < nxseg) {
@@ -162,7 +166,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                 s_scale[tid] = p.x_scales[m0 + tid];
                 s_sumx[tid] = p.x_sums[m0 + tid];
             }
-        } else if (p.prologue == kProInt8Tiled) {
+        } else if (kPlain || p.prologue == kProInt8Tiled) {
             // rows already permuted and spaced like the shared-memory tile: a plain 16-byte copy
             const int chunks_per_row = rs / 16;
             const uint4* src = reinterpret_cast<const uint4*>(p.x_i8 + (size_t)m0 * rs);
@@ -276,7 +280,7 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                     }
                 }
                 base += kMNI;
-                if (kMWarps * base >= pairs) break;
+                if (FORM == kMmaOneBatch || kMWarps * base >= pairs) break;
                 load_batch(s, g, base, wa, wb);
             }
             tr.mark();                                             // 4+: MMAs of a row group done
@@ -324,12 +328,12 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
                     const int sx = s_sumx[out_m];
                     va -= sx;
                     const size_t o = (size_t)(m0 + out_m) * sg.N + n;
-                    if (sg.acc_out) sg.acc_out[o] = va;
+                    if (!kPlain && sg.acc_out) sg.acc_out[o] = va;
                     const float wsa = sg.w_scale;
                     const float ya = __fmul_rn((float)va, __fmul_rn(s_scale[out_m], wsa));
                     if (PAIR) {
                         vb -= sx;
-                        if (p.seg[1].acc_out) p.seg[1].acc_out[o] = vb;
+                        if (!kPlain && p.seg[1].acc_out) p.seg[1].acc_out[o] = vb;
                         const float wsb = p.seg[1].w_scale;
                         const float yb = __fmul_rn((float)vb, __fmul_rn(s_scale[out_m], wsb));
                         if (p.epilogue == LSPK_EPI_SILU_MUL) {
@@ -357,16 +361,25 @@ ternary_linear_mma_kernel(const __grid_constant__ LinearParams p) {
     tr.end();
 }
 
-template <bool PAIR>
-static cudaError_t launch_mma(const LinearParams& p, dim3 grid, size_t smem) {
+template <bool PAIR, int FORM>
+static cudaError_t launch_mma_form(const LinearParams& p, dim3 grid, size_t smem) {
     static bool attr_set = false;
-    auto kern = ternary_linear_mma_kernel<PAIR>;
+    auto kern = ternary_linear_mma_kernel<PAIR, FORM>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
     return launch(kern, grid, dim3(kMThreads), smem, true, p);
+}
+
+template <bool PAIR>
+static cudaError_t launch_mma(const LinearParams& p, dim3 grid, size_t smem) {
+    bool plain = p.prologue == kProInt8Tiled && !p.trace;
+    for (int i = 0; i < p.n_seg; ++i) plain = plain && !p.seg[i].acc_out;
+    if (!plain) return launch_mma_form<PAIR, kMmaAny>(p, grid, smem);
+    return p.chunks <= 2 * kMWarps * kMNI ? launch_mma_form<PAIR, kMmaOneBatch>(p, grid, smem)
+                                          : launch_mma_form<PAIR, kMmaTiled>(p, grid, smem);
 }
 
 // Launch the eight-row kernel.  K is limited by the shared-memory activation tile (8 rows of K bytes).

@@ -29,6 +29,11 @@ __device__ __forceinline__ uint4 ldg_policy(const uint4* p, uint64_t policy) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy));
     return v;
 }
+__device__ __forceinline__ uint32_t ldg_policy(const uint32_t* p, uint64_t policy) {
+    uint32_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(policy));
+    return v;
+}
 
 // Accumulate one 16-byte weight chunk (64 weights) against the matching 64 permuted activations.
 __device__ __forceinline__ void chunk_dot(const uint4& wv, const int4* __restrict__ xp, int acc[4]) {

@@ -46,3 +46,30 @@ def test_plain_forms_equal_the_general_one(n, prologue):
             assert np.array_equal(plain, general, equal_nan=True)
         for w in ws:
             w.free()
+
+
+@pytest.mark.parametrize("M", [2, 8, 9, 40, 130])
+@pytest.mark.parametrize("n", [16, 64, 2560, 4096, 4112, 6912, 8192, 4100])
+def test_many_rows_plain_and_general_forms(n, M):
+    """Rows normalised and quantised on the way into a product, without accumulators (plain forms of the row quantiser and
+    of the product) and with them, and as int8 rows from the quantiser's natural order: one result, bit for bit."""
+    rng = np.random.default_rng(n + M)
+    x = dev.DeviceArray.from_numpy((rng.standard_normal((M, n)) * 3).astype(np.float32))
+    gamma = dev.DeviceArray.from_numpy(synthetic.fp32_to_bf16_u16((1.0 + 0.2 * rng.standard_normal(n)).astype(np.float32)))
+    q, s = dev.DeviceArray((M, n), np.int8), dev.DeviceArray((M,), np.float32)
+    K.check(K.load_library().lspk_rmsnorm_quantize_rows(x.ptr, gamma.ptr, 1, q.ptr, s.ptr, M, n, 1e-5))
+    for sizes, epilogue in (((200, 16, 40), K.EPI_STORE), ((200,), K.EPI_ADD), ((200, 200), K.EPI_RELU2_MUL), ((40, 40), K.EPI_SILU_MUL)):
+        ws = [_weight(rng, N, n) for N in sizes]
+        start = [rng.standard_normal((M, N)).astype(np.float32) for N in sizes]
+        got = []
+        for rows, taps in (("fp32", False), ("fp32", True), ("int8", False), ("int8", True)):
+            outs = [dev.DeviceArray.from_numpy(v) for v in start]
+            accs = [dev.DeviceArray((M, N), np.int32) for N in sizes] if taps else []
+            kw = {"x_f32": x, "gamma": gamma} if rows == "fp32" else {"x_i8": q, "x_scales": s}
+            dev.linear(ws, outs, M, epilogue=epilogue, acc_outs=accs, **kw)
+            got.append([o.numpy() for o in outs])
+        for other in got[1:]:
+            for a, b in zip(got[0], other):
+                assert np.array_equal(a, b, equal_nan=True)
+        for w in ws:
+            w.free()
