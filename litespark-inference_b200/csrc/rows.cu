@@ -217,13 +217,17 @@ __device__ __forceinline__ uint32_t quant_exact(float v, float inv, int k, int K
 // library divisions, two-barrier reductions and a conversion per element took 6 % of the MLP block of 512 rows (49.9 -> 46.9 us)
 // and 7 % of a decode step of eight sequences (1.26 -> 1.16 ms).  A row spread over 640 or 1024 threads, four elements each,
 // is no faster at 8 rows (both 1.18 ms) and slower at 512 (53 us).
-template <int NB>
+// PLAIN   normed rows without a gate or selected weights, whole blocks of 16, permuted output: 11 KB of code (NB = 1; 15 KB at 2)
+//         instead of 25 (42), which each launch of a decode step has to fetch: eight sequences 1.25 -> 1.22 ms a step
+template <int NB, bool PLAIN>
 __global__ void __launch_bounds__(kRowThreads)
 row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gate, const void* __restrict__ gamma_base,
-                      const int* __restrict__ gamma_sel, int gamma_is_bf16, int8_t* __restrict__ out_i8,
-                      float* __restrict__ scales, int K, float eps, float rcp_K, int norm, int perm_kp, int perm_stride,
+                      const int* __restrict__ gamma_sel_in, int gamma_is_bf16, int8_t* __restrict__ out_i8,
+                      float* __restrict__ scales, int K, float eps, float rcp_K, int norm_in, int perm_kp, int perm_stride,
                       int* __restrict__ sums) {
     __shared__ __align__(16) float red[32];
+    const int norm = PLAIN ? 1 : norm_in;
+    const int* gamma_sel = PLAIN ? nullptr : gamma_sel_in;
     const int t = blockIdx.x, tid = threadIdx.x;
     float gm[NB][16];
     auto load_gamma = [&](const void* gamma) {
@@ -234,7 +238,7 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
             for (int q = 0; q < 4; ++q) {
                 const int k = k0 + q * 4;
                 float4 gv = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (k < K) {
+                if ((PLAIN ? k0 : k) < K) {
                     if (gamma_is_bf16) {
                         const uint2 gb = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(gamma) + k));
                         gv.x = __uint_as_float(gb.x << 16);
@@ -267,14 +271,14 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k0 + q * 4 < K) t4 = *reinterpret_cast<const float4*>(src + k0 + q * 4);
+            if ((PLAIN ? k0 : k0 + q * 4) < K) t4 = *reinterpret_cast<const float4*>(src + k0 + q * 4);
             v[nb][q * 4 + 0] = t4.x;
             v[nb][q * 4 + 1] = t4.y;
             v[nb][q * 4 + 2] = t4.z;
             v[nb][q * 4 + 3] = t4.w;
         }
     }
-    if (gate) {
+    if (!PLAIN && gate) {
         const float* gsrc = gate + (size_t)t * K;
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
@@ -282,7 +286,7 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (k0 + q * 4 < K) t4 = *reinterpret_cast<const float4*>(gsrc + k0 + q * 4);
+                if ((PLAIN ? k0 : k0 + q * 4) < K) t4 = *reinterpret_cast<const float4*>(gsrc + k0 + q * 4);
                 v[nb][q * 4 + 0] = __fmul_rn(v[nb][q * 4 + 0], silu_gate(t4.x));
                 v[nb][q * 4 + 1] = __fmul_rn(v[nb][q * 4 + 1], silu_gate(t4.y));
                 v[nb][q * 4 + 2] = __fmul_rn(v[nb][q * 4 + 2], silu_gate(t4.z));
@@ -321,7 +325,7 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
     const float scale = quant_scale_from_absmax(amax);
     const float inv = rcp_rn(scale);
     const int tail_start = K & ~15;
-    const int limit = perm_kp > 0 ? perm_kp : K;
+    const int limit = PLAIN || perm_kp > 0 ? perm_kp : K;
     int sumx = 0;
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
@@ -336,12 +340,17 @@ row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gat
                 all[e & 3] += f;
             }
             const float any = (all[0] + all[1]) + (all[2] + all[3]);
-            if (k0 + 16 > tail_start || !(any == any)) {
+            if (PLAIN && !(any == any)) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                    if (const float f = __fmul_rn(v[nb][e], inv); f != f) w[e] = 0u;
+            }
+            if (!PLAIN && (k0 + 16 > tail_start || !(any == any))) {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) w[e] = quant_exact(v[nb][e], inv, k0 + e, K);
             }
             uint32_t a[4];
-            if (perm_kp > 0) {      // packed in the transposed order
+            if (PLAIN || perm_kp > 0) {      // packed in the transposed order
 #pragma unroll
                 for (int q = 0; q < 4; ++q) a[q] = pack4_bytes(w[q], w[4 + q], w[8 + q], w[12 + q]);
                 *reinterpret_cast<uint4*>(out_i8 + (size_t)t * perm_stride + k0) = make_uint4(a[0], a[1], a[2], a[3]);
@@ -408,11 +417,12 @@ static int launch_rows(const float* x, const void* gamma, int gamma_is_bf16, flo
     if (vec && (mode & 2) && K <= 8192 && (perm_kp == 0 || perm_kp <= 8192)) {
         const int pstride = perm_stride > 0 ? perm_stride : perm_kp;
         const float rcp_K = fma_division_ok((float)K) ? 1.0f / (float)K : 0.0f;
-        const cudaError_t e = K <= 4096 && perm_kp <= 4096
-            ? launch(row_quant_regs_kernel<1>, dim3(T), dim3(kRowThreads), 0, true, x, gate, gamma, gamma_sel, gamma_is_bf16,
-                     out_i8, scales, K, eps, rcp_K, mode & 1, perm_kp, pstride, sums)
-            : launch(row_quant_regs_kernel<2>, dim3(T), dim3(kRowThreads), 0, true, x, gate, gamma, gamma_sel, gamma_is_bf16,
-                     out_i8, scales, K, eps, rcp_K, mode & 1, perm_kp, pstride, sums);
+        const bool one = K <= 4096 && perm_kp <= 4096;
+        const bool plain = (mode & 1) && perm_kp > 0 && K % 16 == 0 && !gate && !gamma_sel;
+        auto kern = plain ? one ? row_quant_regs_kernel<1, true> : row_quant_regs_kernel<2, true>
+                          : one ? row_quant_regs_kernel<1, false> : row_quant_regs_kernel<2, false>;
+        const cudaError_t e = launch(kern, dim3(T), dim3(kRowThreads), 0, true, x, gate, gamma, gamma_sel, gamma_is_bf16, out_i8,
+                                     scales, K, eps, rcp_K, mode & 1, perm_kp, pstride, sums);
         if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "row quantiser launch failed: %s", cudaGetErrorString(e));
         return LSPK_OK;
     }
