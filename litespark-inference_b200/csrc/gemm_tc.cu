@@ -189,15 +189,19 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-// PLAIN   without a trace and without accumulators to hand out
-//         (marks in the K loop of every role and dynamic picks from the accumulators: 7 to 10 KB of code, 7 % of the MLP block of
-//         512 rows, 46.9 -> 43.5 us, 3 % of a prefill of 1531 tokens, 9.59 -> 9.30 ms)
-template <bool PAIR, int TN, bool PLAIN>
+// FORM    kTcAny: every call; kTcPlain: no trace, no accumulators to hand out; with kTcWhole K is not split over a cluster, with
+//         kTcSilu the pair's gate is SiLU, without ReLU^2.
+// What a form leaves out is code that start-up and epilogue would be fetched around: a paired tile of 128 has 24 KB instead of
+// 48, a single one 46 instead of 66.  Marks and taps out: the MLP block of 512 rows 46.9 -> 43.5 us, a prefill of 1531 tokens
+// 9.59 -> 9.30 ms; the split and the other gate out: 42.6 -> 40.7 us and 9.26 -> 9.15 ms.
+enum { kTcAny = 0, kTcPlain = 1, kTcWhole = 2, kTcSilu = 4 };
+template <bool PAIR, int TN, int FORM>
 __global__ void __launch_bounds__(kTcThreads, TcLayout<PAIR, TN>::kHalf ? 2 : 1)
 ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                        const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x,
                        const __grid_constant__ TcParams p) {
     using L = TcLayout<PAIR, TN>;
+    constexpr bool PLAIN = FORM != kTcAny;
     constexpr int FM = L::FM;
     constexpr int kX = L::kX, kA = L::kA, kW = kTcWStages, W = L::kSlab, kBK = kTcBK;
     // instruction descriptor: D = s32, A = B = signed int8 (the weight codes 0, 1, 2 are their own int8 values), both
@@ -228,7 +232,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_
     const int n0 = ((int)blockIdx.x - sg.tile0) * kTcRows;
     const int m0 = blockIdx.y * TN;
     // K split over the cluster: this CTA's K blocks are [kb0, kb0 + nkb)
-    const int splits = gridDim.z, rank = blockIdx.z;
+    const int splits = FORM & kTcWhole ? 1 : gridDim.z, rank = FORM & kTcWhole ? 0 : blockIdx.z;
     const int kb0 = rank * p.kb_per_split;
     const int nkb = min(p.kb_per_split, p.k_blocks - kb0);
 
@@ -488,7 +492,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_
                     for (int j = 0; j < jmax; ++j) g.acc_out[o0 + (size_t)j * g.N] = (int)pick<W>(vg, j);
                 if (!PLAIN && u.acc_out)
                     for (int j = 0; j < jmax; ++j) u.acc_out[o0 + (size_t)j * g.N] = (int)pick<W>(vu, j);
-                if (p.epilogue == LSPK_EPI_SILU_MUL) {
+                if (PLAIN ? (FORM & kTcSilu) != 0 : p.epilogue == LSPK_EPI_SILU_MUL) {
 #pragma unroll
                     for (int j = 0; j < W; ++j) {
                         const float yg = __fmul_rn((float)(int)vg[j], __fmul_rn(y[j], g.w_scale));
@@ -670,11 +674,11 @@ static int activation_map(EncodeTiledFn enc, CUtensorMap* out, int8_t* x, int Kp
     return LSPK_OK;
 }
 
-template <bool PAIR, int TN, bool PLAIN>
+template <bool PAIR, int TN, int FORM>
 static cudaError_t launch_tc_form(const CUtensorMap* mw, const CUtensorMap& mx, const TcParams& p, dim3 grid) {
     constexpr int smem = TcLayout<PAIR, TN>::kSmem;
     static bool attr_set = false;
-    auto kern = ternary_gemm_tc_kernel<PAIR, TN, PLAIN>;
+    auto kern = ternary_gemm_tc_kernel<PAIR, TN, FORM>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
@@ -689,7 +693,13 @@ template <bool PAIR, int TN>
 static cudaError_t launch_tc(const CUtensorMap* mw, const CUtensorMap& mx, const TcParams& p, dim3 grid) {
     bool plain = !p.trace;
     for (int i = 0; i < (PAIR ? 2 : p.n_seg); ++i) plain = plain && !p.seg[i].acc_out;
-    return plain ? launch_tc_form<PAIR, TN, true>(mw, mx, p, grid) : launch_tc_form<PAIR, TN, false>(mw, mx, p, grid);
+    if (!plain) return launch_tc_form<PAIR, TN, kTcAny>(mw, mx, p, grid);
+    if constexpr (PAIR)
+        if (p.epilogue == LSPK_EPI_SILU_MUL)
+            return grid.z > 1 ? launch_tc_form<PAIR, TN, kTcPlain | kTcSilu>(mw, mx, p, grid)
+                              : launch_tc_form<PAIR, TN, kTcPlain | kTcSilu | kTcWhole>(mw, mx, p, grid);
+    return grid.z > 1 ? launch_tc_form<PAIR, TN, kTcPlain>(mw, mx, p, grid)
+                      : launch_tc_form<PAIR, TN, kTcPlain | kTcWhole>(mw, mx, p, grid);
 }
 
 // Token rows per tile and K split of a launch: the plan with the smallest time by a model of a CTA's life in SM cycles,
