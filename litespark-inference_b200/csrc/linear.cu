@@ -55,7 +55,9 @@ __device__ __forceinline__ float cta8_max_nonneg(float v, float* slot) {
 // A decode step walks through five kernels a layer, together more code than an SM's instruction cache holds, so what a launch
 // does not execute costs as well: with the plain forms apart and one set of weight loads the code of q/k/v and o went from 39
 // to 17 KB, of gate/up from 43 to 20 KB, of down from 62 to 24 KB, a decode step at context 128 from 758 to 682 us.
-template <int MT, int NI, int NB, bool PAIR, int PRO>
+// ONCE    a CTA per row group (q/k/v, o, down): no loop, no registers for the next group's weights (decode at context 128 678 ->
+//         667 us a step)
+template <int MT, int NI, int NB, bool PAIR, int PRO, bool ONCE>
 __global__ void __launch_bounds__(kThreads)
 ternary_linear_kernel(const __grid_constant__ LinearParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -302,7 +304,7 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
         // ---- loop over this CTA's row groups: integer dot products, reduction, epilogue ----------------
         while (true) {
             const int next_flat = flat + gridDim.x;
-            const bool has_next = next_flat < p.total_groups;
+            const bool has_next = !ONCE && next_flat < p.total_groups;
             int ns = 0, ng = 0;
             float next_resid = 0.0f;
             if (has_next) {
@@ -417,16 +419,22 @@ static size_t linear_smem_bytes(int MT, int Kp, bool pair) {
     b += 32 * 4 + MT * 4 + MT * kWarps * 4;
     return b;
 }
-template <int NI, int NB, bool PAIR, int PRO>
-static cudaError_t launch_linear(const LinearParams& p, dim3 grid, size_t smem) {
+template <int NI, int NB, bool PAIR, int PRO, bool ONCE>
+static cudaError_t launch_linear_form(const LinearParams& p, dim3 grid, size_t smem) {
     static bool attr_set = false;
-    auto kern = ternary_linear_kernel<1, NI, NB, PAIR, PRO>;
+    auto kern = ternary_linear_kernel<1, NI, NB, PAIR, PRO, ONCE>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
     return launch(kern, grid, dim3(kThreads), smem, true, p);
+}
+template <int NI, int NB, bool PAIR, int PRO>
+static cudaError_t launch_linear(const LinearParams& p, dim3 grid, size_t smem) {
+    if constexpr (PRO != kAnyPrologue)
+        if (p.total_groups <= (int)grid.x) return launch_linear_form<NI, NB, PAIR, PRO, true>(p, grid, smem);
+    return launch_linear_form<NI, NB, PAIR, PRO, false>(p, grid, smem);
 }
 // The plain forms up to K = 8192 have an instantiation each (see the kernel); longer rows are not launch-bound.
 template <int NI, int NB, bool PAIR>
