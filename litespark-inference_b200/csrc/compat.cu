@@ -44,6 +44,87 @@ static bool down(void* dst, const void* src, size_t bytes) {
     return true;
 }
 
+// ---- small calls: pinned, mapped staging ------------------------------------------------------
+// A call of a few rows spends its time on host round trips, not on bytes: copies from and to pageable memory cost 5 to 10 us
+// each, whatever their size, and the wait for the stream as much.  So its arguments are copied (by the CPU) into a pinned
+// buffer that the GPU reads over the bus, its results come back the same way, and a last kernel stores the call's number to a
+// word that the host polls: the seven calls of an MLP block of one row take 192 us instead of 291.  Up to kStageBytes each way,
+// larger calls keep the copies.
+constexpr size_t kStageBytes = 256 * 1024;
+
+__global__ void host_done_kernel(unsigned* flag, unsigned call) {
+    grid_dependency_wait();
+    __threadfence_system();      // the results of the kernel before, then the number
+    asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(flag), "r"(call) : "memory");
+}
+// Mapped host memory -> device memory, for rows that a kernel reads many times.
+__global__ void __launch_bounds__(256) host_fetch_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int n) {
+    grid_dependency_launch();
+    grid_dependency_wait();
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) dst[i] = src[i];
+}
+
+struct HostStage {
+    static constexpr size_t kHead = 256;      // the polled word
+    static constexpr size_t kSlack = 16 * 256;      // regions start at multiples of 256
+    unsigned char *host = nullptr, *dev = nullptr;
+    size_t used = 0;
+    unsigned call = 0;
+    bool failed = false;
+    // Starts a call that moves so many bytes; false: it takes the copies.
+    bool begin(size_t in_bytes, size_t out_bytes) {
+        if (failed || in_bytes > kStageBytes || out_bytes > kStageBytes) return false;
+        if (!host) {
+            void *h = nullptr, *d = nullptr;
+            if (cudaHostAlloc(&h, kHead + 2 * kStageBytes + kSlack, cudaHostAllocMapped) != cudaSuccess ||
+                cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
+                cudaGetLastError();
+                if (h) cudaFreeHost(h);
+                failed = true;
+                return false;
+            }
+            memset(h, 0, kHead);
+            host = static_cast<unsigned char*>(h);
+            dev = static_cast<unsigned char*>(d);
+        }
+        used = kHead;
+        return true;
+    }
+    // The next region: its device address; `h` its host address.
+    void* region(size_t bytes, void** h) {
+        void* d = dev + used;
+        *h = host + used;
+        used += (bytes + 255) / 256 * 256;
+        return d;
+    }
+    const void* put(const void* src, size_t bytes) {
+        void *h, *d = region(bytes, &h);
+        memcpy(h, src, bytes);
+        return d;
+    }
+    // Waits for the kernels enqueued since begin().
+    bool finish() {
+        const unsigned want = ++call;
+        cudaError_t e = launch(host_done_kernel, dim3(1), dim3(1), 0, true, reinterpret_cast<unsigned*>(dev), want);
+        for (unsigned spins = 1; e == cudaSuccess; ++spins) {
+            if (*(volatile unsigned*)host == want) break;
+            if ((spins & 0xfffu) == 0) {      // every so often ask the driver: an error ends the wait
+                const cudaError_t q = cudaStreamQuery(stream());
+                if (q == cudaErrorNotReady) continue;
+                if (q != cudaSuccess || *(volatile unsigned*)host != want) e = q == cudaSuccess ? cudaErrorUnknown : q;
+            }
+        }
+        if (e != cudaSuccess) {
+            fail(LSPK_ERR_CUDA, "host call failed: %s", cudaGetErrorString(e));
+            cudaStreamSynchronize(stream());  // the buffer is the next call's
+            return false;
+        }
+        __sync_synchronize();                 // the results are read after the number
+        return true;
+    }
+};
+static HostStage g_stage;                     // under g_compat_mu
+
 // ---- registry of resident weights / embeddings keyed by host address ------------------------
 struct PackedEntry { lspk_weight_t w; int N, K; };
 struct EmbEntry { void* emb; float* scale; int kind, V, H; };
@@ -74,10 +155,28 @@ static void matmul_host(const int8_t* x, const float* x_scales, const uint8_t* p
     }
     if (!w) return;
     reinterpret_cast<Weight*>(w)->scale = w_scale;
-    int8_t* dx = (int8_t*)slot(S_X, (size_t)T * K);
-    float* dxs = (float*)slot(S_XS, (size_t)T * 4);
-    float* dy = (float*)slot(S_Y, (size_t)T * N * 4);
-    if (dx && dxs && dy && up(dx, x, (size_t)T * K) && up(dxs, x_scales, (size_t)T * 4)) {
+    const size_t xb = ((size_t)T * K + 15) / 16 * 16, sb = ((size_t)T * 4 + 15) / 16 * 16, yb = (size_t)T * N * 4;
+    const bool staged = g_stage.begin(xb + sb, yb);
+    int8_t* dx = (int8_t*)slot(S_X, staged ? xb + sb : (size_t)T * K);
+    float* dxs = staged ? (float*)(dx + xb) : (float*)slot(S_XS, (size_t)T * 4);
+    float* dy = staged ? nullptr : (float*)slot(S_Y, yb);
+    void* y_host = nullptr;
+    bool ok = dx && dxs && (staged || dy);
+    if (ok && staged) {
+        // the rows go to device memory (every CTA of the product reads them), the results straight to the host's
+        void* h;
+        const uint4* src = (const uint4*)g_stage.region(xb + sb, &h);
+        memcpy(h, x, (size_t)T * K);
+        memcpy((char*)h + xb, x_scales, (size_t)T * 4);
+        dy = (float*)g_stage.region(yb, &y_host);
+        const int n = (int)((xb + sb) / 16);
+        const cudaError_t e = launch(host_fetch_kernel, dim3((n + 255) / 256), dim3(256), 0, true, src, (uint4*)dx, n);
+        ok = e == cudaSuccess;
+        if (!ok) fail(LSPK_ERR_CUDA, "host call: launch failed: %s", cudaGetErrorString(e));
+    } else if (ok) {
+        ok = up(dx, x, (size_t)T * K) && up(dxs, x_scales, (size_t)T * 4);
+    }
+    if (ok) {
         lspk_linear_args a = {};
         a.w[0] = w;
         a.out[0] = dy;
@@ -87,7 +186,10 @@ static void matmul_host(const int8_t* x, const float* x_scales, const uint8_t* p
         a.epilogue = LSPK_EPI_STORE;
         a.x_i8 = dx;
         a.x_scales = dxs;
-        if (lspk_linear(&a) == LSPK_OK) down(y, dy, (size_t)T * N * 4);
+        if (lspk_linear(&a) == LSPK_OK) {
+            if (!staged) down(y, dy, yb);
+            else if (g_stage.finish()) memcpy(y, y_host, yb);
+        }
     }
     if (temp) {
         cudaStreamSynchronize(stream());
@@ -100,7 +202,20 @@ static void rows_host(const float* x, const void* gamma, int gamma_is_bf16, floa
     std::lock_guard<std::mutex> lk(g_compat_mu);
     if (ensure_init()) return;
     if (!x || T < 1 || K < 1) { fail(LSPK_ERR_ARG, "row helper: bad arguments (T=%d K=%d)", T, K); return; }
-    const size_t n = (size_t)T * K;
+    const size_t n = (size_t)T * K, gb = gamma ? (size_t)K * (gamma_is_bf16 ? 2 : 4) : 0, ob = (mode & 2) ? n : n * 4;
+    if (g_stage.begin(n * 4 + gb, ob + (size_t)T * 4)) {
+        // every element is read once and written once, by a CTA per row: straight from and to the host's memory
+        const float* sx = (const float*)g_stage.put(x, n * 4);
+        const void* sg = gamma ? g_stage.put(gamma, gb) : nullptr;
+        void *ho, *hs, *d = g_stage.region(ob, &ho), *ds = g_stage.region((size_t)T * 4, &hs);
+        const int rc = mode == 2   ? lspk_quantize_rows(sx, (int8_t*)d, (float*)ds, T, K)
+                       : mode == 1 ? lspk_rmsnorm_rows(sx, sg, gamma_is_bf16, (float*)d, T, K, eps)
+                                   : lspk_rmsnorm_quantize_rows(sx, sg, gamma_is_bf16, (int8_t*)d, (float*)ds, T, K, eps);
+        if (rc != LSPK_OK || !g_stage.finish()) return;
+        memcpy((mode & 2) ? (void*)out_i8 : (void*)out_f32, ho, ob);
+        if (mode & 2) memcpy(scales, hs, (size_t)T * 4);
+        return;
+    }
     float* dx = (float*)slot(S_A, n * 4);
     void* dg = gamma ? slot(S_G, (size_t)K * (gamma_is_bf16 ? 2 : 4)) : nullptr;
     float* dof = (mode & 2) ? nullptr : (float*)slot(S_B, n * 4);
@@ -213,6 +328,12 @@ void relu2_mul_fp32_batched_sm100(const float* gate, const float* up_, float* ou
     if (ensure_init()) return;
     if (!gate || !up_ || !out || T < 1 || K < 1) { fail(LSPK_ERR_ARG, "relu2_mul_sm100: bad arguments"); return; }
     const size_t n = (size_t)T * K;
+    if (g_stage.begin(2 * n * 4, n * 4)) {
+        const float *sg = (const float*)g_stage.put(gate, n * 4), *su = (const float*)g_stage.put(up_, n * 4);
+        void *h, *d = g_stage.region(n * 4, &h);
+        if (lspk_relu2_mul_rows(sg, su, (float*)d, T, K) == LSPK_OK && g_stage.finish()) memcpy(out, h, n * 4);
+        return;
+    }
     float* dg = (float*)slot(S_A, n * 4);
     float* du = (float*)slot(S_B, n * 4);
     float* dout = (float*)slot(S_Y, n * 4);
@@ -227,6 +348,13 @@ void add_inplace_fp32_sm100(float* a, const float* b, int K) {
     std::lock_guard<std::mutex> lk(g_compat_mu);
     if (ensure_init()) return;
     if (!a || !b || K < 1) { fail(LSPK_ERR_ARG, "add_inplace_sm100: bad arguments"); return; }
+    if (g_stage.begin((size_t)K * 8, (size_t)K * 4)) {
+        void *h, *d = g_stage.region((size_t)K * 4, &h);
+        memcpy(h, a, (size_t)K * 4);
+        const float* sb = (const float*)g_stage.put(b, (size_t)K * 4);
+        if (lspk_add_rows((float*)d, sb, (size_t)K) == LSPK_OK && g_stage.finish()) memcpy(a, h, (size_t)K * 4);
+        return;
+    }
     float* da = (float*)slot(S_A, (size_t)K * 4);
     float* db = (float*)slot(S_B, (size_t)K * 4);
     if (!da || !db || !up(da, a, (size_t)K * 4) || !up(db, b, (size_t)K * 4)) return;

@@ -1,0 +1,69 @@
+"""The drop-in calls on host pointers: small calls go through a pinned buffer that the GPU reads and writes over the bus,
+larger ones through copies.  Both sides of the limit (256 KB each way) against the oracle, in place where the reference
+allows it, and from several threads at once."""
+import importlib
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+K = importlib.import_module("litespark_inference_b200.torchless.kernel")
+LIMIT = 256 * 1024
+
+
+@pytest.mark.parametrize("T,n", [(1, 1), (1, 2560), (1, 6912), (1, LIMIT // 8), (1, LIMIT // 8 + 1), (9, 6912), (10, 6912), (26, 2560)])
+def test_elementwise_calls(port, T, n):
+    lib = K.load_library(True)
+    rng = np.random.default_rng(T * n)
+    g, u = (rng.standard_normal((T, n)).astype(np.float32) for _ in range(2))
+    r = np.maximum(g, np.float32(0))
+    out = g.copy()
+    lib.relu2_mul_fp32_batched_sm100(out, u, out, T, n)          # in place
+    assert np.array_equal(out, r * r * u)
+    a = g.ravel().copy()
+    lib.add_inplace_fp32_sm100(a, u.ravel(), a.size)
+    assert np.array_equal(a, g.ravel() + u.ravel())
+
+
+@pytest.mark.parametrize("T,n", [(1, 4), (1, 2560), (1, 8192), (9, 6912), (10, 6912), (25, 2560), (26, 2560)])
+def test_rows_and_products(port, T, n):
+    lib = K.load_library(True)
+    rng = np.random.default_rng(T + n)
+    x = rng.standard_normal((T, n)).astype(np.float32)
+    q, s = np.empty((T, n), np.int8), np.empty(T, np.float32)
+    lib.quantize_activation_batched_sm100(x, q, s, T, n)
+    wq, ws = np.empty_like(q), np.empty_like(s)
+    port.quantize_activation_batched(x, wq, ws)
+    assert np.array_equal(q, wq) and np.array_equal(s, ws)
+    for N in (16, LIMIT // 4 // T, LIMIT // 4 // T + 1):
+        if N * n > 1 << 26:
+            continue
+        packed = rng.integers(0, 3, (N, n // 4), dtype=np.uint8) * np.uint8(0x55)      # four equal weights a byte
+        w = (packed & 3).astype(np.float64) - 1
+        y = np.empty((T, N), np.float32)
+        lib.matmul_lut_sm100_mT(q, s, packed, np.float32(0.5), y, T, N, n)
+        dots = q.astype(np.float64).reshape(T, n // 4, 4).sum(axis=2) @ w.T            # exact: integers below 2^53
+        assert np.array_equal(y, dots.astype(np.float32) * (s * np.float32(0.5))[:, None])
+
+
+def test_calls_from_several_threads():
+    lib = K.load_library(True)
+    rng = np.random.default_rng(0)
+    data = [(rng.standard_normal(n).astype(np.float32), rng.standard_normal(n).astype(np.float32)) for n in (5, 2560, 6912, 40000)]
+    bad = []
+
+    def work(a, b):
+        for _ in range(50):
+            got = a.copy()
+            lib.add_inplace_fp32_sm100(got, b, got.size)
+            if not np.array_equal(got, a + b):
+                bad.append(a.size)
+
+    threads = [threading.Thread(target=work, args=d) for d in data]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
