@@ -580,7 +580,10 @@ int linear_cuda_core(const lspk_linear_args* a) {
     const int tiles = (a->M + MT - 1) / MT;
     p.stream_weights = tiles == 1 ? 1 : 0;
     int ctas = groups;
-    const int per_wave = tiles == 1 ? 2 * sm_count() : (2 * sm_count() + tiles - 1) / tiles;
+    // One row of an unpaired product: three, which its registers allow (a hybrid step, whose Mamba projections have 2 to 4 row
+    // groups per SM, 577 -> 558 us).  Not so the pair: with a CTA for each of 432 groups a decode step takes 672 us, with two
+    // CTAs per SM and a loop 667.
+    const int per_wave = tiles == 1 ? (!pair && a->M == 1 ? 3 : 2) * sm_count() : (2 * sm_count() + tiles - 1) / tiles;
     if (ctas > per_wave) ctas = per_wave > 0 ? per_wave : 1;
     return linear_launch_params(p, MT, pair, ctas, tiles);
 }
