@@ -574,14 +574,14 @@ int linear_cuda_core(const lspk_linear_args* a) {
     p.trace_cap = trace_capacity();
     p.error_flag = device_wait_flag();
     const int MT = a->M == 1 ? 1 : 8;
-    // At most two CTAs per SM when there is a single token tile (measured best on B200: the prologue
-    // runs once per CTA, which then loops over its row groups).  With several token tiles the grid's
+    // With a single token tile at most two CTAs per SM (the prologue runs once per CTA, which then
+    // loops over its row groups).  With several token tiles the grid's
     // second dimension already fills the machine.
     const int tiles = (a->M + MT - 1) / MT;
     p.stream_weights = tiles == 1 ? 1 : 0;
     int ctas = groups;
-    // One row of an unpaired product: three, which its registers allow (a hybrid step, whose Mamba projections have 2 to 4 row
-    // groups per SM, 577 -> 558 us).  Not so the pair: with a CTA for each of 432 groups a decode step takes 672 us, with two
+    // One row of an unpaired product: three, which its registers allow (a hybrid step, whose Mamba input projections have 661 row
+    // groups, 574 -> 560 us).  Not so the pair: with a CTA for each of 432 groups a decode step takes 672 us, with two
     // CTAs per SM and a loop 667.
     const int per_wave = tiles == 1 ? (!pair && a->M == 1 ? 3 : 2) * sm_count() : (2 * sm_count() + tiles - 1) / tiles;
     if (ctas > per_wave) ctas = per_wave > 0 ? per_wave : 1;
