@@ -183,7 +183,8 @@ void matmul_lut_sm100_mT(const int8_t* x, const float* x_scales, const uint8_t* 
 /* kernel.py:252-256  matmul_lut_{T}_prefill (arm argument order) */
 void matmul_lut_sm100_prefill(const int8_t* x, const uint8_t* packed_w, float w_scale,
                               const float* x_scale, float* y, int M, int N, int K);
-/* kernel.py:295-297, 289-291 */
+/* kernel.py:295-297, 289-291.  Null int8 rows are left out (the scales are still returned); null fp32 rows or scales
+ * are a recorded failure. */
 float quantize_activation_sm100(const float* x, int8_t* out, int K);
 void quantize_activation_batched_sm100(const float* x, int8_t* out, float* scales, int T, int K);
 /* kernel.py:307-312, 283-288 */

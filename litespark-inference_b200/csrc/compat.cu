@@ -202,6 +202,7 @@ static void rows_host(const float* x, const void* gamma, int gamma_is_bf16, floa
     std::lock_guard<std::mutex> lk(g_compat_mu);
     if (ensure_init()) return;
     if (!x || T < 1 || K < 1) { fail(LSPK_ERR_ARG, "row helper: bad arguments (T=%d K=%d)", T, K); return; }
+    if ((mode & 2) ? !scales : !out_f32) { fail(LSPK_ERR_ARG, "row helper: null output"); return; }
     const size_t n = (size_t)T * K, gb = gamma ? (size_t)K * (gamma_is_bf16 ? 2 : 4) : 0, ob = (mode & 2) ? n : n * 4;
     if (g_stage.begin(n * 4 + gb, ob + (size_t)T * 4)) {
         // every element is read once and written once, by a CTA per row: straight from and to the host's memory
@@ -212,7 +213,8 @@ static void rows_host(const float* x, const void* gamma, int gamma_is_bf16, floa
                        : mode == 1 ? lspk_rmsnorm_rows(sx, sg, gamma_is_bf16, (float*)d, T, K, eps)
                                    : lspk_rmsnorm_quantize_rows(sx, sg, gamma_is_bf16, (int8_t*)d, (float*)ds, T, K, eps);
         if (rc != LSPK_OK || !g_stage.finish()) return;
-        memcpy((mode & 2) ? (void*)out_i8 : (void*)out_f32, ho, ob);
+        // a caller that wants the scales alone passes no int8 rows
+        if (!(mode & 2) || out_i8) memcpy((mode & 2) ? (void*)out_i8 : (void*)out_f32, ho, ob);
         if (mode & 2) memcpy(scales, hs, (size_t)T * 4);
         return;
     }
@@ -230,7 +232,7 @@ static void rows_host(const float* x, const void* gamma, int gamma_is_bf16, floa
     else rc = lspk_rmsnorm_quantize_rows(dx, dg, gamma_is_bf16, doi, dsc, T, K, eps);
     if (rc != LSPK_OK) return;
     if (mode & 2) {
-        cudaMemcpyAsync(out_i8, doi, n, cudaMemcpyDeviceToHost, stream());
+        if (out_i8) cudaMemcpyAsync(out_i8, doi, n, cudaMemcpyDeviceToHost, stream());
         down(scales, dsc, (size_t)T * 4);
     } else {
         down(out_f32, dof, n * 4);

@@ -1,6 +1,7 @@
 """The drop-in calls on host pointers: small calls go through a pinned buffer that the GPU reads and writes over the bus,
 larger ones through copies.  Both sides of the limit (256 KB each way) against the oracle, in place where the reference
 allows it, and from several threads at once."""
+import ctypes
 import importlib
 import threading
 
@@ -46,6 +47,33 @@ def test_rows_and_products(port, T, n):
         lib.matmul_lut_sm100_mT(q, s, packed, np.float32(0.5), y, T, N, n)
         dots = q.astype(np.float64).reshape(T, n // 4, 4).sum(axis=2) @ w.T            # exact: integers below 2^53
         assert np.array_equal(y, dots.astype(np.float32) * (s * np.float32(0.5))[:, None])
+
+
+@pytest.mark.parametrize("T,n", [(1, 2560), (40, 2560)])
+def test_null_outputs(T, n):
+    """On either side of the limit: a null fp32 row or null scales are recorded as a failure, null int8 rows are left out."""
+    lib = ctypes.CDLL(str(K.library_path()))          # plain pointers, past the array checks of the wrappers
+    lib.lspk_last_error.restype = ctypes.c_char_p
+    x, gamma = np.random.default_rng(n).standard_normal((T, n)).astype(np.float32), np.full(n, 0x3f80, np.uint16)
+    q, s, s_alone = np.empty((T, n), np.int8), np.empty(T, np.float32), np.zeros(T, np.float32)
+    at = lambda a: None if a is None else ctypes.c_void_p(a.ctypes.data)  # noqa: E731
+    eps, rows, width = ctypes.c_float(1e-5), ctypes.c_int(T), ctypes.c_int(n)
+    quantise = lambda o, sc: lib.quantize_activation_batched_sm100(at(x), at(o), at(sc), rows, width)  # noqa: E731
+    norm_quantise = lambda o, sc: lib.rmsnorm_quantize_bf16gamma_batched_sm100(  # noqa: E731
+        at(x), at(gamma), at(o), at(sc), None, rows, width, eps)
+    failing = [lambda: lib.rmsnorm_bf16gamma_fp32_batched_sm100(at(x), at(gamma), None, rows, width, eps),
+               lambda: lib.rmsnorm_fp32gamma_fp32_batched_sm100(at(x), at(x), None, rows, width, eps),
+               lambda: quantise(q, None), lambda: norm_quantise(q, None),
+               lambda: lib.relu2_mul_fp32_batched_sm100(at(x), at(x), None, rows, width)]
+    for call in failing:
+        lib.lspk_clear_error()
+        call()
+        assert lib.lspk_error_count() == 1 and any(m in lib.lspk_last_error() for m in (b"null output", b"bad arguments"))
+    lib.lspk_clear_error()
+    for call in (quantise, norm_quantise):
+        call(q, s)
+        call(None, s_alone)
+        assert lib.lspk_error_count() == 0 and np.array_equal(s, s_alone)
 
 
 def test_calls_from_several_threads():
