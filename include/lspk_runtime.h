@@ -96,6 +96,10 @@ int lspk_debug_expire_wait(int polls);
  * the GPU had none left (0: back to normal). */
 int lspk_debug_allocation_limit(size_t bytes);
 
+/* Test aid: the launch that a one-row lspk_linear(a) would make, which is not made: its CTAs, and how many of them an SM can
+ * hold at once. */
+int lspk_debug_row_launch(const lspk_linear_args* a, int* ctas, int* resident);
+
 /* Test aid: the attention section of one prefill layer on device arrays.  T consecutive rows of one sequence, the first at
  * position *pos (pos + T <= t_max): q [T, Q * D] is rotated in place, the rows' keys (rotated) and values [T, KV * D] are
  * written to the caches [t_max, KV, D] (fp16 or fp32), out [T, Q * D] receives the attention.  rope_cos / rope_sin [t_max, D / 2]. */

@@ -61,9 +61,6 @@ int norm_quant_rows_selected(const float* x, const void* gamma_bf16, const int* 
 int linear_mma_launch(const LinearParams& p, bool pair, int grid_x, int grid_y);
 __host__ __device__ inline int mma_row_stride(int Kp) { return (Kp % 128 == 0) ? Kp + 64 : Kp; }
 
-// Launch the CUDA-core kernel with fully prepared parameters.  mt: rows per CTA tile (1, 2, 4 or 8).
-int linear_launch_params(const LinearParams& p, int mt, bool pair, int grid_x, int grid_y);
-
 // linear.cu: validate + launch the CUDA-core ternary linear kernel on the library stream.
 int linear_cuda_core(const lspk_linear_args* a);
 

@@ -46,6 +46,21 @@ __device__ __forceinline__ float cta8_max_nonneg(float v, float* slot) {
     return fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
 }
 
+// CTAs per SM that a one-row product is launched with at most, by the form of the kernel below (one that has more row groups
+// loops over them).  A CTA that is not resident from the start costs a second run of the prologue without its weights
+// prefetched, so three only where the registers allow it (85 would): 47 to 80 for unpaired products up to K = 4096 and, without a
+// norm or a loop, up to 8192; the others there take 119 to 128.  (Minimum blocks in the launch bounds do not say so for free:
+// with any number there the compiler takes up to 40 registers more.)
+// Two and three per SM, in us (one row, weights not in L2):
+//   K = 2560, norm       N = 6912 5.0 and 4.3, 20480 8.9 and 6.7    (a hybrid step, Mamba projections of 661 groups: 574 and 560)
+//   K = 6912, quantise   N = 5120 5.5 and 5.1,  6912 6.1 and 5.3    (a CTA per group); 13824 8.9 and 11.0 (with the loop)
+//   K = 6912, norm       N = 5120 5.9 and 8.7,  6912 6.6 and 9.3, 13824 9.4 and 13.3; gated N = 6912 11.3 and 18.1
+//   K = 12288, N = 6912  quantise 14.1 and 15.7, norm 20.2 and 25.0
+// The pair keeps two: with a CTA for each of its 432 groups a decode step takes 672 us, with two per SM and the loop 667.
+constexpr int row_ctas_per_sm(bool pair, int ni, int pro, bool once) {
+    return !pair && (ni == 4 || (once && (pro == LSPK_PRO_INT8 || pro == LSPK_PRO_QUANT))) ? 3 : 2;
+}
+
 // MT      token rows per CTA tile
 // NI      16-byte weight loads per lane per batch (covers K <= 4096 at 4, K <= 8192 at 8 in one batch)
 // NB      16-element activation blocks a thread owns in the fp32 prologue (K <= 4096 * NB)
@@ -419,8 +434,13 @@ static size_t linear_smem_bytes(int MT, int Kp, bool pair) {
     b += 32 * 4 + MT * 4 + MT * kWarps * 4;
     return b;
 }
+// A launch, or where `resident` is given what it would be: its grid and how many CTAs of the form an SM holds.
+struct RowLaunch {
+    size_t smem;
+    int ctas, *resident;
+};
 template <int NI, int NB, bool PAIR, int PRO, bool ONCE>
-static cudaError_t launch_linear_form(const LinearParams& p, dim3 grid, size_t smem) {
+static cudaError_t launch_linear_form(const LinearParams& p, RowLaunch& l) {
     static bool attr_set = false;
     auto kern = ternary_linear_kernel<1, NI, NB, PAIR, PRO, ONCE>;
     if (!attr_set) {
@@ -428,46 +448,48 @@ static cudaError_t launch_linear_form(const LinearParams& p, dim3 grid, size_t s
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
-    return launch(kern, grid, dim3(kThreads), smem, true, p);
+    const int most = row_ctas_per_sm(PAIR, NI, PRO, ONCE) * sm_count();
+    l.ctas = p.total_groups < most ? p.total_groups : most;
+    if (l.resident) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(l.resident, kern, kThreads, l.smem);
+    return launch(kern, dim3(l.ctas), dim3(kThreads), l.smem, true, p);
 }
 template <int NI, int NB, bool PAIR, int PRO>
-static cudaError_t launch_linear(const LinearParams& p, dim3 grid, size_t smem) {
+static cudaError_t launch_linear(const LinearParams& p, RowLaunch& l) {
     if constexpr (PRO != kAnyPrologue)
-        if (p.total_groups <= (int)grid.x) return launch_linear_form<NI, NB, PAIR, PRO, true>(p, grid, smem);
-    return launch_linear_form<NI, NB, PAIR, PRO, false>(p, grid, smem);
+        if (p.total_groups <= row_ctas_per_sm(PAIR, NI, PRO, true) * sm_count())
+            return launch_linear_form<NI, NB, PAIR, PRO, true>(p, l);
+    return launch_linear_form<NI, NB, PAIR, PRO, false>(p, l);
 }
 // The plain forms up to K = 8192 have an instantiation each (see the kernel); longer rows are not launch-bound.
 template <int NI, int NB, bool PAIR>
-static cudaError_t launch_linear_pro(const LinearParams& p, dim3 grid, size_t smem) {
+static cudaError_t launch_linear_pro(const LinearParams& p, RowLaunch& l) {
     if constexpr (NB <= 2) {
         bool plain = p.K % 16 == 0 && !p.trace && !p.xq_out && !p.xscale_out;
         for (int i = 0; i < p.n_seg; ++i) plain = plain && !p.seg[i].acc_out;
         if (plain) switch (p.prologue) {
-            case LSPK_PRO_INT8: return launch_linear<NI, NB, PAIR, LSPK_PRO_INT8>(p, grid, smem);
-            case LSPK_PRO_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_QUANT>(p, grid, smem);
-            case LSPK_PRO_RMSNORM_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_RMSNORM_QUANT>(p, grid, smem);
-            case LSPK_PRO_GATED_RMSNORM_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_GATED_RMSNORM_QUANT>(p, grid, smem);
+            case LSPK_PRO_INT8: return launch_linear<NI, NB, PAIR, LSPK_PRO_INT8>(p, l);
+            case LSPK_PRO_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_QUANT>(p, l);
+            case LSPK_PRO_RMSNORM_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_RMSNORM_QUANT>(p, l);
+            case LSPK_PRO_GATED_RMSNORM_QUANT: return launch_linear<NI, NB, PAIR, LSPK_PRO_GATED_RMSNORM_QUANT>(p, l);
         }
     }
-    return launch_linear<NI, NB, PAIR, kAnyPrologue>(p, grid, smem);
+    return launch_linear<NI, NB, PAIR, kAnyPrologue>(p, l);
 }
-static cudaError_t launch_linear_row(const LinearParams& p, dim3 grid, bool pair, size_t smem) {
+static cudaError_t launch_linear_row(const LinearParams& p, RowLaunch& l, bool pair) {
     if (p.chunks <= 64)
-        return pair ? launch_linear_pro<4, 1, true>(p, grid, smem) : launch_linear_pro<4, 1, false>(p, grid, smem);
+        return pair ? launch_linear_pro<4, 1, true>(p, l) : launch_linear_pro<4, 1, false>(p, l);
     if (p.chunks <= 128)
-        return pair ? launch_linear_pro<8, 2, true>(p, grid, smem) : launch_linear_pro<8, 2, false>(p, grid, smem);
-    return pair ? launch_linear_pro<8, 8, true>(p, grid, smem) : launch_linear_pro<8, 8, false>(p, grid, smem);
+        return pair ? launch_linear_pro<8, 2, true>(p, l) : launch_linear_pro<8, 2, false>(p, l);
+    return pair ? launch_linear_pro<8, 8, true>(p, l) : launch_linear_pro<8, 8, false>(p, l);
 }
 
-int linear_launch_params(const LinearParams& p, int mt, bool pair, int grid_x, int grid_y) {
-    // more than one token row per tile: the eight-row mma kernel
-    if (mt > 1) return linear_mma_launch(p, pair, grid_x, grid_y);
-    const int Kp = p.chunks * kWeightsPerChunk;
-    const size_t smem = linear_smem_bytes(1, Kp, pair);
-    LSPK_REQUIRE(smem <= 200 * 1024 && p.chunks <= 512, "linear: K=%d too large (limit 32768)", p.K);
-    const dim3 grid(grid_x, grid_y);
-    const cudaError_t e = launch_linear_row(p, grid, pair, smem);
+// One row.  resident: see RowLaunch.
+static int linear_row(const LinearParams& p, bool pair, int* ctas = nullptr, int* resident = nullptr) {
+    RowLaunch l = {linear_smem_bytes(1, p.chunks * kWeightsPerChunk, pair), 0, resident};
+    LSPK_REQUIRE(l.smem <= 200 * 1024 && p.chunks <= 512, "linear: K=%d too large (limit 32768)", p.K);
+    const cudaError_t e = launch_linear_row(p, l, pair);
     if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "linear launch failed: %s", cudaGetErrorString(e));
+    if (ctas) *ctas = l.ctas;
     return LSPK_OK;
 }
 
@@ -507,8 +529,8 @@ static int check_linear_args(const lspk_linear_args* a) {
 }
 
 // Host-side validation + launch of the CUDA-core kernel.  Used by lspk_linear and by the
-// forward pass.
-int linear_cuda_core(const lspk_linear_args* a) {
+// forward pass.  resident (one row): see RowLaunch.
+static int linear_rows(const lspk_linear_args* a, int* row_ctas, int* resident) {
     if (int rc = check_linear_args(a)) return rc;
     const bool pair = a->epilogue == LSPK_EPI_RELU2_MUL || a->epilogue == LSPK_EPI_SILU_MUL;
     LinearParams p = {};
@@ -573,20 +595,16 @@ int linear_cuda_core(const lspk_linear_args* a) {
     p.trace = trace_buffer();
     p.trace_cap = trace_capacity();
     p.error_flag = device_wait_flag();
-    const int MT = a->M == 1 ? 1 : 8;
-    // With a single token tile at most two CTAs per SM (the prologue runs once per CTA, which then
-    // loops over its row groups).  With several token tiles the grid's
-    // second dimension already fills the machine.
-    const int tiles = (a->M + MT - 1) / MT;
-    p.stream_weights = tiles == 1 ? 1 : 0;
-    int ctas = groups;
-    // One row of an unpaired product: three, which its registers allow (a hybrid step, whose Mamba input projections have 661 row
-    // groups, 574 -> 560 us).  Not so the pair: with a CTA for each of 432 groups a decode step takes 672 us, with two
-    // CTAs per SM and a loop 667.
-    const int per_wave = tiles == 1 ? (!pair && a->M == 1 ? 3 : 2) * sm_count() : (2 * sm_count() + tiles - 1) / tiles;
-    if (ctas > per_wave) ctas = per_wave > 0 ? per_wave : 1;
-    return linear_launch_params(p, MT, pair, ctas, tiles);
+    p.stream_weights = a->M <= LSPK_MAX_GEMV_M ? 1 : 0;
+    if (a->M == 1) return linear_row(p, pair, row_ctas, resident);
+    LSPK_REQUIRE(!resident, "linear: several rows");
+    // Several rows: the eight-row kernel.  With a single token tile at most two CTAs per SM (each loops over its row groups),
+    // with several the grid's second dimension already fills the machine.
+    const int tiles = (a->M + 7) / 8;
+    const int per_wave = tiles == 1 ? 2 * sm_count() : (2 * sm_count() + tiles - 1) / tiles;
+    return linear_mma_launch(p, pair, groups < per_wave ? groups : per_wave > 0 ? per_wave : 1, tiles);
 }
+int linear_cuda_core(const lspk_linear_args* a) { return linear_rows(a, nullptr, nullptr); }
 
 }  // namespace lspk
 
@@ -620,4 +638,10 @@ extern "C" int lspk_linear(const lspk_linear_args* a) {
         if (g_force_path == 2) return fail(LSPK_ERR_ARG, "lspk_linear: shape not supported by the tensor-core path");
     }
     return linear_cuda_core(a);
+}
+
+extern "C" int lspk_debug_row_launch(const lspk_linear_args* a, int* ctas, int* resident) {
+    if (int rc = ensure_init()) return rc;
+    LSPK_REQUIRE(a && ctas && resident, "lspk_debug_row_launch: null argument");
+    return linear_rows(a, ctas, resident);
 }

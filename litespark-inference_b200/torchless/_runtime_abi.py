@@ -34,6 +34,7 @@ SIGNATURES = {
     "lspk_release_parked_states": ([], _ci),
     "lspk_debug_expire_wait": ([_ci], _ci),
     "lspk_debug_prefill_attention": ([_vp] * 9 + [_ci] * 6, _ci),
+    "lspk_debug_row_launch": ([_vp, _vp, _vp], _ci),
     "lspk_debug_allocation_limit": ([_sz], _ci),
 }
 

@@ -1,6 +1,7 @@
 """The plain forms of the one-row product against the general one (which a call takes when it asks for the accumulators):
 both do the same arithmetic in the same order, so outputs are bit-equal.  Lengths around the edges of a form: one block,
 the last block of a thread's share, 4096 and 8192 where the forms change, and those whose scalar tail has no plain form."""
+import ctypes
 import importlib
 
 import numpy as np
@@ -73,3 +74,25 @@ def test_many_rows_plain_and_general_forms(n, M):
                 assert np.array_equal(a, b, equal_nan=True)
         for w in ws:
             w.free()
+
+
+@pytest.mark.parametrize("n", [64, 2560, 4096, 4112, 6912, 8192, 8208, 12288])
+def test_a_row_launch_is_resident_at_once(n):
+    """One row: more than two CTAs per SM only where the registers of the chosen form let an SM hold them."""
+    lib, sms = K.load_library(True), K.load_library(True).lspk_sm_count()
+    x, q, s = dev.DeviceArray((n,), np.float32), dev.DeviceArray((n,), np.int8), dev.DeviceArray((1,), np.float32)
+    g = dev.DeviceArray((n,), np.uint16)
+    for N in (16, 32 * sms, 32 * sms + 16, 48 * sms, 48 * sms + 16, 80 * sms):
+        w = dev.DeviceWeight(np.full((N, n // 4), 0x55, np.uint8), 1.0)
+        y, acc = dev.DeviceArray((N,), np.float32), dev.DeviceArray((N,), np.int32)
+        for prologue in (K.PRO_INT8, K.PRO_QUANT, K.PRO_RMSNORM_QUANT, K.PRO_GATED_RMSNORM_QUANT):
+            for pair, tap in ((False, False), (False, True), (True, False)):
+                a, ctas, resident = K.LinearArgs(), ctypes.c_int(), ctypes.c_int()
+                a.n_mats, a.M, a.prologue, a.epilogue, a.gamma_is_bf16 = 1 + pair, 1, prologue, K.EPI_SILU_MUL * pair, 1
+                a.x_f32, a.x_i8, a.x_scales, a.gamma, a.gate_f32 = x.ptr, q.ptr, s.ptr, g.ptr, x.ptr
+                a.w[0], a.w[1], a.out[0], a.acc_out[0] = w.handle, w.handle if pair else None, y.ptr, acc.ptr if tap else None
+                K.check(lib.lspk_debug_row_launch(ctypes.byref(a), ctypes.byref(ctas), ctypes.byref(resident)))
+                most = max(2, resident.value) * sms
+                assert resident.value >= 1 and 1 <= ctas.value <= most, (N, prologue, pair, tap)
+                assert ctas.value == N // 16 or ctas.value >= 2 * sms
+        w.free()
