@@ -211,7 +211,7 @@ static void rows_host(const float* x, const void* gamma, int gamma_is_bf16, floa
         void *ho, *hs, *d = g_stage.region(ob, &ho), *ds = g_stage.region((size_t)T * 4, &hs);
         const int rc = mode == 2   ? lspk_quantize_rows(sx, (int8_t*)d, (float*)ds, T, K)
                        : mode == 1 ? lspk_rmsnorm_rows(sx, sg, gamma_is_bf16, (float*)d, T, K, eps)
-                                   : lspk_rmsnorm_quantize_rows(sx, sg, gamma_is_bf16, (int8_t*)d, (float*)ds, T, K, eps);
+                                   : rmsnorm_quantize_rows_in_order(sx, sg, gamma_is_bf16, (int8_t*)d, (float*)ds, T, K, eps);
         if (rc != LSPK_OK || !g_stage.finish()) return;
         // a caller that wants the scales alone passes no int8 rows
         if (!(mode & 2) || out_i8) memcpy((mode & 2) ? (void*)out_i8 : (void*)out_f32, ho, ob);

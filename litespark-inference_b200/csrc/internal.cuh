@@ -58,6 +58,10 @@ int quantize_rows_permuted(const lspk_linear_args* a, int K, int Kp, int8_t* out
 // rows in the eight-row tile's layout, and the sum of each.
 int norm_quant_rows_selected(const float* x, const void* gamma_bf16, const int* gamma_sel, int8_t* out, float* scales,
                              int T, int K, float eps, int* tiled_sums = nullptr);
+// rows.cu: lspk_rmsnorm_quantize_rows for norm weights in memory that is written again from call to call.  The kernel requests
+// the norm weights in front of its dependency wait, so this launch does not overlap the one before it.
+int rmsnorm_quantize_rows_in_order(const float* x, const void* gamma, int gamma_is_bf16, int8_t* out, float* scales, int T,
+                                   int K, float eps);
 int linear_mma_launch(const LinearParams& p, bool pair, int grid_x, int grid_y);
 __host__ __device__ inline int mma_row_stride(int Kp) { return (Kp % 128 == 0) ? Kp + 64 : Kp; }
 

@@ -398,7 +398,8 @@ __global__ void add_kernel(float* __restrict__ a, const float* __restrict__ b, s
 
 static int launch_rows(const float* x, const void* gamma, int gamma_is_bf16, float* out_f32, int8_t* out_i8,
                        float* scales, int T, int K, float eps, int mode, const float* gate = nullptr,
-                       const int* gamma_sel = nullptr, int perm_kp = 0, int perm_stride = 0, int* sums = nullptr) {
+                       const int* gamma_sel = nullptr, int perm_kp = 0, int perm_stride = 0, int* sums = nullptr,
+                       bool early = true) {
     if (int rc = ensure_init()) return rc;
     LSPK_REQUIRE(x && T >= 1 && K >= 1, "row helper: bad arguments (T=%d K=%d)", T, K);
     const size_t smem = (size_t)K * sizeof(float);
@@ -421,13 +422,13 @@ static int launch_rows(const float* x, const void* gamma, int gamma_is_bf16, flo
         const bool plain = (mode & 1) && perm_kp > 0 && K % 16 == 0 && !gate && !gamma_sel;
         auto kern = plain ? one ? row_quant_regs_kernel<1, true> : row_quant_regs_kernel<2, true>
                           : one ? row_quant_regs_kernel<1, false> : row_quant_regs_kernel<2, false>;
-        const cudaError_t e = launch(kern, dim3(T), dim3(kRowThreads), 0, true, x, gate, gamma, gamma_sel, gamma_is_bf16, out_i8,
+        const cudaError_t e = launch(kern, dim3(T), dim3(kRowThreads), 0, early, x, gate, gamma, gamma_sel, gamma_is_bf16, out_i8,
                                      scales, K, eps, rcp_K, mode & 1, perm_kp, pstride, sums);
         if (e != cudaSuccess) return fail(LSPK_ERR_CUDA, "row quantiser launch failed: %s", cudaGetErrorString(e));
         return LSPK_OK;
     }
     LSPK_CUDA(launch(vec ? row_norm_quant_kernel<true> : row_norm_quant_kernel<false>, dim3(T), dim3(kRowThreads), smem,
-                     true, x, gate, gamma, gamma_sel, gamma_is_bf16, out_f32, out_i8, scales, K, eps, mode, vec ? perm_kp : 0,
+                     early, x, gate, gamma, gamma_sel, gamma_is_bf16, out_f32, out_i8, scales, K, eps, mode, vec ? perm_kp : 0,
                      perm_stride > 0 ? perm_stride : perm_kp, sums));
     return LSPK_OK;
 }
@@ -484,6 +485,12 @@ int quantize_rows_permuted(const lspk_linear_args* a, int K, int Kp, int8_t* out
         return rc;
     *done = 1;
     return LSPK_OK;
+}
+
+int rmsnorm_quantize_rows_in_order(const float* x, const void* gamma, int gamma_is_bf16, int8_t* out, float* scales, int T,
+                                   int K, float eps) {
+    LSPK_REQUIRE(gamma && out && scales, "rmsnorm_quantize: null argument");
+    return launch_rows(x, gamma, gamma_is_bf16, nullptr, out, scales, T, K, eps, 3, nullptr, nullptr, 0, 0, nullptr, false);
 }
 
 static int grid_for(size_t n, int block) {

@@ -49,6 +49,28 @@ def test_rows_and_products(port, T, n):
         assert np.array_equal(y, dots.astype(np.float32) * (s * np.float32(0.5))[:, None])
 
 
+@pytest.mark.parametrize("T,n", [(1, 16), (1, 2560), (1, 2562), (1, 8192), (1, 12288), (9, 6912), (10, 6912), (24, 2560), (26, 2560)])
+def test_norms_of_changing_weights(port, T, n):
+    """Calls of one shape one behind the other, each with norm weights (and rows) of its own: all pass through the same buffer.
+    The sum of squares is summed in another order than the oracle's: 2e-6 relative, and an element may round the other way."""
+    lib = K.load_library(True)
+    rng = np.random.default_rng(T + n)
+    o, q, s = np.empty((T, n), np.float32), np.empty((T, n), np.int8), np.empty(T, np.float32)
+    wq, ws, tmp = np.empty_like(q), np.empty_like(s), np.empty_like(o)
+    for i in range(12):
+        x = rng.standard_normal((T, n)).astype(np.float32)
+        g32 = ((1 + i) * rng.uniform(0.5, 1.5, n)).astype(np.float32)
+        g16 = (g32.view(np.uint32) >> 16).astype(np.uint16)
+        lib.rmsnorm_quantize_bf16gamma_batched_sm100(x, g16, q, s, tmp, T, n, 1e-5)
+        port.rmsnorm_quantize_batched(x, g16, wq, ws, tmp, 1e-5)
+        assert np.allclose(s, ws, rtol=2e-6, atol=0) and np.abs(q.astype(np.int32) - wq).max() <= 1
+        for norm, gamma in ((lib.rmsnorm_bf16gamma_fp32_batched_sm100, g16), (lib.rmsnorm_fp32gamma_fp32_batched_sm100, g32)):
+            norm(x, gamma, o, T, n, 1e-5)
+            g = g32 if gamma is g32 else (g16.astype(np.uint32) << 16).view(np.float32)
+            wo = (x / np.sqrt((x.astype(np.float64) ** 2).mean(axis=1, keepdims=True) + 1e-5) * g).astype(np.float32)
+            assert np.allclose(o, wo, rtol=2e-6, atol=0)
+
+
 @pytest.mark.parametrize("T,n", [(1, 2560), (40, 2560)])
 def test_null_outputs(T, n):
     """On either side of the limit: a null fp32 row or null scales are recorded as a failure, null int8 rows are left out."""
