@@ -49,7 +49,10 @@ static bool down(void* dst, const void* src, size_t bytes) {
 // each, whatever their size, and the wait for the stream as much.  So its arguments are copied (by the CPU) into a pinned
 // buffer that the GPU reads over the bus, its results come back the same way, and a last kernel stores the call's number to a
 // word that the host polls: the seven calls of an MLP block of one row take 192 us instead of 291.  Up to kStageBytes each way,
-// larger calls keep the copies.
+// larger calls keep the copies.  At the limit every kind of call is ahead, or level (us, copies and staged): add 66 and 35,
+// quantiser of 25 rows of 2560 63 and 39, their norm 66 and 54, product of 9 such rows with 6912 outputs 54 and 41, norm of one
+// row of 51200 85 and 82.  Without it the copies overtake between 0.6 and 1.3 MB: norm of 64 rows of 2560 113 and 128, product
+// of 64 rows 153 and 168.
 constexpr size_t kStageBytes = 256 * 1024;
 
 __global__ void host_done_kernel(unsigned* flag, unsigned call) {
@@ -63,6 +66,14 @@ __global__ void __launch_bounds__(256) host_fetch_kernel(const uint4* __restrict
     grid_dependency_wait();
     for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) dst[i] = src[i];
 }
+
+// Row calls: from so many rows on the norm weights go to device memory first, one launch more.  Read by every row over the bus
+// they cost more than the copies would: 256 rows of 64, norm and quantiser 59 us that way, 50 with copies, 32 so; at 16 rows
+// of 64 ... 2560 23.4 and 37.0 straight from the bus, 24.6 and 39.0 so, level at 24.
+constexpr int kFetchRows = 24;
+// Rows so many that they are as short as a bus access take the copies (16000 rows of one element: 65 us, staged 82; 4096 rows of
+// 4, normed: 41 and 38).
+constexpr int kStageRows = 4096;
 
 struct HostStage {
     static constexpr size_t kHead = 256;      // the polled word
@@ -101,6 +112,16 @@ struct HostStage {
         void *h, *d = region(bytes, &h);
         memcpy(h, src, bytes);
         return d;
+    }
+    // The same into device memory (`dst`, room for `bytes` rounded up to 16): what a kernel reads more than once.
+    const void* fetch(const void* src, size_t bytes, void* dst) {
+        if (!dst) return nullptr;
+        const uint4* d = (const uint4*)put(src, bytes);
+        const int n = (int)((bytes + 15) / 16);
+        const cudaError_t e = launch(host_fetch_kernel, dim3((n + 255) / 256), dim3(256), 0, true, d, (uint4*)dst, n);
+        if (e == cudaSuccess) return dst;
+        fail(LSPK_ERR_CUDA, "host call: launch failed: %s", cudaGetErrorString(e));
+        return nullptr;
     }
     // Waits for the kernels enqueued since begin().
     bool finish() {
@@ -156,7 +177,7 @@ static void matmul_host(const int8_t* x, const float* x_scales, const uint8_t* p
     if (!w) return;
     reinterpret_cast<Weight*>(w)->scale = w_scale;
     const size_t xb = ((size_t)T * K + 15) / 16 * 16, sb = ((size_t)T * 4 + 15) / 16 * 16, yb = (size_t)T * N * 4;
-    const bool staged = g_stage.begin(xb + sb, yb);
+    const bool staged = T <= kStageRows && g_stage.begin(xb + sb, yb);
     int8_t* dx = (int8_t*)slot(S_X, staged ? xb + sb : (size_t)T * K);
     float* dxs = staged ? (float*)(dx + xb) : (float*)slot(S_XS, (size_t)T * 4);
     float* dy = staged ? nullptr : (float*)slot(S_Y, yb);
@@ -204,10 +225,12 @@ static void rows_host(const float* x, const void* gamma, int gamma_is_bf16, floa
     if (!x || T < 1 || K < 1) { fail(LSPK_ERR_ARG, "row helper: bad arguments (T=%d K=%d)", T, K); return; }
     if ((mode & 2) ? !scales : !out_f32) { fail(LSPK_ERR_ARG, "row helper: null output"); return; }
     const size_t n = (size_t)T * K, gb = gamma ? (size_t)K * (gamma_is_bf16 ? 2 : 4) : 0, ob = (mode & 2) ? n : n * 4;
-    if (g_stage.begin(n * 4 + gb, ob + (size_t)T * 4)) {
-        // every element is read once and written once, by a CTA per row: straight from and to the host's memory
+    if (T <= kStageRows && g_stage.begin(n * 4 + gb, ob + (size_t)T * 4)) {
+        // the rows are read once and written once: straight from and to the host's memory.  So are the norm weights of a few
+        // rows; of more, every row would bring them over the bus again.
         const float* sx = (const float*)g_stage.put(x, n * 4);
-        const void* sg = gamma ? g_stage.put(gamma, gb) : nullptr;
+        const void* sg = nullptr;
+        if (gamma && !(sg = T < kFetchRows ? g_stage.put(gamma, gb) : g_stage.fetch(gamma, gb, slot(S_G, gb + 16)))) return;
         void *ho, *hs, *d = g_stage.region(ob, &ho), *ds = g_stage.region((size_t)T * 4, &hs);
         const int rc = mode == 2   ? lspk_quantize_rows(sx, (int8_t*)d, (float*)ds, T, K)
                        : mode == 1 ? lspk_rmsnorm_rows(sx, sg, gamma_is_bf16, (float*)d, T, K, eps)

@@ -49,7 +49,8 @@ def test_rows_and_products(port, T, n):
         assert np.array_equal(y, dots.astype(np.float32) * (s * np.float32(0.5))[:, None])
 
 
-@pytest.mark.parametrize("T,n", [(1, 16), (1, 2560), (1, 2562), (1, 8192), (1, 12288), (9, 6912), (10, 6912), (24, 2560), (26, 2560)])
+@pytest.mark.parametrize("T,n", [(1, 16), (1, 2560), (1, 2562), (1, 8192), (1, 12288), (9, 6912), (10, 6912), (23, 2560), (24, 2560), (26, 2560),
+                                 (24, 2562), (30, 2048), (512, 64), (4096, 4), (4097, 4)])
 def test_norms_of_changing_weights(port, T, n):
     """Calls of one shape one behind the other, each with norm weights (and rows) of its own: all pass through the same buffer.
     The sum of squares is summed in another order than the oracle's: 2e-6 relative, and an element may round the other way."""
