@@ -268,23 +268,21 @@ ternary_linear_kernel(const __grid_constant__ LinearParams p) {
                     const int k0 = b * 16;
                     if (k0 < Kp) {
                         // |v * inv| <= 127 by construction of inv, so the saturation of the reference's
-                        // conversion never acts and round-to-nearest-even can be taken from the adder:
-                        // v + 1.5 * 2^23 leaves the integer in the low mantissa byte.  The words are
-                        // packed directly in the transposed order the dot products read.
+                        // conversion never acts and round-to-nearest-even can be taken from the adder
+                        // (round_to_byte).  The words are packed directly in the transposed order the dot
+                        // products read.
                         uint32_t t[16];
 #pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            t[e] = __float_as_uint(__fadd_rn(__fmul_rn(v[nb][e], inv), 12582912.0f));
+                        for (int e = 0; e < 16; ++e) t[e] = round_to_byte(__fmul_rn(v[nb][e], inv));
                         if (!kPlain && k0 + 16 > tail_start) {
                             // block past the last multiple of 16: the reference's scalar tail rounds halves
                             // away from zero.  The rest of the nearest-even form is exact, so a half that went
-                            // towards zero is told by it; a NaN becomes 0.  Zeros beyond K.
+                            // towards zero is told by it.  Zeros beyond K.
 #pragma unroll
                             for (int e = 0; e < 16; ++e) {
                                 const float x = __fmul_rn(v[nb][e], inv);
-                                const float rest = __fsub_rn(x, __fsub_rn(__uint_as_float(t[e]), 12582912.0f));
+                                const float rest = __fsub_rn(x, (float)(int)(t[e] - kRoundedZero));
                                 if (rest == copysignf(0.5f, x)) t[e] += rest > 0.0f ? 1u : 0xffffffffu;
-                                if (x != x) t[e] = 0u;
                             }
                         }
                         const uint32_t o0 = pack4_bytes(t[0], t[4], t[8], t[12]), o1 = pack4_bytes(t[1], t[5], t[9], t[13]);

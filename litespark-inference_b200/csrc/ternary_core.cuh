@@ -15,6 +15,16 @@ __device__ __forceinline__ void transpose4x4_bytes(uint32_t a0, uint32_t a1, uin
     o3 = __byte_perm(t2, t3, 0x7632);
 }
 
+// x to the nearest integer, halves to even, |x| <= 127, in the low byte of the result; 0 for what is not a number.  Between 0.5
+// and 1 floats are 2^-24 apart, so x * 2^-24 + 0.75, rounded once (the product is exact), is 0.75 with the integer added to its
+// bits; saturation to [0, 1] takes a NaN to 0.
+constexpr uint32_t kRoundedZero = 0x3f400000u;
+__device__ __forceinline__ uint32_t round_to_byte(float x) {
+    float t;
+    asm("fma.rn.sat.f32 %0, %1, 0f33800000, 0f3F400000;" : "=f"(t) : "f"(x));
+    return __float_as_uint(t);
+}
+
 // Weight loads.  Weights that a launch reads once are marked evict-first in L2, so that the KV cache, the activations and the
 // norm weights stay resident from token to token; as a policy of one load instruction, not as two sets of loads.
 __device__ __forceinline__ uint64_t weight_policy(int read_once) {

@@ -84,3 +84,42 @@ def test_rows_that_are_not_finite(port, n):
     ws = port.quantize_activation(clean, want)
     assert s[1] == np.float32(ws) and np.array_equal(q[1], want)
     assert not q[2].any() and s[2] == np.float32(np.float32(1e-5) / np.float32(127.0))
+
+
+@pytest.mark.parametrize("M", [1, 2, 9])
+@pytest.mark.parametrize("n", [60, 64, 2560, 2564, 6912, 6916, 8256])
+def test_products_of_rows_that_are_not_finite(port, n, M):
+    """The same through the products, whose kernels quantise on their own: with and without taps (a form of its own each), with
+    and without a norm.  Every row of a call is the same, so one row and several agree.  The elements that are not a number lie
+    in a whole block of 16 and in the last, shorter one."""
+    rng = np.random.default_rng(n)
+    codes = rng.integers(0, 3, (40, n // 4, 4)).astype(np.uint8)
+    w = dev.DeviceWeight(codes[..., 0] | codes[..., 1] << 2 | codes[..., 2] << 4 | codes[..., 3] << 6, 1.0)
+    plain = codes.reshape(40, n).astype(np.int64) - 1
+    g = np.ones(n, np.float32)
+    g[[7, n - 2]] = np.nan                       # behind a norm: of the weights, since one in the row makes all of it so
+    for bad, norm in ((np.nan, False), (np.inf, False), (np.nan, True)):
+        row = rng.standard_normal(n).astype(np.float32)
+        if not norm:
+            row[[7, n // 2, n - 2]] = bad, -bad, bad
+        kw = {"x_f32": dev.DeviceArray.from_numpy(np.tile(row, (M, 1)))}
+        if norm:
+            kw["gamma"] = dev.DeviceArray.from_numpy(g)
+        y, y_plain, acc = dev.DeviceArray((M, 40), np.float32), dev.DeviceArray((M, 40), np.float32), dev.DeviceArray((M, 40), np.int32)
+        q, s = dev.DeviceArray((M, n), np.int8), dev.DeviceArray((M,), np.float32)
+        dev.linear([w], [y], M, acc_outs=[acc], xq_out=q, xscale_out=s, **kw)
+        dev.linear([w], [y_plain], M, **kw)
+        clean = row if not norm else (row / np.sqrt((row.astype(np.float64) ** 2).mean() + 1e-5)).astype(np.float32)
+        clean = np.where(np.isfinite(clean * g if norm else clean), clean, np.float32(0))
+        want = np.zeros(n, np.int8)
+        ws = np.float32(np.inf) if bad == np.inf else np.float32(port.quantize_activation(clean, want))
+        if bad == np.inf:
+            want[:] = 0
+        assert np.allclose(s.numpy(), ws, rtol=2e-6, atol=0)
+        assert np.abs(q.numpy().astype(int) - want).max() <= (1 if norm else 0) and not q.numpy()[:, ~np.isfinite(g if norm else row)].any()
+        sums = q.numpy().astype(np.int64) @ plain.T
+        assert np.array_equal(acc.numpy(), sums)
+        with np.errstate(invalid="ignore"):
+            out = sums.astype(np.float32) * s.numpy()[:, None]
+        assert np.array_equal(y.numpy(), out, equal_nan=True) and np.array_equal(y_plain.numpy(), out, equal_nan=True)
+    w.free()
