@@ -92,8 +92,8 @@ int lspk_state_step_kernel_count(lspk_state_t s);
  * returns LSPK_ERR_DEVICE_WAIT once and clears it.  Nothing faults and the context stays usable. */
 int lspk_debug_expire_wait(int polls);
 
-/* Test aid for running out of memory: device allocations of more than `bytes` made by the library fail from here on as if
- * the GPU had none left (0: back to normal). */
+/* Test aid for running out of memory: device and pinned allocations of more than `bytes` made by the library fail from here on
+ * as if there was none left (0: back to normal). */
 int lspk_debug_allocation_limit(size_t bytes);
 
 /* Test aid: the launch that a one-row lspk_linear(a) would make, which is not made: its CTAs, and how many of them an SM can

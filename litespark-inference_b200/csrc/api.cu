@@ -62,7 +62,7 @@ static int* g_wait_flag = nullptr;
 int* device_wait_flag() { return g_wait_flag; }
 int bound_device() { return g_device; }
 
-static size_t g_alloc_limit = 0;                    // test aid: device allocations above it fail (0: none do)
+static size_t g_alloc_limit = 0;                    // test aid: allocations above it fail (0: none do)
 
 cudaError_t device_malloc(void** p, size_t bytes) {
     auto attempt = [&]() { return g_alloc_limit && bytes > g_alloc_limit ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes); };
@@ -75,10 +75,11 @@ cudaError_t device_malloc(void** p, size_t bytes) {
 }
 
 cudaError_t pinned_malloc(void** p, size_t bytes) {
-    cudaError_t e = cudaMallocHost(p, bytes);
+    auto attempt = [&]() { return g_alloc_limit && bytes > g_alloc_limit ? cudaErrorMemoryAllocation : cudaMallocHost(p, bytes); };
+    cudaError_t e = attempt();
     if (e == cudaErrorMemoryAllocation && release_parked_states()) {
         cudaGetLastError();
-        e = cudaMallocHost(p, bytes);
+        e = attempt();
     }
     return e;
 }

@@ -81,18 +81,15 @@ struct HostStage {
     unsigned char *host = nullptr, *dev = nullptr;
     size_t used = 0;
     unsigned call = 0;
-    bool failed = false;
     // Starts a call that moves so many bytes; false: it takes the copies.
     bool begin(size_t in_bytes, size_t out_bytes) {
-        if (failed || in_bytes > kStageBytes || out_bytes > kStageBytes) return false;
+        if (in_bytes > kStageBytes || out_bytes > kStageBytes) return false;
         if (!host) {
             void *h = nullptr, *d = nullptr;
-            if (cudaHostAlloc(&h, kHead + 2 * kStageBytes + kSlack, cudaHostAllocMapped) != cudaSuccess ||
-                cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
+            if (pinned_malloc(&h, kHead + 2 * kStageBytes + kSlack) != cudaSuccess || cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
                 cudaGetLastError();
                 if (h) cudaFreeHost(h);
-                failed = true;
-                return false;
+                return false;         // the next call tries again
             }
             memset(h, 0, kHead);
             host = static_cast<unsigned char*>(h);

@@ -172,6 +172,46 @@ def test_memory_of_parked_states_is_bounded_and_given_back():
     _in_own_process(_GIVEN_BACK)
 
 
+_NO_PINNED = """
+import ctypes, importlib
+import numpy as np
+import __graft_entry__ as entry
+entry.load_package()
+name = "litespark_inference_b200.torchless."
+K, rt, synthetic = (importlib.import_module(name + n) for n in ("kernel", "runtime", "synthetic"))
+dm = rt.DeviceModel(synthetic.random_model(synthetic.toy_config(), seed=3))
+lib = dm.lib
+
+def free_bytes():
+    f = ctypes.c_size_t()
+    K.check(lib.lspk_mem_info(ctypes.byref(f), None))
+    return f.value
+
+st = rt.init_state(dm, t_max=8192, batch=24, kv_dtype="fp32")
+size = st.device_bytes
+rt.forward_step(st, np.arange(24, dtype=np.int32))
+st.close()                                                   # parked
+a, b = np.ones(2560, np.float32), np.full(2560, 2, np.float32)
+K.check(lib.lspk_debug_allocation_limit(1000))               # neither a pinned buffer nor device scratch
+before = free_bytes()
+lib.lspk_clear_error()
+lib.add_inplace_fp32_sm100(a, b, a.size)
+assert lib.lspk_error_count() >= 1 and (a == 1).all()
+assert free_bytes() - before > 0.9 * size                    # parked memory was given back before it failed
+K.check(lib.lspk_debug_allocation_limit(0))
+lib.lspk_clear_error()
+lib.add_inplace_fp32_sm100(a, b, a.size)                     # pinned memory is asked for again: no device scratch was made
+before = free_bytes()
+K.check(lib.lspk_debug_allocation_limit(1000))
+lib.relu2_mul_fp32_batched_sm100(a, b, b, 1, a.size)
+assert lib.lspk_error_count() == 0 and (a == 3).all() and (b == 18).all() and free_bytes() == before
+"""
+
+
+def test_small_host_calls_without_pinned_memory():
+    _in_own_process(_NO_PINNED)
+
+
 _SCRATCH_LOST = """
 import ctypes, importlib
 import numpy as np
