@@ -1,6 +1,7 @@
-"""The plain forms of the one-row product against the general one (which a call takes when it asks for the accumulators):
-both do the same arithmetic in the same order, so outputs are bit-equal.  Lengths around the edges of a form: one block,
-the last block of a thread's share, 4096 and 8192 where the forms change, and those whose scalar tail has no plain form."""
+"""The plain forms of the products against the general one (which a call takes when it asks for the accumulators): both do the
+same arithmetic in the same order, so outputs are bit-equal.  Lengths around the edges of a form: one block, the last block
+of a thread's share, 4096 and 8192 where the forms change, and those whose scalar tail has no plain form.  Sizes on either
+side of the grid: a CTA per row group (forms without the loop), and more row groups than CTAs by the number of SMs."""
 import ctypes
 import importlib
 
@@ -14,37 +15,55 @@ K = importlib.import_module("litespark_inference_b200.torchless.kernel")
 synthetic = importlib.import_module("litespark_inference_b200.torchless.synthetic")
 
 
+_TRITS = np.array([a | b << 2 | c << 4 | d << 6 for a in range(3) for b in range(3) for c in range(3) for d in range(3)], np.uint8)
+
+
 def _weight(rng, N, n):
-    codes = rng.integers(0, 3, (N, n // 4, 4)).astype(np.uint8)
-    return dev.DeviceWeight(codes[..., 0] | codes[..., 1] << 2 | codes[..., 2] << 4 | codes[..., 3] << 6, float(rng.uniform(0.5, 2)))
+    return dev.DeviceWeight(_TRITS[rng.integers(0, 81, (N, n // 4), dtype=np.uint8)], float(rng.uniform(0.5, 2)))
+
+
+def _dots(q, w):
+    """Products of int8 rows and a weight's trits; below 2^24, so exact in fp32 in any order."""
+    packed = w.download()
+    trits = np.stack([(packed >> s & 3) for s in (0, 2, 4, 6)], axis=2).reshape(w.N, w.K).astype(np.float32) - 1
+    return q.astype(np.float32) @ trits.T
 
 
 @pytest.mark.parametrize("n", [16, 64, 1008, 2560, 4080, 4096, 4112, 6912, 8176, 8192, 8208, 20, 4100])
 @pytest.mark.parametrize("prologue", ["int8", "quant", "norm bf16", "norm fp32", "gated"])
-def test_plain_forms_equal_the_general_one(n, prologue):
+def test_plain_forms_equal_the_general_one(port, n, prologue):
     rng = np.random.default_rng(n)
     x = dev.DeviceArray.from_numpy((rng.standard_normal(n) * 3).astype(np.float32))
     g = (1.0 + 0.2 * rng.standard_normal(n)).astype(np.float32)
     kw = {"x_f32": x}
+    q, s = np.empty(n, np.int8), np.float32(0.013)
     if prologue == "int8":
-        kw = {"x_i8": dev.DeviceArray.from_numpy(rng.integers(-127, 128, n).astype(np.int8)),
-              "x_scales": dev.DeviceArray.from_numpy(np.float32([0.013]))}
+        q[:] = rng.integers(-127, 128, n)
+        kw = {"x_i8": dev.DeviceArray.from_numpy(q), "x_scales": dev.DeviceArray.from_numpy(np.float32([s]))}
+    elif prologue == "quant":
+        s = np.float32(port.quantize_activation(x.numpy(), q))
     elif prologue != "quant":
         kw["gamma"] = dev.DeviceArray.from_numpy(g if prologue == "norm fp32" else synthetic.fp32_to_bf16_u16(g))
         if prologue == "gated":
             kw["gate_f32"] = dev.DeviceArray.from_numpy(rng.standard_normal(n).astype(np.float32))
-    sizes = {"store": (5000, 16, 40), "add": (4760,), "relu2": (4776, 4776), "silu": (40, 40)}
-    for name, epilogue in (("store", K.EPI_STORE), ("add", K.EPI_ADD), ("relu2", K.EPI_RELU2_MUL), ("silu", K.EPI_SILU_MUL)):
-        ws = [_weight(rng, N, n) for N in sizes[name]]
-        start = [rng.standard_normal(N).astype(np.float32) for N in sizes[name]]
+    sms = K.load_library(True).lspk_sm_count()       # at most three CTAs per SM take a row group of 16 each, of a pair two
+    for sizes, epilogue in (((5000, 16, 40), K.EPI_STORE), ((48 * sms + 8, 16, 40), K.EPI_STORE), ((4760,), K.EPI_ADD),
+                            ((48 * sms + 24,), K.EPI_ADD), ((32 * sms + 24,) * 2, K.EPI_RELU2_MUL), ((40, 40), K.EPI_RELU2_MUL),
+                            ((40, 40), K.EPI_SILU_MUL)):
+        ws = [_weight(rng, N, n) for N in sizes]
+        start = [rng.standard_normal(N).astype(np.float32) for N in sizes]
         got = []
         for taps in (False, True):
             outs = [dev.DeviceArray.from_numpy(s) for s in start]
-            accs = [dev.DeviceArray((N,), np.int32) for N in sizes[name]] if taps else []
+            accs = [dev.DeviceArray((N,), np.int32) for N in sizes] if taps else []
             dev.linear(ws, outs, 1, epilogue=epilogue, acc_outs=accs, **kw)
             got.append([o.numpy() for o in outs])
         for plain, general in zip(*got):
             assert np.array_equal(plain, general, equal_nan=True)
+        if prologue in ("int8", "quant") and epilogue in (K.EPI_STORE, K.EPI_ADD):      # the same roundings in the same order
+            for y, w, v in zip(got[0], ws, start):
+                want = _dots(q, w) * (s * np.float32(w.scale))
+                assert np.array_equal(y, want if epilogue == K.EPI_STORE else v + want)
         for w in ws:
             w.free()
 
@@ -53,13 +72,17 @@ def test_plain_forms_equal_the_general_one(n, prologue):
 @pytest.mark.parametrize("n", [16, 64, 2560, 4096, 4112, 6912, 8192, 4100])
 def test_many_rows_plain_and_general_forms(n, M):
     """Rows normalised and quantised on the way into a product, without accumulators (plain forms of the row quantiser and
-    of the product) and with them, and as int8 rows from the quantiser's natural order: one result, bit for bit."""
+    of the product) and with them, and as int8 rows from the quantiser's natural order: one result, bit for bit, that of
+    the int8 rows."""
     rng = np.random.default_rng(n + M)
     x = dev.DeviceArray.from_numpy((rng.standard_normal((M, n)) * 3).astype(np.float32))
     gamma = dev.DeviceArray.from_numpy(synthetic.fp32_to_bf16_u16((1.0 + 0.2 * rng.standard_normal(n)).astype(np.float32)))
     q, s = dev.DeviceArray((M, n), np.int8), dev.DeviceArray((M,), np.float32)
     K.check(K.load_library().lspk_rmsnorm_quantize_rows(x.ptr, gamma.ptr, 1, q.ptr, s.ptr, M, n, 1e-5))
-    for sizes, epilogue in (((200, 16, 40), K.EPI_STORE), ((200,), K.EPI_ADD), ((200, 200), K.EPI_RELU2_MUL), ((40, 40), K.EPI_SILU_MUL)):
+    many = 32 * K.load_library(True).lspk_sm_count() + 24       # more row groups than the eight-row kernel has CTAs
+    wide = [((many, 16, 40), K.EPI_STORE), ((many,), K.EPI_ADD), ((many, many), K.EPI_RELU2_MUL)] if M <= 9 else []
+    for sizes, epilogue in [((200, 16, 40), K.EPI_STORE), ((200,), K.EPI_ADD), ((200, 200), K.EPI_RELU2_MUL),
+                            ((40, 40), K.EPI_SILU_MUL)] + wide:
         ws = [_weight(rng, N, n) for N in sizes]
         start = [rng.standard_normal((M, N)).astype(np.float32) for N in sizes]
         got = []
@@ -72,6 +95,9 @@ def test_many_rows_plain_and_general_forms(n, M):
         for other in got[1:]:
             for a, b in zip(got[0], other):
                 assert np.array_equal(a, b, equal_nan=True)
+        if epilogue == K.EPI_STORE:
+            for y, w in zip(got[0], ws):
+                assert np.array_equal(y, _dots(q.numpy(), w) * (s.numpy() * np.float32(w.scale))[:, None])
         for w in ws:
             w.free()
 

@@ -45,6 +45,66 @@ def test_gemm_tiles_bit_exact(M, N, Kd, epilogue):
     assert np.array_equal(out.numpy(), want)      # the same roundings in the same order
 
 
+# Every (columns, split) that the plan takes for the products of a 2560 / 6912 layer between 9 and 1531 rows on 148 SMs, named
+# beside it, and the splits of a pair that small matrices take: the plain form of each, which a call without accumulators
+# takes, against the general one and the exact sums (below 2^24, so fp32 holds them in any order of summation).
+@pytest.mark.parametrize("pair,sizes,Kd,M", [
+    (False, (2560, 640, 640), 2560, 9),       # 32 x 4
+    (False, (2560, 640, 640), 2560, 65),      # 64 x 4
+    (False, (2560, 640, 640), 2560, 129),     # 64 x 2
+    (False, (2560, 640, 640), 2560, 257),     # 32 x 1
+    (False, (2560, 640, 640), 2560, 289),     # 96 x 1
+    (False, (2560, 640, 640), 2560, 385),     # 64 x 1
+    (False, (2560,), 6912, 193),              # 32 x 2
+    (False, (2560,), 6912, 225),              # 96 x 2
+    (False, (2560,), 6912, 289),              # 64 x 2
+    (False, (2560,), 6912, 673),              # 128 x 1
+    (False, (2560,), 6912, 1531),             # 128 x 1, the last tile in part
+    (True, (6912, 6912), 2560, 9),           # 32 x 2
+    (True, (6912, 6912), 2560, 33),          # 64 x 2
+    (True, (6912, 6912), 2560, 65),          # 64 x 1
+    (True, (6912, 6912), 2560, 129),         # 96 x 1
+    (True, (6912, 6912), 2560, 193),         # 128 x 1
+    (True, (6912, 6912), 2560, 512),         # 128 x 1
+    (True, (1000, 1000), 2560, 100),         # 32 x 4
+    (True, (1000, 1000), 2560, 129),         # 64 x 4
+])
+def test_gemm_plans_without_taps(pair, sizes, Kd, M):
+    rng = np.random.default_rng(M + Kd)
+    xq, xs = rng.integers(-127, 128, (M, Kd), dtype=np.int8), rng.uniform(0.01, 0.02, M).astype(np.float32)
+    scales = [np.float32(0.75), np.float32(1.25), np.float32(0.5)][:len(sizes)]
+    w = [rng.integers(-1, 2, (N, Kd), dtype=np.int8) for N in sizes]
+    y = [(xq.astype(np.float32) @ a.T.astype(np.float32)) * (xs * s)[:, None] for a, s in zip(w, scales)]
+    W = [dev.DeviceWeight(pack.pack_ternary_4_per_byte(a), float(s)) for a, s in zip(w, scales)]
+    dx, ds = dev.DeviceArray.from_numpy(xq), dev.DeviceArray.from_numpy(xs)
+    start = [rng.standard_normal((M, N)).astype(np.float32) for N in sizes]
+    lib = K.load_library()
+    for epilogue in (K.EPI_RELU2_MUL, K.EPI_SILU_MUL) if pair else (K.EPI_STORE, K.EPI_ADD):
+        got = []
+        for taps in (False, True):
+            outs = [dev.DeviceArray.from_numpy(v) for v in (start[:1] if pair else start)]
+            accs = [dev.DeviceArray((M, N), np.int32) for N in sizes] if taps else []
+            try:
+                K.check(lib.lspk_linear_force_path(2))
+                dev.linear(W, [*outs, None][:len(W)], M, x_i8=dx, x_scales=ds, epilogue=epilogue, acc_outs=accs)
+                K.check(lib.lspk_tc_check_error())
+            finally:
+                lib.lspk_linear_force_path(0)
+            got.append([o.numpy() for o in outs])
+        for plain, general in zip(*got):
+            assert np.array_equal(plain, general)
+        if epilogue == K.EPI_SILU_MUL:      # the exponential's error against the processor's: a few units in the last place
+            with np.errstate(over="ignore"):
+                assert np.allclose(got[0][0], y[0] / (1 + np.exp(-y[0])) * y[1], rtol=1e-5, atol=1e-6)
+        elif pair:
+            assert np.array_equal(got[0][0], np.maximum(y[0], 0) ** 2 * y[1])
+        else:
+            for a, b, v in zip(got[0], y, start):
+                assert np.array_equal(a, b if epilogue == K.EPI_STORE else v + b)
+    for x in W:
+        x.free()
+
+
 @pytest.mark.parametrize("M", [8, 9, 16, 17, 24])
 @pytest.mark.parametrize("Kd", [4, 68, 2560, 4100])          # rows of one word, off the 16-element block, of several trips
 def test_int8_rows_on_either_side_of_the_choice_of_a_kernel(M, Kd):
