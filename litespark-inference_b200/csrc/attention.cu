@@ -1155,21 +1155,24 @@ static size_t attention_group_smem(int D, int t_max, int kv_bytes) {
 
 // When the grouped form pays, by the positions a step attends to (not by the room in the cache: a serving state has a long
 // one and mostly short contexts).  It halves the reads of the cache and takes half the CTAs, of the 256-thread kind.  Measured
-// at 20 / 5 heads of 128, ms per step of the whole decoder, other kernel -> this one:
-//   2 sequences, fp16   1.261 -> 1.237 at 30 keys each, 1.388 -> 1.246 at 1000; fp32 1.168 -> 1.202 at 30, 1.214 -> 1.202 at 300
-//   3                   1.297 -> 1.245 and 1.264 -> 1.208 at 30 keys: always (the other kernel's 480 CTAs are 1.1 waves)
-//   8, fp16             1.245 -> 1.492 at 200 keys, 1.455 -> 1.521 at 700, 1.578 -> 1.546 at 1000, 2.034 -> 1.833 at 2000
-//   8, fp32             1.297 -> 1.404 at 200, 1.393 -> 1.407 at 300, 1.487 -> 1.414 at 400, 2.747 -> 2.126 at 2000
-//   8, one of them long, the others 20 keys: fp16 1.278 -> 1.479 at 1000, 1.508 -> 1.485 at 2000; fp32 1.456 -> 1.389 at 1000
-// The middle between the longest and the mean sequence orders both kinds of batch; with the lines below no batch of 2 to
-// 32 sequences up to 4000 keys is more than 6 % behind the better kernel (by the room in the cache: 40 %).
+// at 20 / 5 heads of 128, ms per step of the whole decoder, other kernel and this one:
+//   2 sequences, fp16   0.985 and 1.048 at 30 keys each, 1.054 and 1.070 at 1000, 1.171 and 1.169 at 2000, 1.398 and 1.364 at 4000
+//                fp32   0.981 and 1.026 at 200, 1.028 and 1.023 at 300, 1.145 and 1.118 at 1000
+//   3                   1.075 and 1.072 at 30 keys, 1.227 and 1.095 at 1000: always (the other kernel's 480 CTAs are 1.1 waves)
+//   8, fp16             1.059 and 1.305 at 200 keys, 1.274 and 1.338 at 700, 1.360 and 1.345 at 800, 1.815 and 1.630 at 2000
+//      fp32             1.106 and 1.214 at 200, 1.215 and 1.225 at 300, 1.296 and 1.225 at 400, 2.514 and 1.914 at 2000
+//   8, one of them long, the others 20 keys: fp16 1.277 and 1.312 at 2000; fp32 1.213 and 1.228 at 800, 1.601 and 1.268 at 2000
+//   32, the same        fp16 2.241 and 2.981 at 4000; fp32 1.977 and 2.629 at 1000, 2.968 and 2.771 at 4000
+// The other kernel's time follows the longest sequence while few are long, and their sum once they fill the machine: the mean
+// sequence, and of what the longest has beyond it the share 2 / T, orders both kinds of batch.  With the lines below no batch
+// measured (2 to 32 sequences, 30 to 4000 keys, even ones and one long among short) is more than 4.2 % behind the better
+// kernel; with the middle between longest and mean sequence it was 33 %.
 bool attention_group_heads(int T, int Q, int KV, int D, int t_max, int kv_is_fp16, long long longest, long long total) {
     if (T < 2 || Q % KV || (Q / KV) % 2 || (D != 64 && D != 128) || attention_group_smem(D, t_max, kv_is_fp16 ? 2 : 4) > 200 * 1024)
         return false;
-    const long long depth = (longest + total / T) / 2;
     if (T == 3) return true;
-    if (T == 2) return kv_is_fp16 || depth >= 275;
-    return depth >= (kv_is_fp16 ? 900 : 275);
+    const long long mean = total / T, depth = mean + 2 * (longest - mean) / T;
+    return depth >= (!kv_is_fp16 ? 300 : T == 2 ? 2000 : 768);
 }
 
 // The phase marks are in instantiations of their own, for a launch with a trace: without them the cluster-split kernel is a tenth

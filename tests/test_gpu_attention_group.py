@@ -48,9 +48,11 @@ def test_grouped_heads_equal_single_sequence(heads, kv_heads, head_dim, lens, t_
 
 
 @pytest.mark.parametrize("kv,lens,t_max", [
-    ("fp32", (270, 268, 271, 266), 2048),            # in the middle of the steps below the two forms change
-    ("fp16", (896, 890, 893, 898, 881), 1000),
-    ("fp32", (100, 440), 500),                       # two sequences, uneven
+    ("fp32", (295, 293, 296, 291), 2048),            # in the middle of the steps below the two forms change
+    ("fp16", (760, 754, 757, 762, 745), 1000),
+    ("fp32", (20, 20, 20, 20, 20, 20, 20, 818), 900),   # one long among short
+    ("fp32", (100, 294), 500),                       # two sequences, uneven
+    ("fp16", (1994, 40), 2100),
     ("fp16", (5, 9), 4000),                          # a long cache with short sequences
 ])
 def test_steps_across_the_change_of_form(kv, lens, t_max):
