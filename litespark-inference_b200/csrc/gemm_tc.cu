@@ -702,15 +702,11 @@ static cudaError_t launch_tc(const CUtensorMap* mw, const CUtensorMap& mx, const
                       : launch_tc_form<PAIR, TN, kTcPlain | kTcWhole>(mw, mx, p, grid);
 }
 
-// Token rows per tile and K split of a launch: the plan with the smallest time by a model of a CTA's life in SM cycles:
+// Token rows per tile and K split of a launch: the plan with the smallest time by a model of a CTA's life in SM cycles,
+// fitted to measured launches (q/k/v, o, gate/up and down of a 2560 / 6912 layer at 32 ... 1531 rows, every plan; the
+// pick is within 7 % of the best measured plan at each, on the best one at 17 of 24):
 //   a K block takes the MMA issue and execution time of the CTAs that share the SM, but not less than one turn of the
-//   pipeline (700 cycles); start-up, first copies and epilogue are paid per round of CTAs, a K split pays its exchange with
-//   every other CTA of the cluster.
-// Fitted to measured launches (int8 rows; q/k/v, o, gate/up and down of a 2560 / 6912 layer, 18 row counts from 9 to 1531,
-// every plan) and tried on 15 row counts between them: there the pick is the best measured plan at 48 of 60, 1.2 % behind
-// it in the mean and 15 % at worst (20 % of all: o at 400 rows).  The constants of the kernel with taps and both gates,
-// 970 cycles a turn and 6200 of start-up, were 5.0 % and 29 % behind there, at worst 40 % (down at 1280 rows: 35.1 us
-// with a split, 25.1 without).
+//   pipeline; start-up, first copies and epilogue are paid per round of CTAs, a K split pays its exchange.
 // Small M therefore takes many narrow tiles and K ranges (all SMs, short chains), large M the widest tiles.
 struct TcPlan {
     int tn, splits, kb_per;
@@ -727,8 +723,8 @@ static TcPlan plan_tiles(int tiles, bool pair, int M, int k_blocks) {
             const int ctas = tiles * ((M + tn - 1) / tn) * splits, per_sm = (ctas + sm_count() - 1) / sm_count();
             const int occ = !pair && tn <= 64 ? 2 : 1, rounds = (per_sm + occ - 1) / occ;
             const double mma = fm * 8 * (tn * 0.47 > 64.0 ? tn * 0.47 : 64.0) * (per_sm < occ ? per_sm : occ);
-            double cost = rounds * (kb_per * (mma > 700.0 ? mma : 700.0) + 5000.0 + 15.5 * fm * tn);
-            cost += (splits - 1) * 20.0 * fm * tn;
+            double cost = rounds * (kb_per * (mma > 970.0 ? mma : 970.0) + 6200.0 + 15.5 * fm * tn);
+            if (splits > 1) cost += 400.0 + 5.0 * fm * tn;
             if (cost < best_cost) {
                 best_cost = cost;
                 best = TcPlan{tn, splits, kb_per};

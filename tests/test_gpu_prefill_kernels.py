@@ -45,31 +45,29 @@ def test_gemm_tiles_bit_exact(M, N, Kd, epilogue):
     assert np.array_equal(out.numpy(), want)      # the same roundings in the same order
 
 
-# Every (columns, split) that the plan takes, named beside it for 148 SMs: at the products of a 2560 / 6912 layer where one of them
-# takes it, else at other sizes.  The plain form of each, which a call without accumulators takes, against the general one
-# and the exact sums (below 2^24, so fp32 holds them in any order of summation).
+# Every (columns, split) that the plan takes for the products of a 2560 / 6912 layer between 9 and 1531 rows on 148 SMs, named
+# beside it, and the splits of a pair that small matrices take: the plain form of each, which a call without accumulators
+# takes, against the general one and the exact sums (below 2^24, so fp32 holds them in any order of summation).
 @pytest.mark.parametrize("pair,sizes,Kd,M", [
     (False, (2560, 640, 640), 2560, 9),       # 32 x 4
-    (False, (2560, 640, 640), 2560, 33),      # 32 x 2
-    (False, (2560, 640, 640), 2560, 65),      # 64 x 2
-    (False, (2560, 640, 640), 2560, 129),     # 96 x 2
-    (False, (2560, 640, 640), 2560, 257),     # 96 x 1
-    (False, (2560, 640, 640), 2560, 385),     # 128 x 1
-    (False, (2560, 640, 640), 2560, 513),     # 64 x 1
-    (False, (2560,), 6912, 97),               # 64 x 4
-    (False, (2560,), 6912, 193),              # 96 x 2
-    (False, (2560,), 6912, 289),              # 128 x 2
+    (False, (2560, 640, 640), 2560, 65),      # 64 x 4
+    (False, (2560, 640, 640), 2560, 129),     # 64 x 2
+    (False, (2560, 640, 640), 2560, 257),     # 32 x 1
+    (False, (2560, 640, 640), 2560, 289),     # 96 x 1
+    (False, (2560, 640, 640), 2560, 385),     # 64 x 1
+    (False, (2560,), 6912, 193),              # 32 x 2
+    (False, (2560,), 6912, 225),              # 96 x 2
+    (False, (2560,), 6912, 289),              # 64 x 2
+    (False, (2560,), 6912, 673),              # 128 x 1
     (False, (2560,), 6912, 1531),             # 128 x 1, the last tile in part
-    (False, (300, 20), 200, 40),              # 32 x 1, one K block
-    (True, (6912, 6912), 2560, 9),            # 32 x 2
-    (True, (6912, 6912), 2560, 33),           # 64 x 2
-    (True, (6912, 6912), 2560, 65),           # 64 x 1
-    (True, (6912, 6912), 2560, 129),          # 96 x 1
-    (True, (6912, 6912), 2560, 193),          # 128 x 1
-    (True, (6912, 6912), 2560, 512),          # 128 x 1
-    (True, (300, 300), 200, 40),              # 32 x 1
-    (True, (128, 128), 4096, 9),              # 32 x 4
-    (True, (2560, 2560), 12288, 37),          # 64 x 4
+    (True, (6912, 6912), 2560, 9),           # 32 x 2
+    (True, (6912, 6912), 2560, 33),          # 64 x 2
+    (True, (6912, 6912), 2560, 65),          # 64 x 1
+    (True, (6912, 6912), 2560, 129),         # 96 x 1
+    (True, (6912, 6912), 2560, 193),         # 128 x 1
+    (True, (6912, 6912), 2560, 512),         # 128 x 1
+    (True, (1000, 1000), 2560, 100),         # 32 x 4
+    (True, (1000, 1000), 2560, 129),         # 64 x 4
 ])
 def test_gemm_plans_without_taps(pair, sizes, Kd, M):
     rng = np.random.default_rng(M + Kd)
