@@ -66,7 +66,9 @@ int lspk_flush_l2(void);                /* overwrite a buffer larger than L2    
 int lspk_timer_start(void);
 int lspk_timer_stop(float* ms_out);
 
-/* In-kernel phase trace (measurement aid): after lspk_trace_begin, CTA 0 of each traced kernel
+/* In-kernel phase trace (measurement aid).  Launches with a trace take the general instantiations of the products and of the
+ * attention, which hold the marks and up to twice the code of the ones that run without: the marks tell how a kernel's phases
+ * compare, not what it takes untraced.  After lspk_trace_begin, CTA 0 of each traced kernel
  * appends a record of 16 uint64 words [kernel id, globaltimer ns at entry, SM clock at phase marks
  * ..., globaltimer ns at exit]; lspk_trace_read copies the records out and clears the counter.
  * A state's CUDA graph captured before the first lspk_trace_begin does not record; a later call with the same or a

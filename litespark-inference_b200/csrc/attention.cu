@@ -1176,7 +1176,7 @@ bool attention_group_heads(int T, int Q, int KV, int D, int t_max, int kv_is_fp1
 }
 
 // The phase marks are in instantiations of their own, for a launch with a trace: without them the cluster-split kernel is a tenth
-// shorter, and a decode step faster by 1 % (one sequence 684 -> 678 us, eight 1.246 -> 1.230 ms).
+// shorter, and a decode step faster by 1 % (one sequence 684 -> 678 us, eight 1.173 -> 1.158 ms).
 template <typename KVT, int D, int VB0, bool TRACE>
 static cudaError_t launch_attention_form(const AttnParams& p, dim3 grid, size_t smem) {
     static bool attr_set = false;

@@ -702,11 +702,14 @@ static cudaError_t launch_tc(const CUtensorMap* mw, const CUtensorMap& mx, const
                       : launch_tc_form<PAIR, TN, kTcPlain | kTcWhole>(mw, mx, p, grid);
 }
 
-// Token rows per tile and K split of a launch: the plan with the smallest time by a model of a CTA's life in SM cycles,
-// fitted to measured launches (q/k/v, o, gate/up and down of a 2560 / 6912 layer at 32 ... 1531 rows, every plan; the
-// pick is within 7 % of the best measured plan at each, on the best one at 17 of 24):
+// Token rows per tile and K split of a launch: the plan with the smallest time by a model of a CTA's life in SM cycles:
 //   a K block takes the MMA issue and execution time of the CTAs that share the SM, but not less than one turn of the
 //   pipeline; start-up, first copies and epilogue are paid per round of CTAs, a K split pays its exchange.
+// The constants were fitted to the kernel before it had plain forms.  Now, called one behind the other (int8 rows; q/k/v, o,
+// gate/up and down of a 2560 / 6912 layer, 33 row counts from 9 to 1531, every plan), the pick is the best measured plan at
+// 84 of 132 and 4 % behind it in the mean; at worst 40 % (down at 1280 rows: 35.1 us split over K, 25.1 with 96 columns and
+// no split).  Constants fitted to such launches are not better for that: in a prefill, between other kernels, they win 3 %
+// at 900 to 1280 tokens and lose 5 % at 600 and 2 % at 48.
 // Small M therefore takes many narrow tiles and K ranges (all SMs, short chains), large M the widest tiles.
 struct TcPlan {
     int tn, splits, kb_per;
@@ -734,11 +737,12 @@ static TcPlan plan_tiles(int tiles, bool pair, int M, int k_blocks) {
     return best;
 }
 
-// Fewest rows this kernel takes: with one eight-row tile the mma.sync kernel (linear_mma.cu) is level with it (33 us for
-// the four products of a layer at 8 rows, here 35), with two it is behind (16 rows: 38 and 34 us; 31 rows: 55 and 36).
+// Fewest rows this kernel takes.  The four products of a layer, rows normalised and quantised on the way: with one eight-row
+// tile the mma.sync kernel (linear_mma.cu) takes 25 us, with two it is behind (9 rows: 33 and 30.5 us here; 16 rows: 32 and
+// 30; 31 rows: 47 and 31).
 constexpr int kTcMinRows = 9;
-// Rows that come as int8 pay one launch more here (permute_rows_kernel) and none there: at 9 to 16 rows the four products
-// of a layer take 29.6 us here and 27.7 there, at 17 to 24 rows 29.5 and 38.9.
+// Rows that come as int8 pay one launch more here (permute_rows_kernel) and none there: called one by one, the four products of
+// a layer take 29 us here and 26.5 there at 9 to 16 rows, 28.7 and 36.2 at 17 to 24.
 constexpr int kTcMinRowsInt8 = 17;
 
 // Tensor-core path: one launch for all matrices of the call (plus the row quantiser in front of it).

@@ -70,8 +70,8 @@ constexpr int row_ctas_per_sm(bool pair, int ni, int pro, bool once) {
 // A decode step walks through five kernels a layer, together more code than an SM's instruction cache holds, so what a launch
 // does not execute costs as well: with the plain forms apart and one set of weight loads the code of q/k/v and o went from 39
 // to 17 KB, of gate/up from 43 to 20 KB, of down from 62 to 24 KB, a decode step at context 128 from 758 to 682 us.
-// ONCE    a CTA per row group (q/k/v, o, down): no loop, no registers for the next group's weights (decode at context 128 678 ->
-//         667 us a step)
+// ONCE    a CTA per row group (q/k/v, o, down): no loop, no registers for the next group's weights (15 and 22 KB; decode at
+//         context 128 678 -> 667 us a step)
 template <int MT, int NI, int NB, bool PAIR, int PRO, bool ONCE>
 __global__ void __launch_bounds__(kThreads)
 ternary_linear_kernel(const __grid_constant__ LinearParams p) {

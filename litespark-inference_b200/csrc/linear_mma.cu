@@ -51,7 +51,7 @@ static_assert(kMWarps == kMT && kMXSegMax <= 32, "row staging maps warp -> row a
 // FORM    kMmaTiled: pre-tiled rows, no trace, no accumulators to hand out; kMmaOneBatch: such rows with chunks for one batch of
 //         weights; kMmaAny: every form, taken from the call.
 // The plain forms are apart because their launches are short and their code cold: 16 and 19 KB (single, paired) of one batch, 18
-// and 22 KB of more, where the general form has 31 and 36; a decode step of eight sequences 1.26 -> 1.20 ms.
+// and 22 KB of more, where the general form has 31 and 36; a decode step of eight sequences 1.18 -> 1.13 ms.
 enum { kMmaAny, kMmaTiled, kMmaOneBatch };
 template <bool PAIR, int FORM>
 __global__ void __launch_bounds__(kMThreads)

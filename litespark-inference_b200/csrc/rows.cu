@@ -216,9 +216,9 @@ __device__ __forceinline__ uint32_t quant_exact(float v, float inv, int k, int K
 // Bound by the latency of the row's arrival and of the serial steps behind it at few rows, by their instructions at many:
 // library divisions, two-barrier reductions and a conversion per element took 6 % of the MLP block of 512 rows (49.9 -> 46.9 us)
 // and 7 % of a decode step of eight sequences (1.26 -> 1.16 ms).  A row spread over 640 or 1024 threads, four elements each,
-// is no faster at 8 rows (both 1.18 ms) and slower at 512 (53 us).
+// is no faster at 8 rows (a step 1.18 ms with either) and slower at 512 (53 us).
 // PLAIN   normed rows without a gate or selected weights, whole blocks of 16, permuted output: 11 KB of code (NB = 1; 15 KB at 2)
-//         instead of 25 (42), which each launch of a decode step has to fetch: eight sequences 1.25 -> 1.22 ms a step
+//         instead of 24 (41), which each launch of a decode step has to fetch: eight sequences 1.18 -> 1.145 ms a step
 template <int NB, bool PLAIN>
 __global__ void __launch_bounds__(kRowThreads)
 row_quant_regs_kernel(const float* __restrict__ x, const float* __restrict__ gate, const void* __restrict__ gamma_base,
