@@ -14,12 +14,17 @@
 // Error against float64, 2-norm, 1531 rows x 20 heads of 128: 3.5e-7 where scores have a spread of 4, and 3.7e-7 in
 // fp32 multiply-adds (attention_rows_kernel); over 16 to 1531 rows and spreads of 1 to 12 it is 0.85 to 1.0 of theirs.
 //
-// One warp owns 16 query rows of one head.  Two splits of the four warps of a CTA:
-//   WK = 1   four row tiles (heads of one KV head first, then positions) share every key / value tile: the form for
-//            long prompts.  480 CTAs at 1531 rows x 20 heads, every key row fetched once per 64 query rows.
-//   WK = 4   one row tile, its keys dealt to the four warps and the four softmax pieces merged at the end: when the
-//            first form would leave SMs without a CTA (128 rows x 20 heads: 40 CTAs, here 160).
-// Bound by the mma.sync rate (three products per term of the dot products): 384 instructions per warp and 64 keys.
+// A warp works on 16 query rows of one head (a row tile) against 32 keys at a time.  WK of the four warps of a CTA share a row tile
+// and deal its keys among themselves; their softmax pieces are merged at the end.  The 4 / WK row tiles of a CTA (heads of one KV
+// head first, then positions) share every key / value tile.  launch_prefill_d chooses.
+//
+// Bound by instructions: on this part mma.sync leaves no room for fp32 arithmetic beside it (a scheduler takes 8.1 cycles for one of
+// them, 12.2 with four independent additions, 13.1 with four packed ones, whatever the number of warps), and a warp forms 192
+// products per 32 keys (1550 cycles) beside some 850 other instructions (1500).  Hence pairs of floats in one instruction, an
+// exponential of few, the queries' terms in registers; 1189 instructions per 32 keys were 1056 then.  Three CTAs per SM (168 registers),
+// products issued in other orders, operands fetched one group ahead, padded instead of permuted tiles: no faster.
+// 20 heads of 128, rotation and attention in us before and now: 16 rows 13.9 -> 11.9, 112 22 -> 13.4, 128 21.9 -> 16.3, 256 33 -> 22,
+// 512 64 -> 40, 800 92 -> 57, 1531 148 -> 140; fp32 cache 512 118 -> 86, 800 168 -> 128, 1531 308.
 #include "internal.cuh"
 
 namespace lspk {
@@ -39,6 +44,47 @@ template <> struct PfTraits<float> {
 // products (row operand term, column operand term), smallest first
 __device__ constexpr int kComboA[2][6] = {{2, 1, 0, 0, 0, 0}, {0, 1, 2, 0, 1, 0}};
 __device__ constexpr int kComboB[2][6] = {{0, 0, 0, 0, 0, 0}, {2, 1, 0, 1, 0, 0}};
+
+// Pairs of floats: one instruction for two of the operations of which a tile has some thousand beside its 384 products.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
+__device__ __forceinline__ f32x2 at2(const float* p) { return pack2(p[0], p[1]); }
+__device__ __forceinline__ void put2(float* p, f32x2 v) { unpack2(v, p[0], p[1]); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// scale * e^d for d <= 0, finite: e^d = 2^t (1 + r) with t = d log2(e) as it rounds and r = d - t ln(2), formed without a
+// rounding that matters from the two parts of ln(2) (|r| < 2^-16 where 2^t is not 0, so the series ends there).  As far off as the
+// instruction's 2^t, 2^-22, like expf; not finite for d = -inf, which the library function takes to 0.
+__device__ __forceinline__ f32x2 exp2x(f32x2 d, float scale) {
+    const f32x2 t = mul2(d, both(1.44269504f));
+    float lo, hi;
+    unpack2(t, lo, hi);
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(lo));
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(hi));
+    f32x2 p = pack2(lo, hi);
+    if (scale != 1.0f) p = mul2(p, both(scale));
+    const f32x2 r = fma2(t, both(1.90465421e-9f), fma2(t, both(-0.693147182f), d));
+    return fma2(p, r, p);
+}
 
 // Three 16-bit terms of a pair of floats, packed for an operand register.
 template <typename KVT>
@@ -60,16 +106,18 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t out[3]) {
         }
     }
 }
+// c = a b (first) or c + a b
 template <typename KVT>
-__device__ __forceinline__ void mma16816(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma16816(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1, bool first) {
+    if (first) c[0] = c[1] = c[2] = c[3] = 0.0f;
     if constexpr (sizeof(KVT) == 2)
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
     else
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void ldsm4(uint32_t r[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -120,23 +168,24 @@ __device__ __noinline__ void attend_row_plain(const float* q, const KVT* k, cons
 template <typename KVT, int D, int WK>
 struct PfLayout {
     static constexpr int kPlanes = PfTraits<KVT>::kPlanes;
-    static constexpr int KT = (WK == 1 ? 64 : 32) / (kPlanes == 1 ? 1 : 2);   // keys of a warp's tile
+    static constexpr int RT = 4 / WK;                                         // row tiles of a CTA
+    static constexpr bool kRing = WK <= 2 && kPlanes == 1;                    // K and V tiles in turn through three buffers
+    static constexpr int KT = kPlanes == 1 ? 32 : WK == 1 ? 32 : 16;          // keys of a warp's tile
     static constexpr int KI = KT * WK;                                        // keys of a CTA's tile
-    static constexpr int kStages = kPlanes == 1 ? 2 : 1;
+    static constexpr int kStages = kPlanes == 1 ? 2 : 1;                      // (without the ring)
     static constexpr int kRowBytes = D * 2;                                   // one term of one row
     static constexpr int kTileBytes = KI * kRowBytes * kPlanes;               // K or V tile
     static constexpr int kQBytes = 16 * kRowBytes * 3;                        // one row tile's three terms
-    static constexpr int kSmem = (4 / WK) * kQBytes + kStages * 2 * kTileBytes;
-    static_assert(WK == 1 || 4 * 16 * D * 4 + 4 * 16 * 8 <= kStages * 2 * kTileBytes, "the merge reuses the tile buffers");
+    static constexpr int kSmem = RT * kQBytes + (kRing ? 3 : kStages * 2) * kTileBytes;
+    static_assert(WK == 1 || 4 * 16 * D * 4 + 4 * 16 * 8 <= (kRing ? 3 : kStages * 2) * kTileBytes, "the merge reuses the tile buffers");
 };
 
-// hg: heads of one KV head that share a CTA (1, 2 or 4; WK = 1 only).
+// hg: heads of one KV head that share a CTA (1, 2 or 4).
 template <typename KVT, int D, int WK>
 __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(const AttnParams p, int hg) {
     using L = PfLayout<KVT, D, WK>;
     constexpr int KT = L::KT, KI = L::KI, RB = L::kRowBytes, kCombos = PfTraits<KVT>::kCombos;
     constexpr int kSet = sizeof(KVT) == 2 ? 0 : 1;
-    constexpr int kQkUnroll = kSet == 0 ? 1 : 2;
     constexpr int kChunkMask = 7;                          // 16-byte chunks of a row are permuted by row & 7
     extern __shared__ __align__(128) unsigned char pf_smem[];
     grid_dependency_launch();
@@ -144,50 +193,60 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = p.Q / p.KV, kd = p.KV * D;
     // heavy row tiles (late positions, many keys) first
-    const int tile_y = (int)gridDim.y - 1 - (int)blockIdx.y;
-    int head, row0, row_last;                              // this warp's head and first row; the CTA's last row
-    if (WK == 1) {
-        const int pt = 4 / hg;                             // position tiles of the CTA
-        head = blockIdx.x * hg + warp % hg;
-        row0 = (tile_y * pt + warp / hg) * 16;
-        row_last = min(p.T, (tile_y + 1) * pt * 16) - 1;
-    } else {
-        head = blockIdx.x;
-        row0 = tile_y * 16;
-        row_last = min(p.T, row0 + 16) - 1;
-    }
-    const int kvh = (int)(WK == 1 ? blockIdx.x * hg : blockIdx.x) / G;
-    unsigned char* qs = pf_smem + (WK == 1 ? warp : 0) * L::kQBytes;
-    unsigned char* kv = pf_smem + (4 / WK) * L::kQBytes;
+    const int tile_y = (int)gridDim.y - 1 - (int)blockIdx.y, tile_x = blockIdx.x;
+    const int rt = warp / WK, wk = warp % WK;              // this warp's row tile in the CTA and its share of the keys
+    const int pt = L::RT / hg;                             // position tiles of the CTA
+    const int head = tile_x * hg + rt % hg, row0 = (tile_y * pt + rt / hg) * 16;
+    const int row_last = min(p.T, (tile_y + 1) * pt * 16) - 1;      // the CTA's last row
+    const int kvh = tile_x * hg / G;
+    unsigned char* qs = pf_smem + rt * L::kQBytes;
+    unsigned char* kv = pf_smem + L::RT * L::kQBytes;
+    float* const factors = reinterpret_cast<float*>(pf_smem + L::kSmem);      // [RT][16], WK > 1
     grid_dependency_wait();
     const int pos0 = p.pos_ptr[0];
     const int n_keys = pos0 + row_last + 1;                // keys any row of the CTA attends to
     const KVT* ck = reinterpret_cast<const KVT*>(p.cache_k) + (size_t)kvh * D;
     const KVT* cv = reinterpret_cast<const KVT*>(p.cache_v) + (size_t)kvh * D;
 
-    auto tile_ptr = [&](int stage, int which) { return kv + (size_t)(stage * 2 + which) * L::kTileBytes; };
-    auto load_tile = [&](int it) {
-        const int k0 = it * KI, stage = it % L::kStages;
-        if constexpr (L::kPlanes == 1) {
+    const int n_it = (n_keys + KI - 1) / KI;
+    auto tile_ptr = [&](int it, int which) {
+        return kv + (size_t)(L::kRing ? (2 * it + which) % 3 : (it % L::kStages) * 2 + which) * L::kTileBytes;
+    };
+    // keys (w = 0) or values of a tile of an fp16 cache, asynchronously
+    auto load_half = [&](int it, int w) {
+        const KVT* src = w ? cv : ck;
+        const uint32_t dst = smem_u32(tile_ptr(it, w));
 #pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const KVT* src = w ? cv : ck;
-                const uint32_t dst = smem_u32(tile_ptr(stage, w));
-                for (int i = tid; i < KI * (D / 8); i += kPfThreads) {
-                    const int r = i / (D / 8), c = i % (D / 8);
-                    const int key = k0 + r;
-                    const void* g = src + (size_t)min(key, n_keys - 1) * kd + c * 8;
-                    const int bytes = key < n_keys ? 16 : 0;       // rows past the last key read as zeros
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * RB + ((c ^ (r & kChunkMask)) << 4)),
-                                 "l"(g), "r"(bytes) : "memory");
-                }
-            }
+        for (int i = tid; i < KI * (D / 8); i += kPfThreads) {
+            const int r = i / (D / 8), c = i % (D / 8);
+            const int key = it * KI + r;
+            const void* g = src + (size_t)min(key, n_keys - 1) * kd + c * 8;
+            const int bytes = key < n_keys ? 16 : 0;       // rows past the last key read as zeros
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * RB + ((c ^ (r & kChunkMask)) << 4)),
+                         "l"(g), "r"(bytes) : "memory");
+        }
+    };
+    // ring: one group of copies per half tile, also behind the last
+    auto ring_load = [&](int t) {
+        if (t < 2 * n_it) load_half(t >> 1, t & 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto ring_step = [&](int t) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                   // half tile t is there for all, and t - 1 is done with
+        ring_load(t + 2);
+    };
+    auto load_tile = [&](int it) {
+        const int k0 = it * KI;
+        if constexpr (L::kPlanes == 1) {
+            load_half(it, 0);
+            load_half(it, 1);
             asm volatile("cp.async.commit_group;" ::: "memory");
         } else {
 #pragma unroll
             for (int w = 0; w < 2; ++w) {
                 const KVT* src = w ? cv : ck;
-                unsigned char* dst = tile_ptr(stage, w);
+                unsigned char* dst = tile_ptr(it, w);
                 for (int i = tid; i < KI * (D / 8); i += kPfThreads) {
                     const int r = i / (D / 8), c = i % (D / 8);
                     const int key = k0 + r;
@@ -210,52 +269,60 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
             }
         }
     };
-    const int n_it = (n_keys + KI - 1) / KI;
-    if (L::kStages == 2) load_tile(0);
+    if (L::kRing) {
+        ring_load(0);
+        ring_load(1);
+    } else if (L::kStages == 2) {
+        load_tile(0);
+    }
 
     // ---- query rows -> three terms in shared memory; with WK = 4 the warps take four rows each ------------------
     float q_unscale_r[2] = {1.0f, 1.0f};                   // rows lane / 4 and lane / 4 + 8
     {
-        constexpr int PER = WK == 1 ? 16 : 4;
+        constexpr int PER = 16 / WK;
         float my = 1.0f;                                   // lane r keeps row r's factor
-        for (int i = 0; i < PER; ++i) {
-            const int r = WK == 1 ? i : warp * 4 + i;
-            const int t = row0 + r;
-            constexpr int EL = D / 32;                     // elements per lane: 2 or 4
-            float v[EL];
+        constexpr int EL = D / 32;                         // elements per lane: 2 or 4
+        // four rows at a time: one after the other, each waits for its own trip to memory and through its maximum
+#pragma unroll 1
+        for (int i0 = 0; i0 < PER; i0 += 4) {
+            float v[4][EL];
 #pragma unroll
-            for (int e = 0; e < EL; ++e) v[e] = 0.0f;
-            if (t < p.T) {
-                const float* src = p.q + (size_t)t * p.Q * D + (size_t)head * D + lane * EL;
+            for (int i = 0; i < 4; ++i) {
+                const int t = row0 + wk * PER + i0 + i;
 #pragma unroll
                 for (int e = 0; e < EL; e += 2) {
-                    const float2 f = *reinterpret_cast<const float2*>(src + e);
-                    v[e] = f.x;
-                    v[e + 1] = f.y;
+                    float2 f = make_float2(0.0f, 0.0f);
+                    if (t < p.T) f = *reinterpret_cast<const float2*>(p.q + (size_t)t * p.Q * D + (size_t)head * D + lane * EL + e);
+                    v[i][e] = f.x;
+                    v[i][e + 1] = f.y;
                 }
             }
-            if (kSet == 0) {
-                float m = 0.0f;
 #pragma unroll
-                for (int e = 0; e < EL; ++e) m = fmaxf(m, fabsf(v[e]));
-                m = warp_max(m);
-                // largest element to [2^13, 2^14): exact scaling by a power of two
-                int ex = m > 0.0f ? 140 - (int)(__float_as_uint(m) >> 23) : 0;
-                ex = max(-100, min(100, ex));
-                const float f = __uint_as_float((uint32_t)(127 + ex) << 23);
+            for (int i = 0; i < 4; ++i) {
+                const int r = wk * PER + i0 + i;
+                if (kSet == 0) {
+                    float m = 0.0f;
 #pragma unroll
-                for (int e = 0; e < EL; ++e) v[e] *= f;
-                if (lane == r) my = __uint_as_float((uint32_t)(127 - ex) << 23);
-                if (WK == 4 && lane == 0) reinterpret_cast<float*>(kv + L::kStages * 2 * L::kTileBytes)[r] = __uint_as_float((uint32_t)(127 - ex) << 23);
-            }
+                    for (int e = 0; e < EL; ++e) m = fmaxf(m, fabsf(v[i][e]));
+                    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));      // m >= 0: ordered like its bits
+                    // largest element to [2^13, 2^14): exact scaling by a power of two
+                    int ex = m > 0.0f ? 140 - (int)(__float_as_uint(m) >> 23) : 0;
+                    ex = max(-100, min(100, ex));
+                    const float f = __uint_as_float((uint32_t)(127 + ex) << 23);
 #pragma unroll
-            for (int e = 0; e < EL; e += 2) {
-                uint32_t t3[3];
-                split3<KVT>(v[e], v[e + 1], t3);
-                const int byte = (lane * EL + e) * 2, c = byte >> 4;
+                    for (int e = 0; e < EL; ++e) v[i][e] *= f;
+                    if (lane == r) my = __uint_as_float((uint32_t)(127 - ex) << 23);
+                    if (WK > 1 && lane == 0) factors[rt * 16 + r] = __uint_as_float((uint32_t)(127 - ex) << 23);
+                }
 #pragma unroll
-                for (int pl = 0; pl < 3; ++pl)
-                    *reinterpret_cast<uint32_t*>(qs + pl * 16 * RB + r * RB + ((c ^ (r & kChunkMask)) << 4) + (byte & 15)) = t3[pl];
+                for (int e = 0; e < EL; e += 2) {
+                    uint32_t t3[3];
+                    split3<KVT>(v[i][e], v[i][e + 1], t3);
+                    const int byte = (lane * EL + e) * 2, c = byte >> 4;
+#pragma unroll
+                    for (int pl = 0; pl < 3; ++pl)
+                        *reinterpret_cast<uint32_t*>(qs + pl * 16 * RB + r * RB + ((c ^ (r & kChunkMask)) << 4) + (byte & 15)) = t3[pl];
+                }
             }
         }
         if (WK == 1) {
@@ -265,9 +332,8 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
         } else {
             __syncthreads();
             if (kSet == 0) {
-                const float* f = reinterpret_cast<const float*>(kv + L::kStages * 2 * L::kTileBytes);
-                q_unscale_r[0] = f[lane >> 2];
-                q_unscale_r[1] = f[(lane >> 2) + 8];
+                q_unscale_r[0] = factors[rt * 16 + (lane >> 2)];
+                q_unscale_r[1] = factors[rt * 16 + (lane >> 2) + 8];
             }
         }
     }
@@ -281,10 +347,28 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
         for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
     float mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.0f, 0.0f};
     const int my_pos[2] = {pos0 + row0 + (lane >> 2), pos0 + row0 + (lane >> 2) + 8};
+    // An fp16 cache leaves the registers to keep the query's terms: fetched for every tile they are 24 of its 56 matrix loads.
+    constexpr bool kKeepQ = kSet == 0;
+    constexpr int kQkUnroll = kKeepQ ? D / 32 : 2;
+    uint32_t qf[kKeepQ ? D / 16 : 2][3][4];
     const uint32_t q_base = smem_u32(qs);
+    auto load_q = [&](uint32_t (&q)[3][4], int ks) {
+#pragma unroll
+        for (int pl = 0; pl < 3; ++pl) {
+            // lanes 0-15: rows 0-15 at chunk 2 ks; lanes 16-31: the same rows at chunk 2 ks + 1
+            const int r = lane & 15, c = ks * 2 + (lane >> 4);
+            ldsm4(q[pl], q_base + pl * 16 * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
+        }
+    };
+    if constexpr (kKeepQ) {
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) load_q(qf[ks], ks);
+    }
 
     for (int it = 0; it < n_it; ++it) {
-        if (L::kStages == 2) {
+        if (L::kRing) {
+            ring_step(2 * it);
+        } else if (L::kStages == 2) {
             if (it + 1 < n_it) {
                 load_tile(it + 1);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -294,113 +378,121 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
         } else {
             load_tile(it);
         }
-        __syncthreads();
-        const int stage = it % L::kStages;
-        const int kw = it * KI + (WK == 1 ? 0 : warp * KT);            // first key of this warp's tile
-        if (kw <= pos0 + min(row0 + 15, p.T - 1) && row0 < p.T) {      // some row of the warp sees some key of the tile
-            const uint32_t kbase = smem_u32(tile_ptr(stage, 0)) + (WK == 1 ? 0 : warp * KT * RB);
-            const uint32_t vbase = smem_u32(tile_ptr(stage, 1)) + (WK == 1 ? 0 : warp * KT * RB);
-            float s[KT / 8][4];
+        if (!L::kRing) __syncthreads();
+        const int kw = it * KI + wk * KT;            // first key of this warp's tile
+        const bool sees = kw <= pos0 + min(row0 + 15, p.T - 1) && row0 < p.T;      // some row of the warp sees some key of the tile
+        float s[KT / 8][4];
 #pragma unroll
-            for (int i = 0; i < KT / 8; ++i)
+        for (int i = 0; i < KT / 8; ++i)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
-            // unrolled as far as the registers of a thread go (D = 128, shared form: whole, 10.16 and 15.40 ms for a prompt of
-            // 1531 rows with an fp16 and an fp32 cache; as here, 10.01 and 14.95)
+            for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
+        if (sees) {
+            const uint32_t kbase = smem_u32(tile_ptr(it, 0)) + wk * KT * RB;
 #pragma unroll kQkUnroll
             for (int kp = 0; kp < D / 32; ++kp) {                      // two k steps: their sums meet before the running one
-                uint32_t qa[2][3][4];
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk)
-#pragma unroll
-                    for (int pl = 0; pl < 3; ++pl) {
-                        // lanes 0-15: rows 0-15 at chunk 2 ks; lanes 16-31: the same rows at chunk 2 ks + 1
-                        const int r = lane & 15, c = (kp * 2 + kk) * 2 + (lane >> 4);
-                        ldsm4(qa[kk][pl], q_base + pl * 16 * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
-                    }
+                if constexpr (!kKeepQ) {
+                    load_q(qf[0], kp * 2);
+                    load_q(qf[1], kp * 2 + 1);
+                }
 #pragma unroll
                 for (int nt = 0; nt < KT / 16; ++nt) {
-                    float c0[2][4], c1[2][4];
+                    float c[2][2][4];                                  // [k step][keys 0-7, 8-15][]
+                    uint32_t kb[2][L::kPlanes][4];
 #pragma unroll
-                    for (int kk = 0; kk < 2; ++kk) {
-                        uint32_t kb[L::kPlanes][4];
+                    for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
                         for (int pl = 0; pl < L::kPlanes; ++pl) {
                             // matrices: keys 0-7 / chunk 0, keys 0-7 / chunk 1, keys 8-15 / chunk 0, keys 8-15 / chunk 1
-                            const int r = nt * 16 + (lane & 7) + ((lane >> 4) << 3), c = (kp * 2 + kk) * 2 + ((lane >> 3) & 1);
-                            ldsm4(kb[pl], kbase + pl * KI * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
+                            const int r = nt * 16 + (lane & 7) + ((lane >> 4) << 3), c8 = (kp * 2 + kk) * 2 + ((lane >> 3) & 1);
+                            ldsm4(kb[kk][pl], kbase + pl * KI * RB + r * RB + ((c8 ^ (r & kChunkMask)) << 4));
                         }
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) c0[kk][e] = c1[kk][e] = 0.0f;
+                    for (int cb = 0; cb < kCombos; ++cb) {
+                        const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
 #pragma unroll
-                        for (int cb = 0; cb < kCombos; ++cb) {
-                            const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
-                            mma16816<KVT>(c0[kk], qa[kk][a], kb[b][0], kb[b][1]);
-                            mma16816<KVT>(c1[kk], qa[kk][a], kb[b][2], kb[b][3]);
-                        }
+                        for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+                                mma16816<KVT>(c[kk][h], qf[(kKeepQ ? kp * 2 : 0) + kk][a], kb[kk][b][2 * h], kb[kk][b][2 * h + 1], cb == 0);
                     }
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        s[nt * 2][e] += c0[0][e] + c0[1][e];
-                        s[nt * 2 + 1][e] += c1[0][e] + c1[1][e];
-                    }
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int e = 0; e < 4; e += 2)
+                            put2(&s[nt * 2 + h][e], add2(at2(&s[nt * 2 + h][e]), add2(at2(&c[0][h][e]), at2(&c[1][h][e]))));
                 }
             }
-            // scale, mask, running maximum
+            // scale, mask, running maximum.  The query's scale is a power of two: one product with both factors rounds as one
+            // with 1 / sqrt(D) alone.  Only the tiles on the diagonal have keys to hide.
+            const f32x2 factor[2] = {both(q_unscale_r[0] * inv_sqrt_d), both(q_unscale_r[1] * inv_sqrt_d)};
+            const bool diagonal = kw + KT - 1 > pos0 + row0;
             float nm[2] = {mx[0], mx[1]};
 #pragma unroll
             for (int i = 0; i < KT / 8; ++i)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int key = kw + i * 8 + (lane & 3) * 2 + (e & 1);
-                    const float v = __fmul_rn(s[i][e] * q_unscale_r[e >> 1], inv_sqrt_d);
-                    s[i][e] = key <= my_pos[e >> 1] ? v : -INFINITY;
-                    nm[e >> 1] = fmaxf(nm[e >> 1], s[i][e]);
-                }
-            float corr[2], base[2];
+                for (int h = 0; h < 2; ++h) put2(&s[i][2 * h], mul2(at2(&s[i][2 * h]), factor[h]));
+            auto hidden = [&](int i, int e) { return kw + i * 8 + (lane & 3) * 2 + (e & 1) > my_pos[e >> 1]; };
+            if (diagonal) {
+#pragma unroll
+                for (int i = 0; i < KT / 8; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (hidden(i, e)) s[i][e] = -INFINITY;
+            }
+#pragma unroll
+            for (int i = 0; i < KT / 8; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) nm[e >> 1] = fmaxf(nm[e >> 1], s[i][e]);
+            float corr[2];
+            f32x2 base[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 nm[h] = fmaxf(nm[h], __shfl_xor_sync(0xffffffffu, nm[h], 1));
                 nm[h] = fmaxf(nm[h], __shfl_xor_sync(0xffffffffu, nm[h], 2));
-                base[h] = nm[h] == -INFINITY ? 0.0f : nm[h];           // a row without keys yet
-                corr[h] = expf(mx[h] - base[h]);
+                const float b = nm[h] == -INFINITY ? 0.0f : nm[h];     // a row without keys yet
+                base[h] = both(-b);
+                corr[h] = expf(mx[h] - b);
                 mx[h] = nm[h];
                 sum[h] *= corr[h];
             }
             // The tile's terms are summed apart: added to the running sums one by one, those of 1531 keys round 383 times in
-            // every lane.  Pairs first where a tile has 64 keys; where it has 32, one by one as they come (pairs: 1.5 % more
-            // time for a prompt of 1024 rows, no less error).
-            float tile_sum[2] = {0.0f, 0.0f};
+            // every lane.
+            f32x2 tile_sum[2] = {both(0.0f), both(0.0f)};
 #pragma unroll
             for (int i = 0; i < KT / 8; ++i)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    s[i][e] = expf(s[i][e] - base[e >> 1]);
-                    if (kSet == 1) tile_sum[e >> 1] += s[i][e];
-                }
-            if (kSet == 0) {
+                for (int h = 0; h < 2; ++h) put2(&s[i][2 * h], exp2x(add2(at2(&s[i][2 * h]), base[h]), kSet == 0 ? kProbScale : 1.0f));
+            if (diagonal) {
 #pragma unroll
-                for (int i = 0; i < KT / 8; ++i) {
-                    tile_sum[0] += s[i][0] + s[i][1];
-                    tile_sum[1] += s[i][2] + s[i][3];
-                }
+                for (int i = 0; i < KT / 8; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (hidden(i, e)) s[i][e] = 0.0f;
             }
-            sum[0] += tile_sum[0];
-            sum[1] += tile_sum[1];
+#pragma unroll
+            for (int i = 0; i < KT / 8; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) tile_sum[h] = add2(tile_sum[h], at2(&s[i][2 * h]));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float lo, hi;
+                unpack2(tile_sum[h], lo, hi);
+                sum[h] += lo + hi;
+            }
             if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
 #pragma unroll
-                for (int i = 0; i < D / 8; ++i) {
-                    o[i][0] *= corr[0];
-                    o[i][1] *= corr[0];
-                    o[i][2] *= corr[1];
-                    o[i][3] *= corr[1];
-                }
+                for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) put2(&o[i][2 * h], mul2(at2(&o[i][2 * h]), both(corr[h])));
             }
+        }
+        if (L::kRing) ring_step(2 * it + 1);
+        if (sees) {
+            const uint32_t vbase = smem_u32(tile_ptr(it, 1)) + wk * KT * RB;
             // o += P V: the score accumulators of 16 keys are the A operand of one k step, two steps where the tile has them
             constexpr int PP = KT >= 32 ? 2 : 1;
 #pragma unroll
             for (int kp = 0; kp < KT / 16 / PP; ++kp) {
-                constexpr float ps = kSet == 0 ? kProbScale : 1.0f;
                 uint32_t pa[PP][3][4];
 #pragma unroll
                 for (int kk = 0; kk < PP; ++kk)
@@ -408,48 +500,49 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
                     for (int j = 0; j < 4; ++j) {
                         const float* sv = s[(kp * PP + kk) * 2 + (j >> 1)];
                         uint32_t t3[3];
-                        split3<KVT>(sv[(j & 1) * 2] * ps, sv[(j & 1) * 2 + 1] * ps, t3);
+                        split3<KVT>(sv[(j & 1) * 2], sv[(j & 1) * 2 + 1], t3);
                         pa[kk][0][j] = t3[0];
                         pa[kk][1][j] = t3[1];
                         pa[kk][2][j] = t3[2];
                     }
 #pragma unroll
                 for (int nt = 0; nt < D / 16; ++nt) {
-                    float c0[PP][4], c1[PP][4];
+                    float c[PP][2][4];
+                    uint32_t vb[PP][L::kPlanes][4];
 #pragma unroll
-                    for (int kk = 0; kk < PP; ++kk) {
-                        uint32_t vb[L::kPlanes][4];
+                    for (int kk = 0; kk < PP; ++kk)
 #pragma unroll
                         for (int pl = 0; pl < L::kPlanes; ++pl) {
                             // matrices (transposed): keys 0-7 / chunk 0, keys 8-15 / chunk 0, keys 0-7 / chunk 1, keys 8-15 / chunk 1
-                            const int r = (kp * PP + kk) * 16 + (lane & 15), c = nt * 2 + (lane >> 4);
-                            ldsm4_t(vb[pl], vbase + pl * KI * RB + r * RB + ((c ^ (r & kChunkMask)) << 4));
+                            const int r = (kp * PP + kk) * 16 + (lane & 15), c8 = nt * 2 + (lane >> 4);
+                            ldsm4_t(vb[kk][pl], vbase + pl * KI * RB + r * RB + ((c8 ^ (r & kChunkMask)) << 4));
                         }
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) c0[kk][e] = c1[kk][e] = 0.0f;
+                    for (int cb = 0; cb < kCombos; ++cb) {
+                        const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
 #pragma unroll
-                        for (int cb = 0; cb < kCombos; ++cb) {
-                            const int a = kComboA[kSet][cb], b = kComboB[kSet][cb];
-                            mma16816<KVT>(c0[kk], pa[kk][a], vb[b][0], vb[b][1]);
-                            mma16816<KVT>(c1[kk], pa[kk][a], vb[b][2], vb[b][3]);
+                        for (int kk = 0; kk < PP; ++kk)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+                                mma16816<KVT>(c[kk][h], pa[kk][a], vb[kk][b][2 * h], vb[kk][b][2 * h + 1], cb == 0);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int e = 0; e < 4; e += 2) {
+                            const f32x2 y = PP == 2 ? add2(at2(&c[0][h][e]), at2(&c[PP - 1][h][e])) : at2(&c[0][h][e]);
+                            put2(&o[nt * 2 + h][e], add2(at2(&o[nt * 2 + h][e]), y));
                         }
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        o[nt * 2][e] += PP == 2 ? c0[0][e] + c0[PP - 1][e] : c0[0][e];
-                        o[nt * 2 + 1][e] += PP == 2 ? c1[0][e] + c1[PP - 1][e] : c1[0][e];
-                    }
                 }
             }
         }
-        __syncthreads();                                   // the tile buffers are refilled next
+        if (!L::kRing) __syncthreads();                    // the tile buffers are refilled next
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
         sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
     }
-    constexpr float unp = kSet == 0 ? 1.0f / kProbScale : 1.0f;
     auto redo_row = [&](int t) {
         const size_t at = (size_t)t * p.Q * D + (size_t)head * D;
         attend_row_plain<KVT, D>(p.q + at, ck, cv, p.out + at, pos0 + t + 1, kd);
@@ -464,7 +557,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
                 float* dst = p.out + (size_t)t * p.Q * D + (size_t)head * D + (lane & 3) * 2;
 #pragma unroll
                 for (int i = 0; i < D / 8; ++i) {
-                    const float2 y = make_float2(__fdiv_rn(o[i][h * 2] * unp, sum[h]), __fdiv_rn(o[i][h * 2 + 1] * unp, sum[h]));
+                    const float2 y = make_float2(__fdiv_rn(o[i][h * 2], sum[h]), __fdiv_rn(o[i][h * 2 + 1], sum[h]));
                     *reinterpret_cast<float2*>(dst + i * 8) = y;
                     finite = finite && fabsf(y.x) < INFINITY && fabsf(y.y) < INFINITY;
                 }
@@ -478,7 +571,11 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
         }
         return;
     }
-    // ---- merge the four warps' softmax pieces -------------------------------------------------------------------
+    // ---- merge the softmax pieces of each row tile's warps -------------------------------------------------------
+    if (L::kRing) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                   // the last tile is done with
+    }
     float* fo = reinterpret_cast<float*>(kv);              // [4][16][D]
     float* fm = fo + 4 * 16 * D;                           // [4][16] maxima, [4][16] sums
 #pragma unroll
@@ -487,45 +584,47 @@ __global__ void __launch_bounds__(kPfThreads, 2) attention_prefill_mma_kernel(co
 #pragma unroll
         for (int i = 0; i < D / 8; ++i)
             *reinterpret_cast<float2*>(fo + (size_t)(warp * 16 + r) * D + i * 8 + (lane & 3) * 2) =
-                make_float2(o[i][h * 2] * unp, o[i][h * 2 + 1] * unp);
+                make_float2(o[i][h * 2], o[i][h * 2 + 1]);
         if ((lane & 3) == 0) {
             fm[warp * 16 + r] = mx[h];
             fm[64 + warp * 16 + r] = sum[h];
         }
     }
     __syncthreads();
-    unsigned redo = 0;                                     // rows that are not finite
-    for (int i = tid; i < 16 * D; i += kPfThreads) {
-        const int r = i / D, d = i % D, t = row0 + r;
-        if (t >= p.T) continue;
-        float M = fm[r];
+    // a warp forms 16 / WK rows of its row tile
+    for (int i = 0; i < 16 / WK; ++i) {
+        const int r = wk * (16 / WK) + i, t = row0 + r;
+        if (t >= p.T) break;
+        const int first = rt * WK;                         // the row tile's first warp
+        float M = fm[first * 16 + r];
 #pragma unroll
-        for (int w = 1; w < 4; ++w) M = fmaxf(M, fm[w * 16 + r]);
-        float den = 0.0f, acc = 0.0f;
+        for (int w = 1; w < WK; ++w) M = fmaxf(M, fm[(first + w) * 16 + r]);
+        float den = 0.0f, wgt[WK];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const float wgt = expf(fm[w * 16 + r] - M);    // 0 for a piece without keys (maximum -inf)
-            den = fmaf(fm[64 + w * 16 + r], wgt, den);
-            acc = fmaf(fo[(size_t)(w * 16 + r) * D + d], wgt, acc);
+        for (int w = 0; w < WK; ++w) {
+            wgt[w] = expf(fm[(first + w) * 16 + r] - M);   // 0 for a piece without keys (maximum -inf)
+            den = fmaf(fm[64 + (first + w) * 16 + r], wgt[w], den);
         }
-        const float y = __fdiv_rn(acc, den);
-        p.out[(size_t)t * p.Q * D + (size_t)head * D + d] = y;
-        redo |= (fabsf(y) < INFINITY ? 0u : 1u) << r;
-    }
-    if (__syncthreads_or((int)redo)) {
-        __shared__ unsigned s_redo;
-        if (tid == 0) s_redo = 0;
-        __syncthreads();
-        if (redo) atomicOr(&s_redo, redo);
-        __syncthreads();
-        for (int r = warp; r < 16; r += 4)
-            if ((s_redo >> r) & 1u) redo_row(row0 + r);
+        bool finite = true;
+#pragma unroll
+        for (int d = lane; d < D; d += 32) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int w = 0; w < WK; ++w) acc = fmaf(fo[(size_t)((first + w) * 16 + r) * D + d], wgt[w], acc);
+            const float y = __fdiv_rn(acc, den);
+            p.out[(size_t)t * p.Q * D + (size_t)head * D + d] = y;
+            finite = finite && fabsf(y) < INFINITY;
+        }
+        if (!__all_sync(0xffffffffu, finite)) {
+            __syncwarp();                                  // the stores above, by other lanes, come first
+            redo_row(t);
+        }
     }
 }
 
 template <typename KVT, int D, int WK>
 static int launch_prefill(const AttnParams& p, dim3 grid, int hg) {
-    constexpr int smem = PfLayout<KVT, D, WK>::kSmem + 64;
+    constexpr int smem = PfLayout<KVT, D, WK>::kSmem + 4 * 16 * 4;
     static bool attr_set = false;
     auto kern = attention_prefill_mma_kernel<KVT, D, WK>;
     if (!attr_set) {
@@ -538,11 +637,26 @@ static int launch_prefill(const AttnParams& p, dim3 grid, int hg) {
 
 template <typename KVT, int D>
 static int launch_prefill_d(const AttnParams& p) {
-    const int G = p.Q / p.KV, hg = G % 4 == 0 ? 4 : G % 2 == 0 ? 2 : 1;
-    const int tiles = (p.T + 15) / 16, pt = 4 / hg;
-    const dim3 shared(p.Q / hg, (tiles + pt - 1) / pt), split(p.Q, tiles);
-    if ((int)(shared.x * shared.y) >= sm_count()) return launch_prefill<KVT, D, 1>(p, shared, hg);
-    return launch_prefill<KVT, D, 4>(p, split, 1);
+    const int G = p.Q / p.KV, tiles = (p.T + 15) / 16, sms = sm_count();
+    // heads of a CTA and its grid where `wk` warps share a row tile's keys
+    auto heads = [&](int wk) { return wk == 1 && G % 4 == 0 ? 4 : wk <= 2 && G % 2 == 0 ? 2 : 1; };
+    auto grid = [&](int wk) {
+        const int pt = 4 / wk / heads(wk);
+        return dim3(p.Q / heads(wk), (tiles + pt - 1) / pt);
+    };
+    auto ctas = [&](int wk) { return (int)(grid(wk).x * grid(wk).y); };
+    // Few CTAs: their keys over more warps.  Rotation and attention in us with 1, 2 and 4 warps per row tile, 20 heads of 128:
+    //   fp16 cache, rows  112  20/16/13    128  22/16/17   160  23/21/18    256  30/22/26    400  41/34/40   640  71/46/69
+    //                    1000 101/79/128  1250 112/114/182  1531 140/152/252
+    //   fp32 cache        400  84/68/61    512 100/86/87    800 168/128/175   1000 206/183/260   1250 252/285/390
+    // so four warps until two would fill the SMs (fp32: twice), but where four need little more than one CTA per SM (128 rows:
+    // 160) two; one warp from 2.7 (2.4) CTAs per SM on, since every key row is then fetched for four row tiles at once.
+    constexpr bool kHalf = sizeof(KVT) == 2;
+    const bool whole = kHalf ? 3 * ctas(1) >= 8 * sms : 5 * ctas(1) >= 12 * sms;
+    const bool halves = kHalf ? ctas(2) >= sms || (ctas(4) > sms && 5 * ctas(4) <= 6 * sms) : ctas(2) >= 2 * sms;
+    if (whole) return launch_prefill<KVT, D, 1>(p, grid(1), heads(1));
+    if (halves) return launch_prefill<KVT, D, 2>(p, grid(2), heads(2));
+    return launch_prefill<KVT, D, 4>(p, grid(4), heads(4));
 }
 
 int attention_prefill_mma(const AttnParams& p, int kv_is_fp16, int* handled) {

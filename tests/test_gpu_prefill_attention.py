@@ -109,3 +109,16 @@ def test_values_that_are_not_finite_stay_where_they_belong(Q, KV, D, T, ctx, kv,
     scale = np.abs(want[ok]).max() if what == "huge values" else 1.0
     # two roundings of the same sums of values of order 1 (of the largest)
     assert np.abs(got[ok] / scale - want[ok] / scale).max() <= 2.0**-18
+
+
+@pytest.mark.parametrize("kv", ["fp16", "fp32"])
+# four, two and one warps per row tile by the CTAs they make (20 heads x 128 rows: two), and heads that share no key rows in pairs
+@pytest.mark.parametrize("Q,KV,D,T,ctx", [(20, 5, 128, 112, 3), (20, 5, 128, 129, 0), (20, 5, 128, 177, 0), (3, 1, 64, 1025, 40),
+                                          (25, 5, 128, 513, 0), (40, 5, 128, 900, 0), (7, 7, 64, 1040, 0)])
+def test_every_split_of_the_rows_and_keys(Q, KV, D, T, ctx, kv):
+    a = Attention(Q, KV, D, T, ctx, kv, 6.0)
+    got, q, ck, cv = a.run(T)
+    plain, _, _, _ = a.run(8)
+    want = a.exact(q, ck, cv)
+    err, ref = (np.linalg.norm(x - want) / np.linalg.norm(want) for x in (got, plain))
+    assert err <= 1.1 * ref + 2e-8                 # as above: two roundings of the same sums
