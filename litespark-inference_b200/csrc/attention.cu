@@ -11,22 +11,13 @@
 #include <cooperative_groups.h>
 #include <stdlib.h>
 
+#include "attention_core.cuh"
 #include "internal.cuh"
 
 namespace lspk {
 
 constexpr int kAttnThreads = 256;
 constexpr int kAttnWarps = kAttnThreads / 32;
-
-template <typename KVT> __device__ __forceinline__ float kv_load(const KVT* p);
-template <> __device__ __forceinline__ float kv_load<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float kv_load<__half>(const __half* p) { return __half2float(*p); }
-template <typename KVT> __device__ __forceinline__ KVT kv_make(float v);
-template <> __device__ __forceinline__ float kv_make<float>(float v) { return v; }
-template <> __device__ __forceinline__ __half kv_make<__half>(float v) { return __float2half_rn(v); }
-template <typename KVT> __device__ __forceinline__ float kv_round(float v);
-template <> __device__ __forceinline__ float kv_round<float>(float v) { return v; }
-template <> __device__ __forceinline__ float kv_round<__half>(float v) { return __half2float(__float2half_rn(v)); }
 
 // Rotate q in place and write rotated k and raw v into the cache, for T rows.  A thread takes V elements of a head and the V they
 // are rotated with (of a row of v: V in each half): it has read all it needs before it writes, and a prompt of few rows spreads
@@ -89,40 +80,6 @@ __global__ void __launch_bounds__(kAttnThreads) rope_store_kernel(const AttnPara
     }
     *reinterpret_cast<Vec*>(dst) = lo;
     *reinterpret_cast<Vec*>(dst + half) = hi;
-}
-
-// 16 bytes of cache row -> fp32 values (8 halves or 4 floats).
-template <typename KVT> struct KvVec;
-template <> struct KvVec<__half> {
-    static constexpr int N = 8;
-    static __device__ __forceinline__ void unpack(const uint4& c, float* f) {
-        const __half2* h = reinterpret_cast<const __half2*>(&c);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 v = __half22float2(h[i]);
-            f[2 * i] = v.x;
-            f[2 * i + 1] = v.y;
-        }
-    }
-};
-template <> struct KvVec<float> {
-    static constexpr int N = 4;
-    static __device__ __forceinline__ void unpack(const uint4& c, float* f) {
-        f[0] = __uint_as_float(c.x);
-        f[1] = __uint_as_float(c.y);
-        f[2] = __uint_as_float(c.z);
-        f[3] = __uint_as_float(c.w);
-    }
-};
-
-// Order-preserving map float -> uint32 (and back), so that a maximum over possibly negative floats
-// can use the integer warp reduction.
-__device__ __forceinline__ uint32_t float_to_ordered(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ordered_to_float(uint32_t u) {
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
 // One CTA per (query head, row).  Built for latency, not bandwidth (one head's K and V are at

@@ -609,6 +609,7 @@ int linear_cuda_core(const lspk_linear_args* a) { return linear_rows(a, nullptr,
 using namespace lspk;
 
 static int g_force_path = 0;   // 0 auto, 1 CUDA-core only, 2 tensor-core only
+int lspk::linear_forced_path() { return g_force_path; }
 
 extern "C" int lspk_linear_force_path(int path) {
     LSPK_REQUIRE(path >= 0 && path <= 2, "lspk_linear_force_path: path must be 0, 1 or 2");

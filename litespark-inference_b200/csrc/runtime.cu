@@ -88,10 +88,10 @@ __global__ void argmax_rows_kernel(const float* __restrict__ logits, int V, unsi
 // End of a decode step: turn the argmax keys into token ids, make them the next step's input,
 // append them to the output list, advance every position, clear the keys.
 // host_pkt (optional, one sequence): mapped host word that receives (count of host-fed steps << 32 | token) in one
-// 8-byte store, so that a host that sees the count has the token.
+// 8-byte store, so that a host that sees the count has the token.  chain_steps (optional): steps whose layers ran as one kernel.
 __global__ void finish_step_kernel(int* __restrict__ ctl, unsigned long long* __restrict__ best,
                                    int* __restrict__ tokens_out, int batch, int out_cap,
-                                   unsigned long long* host_pkt, unsigned* host_seq) {
+                                   unsigned long long* host_pkt, unsigned* host_seq, unsigned* chain_steps) {
     grid_dependency_launch();
     grid_dependency_wait();
     const int b = threadIdx.x;
@@ -111,6 +111,7 @@ __global__ void finish_step_kernel(int* __restrict__ ctl, unsigned long long* __
     }
     __syncthreads();
     if (b == 0) ctl[2 * batch] += 1;
+    if (b == 0 && chain_steps) *chain_steps += 1u;
 }
 
 __global__ void advance_pos_kernel(int* __restrict__ ctl, int seq, int by) {
@@ -131,7 +132,7 @@ int launch_argmax_rows(const float* logits, int rows, int V, unsigned long long*
 }
 int launch_finish_step(int* ctl, unsigned long long* best, int* tokens_out, int batch, int out_cap) {
     LSPK_CUDA(launch(finish_step_kernel, dim3(1), dim3(((batch + 31) / 32) * 32), 0, true, ctl, best, tokens_out,
-                     batch, out_cap, (unsigned long long*)nullptr, (unsigned*)nullptr));
+                     batch, out_cap, (unsigned long long*)nullptr, (unsigned*)nullptr, (unsigned*)nullptr));
     return LSPK_OK;
 }
 
@@ -358,12 +359,10 @@ static int enqueue_step(State* s, bool store_logits, bool host_io = false) {
                      m->emb.kind, (const void*)m->emb.data, (const float*)m->emb.scale, s->x, H, V, (const int*)s->ctl,
                      (const float*)s->rope_cos, (const float*)s->rope_sin, s->rope_cur, m->D() / 2, host_io ? 1 : 0));
     s->rope_cur_valid = true;
-    for (int li = 0; li < c.num_layers; ++li)
-        if (int rc = run_layer(s, li, B, B > 1, 0)) {
-            s->rope_cur_valid = false;
-            return rc;
-        }
+    int rc = s->chained ? decode_chain_launch(s) : LSPK_OK;
+    for (int li = 0; li < c.num_layers && !s->chained && !rc; ++li) rc = run_layer(s, li, B, B > 1, 0);
     s->rope_cur_valid = false;
+    if (rc) return rc;
     const DevTable& head = m->head.data ? m->head : m->emb;
     if (B == 1) {
         if (int rc = lm_head_launch(head.kind, head.data, head.scale, s->x, store_logits ? s->logits : nullptr, 1, V, H,
@@ -377,7 +376,7 @@ static int enqueue_step(State* s, bool store_logits, bool host_io = false) {
     }
     LSPK_CUDA(launch(finish_step_kernel, dim3(1), dim3(((B + 31) / 32) * 32), 0, true, s->ctl, s->best,
                      s->tokens_out, B, s->t_max, host_io ? s->io_pkt_dev : (unsigned long long*)nullptr,
-                     host_io ? s->io_seq_dev : (unsigned*)nullptr));
+                     host_io ? s->io_seq_dev : (unsigned*)nullptr, s->chained ? s->chain : (unsigned*)nullptr));
     return LSPK_OK;
 }
 
@@ -385,7 +384,7 @@ static void destroy_state(State* s) {
     cudaStreamSynchronize(stream());
     for (auto& g : s->graph)
         if (g) cudaGraphExecDestroy(g);
-    void* dev[] = {s->cache_k, s->cache_v, s->rope_cos, s->rope_sin, s->rope_cur, s->ctl, s->best, s->tokens_out, s->x, s->q, s->k,
+    void* dev[] = {s->chain, s->cache_k, s->cache_v, s->rope_cos, s->rope_sin, s->rope_cur, s->ctl, s->best, s->tokens_out, s->x, s->q, s->k,
                    s->v, s->attn, s->inter, s->logits, s->tok_rows};
     for (void* p : dev) cudaFree(p);
     if (s->h_int) cudaFreeHost(s->h_int);
@@ -402,6 +401,7 @@ static int clear_state(State* s) {
     LSPK_CUDA(cudaMemsetAsync(s->cache_v, 0, cache_bytes, stream()));
     LSPK_CUDA(cudaMemsetAsync(s->ctl, 0, (size_t)(2 * s->batch + 1) * 4, stream()));
     LSPK_CUDA(cudaMemsetAsync(s->best, 0, (size_t)s->batch * 8, stream()));
+    LSPK_CUDA(decode_chain_clear(s));
     s->host_pos.assign(s->batch, 0);
     return LSPK_OK;
 }
@@ -418,12 +418,19 @@ static int batch_variant(const State* s, int ahead) {
     return attention_group_heads(s->batch, c.num_heads, c.num_kv_heads, s->m->D(), s->t_max, s->kv_fp16, longest, total) ? 3 : 1;
 }
 
+// The kind of a step of one sequence `ahead` steps from now: with the layers as one kernel where that takes it.
+static int single_variant(State* s, int kind, int ahead) {
+    return decode_chain_fits(s, s->host_pos[0] + ahead + 1) ? kind + 4 : kind;
+}
+
 static int build_graph(State* s, int variant) {
     if (int rc = reserve_rows(s, s->batch)) return rc;
     auto enqueue_variant = [&]() {
+        const int kind = variant & 3;
         s->group_heads = variant == 3;
-        const int rc = enqueue_step(s, variant == 1 || variant == 3, variant == 2);
-        s->group_heads = false;
+        s->chained = variant >= 4;
+        const int rc = enqueue_step(s, kind == 1 || kind == 3, kind == 2);
+        s->group_heads = s->chained = false;
         return rc;
     };
     if (s->graph[variant] && s->graph_gen[variant] == scratch_generation()) return LSPK_OK;
@@ -443,13 +450,16 @@ static int build_graph(State* s, int variant) {
     if (warm_gen != scratch_generation()) {
         const int nctl = 2 * s->batch + 1;
         std::vector<int> saved(nctl);
+        unsigned long long recorded = 0;           // of a trace: the warm-up is none of its steps
         LSPK_CUDA(cudaMemcpyAsync(saved.data(), s->ctl, nctl * sizeof(int), cudaMemcpyDeviceToHost, stream()));
+        if (trace_buffer()) LSPK_CUDA(cudaMemcpyAsync(&recorded, trace_buffer(), 8, cudaMemcpyDeviceToHost, stream()));
         LSPK_CUDA(cudaStreamSynchronize(stream()));
         if (int rc = enqueue_variant()) return rc;
         LSPK_CUDA(cudaStreamSynchronize(stream()));
         LSPK_CUDA(cudaMemcpyAsync(s->ctl, saved.data(), nctl * sizeof(int), cudaMemcpyHostToDevice, stream()));
+        if (trace_buffer()) LSPK_CUDA(cudaMemcpyAsync(trace_buffer(), &recorded, 8, cudaMemcpyHostToDevice, stream()));
         LSPK_CUDA(cudaStreamSynchronize(stream()));
-        if (variant == 2) s->io_seq += 1;          // the warm-up step counted itself on the device
+        if ((variant & 3) == 2) s->io_seq += 1;          // the warm-up step counted itself on the device
         warm_gen = scratch_generation();
     }
 
@@ -795,9 +805,10 @@ int lspk_forward_step(lspk_state_t h, const int* tokens_host, float* logits_host
         // One sequence, token id in, token id out: no copy operations and no stream wait.  The step's first kernel
         // reads the token from mapped pinned memory; its last kernel stores (count << 32 | next token) there.
         *(volatile int*)s->io_tok = tokens_host[0];
-        if (int rc = build_graph(s, 2)) return rc;
+        const int kind = single_variant(s, 2, 0);
+        if (int rc = build_graph(s, kind)) return rc;
         const unsigned want = ++s->io_seq;
-        LSPK_CUDA(cudaGraphLaunch(s->graph[2], stream()));
+        LSPK_CUDA(cudaGraphLaunch(s->graph[kind], stream()));
         unsigned long long pkt = 0;
         for (unsigned spins = 1;; ++spins) {
             pkt = *(volatile unsigned long long*)s->io_pkt;
@@ -818,7 +829,7 @@ int lspk_forward_step(lspk_state_t h, const int* tokens_host, float* logits_host
         s->host_pos[0] += 1;
         return LSPK_OK;
     }
-    const int variant = B > 1 ? batch_variant(s, 0) : logits_host ? 1 : 0;
+    const int variant = B > 1 ? batch_variant(s, 0) : single_variant(s, logits_host ? 1 : 0, 0);
     if (logits_host)
         if (int rc = reserve_host_logits(s)) return rc;
     if (int rc = build_graph(s, variant)) return rc;
@@ -845,8 +856,8 @@ int lspk_decode_greedy(lspk_state_t h, const int* first_tokens_host, int n_steps
         if (s->host_pos[b] + n_steps > s->t_max)
             return fail(LSPK_ERR_STATE, "inference state exhausted: pos=%d + %d steps > t_max=%d", s->host_pos[b],
                         n_steps, s->t_max);
-    // several sequences: positions only grow, so there is one change of kind at most
-    auto variant_at = [&](int i) { return B > 1 ? batch_variant(s, i) : 0; };
+    // positions only grow, so there is one change of kind at most
+    auto variant_at = [&](int i) { return B > 1 ? batch_variant(s, i) : single_variant(s, 0, i); };
     const int kinds[3] = {variant_at(n_steps - 1), variant_at(0), variant_at(n_steps - 1)};
     for (int kind : kinds)      // the last again, should the first have moved scratch
         if (int rc = build_graph(s, kind)) return rc;

@@ -72,10 +72,13 @@ struct State {
     unsigned* io_seq_dev = nullptr;        // device: steps of this kind finished so far
     unsigned io_seq = 0;                   // host: the same count
     // [0] no logits store, [1] with logits, [2] host-fed step, [3] several long sequences: as [1], the attention of two query
-    // heads per CTA
-    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
-    unsigned graph_gen[4] = {0, 0, 0, 0};   // scratch_generation() at capture: a later move of library scratch voids the graph
+    // heads per CTA; [4], [5], [6]: as [0], [1], [2], the layers as one kernel (decode_chain.cu)
+    cudaGraphExec_t graph[7] = {};
+    unsigned graph_gen[7] = {};             // scratch_generation() at capture: a later move of library scratch voids the graph
     bool group_heads = false;            // while the kernels of a step of kind [3] are being enqueued
+    bool chained = false;                // while those of a step of kind [4], [5] or [6] are
+    unsigned* chain = nullptr;           // the words that kernel hands over (decode_chain_fits)
+    int chain_fits = -1;                 // whether it takes this state, -1: not asked yet
     int graph_nodes = 0;
     size_t bytes = 0;
     size_t kv_elem() const { return kv_fp16 ? 2 : 4; }
@@ -86,5 +89,10 @@ struct State {
 // runtime.cu: one transformer layer for `rows` rows held in the state's scratch buffers (see its definition).
 int run_layer(State* s, int li, int rows, bool per_row_seq, int seq, bool skip_attention = false);
 size_t table_bytes(int kind, int V, int H);
+// decode_chain.cu: the layers of a one-sequence step as one kernel.  Whether a step that attends to `keys` positions takes it (makes
+// the state's buffer on first use), the buffer as it has to be before a first step, the launch.
+bool decode_chain_fits(State* s, int keys);
+cudaError_t decode_chain_clear(State* s);
+int decode_chain_launch(State* s);
 
 }  // namespace lspk
