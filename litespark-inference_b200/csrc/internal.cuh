@@ -67,6 +67,7 @@ __host__ __device__ inline int mma_row_stride(int Kp) { return (Kp % 128 == 0) ?
 
 // linear.cu: validate + launch the CUDA-core ternary linear kernel on the library stream.
 int linear_cuda_core(const lspk_linear_args* a);
+int linear_auto(const lspk_linear_args* a);         // or the tensor-core GEMM, by the number of rows (no forced path)
 int linear_forced_path();                           // lspk_linear_force_path's, 0: none
 
 // gemm_tc.cu: tcgen05 tensor-core path for large M.  Returns LSPK_OK and sets *handled = 1 when it

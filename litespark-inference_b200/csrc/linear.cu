@@ -603,6 +603,11 @@ static int linear_rows(const lspk_linear_args* a, int* row_ctas, int* resident) 
     return linear_mma_launch(p, pair, groups < per_wave ? groups : per_wave > 0 ? per_wave : 1, tiles);
 }
 int linear_cuda_core(const lspk_linear_args* a) { return linear_rows(a, nullptr, nullptr); }
+int linear_auto(const lspk_linear_args* a) {
+    int handled = 0;
+    if (int rc = linear_tensor_core(a, &handled, false)) return rc;
+    return handled ? LSPK_OK : linear_cuda_core(a);
+}
 
 }  // namespace lspk
 

@@ -38,3 +38,26 @@ def test_batched_state_update_matches_oracle(port, nheads, B):
             ssm = st[b, layer.conv_dim * 4:].reshape(nheads, 64, 128)
             assert np.allclose(ssm, ost[b].ssm, rtol=1e-4, atol=1e-4 * np.abs(ost[b].ssm).max()), (step, b)
     dmb.free()
+
+
+@pytest.mark.parametrize("B", [8, 9, 16, 33])
+def test_a_sequence_does_not_depend_on_its_batch(B):
+    """Projections of one row, of eight-row tiles and of the tensor-core GEMM: the same integer sums and the same roundings."""
+    cfg = hyb.HybridConfig(hidden_size=256, num_layers=2, vocab_size=64, num_experts=2, intermediate_size=64, nheads=5,
+                           headdim=64, d_state=128)
+    layer = next(L for L in hyb.random_hybrid(cfg, seed=2, norm_jitter=0.1).layers if L.kind == "mamba")
+    dmb = hyb.DeviceMamba(layer, cfg.hidden_size, cfg.rms_norm_eps)
+    x = np.random.default_rng(B).standard_normal((B, cfg.hidden_size)).astype(np.float32)
+
+    def step(rows):
+        state = dev.DeviceArray((len(rows), dmb.state_floats), np.float32)
+        state.fill_bytes(0)
+        dx = dev.DeviceArray.from_numpy(rows)
+        dmb.step(dx, state, dev.DeviceArray.from_numpy(np.zeros(len(rows), np.int32)), len(rows))
+        return dx.numpy(), state.numpy()
+
+    got, states = step(x)
+    for b in (0, B // 2, B - 1):
+        one, state = step(x[b:b + 1])
+        assert np.array_equal(got[b], one[0]) and np.array_equal(states[b], state[0])
+    dmb.free()
