@@ -87,7 +87,8 @@ int lspk_hybrid_step(lspk_hybrid_state_t s, const int* tokens_host, float* logit
 /* n_steps chained greedy steps on the device (argmax feeds the next step); tokens_out_host [n_steps, B]. */
 int lspk_hybrid_decode_greedy(lspk_hybrid_state_t s, const int* first_tokens_host, int n_steps, int* tokens_out_host);
 /* Feed a prompt (one sequence at a time would break lock step, so: the same number of tokens for
- * every sequence, tokens_host [T, B]); the recurrence makes this a loop of T steps on the device. */
+ * every sequence, tokens_host [T, B]).  Positions share their products and the reads of the recurrent state;
+ * results equal those of T steps bit for bit. */
 int lspk_hybrid_prefill(lspk_hybrid_state_t s, const int* tokens_host, int T, int* next_tokens_host);
 int lspk_hybrid_step_kernel_count(lspk_hybrid_state_t s);
 

@@ -91,10 +91,13 @@ int launch_finish_step(int* ctl, unsigned long long* best, int* tokens_out, int 
 struct Moe;
 struct Mamba;
 int moe_reserve(Moe* m, int B);
+size_t moe_scratch_bytes(const Moe* m, int B);
 int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int32_t* acc_gate, int32_t* acc_up,
-                int32_t* acc_down);
+                int32_t* acc_down, void* scratch);
 int mamba_reserve(Mamba* m, int B);
+size_t mamba_scratch_bytes(const Mamba* m, int rows);
 int mamba_step(Mamba* m, float* x, float* state, const int* pos, int B);
+int mamba_prefill(Mamba* m, float* x, float* state, const int* pos, int t0, int T, int B, void* scratch);
 size_t mamba_state_floats(const Mamba* m);
 
 // attention.cu

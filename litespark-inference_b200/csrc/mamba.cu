@@ -20,26 +20,25 @@ struct Mamba {
     lspk_weight_t in_proj = nullptr, out_proj = nullptr;
     float *conv_w = nullptr, *conv_b = nullptr, *A = nullptr, *dt_bias = nullptr, *D = nullptr;
     uint16_t *norm = nullptr, *gnorm = nullptr;
-    int cap_B = 0;
-    float *zx = nullptr, *v = nullptr;      // [B][in_out], [B][d_inner]
+    int cap_B = 0;                          // rows that `scratch` holds
+    void* scratch = nullptr;                // mamba_scratch_bytes(cap_B): [rows][in_out], [rows][d_inner]
     size_t bytes = 0;
     size_t state_floats() const { return (size_t)conv_dim * 4 + (size_t)cfg.nheads * cfg.headdim * cfg.d_state; }
 };
 
 __device__ __forceinline__ float silu_f(float v) { return __fdiv_rn(v, __fadd_rn(expf(-v), 1.0f)); }
 
-// depthwise conv step of one channel (ring of the last four inputs, width 4) + SiLU
-__device__ __forceinline__ float conv_silu(float bias, const float4& taps, const float4& hist, float newv, int pos) {
-    const float h4[4] = {hist.x, hist.y, hist.z, hist.w};
-    const float w4[4] = {taps.x, taps.y, taps.z, taps.w};
-    float acc = bias;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const int sl = (pos - 3 + j) & 3;
-        const float hv = sl == 0 ? h4[0] : sl == 1 ? h4[1] : sl == 2 ? h4[2] : h4[3];
-        acc = __fadd_rn(acc, __fmul_rn(w4[j], hv));
-    }
-    return silu_f(__fadd_rn(acc, __fmul_rn(w4[3], newv)));
+// depthwise conv (width 4) of one channel at one position + SiLU: the three inputs before it, oldest first, and its own
+__device__ __forceinline__ float conv_silu(float bias, const float4& taps, float h0, float h1, float h2, float newv) {
+    float acc = __fadd_rn(bias, __fmul_rn(taps.x, h0));
+    acc = __fadd_rn(acc, __fmul_rn(taps.y, h1));
+    acc = __fadd_rn(acc, __fmul_rn(taps.z, h2));
+    return silu_f(__fadd_rn(acc, __fmul_rn(taps.w, newv)));
+}
+// slot (pos & 3) of a channel's ring of inputs
+__device__ __forceinline__ float ring_at(const float4& ring, int pos) {
+    const int sl = pos & 3;
+    return sl == 0 ? ring.x : sl == 1 ? ring.y : sl == 2 ? ring.z : ring.w;
 }
 // four states of a row: state * dA + dtx * B, and their part of the row's output
 __device__ __forceinline__ void ssu_update(float4& s4, float dA, float dtx, const float4& Bv, const float4& Cv, float& ysum) {
@@ -125,7 +124,7 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     for (int k = 0; k < 2; ++k) {
         if (k == 0 || second) {
             const int idx = tid + 256 * k;
-            const float act = conv_silu(bias[k], taps[k], hist[k], newv[k], pos);
+            const float act = conv_silu(bias[k], taps[k], ring_at(hist[k], pos - 3), ring_at(hist[k], pos - 2), ring_at(hist[k], pos - 1), newv[k]);
             if (idx < ROWS) xs_s[idx] = act;
             else if (idx < ROWS + N) B_s[idx - ROWS] = act;
             else C_s[idx - ROWS - N] = act;
@@ -156,31 +155,149 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     }
 }
 
+// The positions of a prompt, T of every sequence (row t * batch + b of zx), as mamba2_ssu_kernel would take them one by one:
+// the same operations in the same order on every value.  What bounds it: HBM on the state, as there, but read and written once
+// for T positions, then the recurrence's chain.  The convolution has no recurrence (an input and the three before it), so
+// eight positions of every channel are made at once, a thread per channel, with their loads in flight together; the eight
+// steps of the state that follow need no barrier, and each of a row's eight lanes then finishes the output of one position.
+// The ring of inputs is left to mamba2_ring_kernel: other CTAs may not have read it yet.  128 positions of one sequence, 80 heads:
+// 87 us cold (as steps, 128 x 5).
+constexpr int kScan = 8;                       // positions per round: the lanes of a row
+__global__ void __launch_bounds__(256)
+mamba2_scan_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr, int t0, int T,
+                   const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ A,
+                   const float* __restrict__ dt_bias, const float* __restrict__ Dskip, float* __restrict__ vout,
+                   int d_inner, int conv_dim, int in_out, size_t state_floats) {
+    constexpr int P = 64, N = 128, NCH = ROWS + 2 * N;
+    __shared__ __align__(16) float act_s[kScan][NCH];          // x rows, B, C
+    __shared__ float dt_s[kScan], dA_s[kScan];
+    const int batch = gridDim.y, b = blockIdx.y, head = blockIdx.x >> 1, p0 = (blockIdx.x & 1) * ROWS;
+    const int tid = threadIdx.x, seg = tid & 7, p = tid >> 3;
+    grid_dependency_launch();
+    grid_dependency_wait();
+    float4 st[4];
+    float4* const srow = reinterpret_cast<float4*>(state + (size_t)b * state_floats + (size_t)conv_dim * 4 +
+                                                   (size_t)(head * P + p0 + p) * N) + seg;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) st[q] = srow[8 * q];
+    const int pos = pos_ptr[b] + t0;
+    const float dt_b = dt_bias[head], a_head = A[head], d_head = Dskip[head];
+    const float* const zx_b = zx + (size_t)b * in_out;         // row t at t * step
+    const size_t step = (size_t)batch * in_out;
+    // this thread's channels: tid and, the first NCH - 256 threads, a second one
+    const bool second = tid < NCH - 256;
+    int cch[2];
+    float bias[2], h0[2], h1[2], h2[2];
+    float4 taps[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int idx = tid + 256 * k;
+        cch[k] = idx < ROWS ? head * P + p0 + idx : d_inner + (idx - ROWS);
+        if (k == 0 || second) {
+            bias[k] = conv_b[cch[k]];
+            taps[k] = *reinterpret_cast<const float4*>(conv_w + (size_t)cch[k] * 4);
+            const float4 ring = *reinterpret_cast<const float4*>(state + (size_t)b * state_floats + (size_t)cch[k] * 4);
+            h0[k] = ring_at(ring, pos - 3);
+            h1[k] = ring_at(ring, pos - 2);
+            h2[k] = ring_at(ring, pos - 1);
+        }
+    }
+    for (int tb = 0; tb < T; tb += kScan) {
+        const int nt = min(kScan, T - tb);
+        const float* const rows = zx_b + (size_t)tb * step;
+        const float z_gate = seg < nt ? rows[(size_t)seg * step + head * P + p0 + p] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (k == 1 && !second) break;
+            float v[kScan];
+#pragma unroll
+            for (int t = 0; t < kScan; ++t) v[t] = t < nt ? rows[(size_t)t * step + d_inner + cch[k]] : 0.0f;
+#pragma unroll
+            for (int t = 0; t < kScan; ++t) {
+                if (t >= nt) break;
+                act_s[t][tid + 256 * k] = conv_silu(bias[k], taps[k], h0[k], h1[k], h2[k], v[t]);
+                h0[k] = h1[k];
+                h1[k] = h2[k];
+                h2[k] = v[t];
+            }
+        }
+        if (tid >= 256 - kScan && tid - (256 - kScan) < nt) {
+            const int t = tid - (256 - kScan);
+            const float dv = __fadd_rn(rows[(size_t)t * step + d_inner + conv_dim + head], dt_b);
+            const float dt = dv > 20.0f ? dv : log1pf(expf(dv));
+            dt_s[t] = dt;
+            dA_s[t] = expf(__fmul_rn(dt, a_head));
+        }
+        __syncthreads();
+        float mine = 0.0f;
+#pragma unroll 2
+        for (int t = 0; t < nt; ++t) {
+            const float dtx = __fmul_rn(dt_s[t], act_s[t][p]), dA = dA_s[t];
+            const float4* const Bs = reinterpret_cast<const float4*>(&act_s[t][ROWS]) + seg;
+            const float4* const Cs = reinterpret_cast<const float4*>(&act_s[t][ROWS + N]) + seg;
+            float ysum = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ssu_update(st[q], dA, dtx, Bs[8 * q], Cs[8 * q], ysum);
+            ysum = ssu_row_sum(ysum);                          // the same in all eight lanes
+            if (t == seg) mine = ysum;
+        }
+        if (seg < nt) {
+            const float y = __fadd_rn(mine, __fmul_rn(d_head, act_s[seg][p]));
+            vout[((size_t)(tb + seg) * batch + b) * d_inner + head * P + p0 + p] = __fmul_rn(y, silu_f(z_gate));
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) srow[8 * q] = st[q];
+}
+
+// behind mamba2_scan_kernel: the last four of the T positions' convolution inputs into their slots
+__global__ void __launch_bounds__(256)
+mamba2_ring_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr, int t0, int T,
+                   int d_inner, int conv_dim, int in_out, size_t state_floats) {
+    grid_dependency_launch();
+    grid_dependency_wait();
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, batch = gridDim.y;
+    if (c >= conv_dim) return;
+    float* const ring = state + (size_t)b * state_floats + (size_t)c * 4;
+    const int pos = pos_ptr[b] + t0;
+    for (int t = max(0, T - 4); t < T; ++t) ring[(pos + t) & 3] = zx[((size_t)t * batch + b) * in_out + d_inner + c];
+}
+
 size_t mamba_state_floats(const Mamba* m) { return m->state_floats(); }
+
+size_t mamba_scratch_bytes(const Mamba* m, int rows) { return (size_t)rows * (m->in_out + m->d_inner) * 4 + 256; }
 
 int mamba_reserve(Mamba* m, int B) {
     if (B <= m->cap_B) return LSPK_OK;
-    cudaFree(m->zx);
-    cudaFree(m->v);
-    m->zx = m->v = nullptr;
+    cudaFree(m->scratch);
+    m->scratch = nullptr;
+    if (m->cap_B) m->bytes -= mamba_scratch_bytes(m, m->cap_B);
     m->cap_B = 0;
     scratch_moved();
-    LSPK_CUDA(device_malloc((void**)&m->zx, (size_t)B * m->in_out * 4));
-    LSPK_CUDA(device_malloc((void**)&m->v, (size_t)B * m->d_inner * 4));
-    m->bytes += (size_t)B * (m->in_out + m->d_inner) * 4;
+    LSPK_CUDA(device_malloc(&m->scratch, mamba_scratch_bytes(m, B)));
+    m->bytes += mamba_scratch_bytes(m, B);
     m->cap_B = B;
     return LSPK_OK;
 }
 
-int mamba_step(Mamba* m, float* x, float* state, const int* pos, int B) {
+// T positions of B sequences (row t * B + b of x), the first at pos[b] + t0.  scratch (optional): mamba_scratch_bytes(m,
+// T * B) of the caller's, else the layer's own.
+int mamba_prefill(Mamba* m, float* x, float* state, const int* pos, int t0, int T, int B, void* scratch) {
     LSPK_REQUIRE(m && x && state && pos && B >= 1, "mamba_step: bad arguments");
     LSPK_REQUIRE((reinterpret_cast<uintptr_t>(state) & 15) == 0, "mamba_step: the state buffer must be 16-byte aligned");
-    if (int rc = mamba_reserve(m, B)) return rc;
+    const int M = T * B;
+    if (!scratch) {
+        if (int rc = mamba_reserve(m, M)) return rc;
+        scratch = m->scratch;
+    }
+    float* const zx_out = static_cast<float*>(scratch);
+    float* const v = zx_out + ((size_t)M * m->in_out + 63) / 64 * 64;
     lspk_linear_args a = {};
     a.w[0] = m->in_proj;
-    a.out[0] = m->zx;
+    a.out[0] = zx_out;
     a.n_mats = 1;
-    a.M = B;
+    a.M = M;
     a.prologue = LSPK_PRO_RMSNORM_QUANT;
     a.epilogue = LSPK_EPI_STORE;
     a.x_f32 = x;
@@ -191,22 +308,31 @@ int mamba_step(Mamba* m, float* x, float* state, const int* pos, int B) {
     // sixteen the two projections of the hybrid model take 4.3 us less a layer than as two tiles of the eight-row kernel, which
     // expands the weights twice (24 steps of sixteen sequences 32.75 -> 31.55 ms).
     if (int rc = linear_auto(&a)) return rc;
-    LSPK_CUDA(launch(mamba2_ssu_kernel, dim3(m->cfg.nheads * 2, B), dim3(256), 0, true, (const float*)m->zx, state, pos,
-                     (const float*)m->conv_w, (const float*)m->conv_b, (const float*)m->A, (const float*)m->dt_bias,
-                     (const float*)m->D, m->v, m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
+    const float *zx = zx_out, *conv_w = m->conv_w, *conv_b = m->conv_b, *A = m->A, *dt_bias = m->dt_bias, *D = m->D;
+    const dim3 grid(m->cfg.nheads * 2, B);
+    if (T == 1 && t0 == 0) {
+        LSPK_CUDA(launch(mamba2_ssu_kernel, grid, dim3(256), 0, true, zx, state, pos, conv_w, conv_b, A, dt_bias, D, v,
+                         m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
+    } else {
+        LSPK_CUDA(launch(mamba2_scan_kernel, grid, dim3(256), 0, true, zx, state, pos, t0, T, conv_w, conv_b, A, dt_bias, D, v,
+                         m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
+        LSPK_CUDA(launch(mamba2_ring_kernel, dim3((m->conv_dim + 255) / 256, B), dim3(256), 0, true, zx, state, pos, t0, T,
+                         m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
+    }
     lspk_linear_args o = {};
     o.w[0] = m->out_proj;
     o.out[0] = x;
     o.n_mats = 1;
-    o.M = B;
+    o.M = M;
     o.prologue = LSPK_PRO_RMSNORM_QUANT;
     o.epilogue = LSPK_EPI_ADD;
-    o.x_f32 = m->v;
+    o.x_f32 = v;
     o.gamma = m->gnorm;
     o.gamma_is_bf16 = 1;
     o.eps = m->cfg.eps;
     return linear_auto(&o);
 }
+int mamba_step(Mamba* m, float* x, float* state, const int* pos, int B) { return mamba_prefill(m, x, state, pos, 0, 1, B, nullptr); }
 
 }  // namespace lspk
 
@@ -269,7 +395,7 @@ int lspk_mamba_free(lspk_mamba_t h) {
     cudaStreamSynchronize(stream());
     lspk_weight_free(m->in_proj);
     lspk_weight_free(m->out_proj);
-    void* dev[] = {m->conv_w, m->conv_b, m->A, m->dt_bias, m->D, m->norm, m->gnorm, m->zx, m->v};
+    void* dev[] = {m->conv_w, m->conv_b, m->A, m->dt_bias, m->D, m->norm, m->gnorm, m->scratch};
     for (void* p : dev) cudaFree(p);
     delete m;
     return LSPK_OK;

@@ -14,6 +14,7 @@
 //   moe_combine_kernel       x += w_0 y_0 + w_1 y_1
 // The expert matrices live in one device buffer [expert][gate|up|down] in the device chunk layout;
 // an expert with no routed row costs no weight traffic.
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -35,12 +36,36 @@ struct Moe {
     float* router = nullptr;         // [E][H]
     uint16_t* norm = nullptr;        // [H]
     uint16_t* sub_norm = nullptr;    // [E][I]
-    // per-call scratch, sized for cap_B token rows
-    int cap_B = 0;
-    int8_t *xq = nullptr, *xq2 = nullptr;
-    float *xs = nullptr, *xs2 = nullptr, *selw = nullptr, *inter = nullptr, *ydown = nullptr;
-    int *sel = nullptr, *sums = nullptr, *sums2 = nullptr;
+    int cap_B = 0;                   // token rows that `scratch` holds
+    void* scratch = nullptr;         // moe_scratch_bytes(cap_B)
     size_t bytes = 0;
+};
+
+// One call's buffers, carved out of one block
+struct MoeScratch {
+    int8_t *xq, *xq2;
+    float *xs, *xs2, *selw, *inter, *ydown;
+    int *sel, *sums, *sums2;
+    size_t bytes;
+    MoeScratch(const Moe* m, int B, void* block) {
+        const size_t R = 2 * (size_t)B;
+        uint8_t* at = static_cast<uint8_t*>(block);
+        auto take = [&](auto*& p, size_t n) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(at);
+            at += (n * sizeof(*p) + 255) / 256 * 256;
+        };
+        take(xq, (size_t)B * mma_row_stride(m->chunks_gu * kWeightsPerChunk));
+        take(xq2, R * mma_row_stride(m->chunks_d * kWeightsPerChunk));
+        take(sums, (size_t)B);
+        take(sums2, R);
+        take(xs, (size_t)B);
+        take(xs2, R);
+        take(sel, R);
+        take(selw, R);
+        take(inter, R * m->I);
+        take(ydown, R * m->H);
+        bytes = (size_t)(at - static_cast<uint8_t*>(block));
+    }
 };
 
 // One CTA per token row: RMSNorm, quantiser, router logits (one warp per expert, round-robin), softmax
@@ -216,45 +241,30 @@ __global__ void moe_combine_kernel(float* __restrict__ x, const float* __restric
     *reinterpret_cast<float4*>(x + (size_t)t * H + k) = v;
 }
 
-static int moe_alloc(void** p, size_t bytes, Moe* m) {
-    LSPK_CUDA(device_malloc(p, bytes ? bytes : 16));
-    m->bytes += bytes;
-    return LSPK_OK;
-}
+size_t moe_scratch_bytes(const Moe* m, int B) { return MoeScratch(m, B, nullptr).bytes; }
 
-// Make the per-call scratch large enough for B token rows (allocates; call before any graph capture).
+// Make the layer's own scratch large enough for B token rows (allocates; call before any graph capture).
 int moe_reserve(Moe* m, int B) {
     if (B <= m->cap_B) return LSPK_OK;
-    void** old[] = {(void**)&m->xq, (void**)&m->xq2, (void**)&m->xs, (void**)&m->xs2, (void**)&m->selw,
-                    (void**)&m->inter, (void**)&m->ydown, (void**)&m->sel, (void**)&m->sums, (void**)&m->sums2};
-    for (void** p : old) {
-        cudaFree(*p);
-        *p = nullptr;
-    }
-    m->cap_B = 0;               // nothing is held until every buffer below exists
+    cudaFree(m->scratch);
+    m->scratch = nullptr;
+    if (m->cap_B) m->bytes -= moe_scratch_bytes(m, m->cap_B);
+    m->cap_B = 0;
     scratch_moved();
-    const size_t R = 2 * (size_t)B;
-    int rc = 0;
-    const size_t row_gu = mma_row_stride(m->chunks_gu * kWeightsPerChunk), row_d = mma_row_stride(m->chunks_d * kWeightsPerChunk);
-    rc |= moe_alloc((void**)&m->xq, (size_t)B * row_gu, m);
-    rc |= moe_alloc((void**)&m->sums, (size_t)B * 4, m);
-    rc |= moe_alloc((void**)&m->sums2, R * 4, m);
-    rc |= moe_alloc((void**)&m->xs, (size_t)B * 4, m);
-    rc |= moe_alloc((void**)&m->sel, R * 4, m);
-    rc |= moe_alloc((void**)&m->selw, R * 4, m);
-    rc |= moe_alloc((void**)&m->inter, R * m->I * 4, m);
-    rc |= moe_alloc((void**)&m->xq2, R * row_d, m);
-    rc |= moe_alloc((void**)&m->xs2, R * 4, m);
-    rc |= moe_alloc((void**)&m->ydown, R * m->H * 4, m);
-    if (rc) return rc;
+    LSPK_CUDA(device_malloc(&m->scratch, moe_scratch_bytes(m, B)));
+    m->bytes += moe_scratch_bytes(m, B);
     m->cap_B = B;
     return LSPK_OK;
 }
 
+// scratch (optional): moe_scratch_bytes(m, B) of the caller's, else the layer's own
 int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int32_t* acc_gate, int32_t* acc_up,
-                int32_t* acc_down) {
+                int32_t* acc_down, void* scratch) {
     LSPK_REQUIRE(m && x && B >= 1, "moe_forward: bad arguments");
-    if (int rc = moe_reserve(m, B)) return rc;
+    if (!scratch) {
+        if (int rc = moe_reserve(m, B)) return rc;
+    }
+    const MoeScratch c(m, B, scratch ? scratch : m->scratch);
     const int H = m->H, I = m->I, E = m->E, R = 2 * B;
     static bool attr_set = false;
     if (!attr_set) {
@@ -266,8 +276,8 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
     const int staged = (size_t)H * 4 + extra <= 200 * 1024;     // else the router matrix is read where it lies
     LSPK_CUDA(launch(B > 1 ? moe_router_kernel<true> : moe_router_kernel<false>, dim3(B), dim3(kMoeThreads),
                      (size_t)H * 4 + (staged ? extra : 0), true, (const float*)x,
-                     (const uint16_t*)m->norm, (const float*)m->router, m->xq, m->xs, m->sel, m->selw,
-                     m->sums, H, E, m->eps, staged));
+                     (const uint16_t*)m->norm, (const float*)m->router, c.xq, c.xs, c.sel, c.selw,
+                     c.sums, H, E, m->eps, staged));
     if (B == 1) {
         // A single token: its two experts' products are one-row products whose matrices the router has just chosen.
         // Both experts of a stage go through ONE launch of the streamed batch (linear_stream.cu), which reads the
@@ -280,16 +290,16 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
             it = StreamItem{};
             it.w[0] = m->w;
             it.w[1] = m->w + m->mat_stride;
-            it.sel = m->sel + slot;
+            it.sel = c.sel + slot;
             it.sel_stride = 3 * m->mat_stride;
             it.sel_scales = m->scales;
             it.scale_idx[0] = 0;
             it.scale_idx[1] = 1;
-            it.out = m->inter + (size_t)slot * I;
+            it.out = c.inter + (size_t)slot * I;
             it.acc[0] = acc_gate ? acc_gate + (size_t)slot * I : nullptr;
             it.acc[1] = acc_up ? acc_up + (size_t)slot * I : nullptr;
-            it.x = m->xq;
-            it.xs = m->xs;
+            it.x = c.xq;
+            it.xs = c.xs;
             it.N = I;
             it.K = H;
             it.chunks = m->chunks_gu;
@@ -298,20 +308,20 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
             it.epilogue = LSPK_EPI_RELU2_MUL;
         }
         if (int rc = stream_launch(&sp)) return rc;
-        if (int rc = norm_quant_rows_selected(m->inter, m->sub_norm, m->sel, m->xq2, m->xs2, R, I, m->eps)) return rc;
+        if (int rc = norm_quant_rows_selected(c.inter, m->sub_norm, c.sel, c.xq2, c.xs2, R, I, m->eps)) return rc;
         for (int slot = 0; slot < 2; ++slot) {
             StreamItem& it = sp.it[slot];
             it = StreamItem{};
             it.w[0] = m->w + 2 * m->mat_stride;
-            it.sel = m->sel + slot;
+            it.sel = c.sel + slot;
             it.sel_stride = 3 * m->mat_stride;
             it.sel_scales = m->scales;
             it.scale_idx[0] = 2;
             it.scale_idx[1] = 2;
-            it.out = m->ydown + (size_t)slot * H;
+            it.out = c.ydown + (size_t)slot * H;
             it.acc[0] = acc_down ? acc_down + (size_t)slot * H : nullptr;
-            it.x = m->xq2 + (size_t)slot * I;
-            it.xs = m->xs2 + slot;
+            it.x = c.xq2 + (size_t)slot * I;
+            it.xs = c.xs2 + slot;
             it.N = H;
             it.K = I;
             it.chunks = m->chunks_d;
@@ -321,9 +331,9 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
         }
         sp.sel_ready = 1;              // as for several tokens below: requested under the quantiser
         if (int rc = stream_launch(&sp)) return rc;
-        LSPK_CUDA(launch(moe_combine_kernel, dim3(B, (H + 511) / 512), dim3(128), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
-        if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, m->sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
-        if (selw_out) LSPK_CUDA(cudaMemcpyAsync(selw_out, m->selw, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
+        LSPK_CUDA(launch(moe_combine_kernel, dim3(B, (H + 511) / 512), dim3(128), 0, true, x, (const float*)c.ydown, (const float*)c.selw, H));
+        if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, c.sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
+        if (selw_out) LSPK_CUDA(cudaMemcpyAsync(selw_out, c.selw, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
         return LSPK_OK;
     }
 
@@ -331,18 +341,18 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
     ExpertStreamParams p = {};
     p.w_stride = 3 * m->mat_stride;
     p.scales = m->scales;
-    p.sel = m->sel;
+    p.sel = c.sel;
     p.R = R;
     p.E = E;
     p.w[0] = m->w;
     p.w[1] = m->w + m->mat_stride;
     p.scale_idx[0] = 0;
     p.scale_idx[1] = 1;
-    p.x = m->xq;
-    p.xs = m->xs;
-    p.x_sums = m->sums;
+    p.x = c.xq;
+    p.xs = c.xs;
+    p.x_sums = c.sums;
     p.in_shift = 1;                    // routed row 2*token + slot reads token's activations
-    p.out = m->inter;
+    p.out = c.inter;
     p.acc[0] = acc_gate;
     p.acc[1] = acc_up;
     p.N = I;
@@ -351,19 +361,19 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
     p.groups = m->groups_gu;
     if (int rc = expert_stream_launch(p, true)) return rc;
     // SubLN + quantiser per routed row, with the row's expert's norm weights
-    int* const sums2 = I % 8 == 0 ? m->sums2 : nullptr;      // else natural rows: an expert's norm weights are not 16-byte aligned
-    if (int rc = norm_quant_rows_selected(m->inter, m->sub_norm, m->sel, m->xq2, m->xs2, R, I, m->eps, sums2)) return rc;
+    int* const sums2 = I % 8 == 0 ? c.sums2 : nullptr;      // else natural rows: an expert's norm weights are not 16-byte aligned
+    if (int rc = norm_quant_rows_selected(c.inter, m->sub_norm, c.sel, c.xq2, c.xs2, R, I, m->eps, sums2)) return rc;
     // The quantiser lets its successor start only once gate / up has ended (norm_quant_rows_selected), the router long
     // before: the down matrices are requested under the quantiser.
     p.sel_ready = 1;
     p.w[0] = m->w + 2 * m->mat_stride;
     p.w[1] = nullptr;
     p.scale_idx[0] = 2;
-    p.x = m->xq2;
-    p.xs = m->xs2;
+    p.x = c.xq2;
+    p.xs = c.xs2;
     p.x_sums = sums2;
     p.in_shift = 0;
-    p.out = m->ydown;
+    p.out = c.ydown;
     p.acc[0] = acc_down;
     p.acc[1] = nullptr;
     p.N = H;
@@ -371,9 +381,9 @@ int moe_forward(Moe* m, float* x, int B, int32_t* sel_out, float* selw_out, int3
     p.chunks = m->chunks_d;
     p.groups = m->groups_d;
     if (int rc = expert_stream_launch(p, false)) return rc;
-    LSPK_CUDA(launch(moe_combine_kernel, dim3(B, (H + 511) / 512), dim3(128), 0, true, x, (const float*)m->ydown, (const float*)m->selw, H));
-    if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, m->sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
-    if (selw_out) LSPK_CUDA(cudaMemcpyAsync(selw_out, m->selw, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
+    LSPK_CUDA(launch(moe_combine_kernel, dim3(B, (H + 511) / 512), dim3(128), 0, true, x, (const float*)c.ydown, (const float*)c.selw, H));
+    if (sel_out) LSPK_CUDA(cudaMemcpyAsync(sel_out, c.sel, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
+    if (selw_out) LSPK_CUDA(cudaMemcpyAsync(selw_out, c.selw, (size_t)R * 4, cudaMemcpyDeviceToDevice, stream()));
     return LSPK_OK;
 }
 
@@ -443,8 +453,7 @@ int lspk_moe_free(lspk_moe_t h) {
     if (!h) return LSPK_OK;
     Moe* m = reinterpret_cast<Moe*>(h);
     cudaStreamSynchronize(stream());
-    void* dev[] = {m->w, m->scales, m->router, m->norm, m->sub_norm, m->xq, m->xq2, m->xs, m->xs2, m->selw,
-                   m->inter, m->ydown, m->sel, m->sums, m->sums2};
+    void* dev[] = {m->w, m->scales, m->router, m->norm, m->sub_norm, m->scratch};
     for (void* p : dev) cudaFree(p);
     delete m;
     return LSPK_OK;
@@ -455,7 +464,7 @@ size_t lspk_moe_device_bytes(lspk_moe_t h) { return h ? reinterpret_cast<Moe*>(h
 int lspk_moe_forward(lspk_moe_t h, float* x_dev, int B, int32_t* sel_out, float* selw_out, int32_t* acc_gate_out,
                      int32_t* acc_up_out, int32_t* acc_down_out) {
     if (int rc = ensure_init()) return rc;
-    return moe_forward(reinterpret_cast<Moe*>(h), x_dev, B, sel_out, selw_out, acc_gate_out, acc_up_out, acc_down_out);
+    return moe_forward(reinterpret_cast<Moe*>(h), x_dev, B, sel_out, selw_out, acc_gate_out, acc_up_out, acc_down_out, nullptr);
 }
 
 }  // extern "C"

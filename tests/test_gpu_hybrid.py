@@ -258,3 +258,27 @@ def test_hybrid_full_depth_steps_match_oracle(oracle, port):
         assert np.median(errs) <= 0.5
     st.close()
     d.close()
+
+
+@pytest.mark.parametrize("B,T", [(1, 2), (1, 9), (1, 515), (3, 5), (16, 17), (64, 9), (513, 2)])
+def test_prefill_equals_the_steps(B, T):
+    """Positions of a prompt together (in passes, the last one shorter) or one by one: the same bits, twice in a row."""
+    cfg = hyb.HybridConfig(hidden_size=256, num_layers=4, vocab_size=96, num_experts=4, intermediate_size=192, nheads=4,
+                           headdim=64, d_state=128)
+    d = hyb.DeviceHybrid(hyb.random_hybrid(cfg, seed=5, norm_jitter=0.1))
+    rng = np.random.default_rng(100 * B + T)
+    prompt = rng.integers(0, cfg.vocab_size, (T, B)).astype(np.int32)
+    more = rng.integers(0, cfg.vocab_size, (T, B)).astype(np.int32)
+    together, single = hyb.HybridState(d, B, 8), hyb.HybridState(d, B, 8)
+    for part in (prompt, more):
+        got = together.prefill(part)
+        for t in range(T):
+            want = single.step(part[t])
+        assert np.array_equal(got, want)
+        if B == 1:
+            a, b = together.step(part[0], want_logits=True), single.step(part[0], want_logits=True)
+            assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    assert np.array_equal(together.decode_greedy(got, 5), single.decode_greedy(got, 5))
+    for st in (together, single):
+        st.close()
+    d.close()
