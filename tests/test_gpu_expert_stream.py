@@ -77,3 +77,23 @@ def test_many_passes_equal_single_tokens():
         dm.forward(one, 1)
         assert np.array_equal(one.numpy()[0], runs[0][t]), t
     dm.free()
+
+
+@pytest.mark.parametrize("hidden,inter", [(320, 200), (64, 4864), (5120, 64)])     # passes of 32 rows; down of 16; gate / up of 16
+@pytest.mark.parametrize("B", [41, 48, 57, 64, 65, 81])
+def test_passes_of_several_tiles(hidden, inter, B):
+    """Two experts, so that each has every token's row: tiles and passes that end anywhere.  Integer sums and the same
+    roundings in every form, so each row as the one-token kernels compute it."""
+    cfg = hyb.HybridConfig(hidden_size=hidden, num_layers=2, vocab_size=64, num_experts=2, intermediate_size=inter, nheads=2,
+                           headdim=64, d_state=128)
+    layer = next(L for L in hyb.random_hybrid(cfg, seed=3, norm_jitter=0.1).layers if L.kind == "moe")
+    dm = hyb.DeviceMoE(layer, cfg.rms_norm_eps)
+    x = np.random.default_rng(B).standard_normal((B, hidden)).astype(np.float32)
+    dx = dev.DeviceArray.from_numpy(x)
+    dm.forward(dx, B)
+    got = dx.numpy()
+    for t in range(B):
+        one = dev.DeviceArray.from_numpy(x[t:t + 1])
+        dm.forward(one, 1)
+        assert np.array_equal(one.numpy()[0], got[t]), t
+    dm.free()
