@@ -21,7 +21,7 @@ struct Mamba {
     float *conv_w = nullptr, *conv_b = nullptr, *A = nullptr, *dt_bias = nullptr, *D = nullptr;
     uint16_t *norm = nullptr, *gnorm = nullptr;
     int cap_B = 0;                          // rows that `scratch` holds
-    void* scratch = nullptr;                // mamba_scratch_bytes(cap_B): [rows][in_out], [rows][d_inner]
+    void* scratch = nullptr;                // mamba_scratch_bytes(cap_B): [rows][in_out], [rows][d_inner], a prompt's activations
     size_t bytes = 0;
     size_t state_floats() const { return (size_t)conv_dim * 4 + (size_t)cfg.nheads * cfg.headdim * cfg.d_state; }
 };
@@ -155,118 +155,157 @@ mamba2_ssu_kernel(const float* __restrict__ zx, float* __restrict__ state, const
     }
 }
 
-// The positions of a prompt, T of every sequence (row t * batch + b of zx), as mamba2_ssu_kernel would take them one by one:
-// the same operations in the same order on every value.  What bounds it: HBM on the state, as there, but read and written once
-// for T positions, then the recurrence's chain.  The convolution has no recurrence (an input and the three before it), so
-// eight positions of every channel are made at once, a thread per channel, with their loads in flight together; the eight
-// steps of the state that follow need no barrier, and each of a row's eight lanes then finishes the output of one position.
-// The ring of inputs is left to mamba2_ring_kernel: other CTAs may not have read it yet.  128 positions of one sequence, 80 heads:
-// 87 us cold (as steps, 128 x 5).
-constexpr int kScan = 8;                       // positions per round: the lanes of a row
+// The positions of a prompt, T of every sequence (row t * batch + b of zx), in two kernels: the same operations in the same
+// order on every value as mamba2_ssu_kernel's, position by position.
+//
+// mamba2_conv_kernel: what has no recurrence (the convolution is of an input and the three before it) for all positions side by
+// side, a thread per channel and eight positions; behind the channels of a row, every head's dt and dA.
+constexpr int kScan = 8;                       // positions of a round
+__host__ __device__ inline int act_stride(int conv_dim, int nheads) { return (conv_dim + 2 * nheads + 3) / 4 * 4; }
 __global__ void __launch_bounds__(256)
-mamba2_scan_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr, int t0, int T,
+mamba2_conv_kernel(const float* __restrict__ zx, const float* __restrict__ state, const int* __restrict__ pos_ptr, int t0, int T,
                    const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ A,
-                   const float* __restrict__ dt_bias, const float* __restrict__ Dskip, float* __restrict__ vout,
-                   int d_inner, int conv_dim, int in_out, size_t state_floats) {
-    constexpr int P = 64, N = 128, NCH = ROWS + 2 * N;
-    __shared__ __align__(16) float act_s[kScan][NCH];          // x rows, B, C
-    __shared__ float dt_s[kScan], dA_s[kScan];
-    const int batch = gridDim.y, b = blockIdx.y, head = blockIdx.x >> 1, p0 = (blockIdx.x & 1) * ROWS;
-    const int tid = threadIdx.x, seg = tid & 7, p = tid >> 3;
+                   const float* __restrict__ dt_bias, float* __restrict__ act, int nheads, int d_inner, int conv_dim, int in_out,
+                   size_t state_floats) {
+    const int c = blockIdx.x * 256 + threadIdx.x, batch = gridDim.y, b = blockIdx.y, tb = blockIdx.z * kScan;
+    const int nt = min(kScan, T - tb);
     grid_dependency_launch();
     grid_dependency_wait();
+    if (c >= conv_dim + nheads) return;
+    const size_t step = (size_t)batch * in_out, astep = (size_t)batch * act_stride(conv_dim, nheads);
+    const float* const raw = zx + ((size_t)tb * batch + b) * in_out + d_inner + c;
+    float* const out = act + ((size_t)tb * batch + b) * act_stride(conv_dim, nheads) + c;
+    float v[kScan];
+#pragma unroll
+    for (int t = 0; t < kScan; ++t) v[t] = t < nt ? raw[t * step] : 0.0f;
+    if (c >= conv_dim) {
+        const float dt_b = dt_bias[c - conv_dim], a_head = A[c - conv_dim];
+#pragma unroll
+        for (int t = 0; t < kScan; ++t) {
+            if (t >= nt) break;
+            const float dv = __fadd_rn(v[t], dt_b);
+            const float dt = dv > 20.0f ? dv : log1pf(expf(dv));
+            out[t * astep] = dt;
+            out[t * astep + nheads] = expf(__fmul_rn(dt, a_head));
+        }
+        return;
+    }
+    const float bias = conv_b[c];
+    const float4 taps = *reinterpret_cast<const float4*>(conv_w + (size_t)c * 4);
+    float h0, h1, h2;
+    if (tb == 0) {
+        const float4 ring = *reinterpret_cast<const float4*>(state + (size_t)b * state_floats + (size_t)c * 4);
+        const int pos = pos_ptr[b] + t0;
+        h0 = ring_at(ring, pos - 3);
+        h1 = ring_at(ring, pos - 2);
+        h2 = ring_at(ring, pos - 1);
+    } else {
+        h0 = *(raw - 3 * step);
+        h1 = *(raw - 2 * step);
+        h2 = *(raw - step);
+    }
+#pragma unroll
+    for (int t = 0; t < kScan; ++t) {
+        if (t >= nt) break;
+        out[t * astep] = conv_silu(bias, taps, h0, h1, h2, v[t]);
+        h0 = h1;
+        h1 = h2;
+        h2 = v[t];
+    }
+}
+
+// mamba2_scan_kernel: the recurrence, RW rows of a head's state per CTA, eight lanes a row as in mamba2_ssu_kernel, the state in
+// registers from the first position to the last.  What bounds it: HBM on the state, read and written once for T positions,
+// then the latency of a row's sums with few warps on an SM (pairs of floats in one instruction were no faster, and the
+// compiler fused their products and sums, which the steps' arithmetic does not).  Eight positions' inputs come into shared
+// memory under the eight before them; the steps of a round need no barrier, and each of a row's lanes finishes the output of one
+// position.  Few sequences take 8 rows a CTA, which spread evenly over the SMs, many take 32, which share the rows of B and C:
+// a prompt of 128 tokens of one sequence 2.30 : 2.48 ms, of 512 6.2 : 6.8, of 2 tokens of sixty-four 3.86 : 3.70.
+// 128 positions of one sequence, 80 heads: 44 + 5 us (87 with the convolution inside the recurrence's rounds, 160 CTAs).
+template <int RW>
+__global__ void __launch_bounds__(8 * RW)
+mamba2_scan_kernel(const float* __restrict__ zx, const float* __restrict__ act, float* __restrict__ state,
+                   const int* __restrict__ pos_ptr, int t0, int T, const float* __restrict__ Dskip, float* __restrict__ vout, int nheads,
+                   int d_inner, int conv_dim, int in_out, size_t state_floats) {
+    constexpr int P = 64, N = 128, THREADS = 8 * RW, PIECES = (RW + 2 * N) / 4;       // 16-byte pieces of a position
+    __shared__ __align__(16) float act_s[2][kScan][RW + 2 * N];                       // x rows, B, C
+    __shared__ float dt_s[2][kScan], dA_s[2][kScan];
+    const int batch = gridDim.y, b = blockIdx.y, head = blockIdx.x / (P / RW), p0 = blockIdx.x % (P / RW) * RW;
+    const int tid = threadIdx.x, seg = tid & 7, p = tid >> 3;
+    const size_t astride = act_stride(conv_dim, nheads), astep = (size_t)batch * astride, step = (size_t)batch * in_out;
+    grid_dependency_launch();
+    grid_dependency_wait();
+    const float* const act_b = act + (size_t)b * astride;
+    auto request = [&](int tb, int buf) {
+        const int nt = min(kScan, T - tb);
+        for (int i = tid; i < nt * PIECES; i += THREADS) {
+            const int t = i / PIECES, k = i % PIECES;
+            const float* src = act_b + (size_t)(tb + t) * astep + (k < RW / 4 ? head * P + p0 + 4 * k : d_inner + 4 * k - RW);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&act_s[buf][t][4 * k])), "l"(src) : "memory");
+        }
+        if (tid < nt) {
+            const float* src = act_b + (size_t)(tb + tid) * astep + conv_dim + head;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&dt_s[buf][tid])), "l"(src) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&dA_s[buf][tid])), "l"(src + nheads) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    request(0, 0);
     float4 st[4];
     float4* const srow = reinterpret_cast<float4*>(state + (size_t)b * state_floats + (size_t)conv_dim * 4 +
                                                    (size_t)(head * P + p0 + p) * N) + seg;
 #pragma unroll
     for (int q = 0; q < 4; ++q) st[q] = srow[8 * q];
-    const int pos = pos_ptr[b] + t0;
-    const float dt_b = dt_bias[head], a_head = A[head], d_head = Dskip[head];
-    const float* const zx_b = zx + (size_t)b * in_out;         // row t at t * step
-    const size_t step = (size_t)batch * in_out;
-    // this thread's channels: tid and, the first NCH - 256 threads, a second one
-    const bool second = tid < NCH - 256;
-    int cch[2];
-    float bias[2], h0[2], h1[2], h2[2];
-    float4 taps[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int idx = tid + 256 * k;
-        cch[k] = idx < ROWS ? head * P + p0 + idx : d_inner + (idx - ROWS);
-        if (k == 0 || second) {
-            bias[k] = conv_b[cch[k]];
-            taps[k] = *reinterpret_cast<const float4*>(conv_w + (size_t)cch[k] * 4);
-            const float4 ring = *reinterpret_cast<const float4*>(state + (size_t)b * state_floats + (size_t)cch[k] * 4);
-            h0[k] = ring_at(ring, pos - 3);
-            h1[k] = ring_at(ring, pos - 2);
-            h2[k] = ring_at(ring, pos - 1);
-        }
-    }
-    for (int tb = 0; tb < T; tb += kScan) {
+    const float d_head = Dskip[head];
+    int buf = 0;
+    for (int tb = 0; tb < T; tb += kScan, buf ^= 1) {
         const int nt = min(kScan, T - tb);
-        const float* const rows = zx_b + (size_t)tb * step;
-        const float z_gate = seg < nt ? rows[(size_t)seg * step + head * P + p0 + p] : 0.0f;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            if (k == 1 && !second) break;
-            float v[kScan];
-#pragma unroll
-            for (int t = 0; t < kScan; ++t) v[t] = t < nt ? rows[(size_t)t * step + d_inner + cch[k]] : 0.0f;
-#pragma unroll
-            for (int t = 0; t < kScan; ++t) {
-                if (t >= nt) break;
-                act_s[t][tid + 256 * k] = conv_silu(bias[k], taps[k], h0[k], h1[k], h2[k], v[t]);
-                h0[k] = h1[k];
-                h1[k] = h2[k];
-                h2[k] = v[t];
-            }
-        }
-        if (tid >= 256 - kScan && tid - (256 - kScan) < nt) {
-            const int t = tid - (256 - kScan);
-            const float dv = __fadd_rn(rows[(size_t)t * step + d_inner + conv_dim + head], dt_b);
-            const float dt = dv > 20.0f ? dv : log1pf(expf(dv));
-            dt_s[t] = dt;
-            dA_s[t] = expf(__fmul_rn(dt, a_head));
+        const float z_gate = seg < nt ? zx[((size_t)(tb + seg) * batch + b) * in_out + head * P + p0 + p] : 0.0f;
+        if (tb + kScan < T) {
+            request(tb + kScan, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
         float mine = 0.0f;
-#pragma unroll 2
-        for (int t = 0; t < nt; ++t) {
-            const float dtx = __fmul_rn(dt_s[t], act_s[t][p]), dA = dA_s[t];
-            const float4* const Bs = reinterpret_cast<const float4*>(&act_s[t][ROWS]) + seg;
-            const float4* const Cs = reinterpret_cast<const float4*>(&act_s[t][ROWS + N]) + seg;
+        auto position = [&](int t) {
+            const float dtx = __fmul_rn(dt_s[buf][t], act_s[buf][t][p]), dA = dA_s[buf][t];
+            const float4* const Bs = reinterpret_cast<const float4*>(&act_s[buf][t][RW]) + seg;
+            const float4* const Cs = reinterpret_cast<const float4*>(&act_s[buf][t][RW + N]) + seg;
             float ysum = 0.0f;
 #pragma unroll
             for (int q = 0; q < 4; ++q) ssu_update(st[q], dA, dtx, Bs[8 * q], Cs[8 * q], ysum);
             ysum = ssu_row_sum(ysum);                          // the same in all eight lanes
             if (t == seg) mine = ysum;
+        };
+        if (nt == kScan) {
+#pragma unroll
+            for (int t = 0; t < kScan; ++t) position(t);
+        } else {
+            for (int t = 0; t < nt; ++t) position(t);
         }
         if (seg < nt) {
-            const float y = __fadd_rn(mine, __fmul_rn(d_head, act_s[seg][p]));
+            const float y = __fadd_rn(mine, __fmul_rn(d_head, act_s[buf][seg][p]));
             vout[((size_t)(tb + seg) * batch + b) * d_inner + head * P + p0 + p] = __fmul_rn(y, silu_f(z_gate));
         }
         __syncthreads();
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) srow[8 * q] = st[q];
-}
-
-// behind mamba2_scan_kernel: the last four of the T positions' convolution inputs into their slots
-__global__ void __launch_bounds__(256)
-mamba2_ring_kernel(const float* __restrict__ zx, float* __restrict__ state, const int* __restrict__ pos_ptr, int t0, int T,
-                   int d_inner, int conv_dim, int in_out, size_t state_floats) {
-    grid_dependency_launch();
-    grid_dependency_wait();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, batch = gridDim.y;
-    if (c >= conv_dim) return;
-    float* const ring = state + (size_t)b * state_floats + (size_t)c * 4;
-    const int pos = pos_ptr[b] + t0;
-    for (int t = max(0, T - 4); t < T; ++t) ring[(pos + t) & 3] = zx[((size_t)t * batch + b) * in_out + d_inner + c];
+    // the last four inputs of the convolution into their slots: this CTA's x channels, and B and C for the first
+    const int pos = pos_ptr[b] + t0, channels = blockIdx.x == 0 ? RW + 2 * N : RW;
+    for (int i = tid; i < 4 * channels; i += THREADS) {
+        const int t = T - 4 + (i & 3), k = i >> 2, c = k < RW ? head * P + p0 + k : d_inner + k - RW;
+        if (t >= 0) state[(size_t)b * state_floats + (size_t)c * 4 + ((pos + t) & 3)] = zx[(size_t)t * step + (size_t)b * in_out + d_inner + c];
+    }
 }
 
 size_t mamba_state_floats(const Mamba* m) { return m->state_floats(); }
 
-size_t mamba_scratch_bytes(const Mamba* m, int rows) { return (size_t)rows * (m->in_out + m->d_inner) * 4 + 256; }
+size_t mamba_scratch_bytes(const Mamba* m, int rows) {
+    return (size_t)rows * (m->in_out + m->d_inner + act_stride(m->conv_dim, m->cfg.nheads)) * 4 + 512;
+}
 
 int mamba_reserve(Mamba* m, int B) {
     if (B <= m->cap_B) return LSPK_OK;
@@ -309,15 +348,19 @@ int mamba_prefill(Mamba* m, float* x, float* state, const int* pos, int t0, int 
     // expands the weights twice (24 steps of sixteen sequences 32.75 -> 31.55 ms).
     if (int rc = linear_auto(&a)) return rc;
     const float *zx = zx_out, *conv_w = m->conv_w, *conv_b = m->conv_b, *A = m->A, *dt_bias = m->dt_bias, *D = m->D;
-    const dim3 grid(m->cfg.nheads * 2, B);
     if (T == 1 && t0 == 0) {
-        LSPK_CUDA(launch(mamba2_ssu_kernel, grid, dim3(256), 0, true, zx, state, pos, conv_w, conv_b, A, dt_bias, D, v,
+        LSPK_CUDA(launch(mamba2_ssu_kernel, dim3(m->cfg.nheads * 2, B), dim3(256), 0, true, zx, state, pos, conv_w, conv_b, A, dt_bias, D, v,
                          m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
     } else {
-        LSPK_CUDA(launch(mamba2_scan_kernel, grid, dim3(256), 0, true, zx, state, pos, t0, T, conv_w, conv_b, A, dt_bias, D, v,
-                         m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
-        LSPK_CUDA(launch(mamba2_ring_kernel, dim3((m->conv_dim + 255) / 256, B), dim3(256), 0, true, zx, state, pos, t0, T,
-                         m->d_inner, m->conv_dim, m->in_out, m->state_floats()));
+        float* const act = v + ((size_t)M * m->d_inner + 63) / 64 * 64;
+        const int nheads = m->cfg.nheads;
+        LSPK_CUDA(launch(mamba2_conv_kernel, dim3((m->conv_dim + nheads + 255) / 256, B, (T + kScan - 1) / kScan), dim3(256), 0, true, zx,
+                         (const float*)state, pos, t0, T, conv_w, conv_b, A, dt_bias, act, nheads, m->d_inner, m->conv_dim, m->in_out,
+                         m->state_floats()));
+        const bool few = 2 * nheads * B < 2 * sm_count();
+        LSPK_CUDA(launch(few ? mamba2_scan_kernel<8> : mamba2_scan_kernel<32>, dim3(nheads * (few ? 8 : 2), B), dim3(few ? 64 : 256), 0,
+                         true, zx, (const float*)act, state, pos, t0, T, D, v, nheads, m->d_inner, m->conv_dim, m->in_out,
+                         m->state_floats()));
     }
     lspk_linear_args o = {};
     o.w[0] = m->out_proj;

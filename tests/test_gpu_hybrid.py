@@ -260,7 +260,7 @@ def test_hybrid_full_depth_steps_match_oracle(oracle, port):
     d.close()
 
 
-@pytest.mark.parametrize("B,T", [(1, 2), (1, 9), (1, 515), (3, 5), (16, 17), (64, 9), (513, 2)])
+@pytest.mark.parametrize("B,T", [(1, 2), (1, 9), (1, 515), (2, 16), (3, 5), (16, 17), (64, 9), (513, 2)])
 def test_prefill_equals_the_steps(B, T):
     """Positions of a prompt together (in passes, the last one shorter) or one by one: the same bits, twice in a row."""
     cfg = hyb.HybridConfig(hidden_size=256, num_layers=4, vocab_size=96, num_experts=4, intermediate_size=192, nheads=4,
