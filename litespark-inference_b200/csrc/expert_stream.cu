@@ -377,6 +377,9 @@ static int expert_slots(int chunks, int tiles) {
     return slots < kESlotsMax ? slots : kESlotsMax;
 }
 
+// four slots and more beside eight rows keep the ring turning (K up to about 24000); the model shapes have 24 to 29
+static bool expert_ring_fits(int chunks) { return expert_row_bytes(chunks, 1) + 30 * 1024 <= (size_t)kESmem; }
+
 int expert_stream_launch(ExpertStreamParams p, bool pair) {
     // Passes of several tiles where experts have some forty rows or more on average and eight slots are left beside the
     // rows (K of 2560: four tiles, of 6912: two).  A MoE layer of eight experts of 6912 x 2560, one tile against these, us:
@@ -384,8 +387,7 @@ int expert_stream_launch(ExpertStreamParams p, bool pair) {
     int tiles = 1;
     if (p.R > 40 * p.E) tiles = expert_slots(p.chunks, 4) >= 8 ? 4 : expert_slots(p.chunks, 2) >= 8 ? 2 : 1;
     p.slots = expert_slots(p.chunks, tiles);
-    // three slots keep the ring turning at the longest rows (K of about 24000); the model shapes have 24 to 29
-    LSPK_REQUIRE(p.slots >= 3, "expert products: K=%d too large for eight rows in shared memory (limit about 24000)", p.K);
+    LSPK_REQUIRE(expert_ring_fits(p.chunks), "expert products: K=%d too large for eight rows in shared memory (limit about 24000)", p.K);
     p.cps = kEStageChunks / (pair ? 2 : 1);
     p.sub = (p.chunks + p.cps - 1) / p.cps;
     p.error_flag = device_wait_flag();
@@ -406,8 +408,8 @@ int expert_stream_launch(ExpertStreamParams p, bool pair) {
 extern "C" int lspk_debug_expert_stage(int K, int stage, int* slot_out, int* producer_out) {
     using namespace lspk;
     LSPK_REQUIRE(K >= 4 && stage >= 0 && slot_out && producer_out, "lspk_debug_expert_stage: bad arguments");
-    const int slots = expert_slots((K + kWeightsPerChunk - 1) / kWeightsPerChunk, 1);
-    LSPK_REQUIRE(slots >= 3, "lspk_debug_expert_stage: K=%d has no ring", K);
+    const int chunks = (K + kWeightsPerChunk - 1) / kWeightsPerChunk, slots = expert_slots(chunks, 1);
+    LSPK_REQUIRE(expert_ring_fits(chunks), "lspk_debug_expert_stage: K=%d has no ring", K);
     *slot_out = stage % slots;
     *producer_out = e_producer_of_slot(*slot_out);
     return LSPK_OK;
