@@ -282,3 +282,25 @@ def test_prefill_equals_the_steps(B, T):
     for st in (together, single):
         st.close()
     d.close()
+
+
+# a few tiles of the table for some warps, a second and a third tile for some; the shortest rows whose terms go in halves,
+# the model's, long ones
+@pytest.mark.parametrize("B,V,H", [(9, 67, 2112), (16, 37921, 2560), (13, 80003, 2560), (16, 37921, 3136)])
+def test_greedy_choice_of_nine_to_sixteen(B, V, H):
+    """The LM head that takes the halves of its rows in turn has the sums of the one that takes eight rows: the same choices."""
+    cfg = hyb.HybridConfig(hidden_size=H, num_layers=2, vocab_size=V, num_experts=2, intermediate_size=64, nheads=2, headdim=64,
+                           d_state=128)
+    d = hyb.DeviceHybrid(hyb.random_hybrid(cfg, seed=V, norm_jitter=0.1, fast=True))
+    first = np.random.default_rng(B).integers(0, V, B).astype(np.int32)
+
+    def greedy(tokens):
+        st = hyb.HybridState(d, len(tokens), 4)
+        out = st.decode_greedy(tokens, 4)
+        st.close()
+        return out
+
+    together = greedy(first)
+    assert np.array_equal(together[:, :8], greedy(first[:8])) and np.array_equal(together[:, B - 8:], greedy(first[B - 8:]))
+    assert len(np.unique(together)) > 8
+    d.close()
